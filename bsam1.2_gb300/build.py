@@ -35,6 +35,7 @@ UNITS = {
     "hier.cu": [],
     "ghostc.cpp": [],
     "pool.cpp": [],
+    "uni.cpp": [],
     "regrid.cpp": [],
     "io.cu": ["--fmad=false"],
     "frames.cpp": [],

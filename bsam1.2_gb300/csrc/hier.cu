@@ -15,6 +15,7 @@
 #include "hier.h"
 #include "box.h"
 #include "mixed.h"
+#include "uni.h"
 
 using namespace bsamg;
 
@@ -100,7 +101,10 @@ int enq_op(Hier& H, int level, int kind, int op, int arg) {
 
 int enq_relax(Hier& H, int level, int ipass) { return enq_op(H, level, kKindColor, kTRelax, ipass); }
 
+const PluginUni& uni64(const Hier& H) { return find_plugin(H.problem)->fp64->uni; }
+
 int enq_set_ghost(Hier& H, int level, int ipass) {
+  if (uni_level(H, level)) return after_launch(H, uni64(H).ghost(H.lc(), H.ubc, H.hP[uni_patch(H, level)]));
   LevelT& L = H.L(level);
   GhostProg& g = L.gp[ipass];
   int nst = (int)g.stage_off.size() - 1;
@@ -120,6 +124,11 @@ int enq_set_ghost(Hier& H, int level, int ipass) {
 int enq_level_relax(Hier& H, int level, int nsmooth) {
   for (int pass = 1; pass <= nsmooth; pass++)
     for (int rb = 1; rb <= 2; rb++) {
+      if (uni_level(H, level)) {  // the sweep writes its cells' ghosts too
+        const int p = uni_patch(H, level);
+        RET(after_launch(H, uni64(H).relax(H.lc(), H.ubc, p, H.hP[p], rb, pass == nsmooth)));
+        continue;
+      }
       RET(enq_relax(H, level, rb));
       RET(enq_set_ghost(H, level, rb));
     }
@@ -128,6 +137,21 @@ int enq_level_relax(Hier& H, int level, int nsmooth) {
 
 // AFASVcycle, afasroutines.f90:495-529
 int enq_vcycle(Hier& H, int level, int minlevel, int nsmooth) {
+  if (uni_level(H, level)) {
+    const PluginUni& U = uni64(H);
+    const Hier::UniPlan* pl = uni_plan(H, U, level, minlevel, nsmooth);
+    if (pl && pl->top == level) {  // the rest of the V-cycle in one cluster launch
+      const int n = U.cycle(H.lc(), pl->A, pl->smem);
+      return n < 0 ? cuda_fail(cudaGetLastError(), "coarse V-cycle launch") : after_launch(H, n);
+    }
+    RET(enq_level_relax(H, level, nsmooth));
+    if (level == minlevel) return BSAMG_OK;
+    const int p = uni_patch(H, level), u = uni_patch(H, level - 1);
+    RET(after_launch(H, U.restrict_load(H.lc(), H.ubc, p, H.hP[p], H.hP[u])));
+    RET(enq_vcycle(H, level - 1, minlevel, nsmooth));
+    RET(after_launch(H, U.correct(H.lc(), H.ubc, H.hP[p], H.hP[u])));
+    return enq_level_relax(H, level, nsmooth);
+  }
   if (!H.rec && level <= H.tail_level && level >= minlevel) {
     auto it = H.fp_tail_progs.find(std::make_tuple(level, minlevel, nsmooth));
     if (it != H.fp_tail_progs.end())  // the rest of the V-cycle in one block
@@ -217,6 +241,7 @@ int fp_prepare_tail(Hier& H, int finest, int minlevel, int nsmooth) {
 // FillDown, afasroutines.f90:236-254 (field 1 = source, 2 = solution)
 int enq_fill_down_from(Hier& H, int field, int finest, int minlevel) {
   for (int level = finest; level >= minlevel + 1; level--) {
+    if (uni_level(H, level)) return uni_enq_fill(H, uni64(H), field == 2 ? 1 : 2, level, minlevel);
     if (!H.rec && level <= H.tail_level) {
       auto it = H.fp_tail_progs.find(std::make_tuple(level, minlevel, -field));
       if (it != H.fp_tail_progs.end())  // the remaining levels in one block
@@ -272,13 +297,24 @@ int enq_copy_q_to_qold(Hier& H, int minlevel, int finest) {
   return BSAMG_OK;
 }
 
+// the part of FillDown that enq_iteration leaves to the end of the loop
+int finish_fill_down(Hier& H, int finest, int minlevel) {
+  if (!H.uni) return BSAMG_OK;
+  if (finest > 0) RET(enq_fill_down(H, 1, finest, 0));
+  return uni_enq_fill(H, uni64(H), 3, 0, minlevel);
+}
+
 // One V-cycle iteration body of MultigridIterations (afasroutines.f90:81-104)
 // followed by a copy of the norm to pinned host memory.
 int enq_iteration(Hier& H, int finest, int minlevel, int nsmooth, int errortype) {
   RET(enq_vcycle(H, finest, minlevel, nsmooth));
-  RET(enq_fill_down(H, 2, finest, minlevel));
+  // With uniform levels <= 0 the next V-cycle writes q and f below level 0,
+  // and f under every finer patch, before it reads them (RestrictSolution and
+  // CoarseLoadingFunction cover them whole), so FillDown of those is done
+  // once, after the last cycle (finish_fill_down).
+  RET(enq_fill_down(H, 2, finest, H.uni ? std::max(0, minlevel) : minlevel));
   RET(enq_update_source(H, finest));
-  RET(enq_fill_down(H, 1, finest, minlevel));
+  if (!H.uni) RET(enq_fill_down(H, 1, finest, minlevel));
   RET(enq_norm(H, finest, errortype));
   CK(cudaMemcpyAsync(H.h_norm, H.d_norm, 2 * sizeof(double), cudaMemcpyDeviceToHost, H.s));
   CK(cudaMemcpyAsync(H.h_nonfinite, H.d_nonfinite, sizeof(int), cudaMemcpyDeviceToHost, H.s));
@@ -491,11 +527,12 @@ int multigrid_iterations(Hier& H, int finest, int minlevel, int nsmooth, int max
   // the periodic-box mixed path forms f from qold itself
   if (mode == BSAMG_MODE_MIXED && H.box)
     return box_iterations(H, finest, minlevel, nsmooth, maxvcycles, tol, errortype, strict, ncycles, residuals);
-  RET(fp_prepare_tail(H, finest, minlevel, nsmooth));
-  RET(enq_fill_down(H, 2, finest, minlevel));
+  if (!H.uni) RET(fp_prepare_tail(H, finest, minlevel, nsmooth));
+  const bool late = H.uni && mode == BSAMG_MODE_FP64;  // see enq_iteration
+  RET(enq_fill_down(H, 2, finest, late ? 0 : minlevel));
   RET(enq_get_source(H, finest));
   RET(enq_update_source(H, finest));
-  RET(enq_fill_down(H, 1, finest, minlevel));
+  if (!late) RET(enq_fill_down(H, 1, finest, minlevel));
   if (mode == BSAMG_MODE_MIXED)
     return mixed_iterations(H, finest, minlevel, nsmooth, maxvcycles, tol, errortype, strict, ncycles, residuals);
   Hier::GraphRec* gr = nullptr;
@@ -507,9 +544,10 @@ int multigrid_iterations(Hier& H, int finest, int minlevel, int nsmooth, int max
     RET(replay(H, gr));
     r = H.h_norm[0];
     if (residuals) residuals[it - 1] = r;
-    RET(check_nonfinite(H));
-    if (r < tol) break;
+    if (check_nonfinite(H) || r < tol) break;
   }
+  RET(finish_fill_down(H, finest, minlevel));
+  RET(check_nonfinite(H));
   bool conv = it <= maxvcycles;
   if (ncycles) *ncycles = conv ? it : maxvcycles;
   if (!conv && strict) return BSAMG_ERR_NOT_CONVERGED;
@@ -708,6 +746,8 @@ int commit(Hier& H) {
       for (int f = 0; f < 2 * H.ndims; f++) w = w && P.mthbc[f] == 2;
     for (int v = 0; v < H.nrvars; v++) w = w && H.pp.qpo[v] == 0.0;
     H.box = box_eligible(H, w);
+    H.uni = uni_eligible(H);
+    if (H.uni) H.ubc = uni_bc(H);
   }
 
   // pool layout: [q...][qold...][qc...][f...][rf...][ftmp...]

@@ -86,6 +86,16 @@ struct Hier {
   Blk* mx_prep_coarse = nullptr;              // interior lists of all levels < 0
   int mx_prep_coarse_n = 0;
   std::vector<Blk> h_mx_norm_blk[kNLev], h_mx_prep_coarse;  // host copies of the two
+  // uniform levels (uni.h): levels <= 0 are single patches whose ghosts the
+  // operations themselves write; the cluster plans per (level, minlevel,
+  // nsmooth, bytes a value)
+  bool uni = false;
+  UniBC ubc{};
+  struct UniPlan {
+    UniCycle A;
+    int smem, top;  // top: the level the cluster's V-cycle starts at
+  };
+  std::map<std::tuple<int, int, int, int>, UniPlan> uni_plans;
   // coarse tail of the V-cycle (levels <= tail_level run in one CTA); the
   // recorded programs per (minlevel, nsmooth): device phases and their count
   int tail_level = -kMaxDepth - 2;

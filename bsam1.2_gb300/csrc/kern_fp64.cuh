@@ -12,6 +12,7 @@
 #include <cuda_runtime.h>
 
 #include "cellops.cuh"
+#include "kern_uni.cuh"
 #include "launch.h"
 #include "plugin.h"
 
@@ -431,6 +432,97 @@ __global__ void __launch_bounds__(kBlock) k_tail_smem(const PatchDev* __restrict
   }
 }
 
+// Uniform levels in FP64 (kern_uni.cuh)
+template <class PL>
+struct Uni64 {
+  using T = double;
+  using Par = ProbParams;
+  struct Mem {
+    double* pool;
+  };
+  static constexpr int NV = PL::kNV;
+  static constexpr bool kStoreRf = true;
+  static constexpr bool kOld = UsesQold<PL>::value;
+  static constexpr int kXPlanes = kOld ? NV : 0, kXGhosted = 1;
+  static Mem mem(const LaunchCtx& c) { return Mem{c.pool}; }
+  static Par par(const LaunchCtx& c) { return c.pp; }
+
+  // SelfPeriodicBC's offset across the x faces (boundary.f90:480-577): the
+  // image beyond the high face (s = 1) and beyond the low one (s = 2)
+  __device__ __forceinline__ static double shift(double w, int s, int v, const Par& pp) {
+    if (s == 0) return w;
+    if (__double_as_longlong(pp.qpo[v]) == 0)  // + 0.0 turns -0.0 into 0.0, - 0.0 changes nothing
+      return s == 1 && __double_as_longlong(w) == (long long)(1ull << 63) ? 0.0 : w;
+    return s == 1 ? w + pp.qpo[v] : w - pp.qpo[v];
+  }
+  __device__ __forceinline__ static double wall(double u, int mask, int v) {
+    return ((mask >> v) & 1) ? 2.0 - u : (((mask >> (8 + v)) & 1) ? -u : u);
+  }
+  __device__ __forceinline__ static int ipass(int colour, bool) { return colour; }
+  __device__ __forceinline__ static void bind(uni::View<double>& V, const PatchDev& p, const Mem& m) {
+    V.q = m.pool + p.oq;
+    V.f = m.pool + p.of;
+    V.c = m.pool + p.oqc;
+    V.x = m.pool + p.oqold;
+  }
+  __device__ __forceinline__ static double* rf(const PatchDev& p, const Mem& m) { return m.pool + p.orf; }
+  template <int DIM>
+  __device__ __forceinline__ static void relax(const uni::View<double>& V, int c, int fc, int, const PatchDev& P,
+                                               const Par& pp) {
+    Cell64 x;
+    x.q = V.q;
+    x.f = V.f;
+    x.qold = kOld ? V.x : V.q;
+    x.c = c;
+    x.fc = fc;
+    x.sy = V.g.sy;
+    x.sz = V.g.sz;
+    x.sq = V.g.sq;
+    x.sf = V.sf;
+    PL::template relax<DIM>(x, P.c, pp);
+  }
+  template <int DIM>
+  __device__ __forceinline__ static void op(const double* a, int c, const uni::Geo& g, const uni::View<double>& X,
+                                            int xc, int, const PatchDev& P, const Par& pp, double* r) {
+    const double* qo = kOld ? X.x + xc : a;
+    PL::template op<DIM>(a, c, g.sy, g.sz, g.sq, QoldView{qo, X.g.sy, X.g.sz, X.g.sq}, P.c, pp, r);
+  }
+  template <int DIM>
+  __device__ __forceinline__ static void restrict_base(const uni::View<double>&, const uni::View<double>&, int, int,
+                                                       int, int) {}
+  // the top level's q and f and every level's qold in; every level's q, f,
+  // coarse image out
+  template <int DIM>
+  __device__ __forceinline__ static void stage_in(const UniCycle& A, int rank, const PatchDev* sp, const Mem& m) {
+    uni::Part pt;
+    for (int x = 0; x < A.nl; x++) {
+      if (!A.L[x].mul && rank) break;
+      const uni::View<double> V = uni::slab_view<Uni64, DIM, false>(A, x, rank, pt);
+      const PatchDev& p = sp[x];
+      if (x == 0) {
+        uni::copy_rows<double, DIM>(V.q, V.g, m.pool + p.oq, p.sq, NV, 0, V.g.nr + 1, false);
+        uni::copy_inner<double, DIM>(V.f, V.g, V.sf, m.pool + p.of, p.sf, NV, false);
+      }
+      if (kOld) uni::copy_rows<double, DIM>(V.x, V.g, m.pool + p.oqold, p.sq, NV, 0, V.g.nr + 1, false);
+    }
+  }
+  template <int DIM>
+  __device__ __forceinline__ static void stage_out(const UniCycle& A, int rank, const PatchDev* sp, const Mem& m) {
+    uni::Part pt;
+    for (int x = 0; x < A.nl; x++) {
+      if (!A.L[x].mul && rank) break;
+      const uni::View<double> V = uni::slab_view<Uni64, DIM, false>(A, x, rank, pt);
+      const PatchDev& p = sp[x];
+      const bool first = V.g.r0 == 0, last = V.g.r0 + V.g.nr == V.g.N;
+      uni::copy_rows<double, DIM>(V.q, V.g, m.pool + p.oq, p.sq, NV, first ? 0 : 1, last ? V.g.nr + 1 : V.g.nr, true);
+      if (x) uni::copy_inner<double, DIM>(V.f, V.g, V.sf, m.pool + p.of, p.sf, NV, true);
+      if (x + 1 < A.nl)
+        uni::copy_rows<double, DIM>(V.c, V.gc, m.pool + p.oqc, p.sc, NV, first ? 0 : 1, last ? V.gc.nr + 1 : V.gc.nr,
+                                    true);
+    }
+  }
+};
+
 // The launchers of one plugin's FP64 kernels (the table the plugin registers)
 template <class PL>
 struct Fp64Launchers {
@@ -493,7 +585,8 @@ const PluginFp64* fp64_ops() {
   static const PluginFp64 ops = {&Fp64Launchers<PL>::relax,        &Fp64Launchers<PL>::coarse_load,
                                  &Fp64Launchers<PL>::norm_partial, &Fp64Launchers<PL>::get_source,
                                  &Fp64Launchers<PL>::update_source, &Fp64Launchers<PL>::tail,
-                                 &Fp64Launchers<PL>::tail_smem,    &Fp64Launchers<PL>::tail_smem_attributes};
+                                 &Fp64Launchers<PL>::tail_smem,    &Fp64Launchers<PL>::tail_smem_attributes,
+                                 uni::UniLaunchers<Uni64<PL>>::table()};
   return &ops;
 }
 

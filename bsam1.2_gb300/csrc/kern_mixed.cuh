@@ -8,6 +8,7 @@
 #include <cuda_runtime.h>
 
 #include "cellops.cuh"
+#include "kern_uni.cuh"
 #include "launch.h"
 #include "plugin.h"
 
@@ -481,6 +482,85 @@ __global__ void __launch_bounds__(kBlock) k_mx_tail_smem(const PatchDev* __restr
 namespace bsamg {
 namespace mx {
 
+// Uniform levels of the correction cycle (kern_uni.cuh): e, its coarse
+// image, g and the frozen base planes, FP32; boundary conditions in
+// homogeneous form
+template <class PL>
+struct Uni32 {
+  using T = float;
+  using Par = MxParams;
+  struct Mem {
+    float* fpool;
+  };
+  static constexpr int NV = PL::kNV;
+  static constexpr bool kStoreRf = false;
+  static constexpr int kXPlanes = PL::kMxBase, kXGhosted = 0;
+  static Mem mem(const LaunchCtx& c) { return Mem{c.fpool}; }
+  static Par par(const LaunchCtx& c) { return PL::mx_params(c.pp); }
+
+  __device__ __forceinline__ static float shift(float w, int, int, const Par&) { return w; }  // qpo cancels
+  __device__ __forceinline__ static float wall(float u, int mask, int v) { return ((mask >> v) & 0x101) ? -u : u; }
+  __device__ __forceinline__ static int ipass(int colour, bool coarsest) {
+    return coarsest ? colour | kRelax64 : colour;
+  }
+  __device__ __forceinline__ static void bind(uni::View<float>& V, const PatchDev& p, const Mem& m) {
+    V.q = m.fpool + p.eq;
+    V.f = m.fpool + p.eg;
+    V.c = m.fpool + p.ecq;
+    V.x = m.fpool + p.ephi;
+  }
+  __device__ __forceinline__ static float* rf(const PatchDev&, const Mem&) { return nullptr; }
+  template <int DIM>
+  __device__ __forceinline__ static void relax(const uni::View<float>& V, int c, int fc, int ipass, const PatchDev& P,
+                                               const Par& mp) {
+    Cell32 x;
+    x.e = V.q;
+    x.g = V.f;
+    x.base = V.x;
+    x.c = c;
+    x.fc = fc;
+    x.sy = V.g.sy;
+    x.sz = V.g.sz;
+    x.sq = V.g.sq;
+    x.sf = V.sf;
+    if (ipass & kRelax64) PL::template mx_relax<DIM, double>(x, P.c, mp);
+    else PL::template mx_relax<DIM, float>(x, P.cf, mp);
+  }
+  template <int DIM>
+  __device__ __forceinline__ static void op(const float* a, int c, const uni::Geo& g, const uni::View<float>& X, int,
+                                            int fc, const PatchDev& P, const Par& mp, float* r) {
+    PL::template mx_op<DIM>(a, c, g.sy, g.sz, g.sq, X.x, fc, X.sf, P.cf, mp, r);
+  }
+  template <int DIM>
+  __device__ __forceinline__ static void restrict_base(const uni::View<float>&, const uni::View<float>&, int, int, int,
+                                                       int) {}
+  // the top level's e and g and every level's base planes in; the top
+  // level's e out (nothing reads the coarse corrections after the cycle)
+  template <int DIM>
+  __device__ __forceinline__ static void stage_in(const UniCycle& A, int rank, const PatchDev* sp, const Mem& m) {
+    uni::Part pt;
+    for (int x = 0; x < A.nl; x++) {
+      if (!A.L[x].mul && rank) break;
+      const uni::View<float> V = uni::slab_view<Uni32, DIM, false>(A, x, rank, pt);
+      const PatchDev& p = sp[x];
+      if (x == 0) {
+        uni::copy_rows<float, DIM>(V.q, V.g, m.fpool + p.eq, p.sq, NV, 0, V.g.nr + 1, false);
+        uni::copy_inner<float, DIM>(V.f, V.g, V.sf, m.fpool + p.eg, p.sf, NV, false);
+      }
+      uni::copy_inner<float, DIM>(V.x, V.g, V.sf, m.fpool + p.ephi, p.sf, kXPlanes, false);
+    }
+  }
+  template <int DIM>
+  __device__ __forceinline__ static void stage_out(const UniCycle& A, int rank, const PatchDev* sp, const Mem& m) {
+    uni::Part pt;
+    if (!A.L[0].mul && rank) return;
+    const uni::View<float> V = uni::slab_view<Uni32, DIM, false>(A, 0, rank, pt);
+    const bool first = V.g.r0 == 0, last = V.g.r0 + V.g.nr == V.g.N;
+    uni::copy_rows<float, DIM>(V.q, V.g, m.fpool + sp[0].eq, sp[0].sq, NV, first ? 0 : 1,
+                               last ? V.g.nr + 1 : V.g.nr, true);
+  }
+};
+
 // The launchers of one plugin's correction-form kernels (the table the
 // plugin registers)
 template <class PL>
@@ -624,7 +704,8 @@ const PluginMixed* mixed_ops() {
   static const PluginMixed ops = {PL::kMxBase,           PL::kMxUpdate,          &Launchers<PL>::prep,
                                   &Launchers<PL>::relax, &Launchers<PL>::coarse_load, &Launchers<PL>::track,
                                   &Launchers<PL>::norm,  &Launchers<PL>::tail,   &Launchers<PL>::tail_smem_attributes,
-                                  &Launchers<PL>::solve, &Launchers<PL>::solve_setup};
+                                  &Launchers<PL>::solve, &Launchers<PL>::solve_setup,
+                                  uni::UniLaunchers<Uni32<PL>>::table()};
   return &ops;
 }
 

@@ -118,6 +118,63 @@ struct SolveShape {
   int tile;  // units per tile of the FP32 work lists (32, 64, 128 or 256)
 };
 
+// Uniform levels (kern_uni.cuh).  UniBC: per dimension 0 periodic, 1
+// physical faces (UserBC with the plugin's mask).
+struct UniBC {
+  int phys[3];
+  int mask;
+};
+// Division by d as a multiplication by m = ceil(2^32 / d) (0: d = 1)
+struct UniDiv {
+  int d;
+  unsigned m;
+};
+// the divisors of a level's index decoding: (n0+1)/2, n0, n1, the ghosted
+// extents, the coarse image's interior, +1 and ghosted extents, and the cells
+// of a plane's frame (3D) of the level and of its coarse image
+struct UniDim {
+  UniDiv hx, n0, n1, e0, c0, c1, cp0, cp1, ce0, ce1, ring, cring;
+};
+inline UniDim uni_dim(const int* n) {
+  auto dv = [](int d) { return UniDiv{d, d <= 1 ? 0u : 0xFFFFFFFFu / (unsigned)d + 1u}; };
+  const int c0 = n[0] / 2, c1 = n[1] / 2;
+  return UniDim{dv((n[0] + 1) / 2), dv(n[0]), dv(n[1]), dv(n[0] + 2), dv(c0 > 0 ? c0 : 1), dv(c1 > 0 ? c1 : 1),
+                dv(c0 + 1), dv(c1 + 1), dv(c0 + 2), dv(c1 + 2), dv(2 * (n[0] + 2) + 2 * n[1]),
+                dv(2 * (c0 + 2) + 2 * c1)};
+}
+// a level's table entry and divisors, as a kernel argument
+struct UniPatch {
+  PatchDev p;
+  UniDim d;
+};
+inline UniPatch uni_patch_of(const PatchDev& p) { return UniPatch{p, uni_dim(p.mx)}; }
+// One level of a cluster's V-cycle: its patch, extents, the most rows of the
+// slowest dimension a CTA holds, the rows per row of the partition (0: CTA 0
+// holds the level alone) and where its arrays start in every CTA's shared
+// memory (elements): q, f, the coarse image, and the frozen data (qold or
+// base planes).
+struct UniLev {
+  int patch;
+  int n[3];
+  int maxr, mul;
+  int q, f, c, x;
+  UniDim d;
+};
+// the partition's rows of one CTA
+struct UniRank {
+  short row0, rows;
+};
+struct UniCycle {
+  UniLev L[kNLev];  // finest first
+  UniRank R[16];
+  int nl, ctas, threads, nsmooth;
+  int scratch;      // start of a CTA's residual scratch (elements)
+  UniBC bc;
+};
+constexpr int kUniThreads = 512;           // most threads of a CTA
+constexpr int kUniFillThreads = 1024;
+constexpr int kUniSmemMax = 200 * 1024;    // dynamic shared memory of a CTA
+
 // A contiguous run of pool elements staged in shared memory by a tail
 // kernel: pool[g .. g+n) <-> smem[s .. s+n); written back when out != 0.
 struct StageSeg {

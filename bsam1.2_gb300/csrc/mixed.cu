@@ -33,6 +33,7 @@
 #include "kern_mixed.cuh"
 #include "box.h"
 #include "mixed.h"
+#include "uni.h"
 
 namespace bsamg {
 
@@ -124,7 +125,10 @@ bool has_mixed(const Hier& H) {
 // the tail program being recorded (mx_vcycle records instead of launching)
 std::vector<TailPhase>* rec_of(Hier& H) { return static_cast<std::vector<TailPhase>*>(H.rec); }
 
+const PluginUni& uni32(const Hier& H) { return mxp(H).uni; }
+
 int mx_set_ghost(Hier& H, int level, int ipass) {
+  if (uni_level(H, level)) return after_launch(H, uni32(H).ghost(H.lc(), H.ubc, H.hP[uni_patch(H, level)]));
   GhostProg& g = H.L(level).gp[ipass];
   int nst = (int)g.stage_off.size() - 1;
   if (nst <= 0) return BSAMG_OK;
@@ -171,6 +175,12 @@ int mx_op(Hier& H, int level, int kind, int op, int arg) {
 int mx_level_relax(Hier& H, int level, int nsmooth, bool coarse) {
   for (int pass = 1; pass <= nsmooth; pass++)
     for (int rb = 1; rb <= 2; rb++) {
+      if (uni_level(H, level)) {  // the sweep writes its cells' ghosts too
+        const int p = uni_patch(H, level);
+        int ru = after_launch(H, uni32(H).relax(H.lc(), H.ubc, p, H.hP[p], coarse ? rb | kRelax64 : rb, pass == nsmooth));
+        if (ru) return ru;
+        continue;
+      }
       int r = mx_op(H, level, kKindColor, kTRelax, coarse ? rb | kRelax64 : rb);
       if (!r) r = mx_set_ghost(H, level, rb);
       if (r) return r;
@@ -179,6 +189,21 @@ int mx_level_relax(Hier& H, int level, int nsmooth, bool coarse) {
 }
 
 int mx_vcycle(Hier& H, int level, int minlevel, int nsmooth) {
+  if (uni_level(H, level)) {
+    const PluginUni& U = uni32(H);
+    const Hier::UniPlan* pl = uni_plan(H, U, level, minlevel, nsmooth);
+    if (pl && pl->top == level) {  // the rest of the V-cycle in one cluster launch
+      const int n = U.cycle(H.lc(), pl->A, pl->smem);
+      return n < 0 ? cuda_fail(cudaGetLastError(), "coarse V-cycle launch") : after_launch(H, n);
+    }
+    int r = mx_level_relax(H, level, nsmooth, level == minlevel);
+    if (r || level == minlevel) return r;
+    const int p = uni_patch(H, level), u = uni_patch(H, level - 1);
+    if ((r = after_launch(H, U.restrict_load(H.lc(), H.ubc, p, H.hP[p], H.hP[u])))) return r;
+    if ((r = mx_vcycle(H, level - 1, minlevel, nsmooth))) return r;
+    if ((r = after_launch(H, U.correct(H.lc(), H.ubc, H.hP[p], H.hP[u])))) return r;
+    return mx_level_relax(H, level, nsmooth, false);
+  }
   if (!H.rec && level <= H.tail_level && level >= minlevel) {
     auto it = H.mx_tail_progs.find(std::make_tuple(level, minlevel, nsmooth));
     if (it != H.mx_tail_progs.end()) {  // the whole V-cycle from here down in one CTA
@@ -336,7 +361,8 @@ int mx_iteration(Hier& H, int finest, int minlevel, int nsmooth, int errortype, 
   int r__ = 0;
   // e of levels >= 0 was cleared by the previous update pass (or by
   // mixed_iterations before the first cycle); clear the coarse ones
-  if (H.e_coarse_len) {
+  // (uniform coarse levels are written whole before they are read)
+  if (H.e_coarse_len && !H.uni) {
     cudaError_t ce = cudaMemsetAsync(H.fpool + H.e_coarse_off, 0, H.e_coarse_len * sizeof(float), H.s);
     if (ce != cudaSuccess) return cuda_fail(ce, "cudaMemsetAsync(e)");
   }
@@ -1135,7 +1161,7 @@ int mixed_iterations(Hier& H, int finest, int minlevel, int nsmooth, int maxvcyc
   if ((r = to_host(H))) return r;
   if (int rw = stream_wait(H)) return rw;
   double r_sync = H.h_norm[0];  // FP64 residual the current g was taken from
-  if ((r = mx_prepare_tail(H, finest, minlevel, nsmooth))) return r;
+  if (!H.uni && (r = mx_prepare_tail(H, finest, minlevel, nsmooth))) return r;
   Hier::GraphRec *ga = nullptr, *gt = nullptr, *gv = nullptr;
   auto key = [&](int m) { return std::make_tuple(m, finest, minlevel, nsmooth, errortype); };
   if ((r = capture_graph(H, key(11), [&] { return mx_iteration(H, finest, minlevel, nsmooth, errortype, true); },

@@ -29,6 +29,8 @@
 //   static void coefficients(const ProbParams&, int ndims, double h, double c[4]);
 //   static int bc_mask(int ndims);     // bits 0-7: 2 - q, bits 8-15: -q
 //   static int stats(int ndims);       // bit 0: integral of phi, bit 1: CH energy
+//   // optional: false when relax and op read nothing of qold (default true)
+//   static constexpr bool kQold;
 //   // device, FP64, evaluated in the reference's order (the FP64 part of a
 //   // plugin file is compiled with --fmad=false):
 //   template <int DIM> __device__ static void relax(const Cell64&, const double* c, const ProbParams&);
@@ -98,6 +100,22 @@ struct MxParams {
   float p[4];
 };
 
+// Launchers of the uniform-level operations (kern_uni.cuh) of one path: the
+// FP64 path's, or the correction cycle's.  p and u are the host's table
+// entries of a level's patch and of its parent.
+struct PluginUni {
+  int nv, nx, x_ghosted, elem;  // variables, planes of the frozen data and whether they are ghosted, bytes a value
+  // full: the sweep's edge and corner images too (the last sweep of a smoothing)
+  int (*relax)(const LaunchCtx&, const UniBC&, int patch, const PatchDev& p, int ipass, int full);
+  int (*restrict_load)(const LaunchCtx&, const UniBC&, int patch, const PatchDev& p, const PatchDev& u);
+  int (*correct)(const LaunchCtx&, const UniBC&, const PatchDev& p, const PatchDev& u);
+  int (*ghost)(const LaunchCtx&, const UniBC&, const PatchDev& p);
+  int (*fill)(const LaunchCtx&, const UniBC&, const PatchDev& p, const PatchDev& u, int fields);
+  int (*fill_small)(const LaunchCtx&, const UniCycle& A, int fields);
+  int (*cycle)(const LaunchCtx&, const UniCycle& A, int smem);
+  int (*cycle_fit)(int ndims, int ctas, int smem);
+};
+
 // Launchers of the plain FP64 path's plugin-dependent kernels.
 struct PluginFp64 {
   int (*relax)(const LaunchCtx&, const Blk*, int nblk, int ipass);
@@ -109,6 +127,7 @@ struct PluginFp64 {
   int (*tail_smem)(const LaunchCtx&, const PatchDev* shadow, const TailPhase*, int nph, const StageSeg*, int nsegs,
                    int smem_bytes);
   int (*tail_smem_attributes)();
+  PluginUni uni;
 };
 
 // Launchers of the mixed path's plugin-dependent kernels (the correction
@@ -138,6 +157,17 @@ struct PluginMixed {
   // (0: the shape cannot run)
   int (*solve)(const MxLaunch&, const void* image, SolveImage, SolveCtl*, double* res, double* partial, SolveShape);
   int (*solve_setup)(int ndims, SolveShape);
+  PluginUni uni;
+};
+
+// PL::kQold where the plugin states it, else true
+template <class PL, class = void>
+struct UsesQold {
+  static constexpr bool value = true;
+};
+template <class PL>
+struct UsesQold<PL, decltype((void)PL::kQold)> {
+  static constexpr bool value = PL::kQold;
 };
 
 struct Plugin {

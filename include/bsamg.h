@@ -301,14 +301,17 @@ int bsamg_hier_reset(bsamg_hier* h);
  * and the four-row sweeps elsewhere.  0, 1 and 3 give the same bits.
  * Drops the hierarchy's captured graphs. */
 int bsamg_set_box_sweep(bsamg_hier* h, int kind);
-/* Tuning (no reference counterpart): the mixed V-cycle runs its coarse
- * tail -- the levels from minlevel up to the highest one at which the
- * levels together hold at most `cells` interior cells -- inside one thread
- * block, one launch instead of ~20 per level; results are bit-identical.
- * Default 2048, where one block is still as fast as the launches it
- * replaces; a larger value trades a single run's latency for throughput
- * when many hierarchies share the GPU.  0 disables.  Drops the hierarchy's
- * captured graphs. */
+/* Tuning (no reference counterpart): how the coarse end of a V-cycle runs.
+ * On uniform levels (levels <= 0 that are one patch each, every dimension
+ * periodic or between walls, one ghost layer) any cells > 0 runs the levels
+ * of up to 6144 (FP64) or 40960 (correction cycle) cells in one launch of a
+ * thread-block cluster.  On other hierarchies the coarse tail -- the levels
+ * from minlevel up to the highest one at which the levels together hold at
+ * most `cells` interior cells -- runs inside one thread block, one launch
+ * instead of ~20 per level.  Results are bit-identical.  Default 2048; a
+ * larger value trades a single run's latency for throughput when many
+ * hierarchies share the GPU.  0: every operation its own launch.  Drops the
+ * hierarchy's captured graphs. */
 int bsamg_set_tail_cells(bsamg_hier* h, long long cells);
 /* Tuning (no reference counterpart; replaces the loop of
  * MultigridIterations, afasroutines.f90:78-104, and the ApplyOnLevel loops
