@@ -39,7 +39,9 @@
 #include <functional>
 
 #include "box.h"
+#include "kern_uni.cuh"
 #include "launch.h"
+#include "uni.h"
 
 namespace bsamg {
 
@@ -260,54 +262,46 @@ __device__ __forceinline__ void cta_sum2(float s0, float s1, double* partial) {
 // contract:  a21 = -3 (pb + xv)^2 - tmp3,  b1 = g0 + c0 s1,
 // b2 = g1 - c1 s0 - xv^2 (3 pb + 2 xv),  det = 1 - a12 a21,
 // e0 = (b1 - a12 b2) / det,  e1 = (b2 - a21 b1) / det.
+__device__ __forceinline__ void newton_cell(float c0, float c1, float tmp3, float a12, float pb, float xv, float s0,
+                                            float s1, float g0, float g1, float& r0, float& r1) {
+  const float w = __fadd_rn(pb, xv);
+  const float a21 = __fmaf_rn(__fmul_rn(-3.0f, w), w, -tmp3);
+  const float b1 = __fmaf_rn(c0, s1, g0);
+  const float t = __fmaf_rn(3.0f, pb, __fmul_rn(2.0f, xv));
+  const float b2 = __fmaf_rn(-__fmul_rn(xv, xv), t, __fmaf_rn(-c1, s0, g1));
+  const float rdet = __frcp_rn(__fmaf_rn(-a12, a21, 1.0f));
+  r0 = __fmul_rn(__fmaf_rn(-a12, b2, b1), rdet);
+  r1 = __fmul_rn(__fmaf_rn(-a21, b1, b2), rdet);
+}
 __device__ __forceinline__ void newton_cell(const BoxLev& L, float pb, float xv, float s0, float s1, float g0,
                                             float g1, float& r0, float& r1) {
-  const float w = __fadd_rn(pb, xv);
-  const float a21 = __fmaf_rn(__fmul_rn(-3.0f, w), w, -L.tmp3);
-  const float b1 = __fmaf_rn(L.c0, s1, g0);
-  const float t = __fmaf_rn(3.0f, pb, __fmul_rn(2.0f, xv));
-  const float b2 = __fmaf_rn(-__fmul_rn(xv, xv), t, __fmaf_rn(-L.c1, s0, g1));
-  const float rdet = __frcp_rn(__fmaf_rn(-L.a12, a21, 1.0f));
-  r0 = __fmul_rn(__fmaf_rn(-L.a12, b2, b1), rdet);
-  r1 = __fmul_rn(__fmaf_rn(-a21, b1, b2), rdet);
+  newton_cell(L.c0, L.c1, L.tmp3, L.a12, pb, xv, s0, s1, g0, g1, r0, r1);
 }
 
 // One cell of a colour half-sweep of the correction smoother (RelaxGrid2D/3D
-// in correction form, see mixed.cu k_mx_relax).  first = 1: e of both
-// colours counts as zero (first half-sweep of a cycle); first = 2: the own
-// colour's e counts as zero (second half-sweep).  Arithmetic T: float, or
-// double with the FP64 coefficients on the coarsest level (FP32 storage).
-template <int DIM, typename T = float>
-__device__ __forceinline__ void relax_at(float* __restrict__ fp, const BoxLev& L, int c, int first, int h, int y,
-                                         int z) {
-  constexpr bool D = sizeof(T) == sizeof(double);
-  const T c0 = D ? T(L.cd[0]) : T(L.c0), c1 = D ? T(L.cd[1]) : T(L.c1);
-  const T tmp3 = D ? T(L.cd[2]) : T(L.tmp3), a12 = D ? T(L.cd[3]) : T(L.a12);
+// in correction form, see mixed.cu k_mx_relax) in FP64 arithmetic with the
+// FP64 coefficients (FP32 storage).  first = 1: e of both colours counts as
+// zero (first half-sweep of a cycle); first = 2: the own colour's e counts as
+// zero (second half-sweep).
+template <int DIM>
+__device__ __forceinline__ void relax64_at(float* __restrict__ fp, const BoxLev& L, int c, int first, int h, int y,
+                                           int z) {
   V2 E = var2(fp, L.oe, L.half), G = var2(fp, L.og, L.half);
-  const float* PB = fp + L.opb;
   int x = 2 * h + ((c + y + z + (DIM == 3 ? 1 : 0)) & 1);
   Loc<DIM> l(L, x, y, z);
-  T pb = PB[l.own];
-  T s0 = T(0), s1 = T(0), xv = T(0);
+  double pb = fp[L.opb + l.own], s0 = 0.0, s1 = 0.0, xv = 0.0;
   if (first != 1) {
-    s0 = nsum<DIM, T>(E.v0, l);
-    s1 = nsum<DIM, T>(E.v1, l);
+    s0 = nsum<DIM, double>(E.v0, l);
+    s1 = nsum<DIM, double>(E.v1, l);
     if (first == 0) xv = E.v0[l.own];
   }
-  if constexpr (!D) {
-    float r0, r1;
-    newton_cell(L, pb, xv, s0, s1, G.v0[l.own], G.v1[l.own], r0, r1);
-    E.v0[l.own] = r0;
-    E.v1[l.own] = r1;
-  } else {
-    T w = pb + xv;
-    T a21 = T(-3) * w * w - tmp3;
-    T b1 = T(G.v0[l.own]) + c0 * s1;
-    T b2 = T(G.v1[l.own]) - c1 * s0 - xv * xv * (T(3) * pb + T(2) * xv);
-    T rdet = T(1) / (T(1) - a12 * a21);
-    E.v0[l.own] = (float)((b1 - a12 * b2) * rdet);
-    E.v1[l.own] = (float)((b2 - a21 * b1) * rdet);
-  }
+  double w = pb + xv;
+  double a21 = -3.0 * w * w - L.cd[2];
+  double b1 = G.v0[l.own] + L.cd[0] * s1;
+  double b2 = G.v1[l.own] - L.cd[1] * s0 - xv * xv * (3.0 * pb + 2.0 * xv);
+  double rdet = 1.0 / (1.0 - L.cd[3] * a21);
+  E.v0[l.own] = (float)((b1 - L.cd[3] * b2) * rdet);
+  E.v1[l.own] = (float)((b2 - a21 * b1) * rdet);
 }
 
 // the FP64 smoother over a whole level (the coarsest level of a V-cycle
@@ -316,7 +310,7 @@ template <int DIM>
 __global__ void __launch_bounds__(256) k_bx_relax64(float* __restrict__ fp, BoxLev L, int c, int first) {
   int h = blockIdx.x * blockDim.x + threadIdx.x;
   int y = blockIdx.y * blockDim.y + threadIdx.y;
-  if (h < L.hh && y < L.n[1]) relax_at<DIM, double>(fp, L, c, first, h, y, blockIdx.z);
+  if (h < L.hh && y < L.n[1]) relax64_at<DIM>(fp, L, c, first, h, y, blockIdx.z);
 }
 
 // Full-grid sweep: each thread takes position h of rows R*yp .. R*yp+R-1
@@ -364,8 +358,8 @@ __global__ void __launch_bounds__(256, MINB) k_bx_relax(float* __restrict__ fp, 
 // z+1 (periodic wrap).  Persistent CTAs walk the tiles plane by plane, the
 // next tile's rows in flight while the current one is computed, so the
 // memory system always has whole rows outstanding instead of one word per
-// thread.  The cell update is relax_at's (newton_cell); the six neighbours
-// are summed left to right, where relax_at adds the two z-neighbours as a
+// thread.  The cell update is k_bx_relax's (newton_cell); the six neighbours
+// are summed left to right, where that adds the two z-neighbours as a
 // pair, so the values agree to rounding, not bit for bit.
 constexpr int kTileThreads = 256;
 constexpr long long kWaitLimit = 1ll << 24;  // mbarrier polls before giving up
@@ -742,61 +736,6 @@ __global__ void __launch_bounds__(NT, 1) k_bx_smooth(float* __restrict__ fp, Box
     for (int b = 0; b < NSL; b++) mbar_wait(smem_addr(&bar[b]), 0u), mbar_wait(smem_addr(&bar[b]), 1u);
 }
 
-// RestrictSolution on e and on the base field: coarse e = ec = R(e_fine),
-// coarse pb = R(pb_fine); one coarse cell
-template <int DIM>
-__device__ __forceinline__ void restrict_at(float* __restrict__ fp, const BoxLev& F, const BoxLev& C, int X, int Y,
-                                            int Z) {
-  V2 Ef = var2(fp, F.oe, F.half);
-  const float* PBf = fp + F.opb;
-  float s[3] = {0.f, 0.f, 0.f};
-  const int nz = DIM == 3 ? 2 : 1;
-  for (int dz = 0; dz < nz; dz++)
-    for (int dy = 0; dy < 2; dy++) {
-      unsigned y = 2 * Y + dy, z = DIM == 3 ? 2 * Z + dz : 0;
-      unsigned r = (z * (unsigned)F.n[1] + y) * (unsigned)F.hh + (unsigned)X;  // both fine cells sit at x/2 = X
-      for (int c = 0; c < 2; c++) {
-        unsigned i = r + (c ? (unsigned)F.half : 0u);
-        s[0] += Ef.v0[i];
-        s[1] += Ef.v1[i];
-        s[2] += PBf[i];
-      }
-    }
-  const float w = DIM == 2 ? 0.25f : 0.125f;
-  Loc<DIM> lc(C, X, Y, Z);
-  V2 Ec = var2(fp, C.oe, C.half), ECc = var2(fp, C.oec, C.half);
-  Ec.v0[lc.own] = ECc.v0[lc.own] = s[0] * w;
-  Ec.v1[lc.own] = ECc.v1[lc.own] = s[1] * w;
-  fp[C.opb + lc.own] = s[2] * w;
-}
-
-// CoarseLoadingFunction on the correction: coarse g = R(g - M(e)) + M_c(ec)
-template <int DIM>
-__device__ __forceinline__ void coarse_load_at(float* __restrict__ fp, const BoxLev& F, const BoxLev& C, int X, int Y,
-                                               int Z) {
-  V2 Ef = var2(fp, F.oe, F.half), Gf = var2(fp, F.og, F.half);
-  const float* PBf = fp + F.opb;
-  float R0 = 0.f, R1 = 0.f;
-  const int nz = DIM == 3 ? 2 : 1;
-  for (int dz = 0; dz < nz; dz++)
-    for (int dy = 0; dy < 2; dy++)
-      for (int dx = 0; dx < 2; dx++) {
-        Loc<DIM> l(F, 2 * X + dx, 2 * Y + dy, DIM == 3 ? 2 * Z + dz : 0);
-        float m0, m1;
-        mop<DIM>(Ef, F, l, PBf[l.own], m0, m1);
-        R0 += Gf.v0[l.own] - m0;
-        R1 += Gf.v1[l.own] - m1;
-      }
-  const float w = DIM == 2 ? 0.25f : 0.125f;
-  Loc<DIM> lc(C, X, Y, Z);
-  // M_c(ec): the coarse operator on the restricted correction
-  V2 ECc = var2(fp, C.oec, C.half), Gc = var2(fp, C.og, C.half);
-  float m0, m1;
-  mop<DIM>(ECc, C, lc, fp[C.opb + lc.own], m0, m1);
-  Gc.v0[lc.own] = R0 * w + m0;
-  Gc.v1[lc.own] = R1 * w + m1;
-}
-
 // RestrictSolution and the fine half of CoarseLoadingFunction in one pass
 // over the fine cells: coarse e = ec = R(e), coarse pb = R(pb) and coarse
 // g = R(g - M(e)); the coarse operator M_c(ec) needs the neighbours' ec, so
@@ -921,136 +860,505 @@ __global__ void __launch_bounds__(256) k_bx_prolong(float* __restrict__ fp, BoxL
   if (X < C.n[0] && Y < C.n[1]) prolong_at<DIM>(fp, F, C, X, Y, blockIdx.z);
 }
 
-// The V-cycle on the coarse end of the hierarchy (levels with at most
-// kSmallCells cells) in one CTA: the same phases as bx_vcycle, separated by
-// __syncthreads() instead of kernel boundaries, so a cycle spends one launch
-// instead of eleven per level on grids too small to fill the GPU.
-constexpr int kSmallCells = 8192;
-constexpr int kSmallThreads = 512;
-struct SmallLevels {
-  BoxLev L[kNLev];  // L[0] the top (finest) small level, then coarser
-  int n;
+// ---------------------------------------------------------------------------
+// The coarse levels of the V-cycle in one launch of a thread-block cluster.
+// Every CTA holds a slab of rows (the slowest dimension) of each level in
+// shared memory, in natural order with one halo row at each side of e and ec;
+// a CTA writes its boundary rows into its neighbours' halos as it computes
+// them (distributed shared memory), so all reads are local and a sweep costs
+// one cluster barrier.  Levels too small to share out are CTA 0's.
+//
+// A thread owns pairs of x-neighbours (2h, 2h+1), one cell of each colour,
+// and keeps their e, g and pb in registers through a smoothing: a sweep reads
+// the five (2D: three) neighbours outside the pair, updates and stores.  What
+// surrounds the sweeps runs on the same registers: on the way down the
+// coarse equation's M_c(ec) is added to g at the start and the residual
+// g - M(e) that the coarse level averages is formed at the end; on the way up
+// the prolonged correction is added at the start and e - ec, which the finer
+// level prolongs, is left in ec at the end.
+//
+// Bound by latency: about 60 instructions a sweep and pair, a barrier of the
+// cluster (0.3-0.5 us) or of the CTA (0.06 us), and on the coarsest level the
+// FP64 unit, which takes 64 cycles a warp instruction however few lanes work.
+// It took the place of one CTA on the levels up to 8192 cells (38 us for
+// 64^2 .. 2^2) with a launch per sweep above: ten steps at 128^2 7.8 -> 5.95
+// ms, five at 64^3 4.65 -> 4.15 ms, eight at 32^2 3.01 -> 2.68 ms, the same
+// bits.
+struct CycLev {
+  int n0, n1, N;       // extents (n1: 3D), rows
+  int maxr, mul;       // rows a CTA holds at most, rows per row of the partition (0: CTA 0 alone)
+  int e, ec, g, pb;    // starts in shared memory (floats)
+  int by_colour;       // order of the restriction's sums (see cyc_smooth)
+  float c0, c1, tmp3, a12;
+  UniDiv hx, d1, hc, dc1;  // divisors: pairs of a row, n1, coarse cells of a row, coarse n1
 };
+struct Cyc {
+  CycLev L[kNLev];     // finest first
+  UniRank R[16];
+  int nl, ctas, nsmooth, scratch;
+  double cd[4];        // the coarsest level's coefficients in FP64
+};
+constexpr int kCycThreads = 512, kCycPairs = 2;  // threads of a CTA, most pairs a thread holds
+extern __shared__ __align__(16) float csm[];
 
-// q = i / n, r = i % n for i >= 0: a shift and a mask when n is a power of
-// two (every extent of a periodic box level here; the branch is uniform
-// across the CTA), the division otherwise
-__device__ __forceinline__ void divmod(int i, int n, int& q, int& r) {
-  if ((n & (n - 1)) == 0) {
-    q = i >> (__ffs(n) - 1);
-    r = i & (n - 1);
+// This CTA's part of a level.
+struct Slab {
+  int n0, n1, N, r0, nr;
+  int plane, var, ivar;  // floats of a row's plane, of a variable with halos, of an interior variable
+  bool shared;
+  int lo, hi, lo_rows;   // neighbours (around the domain) and the rows of the one below
+  float *e, *ec, *g, *pb;
+};
+template <int DIM, bool REMOTE>
+__device__ __forceinline__ Slab slab(const Cyc& A, int x, int rank) {
+  const CycLev& L = A.L[x];
+  Slab S;
+  float* sm = csm;
+  S.n0 = L.n0, S.n1 = L.n1, S.N = L.N, S.r0 = 0, S.nr = L.N;
+  S.shared = L.mul != 0;
+  S.lo = S.hi = 0, S.lo_rows = L.N;
+  if (S.shared) {
+    S.r0 = A.R[rank].row0 * L.mul;
+    S.nr = A.R[rank].rows * L.mul;
+    S.lo = rank ? rank - 1 : A.ctas - 1;
+    S.hi = rank + 1 < A.ctas ? rank + 1 : 0;
+    S.lo_rows = A.R[S.lo].rows * L.mul;
+  } else if (REMOTE && rank) {
+    sm = uni::on_rank(sm, 0);
+  }
+  S.plane = DIM == 3 ? L.n0 * L.n1 : L.n0;
+  S.var = S.plane * (L.maxr + 2);
+  S.ivar = S.plane * L.maxr;
+  S.e = sm + L.e, S.ec = sm + L.ec, S.g = sm + L.g, S.pb = sm + L.pb;
+  return S;
+}
+
+// Where a value of a halo array at local row `row` of a slab goes besides
+// its own place: rows 1 and nr of a shared level into the neighbours' halos.
+// (A level one CTA holds wraps its rows when read.)
+struct HaloOut {
+  float *lo, *hi;   // the array in the neighbours' shared memory
+  int dlo, dhi;     // from a cell of row 1 (nr) to its image there
+};
+__device__ __forceinline__ HaloOut halo_out(const Slab& S, float* a) {
+  HaloOut h{nullptr, nullptr, 0, 0};
+  if (S.shared) {
+    h.lo = uni::on_rank(a, S.lo);
+    h.hi = uni::on_rank(a, S.hi);
+    h.dlo = S.lo_rows * S.plane;
+    h.dhi = -S.nr * S.plane;
+  }
+  return h;
+}
+__device__ __forceinline__ void halo_put(const Slab& S, const HaloOut& h, int row, int at, float v) {
+  if (!S.shared) return;
+  if (row == 1) h.lo[at + h.dlo] = v;
+  if (row == S.nr) h.hi[at + h.dhi] = v;
+}
+
+// A pair of cells (2h, 2h+1) of local row `row` (and y): its place in the
+// halo arrays and the interior ones, the steps to the x-neighbours beyond the
+// pair and to the other rows, and which of its cells has colour 0.
+struct Pair {
+  int at, in, row;
+  int xl, xr, ym, yp, rm, rp;
+  int b0;  // the colour-0 cell is at at + b0
+};
+template <int DIM>
+__device__ __forceinline__ Pair pair_of(const Slab& S, const CycLev& L, int u) {
+  Pair p;
+  int r, h, y = 0, k;
+  uni::fdivmod(u, L.hx, r, h);
+  if (DIM == 3) uni::fdivmod(r, L.d1, k, y);
+  else k = r;
+  p.row = k + 1;
+  const int base = DIM == 3 ? y * S.n0 + 2 * h : 2 * h;
+  p.at = p.row * S.plane + base;
+  p.in = k * S.plane + base;
+  p.xl = h ? -1 : S.n0 - 1;
+  p.xr = 2 * h + 2 < S.n0 ? 1 : 1 - S.n0;
+  p.ym = y ? -S.n0 : (S.n1 - 1) * S.n0;
+  p.yp = y + 1 < S.n1 ? S.n0 : -(S.n1 - 1) * S.n0;
+  p.rm = S.shared || k ? -S.plane : (S.nr - 1) * S.plane;
+  p.rp = S.shared || k + 1 < S.nr ? S.plane : -(S.nr - 1) * S.plane;
+  p.b0 = (y + k + S.r0 + (DIM == 3 ? 1 : 0)) & 1;
+  return p;
+}
+// sum over the neighbours of the pair's cell at at + b, `other` the pair's other cell
+template <int DIM, typename T>
+__device__ __forceinline__ T pair_sum(const float* a, const Pair& p, int b, T other) {
+  const float* c = a + p.at + b;
+  T s = T(b ? c[p.xr] : c[p.xl]) + other;
+  if (DIM == 3) {
+    s = s + T(c[p.ym]) + T(c[p.yp]);
+    s += T(c[p.rm]) + T(c[p.rp]);
   } else {
-    q = i / n;
-    r = i - q * n;
+    s = s + T(c[p.rm]) + T(c[p.rp]);
   }
-}
-// linear index j of an n0 x n1 x n2 grid -> (x, y, z)
-__device__ __forceinline__ void unflatten(int j, int n0, int n1, int& x, int& y, int& z) {
-  int r;
-  divmod(j, n0, r, x);
-  divmod(r, n1, z, y);
+  return s;
 }
 
-template <int DIM, typename T = float>
-__device__ __forceinline__ void small_relax(float* fp, const BoxLev& L, int nsmooth, bool fresh) {
-  int cnt = L.hh * L.n[1] * L.n[2];
-  for (int pass = 1; pass <= nsmooth; pass++)
-    for (int c = 0; c < 2; c++) {
-      int first = (fresh && pass == 1) ? c + 1 : 0;
-      for (int i = threadIdx.x; i < cnt; i += blockDim.x) {
-        int h, y, z;
-        unflatten(i, L.hh, L.n[1], h, y, z);
-        relax_at<DIM, T>(fp, L, c, first, h, y, z);
+// What a smoothing does before its sweeps and after them.
+enum CycBegin { kTop = 0, kDown = 1, kUp = 2 };
+
+// One smoothing of this CTA's slab of level x (see above), K pairs a thread.
+// sync: the level's barrier.  C: the parent level's slab.  The caller's
+// barrier follows the call.
+template <int DIM, int K, typename F>
+__device__ __forceinline__ void cyc_smooth(const Cyc& A, int x, const Slab& S, const Slab& C, int begin, bool restrict_,
+                                           bool emit, int t, int nt, F&& sync) {
+  const CycLev& L = A.L[x];
+  const int units = (S.n0 >> 1) * (DIM == 3 ? S.n1 : 1) * S.nr;
+  float *E0 = S.e, *E1 = S.e + S.var;
+  const HaloOut H0 = halo_out(S, E0), H1 = halo_out(S, E1);
+  Pair p[K];
+  bool on[K];
+  float e[K][2][2], g[K][2][2], pb[K][2];  // [cell of the pair][variable]
+#pragma unroll
+  for (int q = 0; q < K; q++) {
+    on[q] = t + q * nt < units;
+    if (!on[q]) continue;
+    p[q] = pair_of<DIM>(S, L, t + q * nt);
+#pragma unroll
+    for (int b = 0; b < 2; b++) {
+      e[q][b][0] = E0[p[q].at + b];
+      e[q][b][1] = E1[p[q].at + b];
+      g[q][b][0] = S.g[p[q].in + b];
+      g[q][b][1] = S.g[S.ivar + p[q].in + b];
+      pb[q][b] = S.pb[p[q].in + b];
+    }
+  }
+  const float kc = DIM == 2 ? 4.0f : 6.0f;
+  auto mop_pair = [&](int q, int b, float& m0, float& m1) {  // M(e) at a cell (mop)
+    const float xx = e[q][b][0], y = e[q][b][1];
+    const float s0 = pair_sum<DIM, float>(E0, p[q], b, e[q][1 - b][0]);
+    const float s1 = pair_sum<DIM, float>(E1, p[q], b, e[q][1 - b][1]);
+    m0 = xx - L.c0 * (s1 - kc * y);
+    m1 = y - xx * (3.0f * pb[q][b] * (pb[q][b] + xx) + xx * xx) + L.c1 * (s0 - kc * xx);
+  };
+  if (begin == kDown) {  // g = R(g - M(e)) (left by the finer level) + M_c(ec); e is ec here
+#pragma unroll
+    for (int q = 0; q < K; q++)
+      if (on[q]) {
+        float m[2][2];
+#pragma unroll
+        for (int b = 0; b < 2; b++) mop_pair(q, b, m[b][0], m[b][1]);
+#pragma unroll
+        for (int b = 0; b < 2; b++)
+#pragma unroll
+          for (int v = 0; v < 2; v++) {
+            g[q][b][v] += m[b][v];
+            S.g[v * S.ivar + p[q].in + b] = g[q][b][v];
+          }
       }
-      __syncthreads();
-    }
-}
-
-template <int DIM>
-__device__ __forceinline__ void small_cycle(float* fp, const SmallLevels& S, int nsmooth, int fresh) {
-  for (int i = 0; i < S.n; i++) {
-    const BoxLev& F = S.L[i];
-    if (i == S.n - 1) {  // the coarsest level: FP64 arithmetic
-      small_relax<DIM, double>(fp, F, nsmooth, fresh && i == 0);
-      break;
-    }
-    small_relax<DIM>(fp, F, nsmooth, fresh && i == 0);
-    const BoxLev& C = S.L[i + 1];
-    int cnt = C.n[0] * C.n[1] * C.n[2];
-    for (int j = threadIdx.x; j < cnt; j += blockDim.x) {
-      int X, Y, Z;
-      unflatten(j, C.n[0], C.n[1], X, Y, Z);
-      restrict_at<DIM>(fp, F, C, X, Y, Z);
-    }
-    __syncthreads();
-    for (int j = threadIdx.x; j < cnt; j += blockDim.x) {
-      int X, Y, Z;
-      unflatten(j, C.n[0], C.n[1], X, Y, Z);
-      coarse_load_at<DIM>(fp, F, C, X, Y, Z);
-    }
-    __syncthreads();
+    sync();
   }
-  for (int i = S.n - 2; i >= 0; i--) {
-    const BoxLev &F = S.L[i], &C = S.L[i + 1];
-    int cnt = C.n[0] * C.n[1] * C.n[2];
-    for (int j = threadIdx.x; j < cnt; j += blockDim.x) {
-      int X, Y, Z;
-      unflatten(j, C.n[0], C.n[1], X, Y, Z);
-      prolong_at<DIM>(fp, F, C, X, Y, Z);
-    }
-    __syncthreads();
-    small_relax<DIM>(fp, F, nsmooth, false);
+  if (begin == kUp) {  // e += P(e_c - ec), the difference in the parent's ec
+#pragma unroll
+    for (int q = 0; q < K; q++)
+      if (on[q]) {
+        const int u = t + q * nt;
+        int r, h, y = 0, k;
+        uni::fdivmod(u, L.hx, r, h);
+        if (DIM == 3) uni::fdivmod(r, L.d1, k, y);
+        else k = r;
+        const int z = k + S.r0;  // global row
+        // coarse columns h-1, h, h+1 and, per dimension, the near and the far coarse cell
+        const int xm = h ? h - 1 : C.n0 - 1, xp = h + 1 < C.n0 ? h + 1 : 0;
+        const int yn = y >> 1, yf = (y & 1) ? (yn + 1 < C.n1 ? yn + 1 : 0) : (yn ? yn - 1 : C.n1 - 1);
+        // local coarse rows (row 1 is the slab's first; shared slabs have halo rows)
+        const int zn = (z >> 1) - C.r0 + 1;
+        int zf = (z & 1) ? zn + 1 : zn - 1;
+        if (!C.shared) zf = zf < 1 ? C.nr : (zf > C.nr ? 1 : zf);
+        auto xstage = [&](const float* a, int yy, int zz, float& lo, float& hi) {
+          const float* c = a + zz * C.plane + (DIM == 3 ? yy * C.n0 : 0);
+          const float v0 = c[xm], v1 = c[h], v2 = c[xp];
+          lo = v0 + 3.0f * v1;  // cell 2h
+          hi = 3.0f * v1 + v2;  // cell 2h+1
+        };
+#pragma unroll
+        for (int v = 0; v < 2; v++) {
+          const float* a = C.ec + v * C.var;
+          float lo, hi, l2, h2;
+          if (DIM == 3) {
+            float a0, a1, b0, b1;
+            xstage(a, yn, zn, a0, a1);
+            xstage(a, yf, zn, b0, b1);
+            lo = 3.0f * a0 + b0, hi = 3.0f * a1 + b1;
+            xstage(a, yn, zf, a0, a1);
+            xstage(a, yf, zf, b0, b1);
+            l2 = 3.0f * a0 + b0, h2 = 3.0f * a1 + b1;
+          } else {
+            xstage(a, 0, zn, lo, hi);
+            xstage(a, 0, zf, l2, h2);
+          }
+          const float w = DIM == 3 ? 1.0f / 64.0f : 1.0f / 16.0f;
+          e[q][0][v] += (3.0f * lo + l2) * w;
+          e[q][1][v] += (3.0f * hi + h2) * w;
+#pragma unroll
+          for (int b = 0; b < 2; b++) {
+            (v ? E1 : E0)[p[q].at + b] = e[q][b][v];
+            halo_put(S, v ? H1 : H0, p[q].row, p[q].at + b, e[q][b][v]);
+          }
+        }
+      }
+    sync();
   }
-}
-
-template <int DIM>
-__global__ void __launch_bounds__(kSmallThreads) k_bx_small_vcycle(float* __restrict__ fp, SmallLevels S, int nsmooth,
-                                                                   int fresh) {
-  small_cycle<DIM>(fp, S, nsmooth, fresh);
-}
-
-// The same cycle on a copy in shared memory: the small levels' arrays are
-// one contiguous range of the pool, fp[lo, lo + nf) (levels are laid out
-// finest first, every array start a multiple of 64 floats), so the CTA
-// copies the range in, cycles on it with S's offsets taken relative to lo,
-// and copies it back.  Every phase then waits on shared memory instead of
-// L2.
-constexpr int kSmallSmemMax = 200 * 1024;
-template <int DIM>
-__global__ void __launch_bounds__(kSmallThreads) k_bx_small_vcycle_smem(float* __restrict__ fp, SmallLevels S,
-                                                                        long long lo, int nf, int nsmooth, int fresh) {
-  extern __shared__ float4 sm4[];
-  float4* g4 = reinterpret_cast<float4*>(fp + lo);
-  for (int i = threadIdx.x; i < nf / 4; i += blockDim.x) sm4[i] = g4[i];
+  for (int s = 0; s < 2 * A.nsmooth; s++) {
+    const int c = s & 1;
+#pragma unroll
+    for (int q = 0; q < K; q++)
+      if (on[q]) {
+        const int b = p[q].b0 ^ c;
+        const float o0 = b ? e[q][0][0] : e[q][1][0], o1 = b ? e[q][0][1] : e[q][1][1];
+        const float s0 = pair_sum<DIM, float>(E0, p[q], b, o0), s1 = pair_sum<DIM, float>(E1, p[q], b, o1);
+        float r0, r1;
+        newton_cell(L.c0, L.c1, L.tmp3, L.a12, b ? pb[q][1] : pb[q][0], b ? e[q][1][0] : e[q][0][0], s0, s1,
+                    b ? g[q][1][0] : g[q][0][0], b ? g[q][1][1] : g[q][0][1], r0, r1);
+        if (b) e[q][1][0] = r0, e[q][1][1] = r1;
+        else e[q][0][0] = r0, e[q][0][1] = r1;
+        E0[p[q].at + b] = r0;
+        E1[p[q].at + b] = r1;
+        halo_put(S, H0, p[q].row, p[q].at + b, r0);
+        halo_put(S, H1, p[q].row, p[q].at + b, r1);
+      }
+    if (s + 1 < 2 * A.nsmooth || restrict_) sync();
+  }
+  if (emit) {  // ec = e - ec, for the finer level's prolongation
+    const HaloOut C0 = halo_out(S, S.ec), C1 = halo_out(S, S.ec + S.var);
+#pragma unroll
+    for (int q = 0; q < K; q++)
+      if (on[q])
+#pragma unroll
+        for (int b = 0; b < 2; b++)
+#pragma unroll
+          for (int v = 0; v < 2; v++) {
+            float* d = S.ec + v * S.var + p[q].at + b;
+            const float w = e[q][b][v] - *d;
+            *d = w;
+            halo_put(S, v ? C1 : C0, p[q].row, p[q].at + b, w);
+          }
+  }
+  if (!restrict_) return;
+  // the residual g - M(e), which the coarse cells average
+  float* const sc = csm + A.scratch;
+#pragma unroll
+  for (int q = 0; q < K; q++)
+    if (on[q]) {
+#pragma unroll
+      for (int b = 0; b < 2; b++) {
+        float m0, m1;
+        mop_pair(q, b, m0, m1);
+        sc[p[q].in + b] = g[q][b][0] - m0;
+        sc[S.ivar + p[q].in + b] = g[q][b][1] - m1;
+      }
+    }
   __syncthreads();
-  small_cycle<DIM>(reinterpret_cast<float*>(sm4), S, nsmooth, fresh);
-  __syncthreads();
-  for (int i = threadIdx.x; i < nf / 4; i += blockDim.x) g4[i] = sm4[i];
+  // RestrictSolution and the fine half of CoarseLoadingFunction
+  const int cu = units >> (DIM == 3 ? 2 : 1);
+  const float w = DIM == 3 ? 0.125f : 0.25f;
+  const HaloOut C0 = halo_out(C, C.e), C1 = halo_out(C, C.e + C.var);
+  const HaloOut D0 = halo_out(C, C.ec), D1 = halo_out(C, C.ec + C.var);
+  for (int u = t; u < cu; u += nt) {
+    int r, X, Y = 0, Z;
+    uni::fdivmod(u, L.hc, r, X);
+    if (DIM == 3) uni::fdivmod(r, L.dc1, Z, Y);
+    else Z = r;
+    float a[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int dz = 0; dz < 2; dz++)
+#pragma unroll
+      for (int dy = 0; dy < (DIM == 3 ? 2 : 1); dy++) {
+        const int k = 2 * Z + dz, y = 2 * Y + dy;
+        const int in = k * S.plane + (DIM == 3 ? y * S.n0 : 0) + 2 * X, at = in + S.plane;
+        // a row's two cells of e and pb: colour 0 first on small levels, else left to right
+        const int b = L.by_colour ? (y + k + S.r0 + (DIM == 3 ? 1 : 0)) & 1 : 0;
+        a[0] += E0[at + b];
+        a[0] += E0[at + 1 - b];
+        a[1] += E1[at + b];
+        a[1] += E1[at + 1 - b];
+        a[2] += S.pb[in + b];
+        a[2] += S.pb[in + 1 - b];
+        a[3] += sc[in];
+        a[3] += sc[in + 1];
+        a[4] += sc[S.ivar + in];
+        a[4] += sc[S.ivar + in + 1];
+      }
+#pragma unroll
+    for (int v = 0; v < 5; v++) a[v] *= w;
+    const int row = Z + (S.r0 >> 1) - C.r0 + 1;
+    const int in = (row - 1) * C.plane + (DIM == 3 ? Y * C.n0 : 0) + X, at = in + C.plane;
+    C.e[at] = a[0];
+    C.e[C.var + at] = a[1];
+    C.ec[at] = a[0];
+    C.ec[C.var + at] = a[1];
+    halo_put(C, C0, row, at, a[0]);
+    halo_put(C, C1, row, at, a[1]);
+    halo_put(C, D0, row, at, a[0]);
+    halo_put(C, D1, row, at, a[1]);
+    C.pb[in] = a[2];
+    C.g[in] = a[3];
+    C.g[C.ivar + in] = a[4];
+  }
 }
 
-// The pool range [lo, hi) of the small levels' arrays, S rebased to lo.
-// False when it does not fit kSmallSmemMax.
-bool small_in_smem(SmallLevels& S, long long& lo, int& nf) {
-  lo = S.L[0].oe;
-  long long hi = 0;
-  for (int i = 0; i < S.n; i++) {
-    const BoxLev& L = S.L[i];
-    long long ends[4] = {L.oe + 4 * L.half, L.og + 4 * L.half,
-                         L.opb + (L.oec < 0 ? 4 : 2) * L.half, L.oec < 0 ? 0 : L.oec + 4 * L.half};
-    for (long long e : ends) hi = std::max(hi, e);
-    lo = std::min({lo, L.oe, L.og, L.opb, L.oec < 0 ? lo : L.oec});
+// The coarsest level, smoothed in FP64 arithmetic (FP32 storage): one pair a
+// thread.  Values are widened by bit operations, which leave the FP64 unit
+// to the arithmetic.
+template <int DIM, typename F>
+__device__ __forceinline__ void cyc_coarsest(const Cyc& A, int x, const Slab& S, bool down, bool emit, int t,
+                                             F&& sync) {
+  const CycLev& L = A.L[x];
+  const int units = (S.n0 >> 1) * (DIM == 3 ? S.n1 : 1) * S.nr;
+  float *E0 = S.e, *E1 = S.e + S.var;
+  const bool on = t < units;
+  Pair p;
+  float e[2][2], g[2][2], pb[2];
+  const HaloOut H0 = halo_out(S, E0), H1 = halo_out(S, E1);
+  if (on) {
+    p = pair_of<DIM>(S, L, t);
+    const float kc = DIM == 2 ? 4.0f : 6.0f;
+#pragma unroll
+    for (int b = 0; b < 2; b++) {
+      e[b][0] = E0[p.at + b];
+      e[b][1] = E1[p.at + b];
+      g[b][0] = S.g[p.in + b];
+      g[b][1] = S.g[S.ivar + p.in + b];
+      pb[b] = S.pb[p.in + b];
+    }
+    if (down) {
+#pragma unroll
+      for (int b = 0; b < 2; b++) {
+        const float xx = e[b][0], y = e[b][1];
+        const float s0 = pair_sum<DIM, float>(E0, p, b, e[1 - b][0]);
+        const float s1 = pair_sum<DIM, float>(E1, p, b, e[1 - b][1]);
+        g[b][0] += xx - L.c0 * (s1 - kc * y);
+        g[b][1] += y - xx * (3.0f * pb[b] * (pb[b] + xx) + xx * xx) + L.c1 * (s0 - kc * xx);
+      }
+    }
   }
-  hi = (hi + 63) & ~63LL;
-  if (lo % 4 || (hi - lo) * (long long)sizeof(float) > kSmallSmemMax) return false;
-  nf = (int)(hi - lo);
-  for (int i = 0; i < S.n; i++) {
-    BoxLev& L = S.L[i];
-    L.oe -= lo;
-    L.og -= lo;
-    L.opb -= lo;
-    if (L.oec >= 0) L.oec -= lo;
+  if (down) sync();
+  for (int s = 0; s < 2 * A.nsmooth; s++) {
+    if (on) {
+      const int b = p.b0 ^ (s & 1);
+      auto dsum = [&](const float* a, float other) {
+        const float* c = a + p.at + b;
+        double q = f2d(b ? c[p.xr] : c[p.xl]) + f2d(other);
+        if (DIM == 2) return q + f2d(c[p.rm]) + f2d(c[p.rp]);
+        q = q + f2d(c[p.ym]) + f2d(c[p.yp]);
+        return q + (f2d(c[p.rm]) + f2d(c[p.rp]));
+      };
+      const double s0 = dsum(E0, b ? e[0][0] : e[1][0]), s1 = dsum(E1, b ? e[0][1] : e[1][1]);
+      const double pbd = f2d(b ? pb[1] : pb[0]), xv = f2d(b ? e[1][0] : e[0][0]);
+      const double w = pbd + xv;
+      const double a21 = -3.0 * w * w - A.cd[2];
+      const double b1 = f2d(b ? g[1][0] : g[0][0]) + A.cd[0] * s1;
+      const double b2 = f2d(b ? g[1][1] : g[0][1]) - A.cd[1] * s0 - xv * xv * (3.0 * pbd + 2.0 * xv);
+      const double rdet = __drcp_rn(1.0 - A.cd[3] * a21);
+      const float r0 = (float)((b1 - A.cd[3] * b2) * rdet), r1 = (float)((b2 - a21 * b1) * rdet);
+      if (b) e[1][0] = r0, e[1][1] = r1;
+      else e[0][0] = r0, e[0][1] = r1;
+      E0[p.at + b] = r0;
+      E1[p.at + b] = r1;
+      halo_put(S, H0, p.row, p.at + b, r0);
+      halo_put(S, H1, p.row, p.at + b, r1);
+    }
+    if (s + 1 < 2 * A.nsmooth) sync();
   }
-  return true;
+  if (emit && on) {
+    const HaloOut C0 = halo_out(S, S.ec), C1 = halo_out(S, S.ec + S.var);
+#pragma unroll
+    for (int b = 0; b < 2; b++)
+#pragma unroll
+      for (int v = 0; v < 2; v++) {
+        float* d = S.ec + v * S.var + p.at + b;
+        const float w = e[b][v] - *d;
+        *d = w;
+        halo_put(S, v ? C1 : C0, p.row, p.at + b, w);
+      }
+  }
+}
+
+template <int DIM>
+__global__ void __launch_bounds__(kCycThreads, 1) k_bx_cycle(float* __restrict__ fp, const __grid_constant__ Cyc A,
+                                                             BoxLev T, int fresh) {
+  const int rank = A.ctas > 1 ? uni::my_rank() : 0;
+  const int t = threadIdx.x, nt = blockDim.x;
+  auto all = [&] {
+    if (A.ctas > 1) uni::cluster_sync();
+    else __syncthreads();
+  };
+  {  // the top level: e (halo rows too; zero when fresh), g and pb from the colour-split arrays, a pair a thread
+    const Slab S = slab<DIM, false>(A, 0, rank);
+    const CycLev& L = A.L[0];
+    const V2 E = var2(fp, T.oe, T.half), G = var2(fp, T.og, T.half);
+    const int pr = (S.n0 >> 1) * (DIM == 3 ? S.n1 : 1);
+    if (S.shared || rank == 0)
+      for (int u = t; u < pr * (S.nr + 2); u += nt) {
+        int r, h, y = 0, k;
+        uni::fdivmod(u, L.hx, r, h);
+        if (DIM == 3) uni::fdivmod(r, L.d1, k, y);
+        else k = r;
+        int z = k + S.r0 - 1;
+        z = z < 0 ? z + S.N : (z >= S.N ? z - S.N : z);
+        const unsigned q = ((unsigned)z * (DIM == 3 ? S.n1 : 1) + y) * T.hh + h;
+        const int c = DIM == 3 ? (y + z + 1) & 1 : z & 1;  // colour of cell 2h
+        const unsigned i0 = q + (c ? (unsigned)T.half : 0u), i1 = q + (c ? 0u : (unsigned)T.half);
+        const int at = k * S.plane + (DIM == 3 ? y * S.n0 : 0) + 2 * h;
+        float v[4] = {0.f, 0.f, 0.f, 0.f};
+        if (!fresh) v[0] = E.v0[i0], v[1] = E.v0[i1], v[2] = E.v1[i0], v[3] = E.v1[i1];
+        S.e[at] = v[0], S.e[at + 1] = v[1];
+        S.e[S.var + at] = v[2], S.e[S.var + at + 1] = v[3];
+        if (k >= 1 && k <= S.nr) {
+          const int in = at - S.plane;
+          S.g[in] = G.v0[i0], S.g[in + 1] = G.v0[i1];
+          S.g[S.ivar + in] = G.v1[i0], S.g[S.ivar + in + 1] = G.v1[i1];
+          S.pb[in] = fp[T.opb + i0], S.pb[in + 1] = fp[T.opb + i1];
+        }
+      }
+  }
+  all();
+  auto smooth = [&](int x, int begin, bool restrict_, bool emit) {
+    const Slab S = slab<DIM, false>(A, x, rank);
+    const Slab C = x + 1 < A.nl ? slab<DIM, true>(A, x + 1, rank) : S;
+    auto sync = [&] {
+      if (S.shared) uni::cluster_sync();
+      else __syncthreads();
+    };
+    const int units = (S.n0 >> 1) * (DIM == 3 ? S.n1 : 1) * A.L[x].maxr;
+    if (x == A.nl - 1) cyc_coarsest<DIM>(A, x, S, begin == kDown, emit, t, sync);
+    else if (units <= nt) cyc_smooth<DIM, 1>(A, x, S, C, begin, restrict_, emit, t, nt, sync);
+    else cyc_smooth<DIM, kCycPairs>(A, x, S, C, begin, restrict_, emit, t, nt, sync);
+    // what the next level reads has been written
+    if (S.shared) uni::cluster_sync();
+    else __syncthreads();
+  };
+  for (int x = 0; x < A.nl; x++) {
+    if (!A.L[x].mul && rank) break;
+    smooth(x, x ? kDown : kTop, x + 1 < A.nl, x && x + 1 == A.nl);
+  }
+  for (int x = A.nl - 2; x >= 0; x--) {
+    if (!A.L[x].mul && rank) continue;
+    if (A.L[x].mul && !A.L[x + 1].mul) all();  // CTA 0 has finished the levels it holds
+    smooth(x, kUp, false, x > 0);
+  }
+  const Slab S = slab<DIM, false>(A, 0, rank);
+  const CycLev& L = A.L[0];
+  const V2 E = var2(fp, T.oe, T.half);
+  if (S.shared || rank == 0)
+    for (int u = t; u < (S.n0 >> 1) * (DIM == 3 ? S.n1 : 1) * S.nr; u += nt) {
+      const Pair p = pair_of<DIM>(S, L, u);
+      int r, h;
+      uni::fdivmod(u, L.hx, r, h);
+      const unsigned q = ((unsigned)S.r0 * (DIM == 3 ? S.n1 : 1) + r) * T.hh + h;
+#pragma unroll
+      for (int b = 0; b < 2; b++) {
+        const unsigned i = q + ((b ^ p.b0) ? (unsigned)T.half : 0u);
+        E.v0[i] = S.e[p.at + b];
+        E.v1[i] = S.e[S.var + p.at + b];
+      }
+    }
+  all();  // a CTA's shared memory stays while another may still write a halo
 }
 
 // After a cycle on the finest level: tracked residual g <- g - M(e) (M at
@@ -1397,32 +1705,135 @@ int bx_level_relax(Hier& H, int level, int nsmooth, bool fresh, bool coarse = fa
   return BSAMG_OK;
 }
 
-// AFASVcycle (afasroutines.f90:495-529) on the correction
-int bx_vcycle(Hier& H, int level, int minlevel, int nsmooth, bool fresh) {
-  if (2 * B(H, level).half <= kSmallCells) {
-    SmallLevels S{};
-    for (int l = level; l >= minlevel; l--) S.L[S.n++] = B(H, l);
-    long long lo;
-    int nf;
-    if (small_in_smem(S, lo, nf)) {
-      static std::atomic<unsigned long long> attr[2];  // the kernels' shared-memory limit, per device
-      if (needs_setup(attr[H.ndims - 2], H.ctx->device)) {
-        cudaError_t e = H.ndims == 2 ? cudaFuncSetAttribute(k_bx_small_vcycle_smem<2>,
-                                                            cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallSmemMax)
-                                     : cudaFuncSetAttribute(k_bx_small_vcycle_smem<3>,
-                                                            cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallSmemMax);
-        if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(k_bx_small_vcycle_smem)");
-        mark_setup(attr[H.ndims - 2], H.ctx->device);
+// clusters of `ctas` CTAs with smem bytes that fit at once; raises the
+// kernel's limits
+int cycle_fit(int ndims, int ctas, int smem) {
+  auto fit = [&](auto k) {
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) return 0;
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kUniSmemMax) != cudaSuccess) return 0;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(kCycThreads);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = ctas;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess) return 0;
+    return n;
+  };
+  const int n = ndims == 2 ? fit(k_bx_cycle<2>) : fit(k_bx_cycle<3>);
+  cudaGetLastError();  // a shape that does not fit is an answer, not an error
+  return n;
+}
+
+// The cluster's plan for the levels top .. minlevel with the first `share`
+// of them shared out; false when it does not fit (shared memory, pairs a
+// thread, the coarsest level's one pair a thread)
+bool cycle_layout(Hier& H, int top, int minlevel, int nsmooth, int share, Cyc& A, int* smem) {
+  const int D = H.ndims;
+  A = Cyc{};
+  A.nl = top - minlevel + 1;
+  A.nsmooth = nsmooth;
+  A.ctas = 1;
+  int nc = 1;
+  if (share) {
+    // whole rows of the first level CTA 0 holds (each CTA restricts whole
+    // coarse rows), or of the last level when all are shared
+    nc = B(H, top - std::min(share, A.nl - 1)).n[D - 1];
+    A.ctas = std::min(16, nc);
+    if (A.ctas < 2) return false;
+  }
+  int most = 0;
+  for (int r = 0; r < A.ctas; r++) {
+    const int a = r * nc / A.ctas, b = (r + 1) * nc / A.ctas;
+    A.R[r] = UniRank{(short)a, (short)(b - a)};
+    most = std::max(most, b - a);
+  }
+  long long o = 0, scratch = 0;
+  auto add = [&](long long n) {
+    const long long at = o;
+    o += (n + 3) & ~3LL;
+    return (int)at;
+  };
+  auto dv = [](int d) { return UniDiv{d, d <= 1 ? 0u : 0xFFFFFFFFu / (unsigned)d + 1u}; };
+  for (int x = 0; x < A.nl; x++) {
+    const BoxLev& P = B(H, top - x);
+    CycLev& L = A.L[x];
+    L.n0 = P.n[0], L.n1 = P.n[1], L.N = P.n[D - 1];
+    L.mul = x < share ? 1 << (std::min(share, A.nl - 1) - x) : 0;
+    L.maxr = L.mul ? most * L.mul : L.N;
+    const long long plane = (long long)P.n[0] * (D == 3 ? P.n[1] : 1);
+    const long long pairs = plane / 2 * L.maxr;
+    if (pairs > kCycThreads * (x + 1 < A.nl ? kCycPairs : 1)) return false;
+    L.e = add(2 * plane * (L.maxr + 2));
+    L.ec = x ? add(2 * plane * (L.maxr + 2)) : 0;
+    L.g = add(2 * plane * L.maxr);
+    L.pb = add(plane * L.maxr);
+    L.c0 = P.c0, L.c1 = P.c1, L.tmp3 = P.tmp3, L.a12 = P.a12;
+    L.hx = dv(P.n[0] / 2), L.d1 = dv(P.n[1]), L.hc = dv(P.n[0] / 2), L.dc1 = dv(std::max(1, P.n[1] / 2));
+    // the sums of the restriction keep the order of each size of level: small
+    // levels colour by colour, the others as k_bx_restrict_load
+    L.by_colour = 2 * P.half <= 8192;
+    if (x + 1 < A.nl) scratch = std::max(scratch, 4 * pairs);
+    if (o * 4 > kUniSmemMax) return false;
+  }
+  A.scratch = add(scratch);
+  for (int v = 0; v < 4; v++) A.cd[v] = B(H, minlevel).cd[v];
+  *smem = (int)(o * 4);
+  return *smem <= kUniSmemMax;
+}
+
+// The level from which the V-cycle runs in the cluster (the highest that
+// fits, or none), and the split of its levels: the cheapest by a model of a
+// sweep -- a barrier of the cluster or of the CTA and the issue slots of
+// about 70 instructions a pair.
+bool cycle_plan(Hier& H, int level, int minlevel, int nsmooth, Cyc& best, int* smem, int* at) {
+  for (int top = level; top >= minlevel; top--) {
+    double best_us = 0.0;
+    for (int share = 0; share <= top - minlevel + 1; share++) {
+      Cyc A;
+      int sm = 0;
+      if (!cycle_layout(H, top, minlevel, nsmooth, share, A, &sm) || cycle_fit(H.ndims, A.ctas, sm) < 1) continue;
+      double us = 0.0;
+      for (int x = 0; x < A.nl; x++) {
+        const double pairs = (double)B(H, top - x).half / (x < share ? A.ctas : 1);
+        us += (x < share ? 0.75 : 0.3) + pairs * 70 / 32 / 4 / 2000.0 * 1.5;
       }
-      size_t smem = (size_t)nf * sizeof(float);
-      if (H.ndims == 2)
-        k_bx_small_vcycle_smem<2><<<1, kSmallThreads, smem, H.s>>>(H.fpool, S, lo, nf, nsmooth, fresh ? 1 : 0);
-      else
-        k_bx_small_vcycle_smem<3><<<1, kSmallThreads, smem, H.s>>>(H.fpool, S, lo, nf, nsmooth, fresh ? 1 : 0);
-      return after_launch(H, 1);
+      if (best_us > 0.0 && us >= best_us) continue;
+      best_us = us;
+      best = A;
+      *smem = sm;
+      *at = top;
     }
-    if (H.ndims == 2) k_bx_small_vcycle<2><<<1, kSmallThreads, 0, H.s>>>(H.fpool, S, nsmooth, fresh ? 1 : 0);
-    else k_bx_small_vcycle<3><<<1, kSmallThreads, 0, H.s>>>(H.fpool, S, nsmooth, fresh ? 1 : 0);
+    if (best_us > 0.0) return true;
+  }
+  return false;
+}
+
+// AFASVcycle (afasroutines.f90:495-529) on the correction
+int bx_vcycle_from(Hier& H, int level, int minlevel, int nsmooth, bool fresh, const Cyc& cyc, int cyc_smem, int cyc_at) {
+  if (level <= cyc_at) {  // the rest of the V-cycle in one cluster launch
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(cyc.ctas);
+    cfg.blockDim = dim3(kCycThreads);
+    cfg.dynamicSmemBytes = cyc_smem;
+    cfg.stream = H.s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = cyc.ctas;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    const BoxLev& T = B(H, level);
+    cudaError_t e = H.ndims == 2 ? cudaLaunchKernelEx(&cfg, k_bx_cycle<2>, H.fpool, cyc, T, fresh ? 1 : 0)
+                                 : cudaLaunchKernelEx(&cfg, k_bx_cycle<3>, H.fpool, cyc, T, fresh ? 1 : 0);
+    if (e != cudaSuccess) return cuda_fail(e, "coarse V-cycle launch");
     return after_launch(H, 1);
   }
   if (level > minlevel && smooth_applies(H, B(H, level), nsmooth)) {
@@ -1436,7 +1847,7 @@ int bx_vcycle(Hier& H, int level, int minlevel, int nsmooth, bool fresh) {
     if (r) return r;
     BX_LAUNCH(H, sc, k_bx_restrict_load, H.fpool, Fb, C);
     BX_LAUNCH(H, sc, k_bx_coarse_op, H.fpool, C);
-    if ((r = bx_vcycle(H, level - 1, minlevel, nsmooth, false))) return r;
+    if ((r = bx_vcycle_from(H, level - 1, minlevel, nsmooth, false, cyc, cyc_smem, cyc_at))) return r;
     BX_LAUNCH(H, sc, k_bx_prolong, H.fpool, Fb, C);
     return bx_smooth(H, Fb, F.oe, false);
   }
@@ -1447,11 +1858,18 @@ int bx_vcycle(Hier& H, int level, int minlevel, int nsmooth, bool fresh) {
     Launch sc = shape(C.n[0], C.n[1], C.n[2]);
     BX_LAUNCH(H, sc, k_bx_restrict_load, H.fpool, F, C);
     BX_LAUNCH(H, sc, k_bx_coarse_op, H.fpool, C);
-    if ((r = bx_vcycle(H, level - 1, minlevel, nsmooth, false))) return r;
+    if ((r = bx_vcycle_from(H, level - 1, minlevel, nsmooth, false, cyc, cyc_smem, cyc_at))) return r;
     BX_LAUNCH(H, sc, k_bx_prolong, H.fpool, F, C);
     if ((r = bx_level_relax(H, level, nsmooth, false))) return r;
   }
   return BSAMG_OK;
+}
+
+int bx_vcycle(Hier& H, int level, int minlevel, int nsmooth, bool fresh) {
+  Cyc cyc;
+  int smem = 0, at = minlevel - 1;
+  cycle_plan(H, level, minlevel, nsmooth, cyc, &smem, &at);
+  return bx_vcycle_from(H, level, minlevel, nsmooth, fresh, cyc, smem, at);
 }
 
 int bx_finish(Hier& H, int finest, long long nparts, int errortype, bool to_host = true) {

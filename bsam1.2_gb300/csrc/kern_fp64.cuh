@@ -487,9 +487,6 @@ struct Uni64 {
     const double* qo = kOld ? X.x + xc : a;
     PL::template op<DIM>(a, c, g.sy, g.sz, g.sq, QoldView{qo, X.g.sy, X.g.sz, X.g.sq}, P.c, pp, r);
   }
-  template <int DIM>
-  __device__ __forceinline__ static void restrict_base(const uni::View<double>&, const uni::View<double>&, int, int,
-                                                       int, int) {}
   // the top level's q and f and every level's qold in; every level's q, f,
   // coarse image out
   template <int DIM>

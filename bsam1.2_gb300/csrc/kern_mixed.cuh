@@ -531,9 +531,6 @@ struct Uni32 {
                                             int fc, const PatchDev& P, const Par& mp, float* r) {
     PL::template mx_op<DIM>(a, c, g.sy, g.sz, g.sq, X.x, fc, X.sf, P.cf, mp, r);
   }
-  template <int DIM>
-  __device__ __forceinline__ static void restrict_base(const uni::View<float>&, const uni::View<float>&, int, int, int,
-                                                       int) {}
   // the top level's e and g and every level's base planes in; the top
   // level's e out (nothing reads the coarse corrections after the cycle)
   template <int DIM>

@@ -828,7 +828,6 @@ __device__ __forceinline__ void restrict_slab(const View<typename TR::T>& V, con
     }
     push_slab<TR, DIM>(V.c, gc, E, ci, cj, ck, w, bc, par);
     push_slab<TR, DIM>(U.q, U.g, EU, ci, pj, pk, w, bc, par);
-    TR::template restrict_base<DIM>(V, U, ci, cj, ck, up);
   }
 }
 

@@ -133,12 +133,12 @@ struct UniDiv {
 // extents, the coarse image's interior, +1 and ghosted extents, and the cells
 // of a plane's frame (3D) of the level and of its coarse image
 struct UniDim {
-  UniDiv hx, n0, n1, e0, c0, c1, cp0, cp1, ce0, ce1, ring, cring;
+  UniDiv hx, n0, n1, e0, e1, c0, c1, cp0, cp1, ce0, ce1, ring, cring;
 };
 inline UniDim uni_dim(const int* n) {
   auto dv = [](int d) { return UniDiv{d, d <= 1 ? 0u : 0xFFFFFFFFu / (unsigned)d + 1u}; };
   const int c0 = n[0] / 2, c1 = n[1] / 2;
-  return UniDim{dv((n[0] + 1) / 2), dv(n[0]), dv(n[1]), dv(n[0] + 2), dv(c0 > 0 ? c0 : 1), dv(c1 > 0 ? c1 : 1),
+  return UniDim{dv((n[0] + 1) / 2), dv(n[0]), dv(n[1]), dv(n[0] + 2), dv(n[1] + 2), dv(c0 > 0 ? c0 : 1), dv(c1 > 0 ? c1 : 1),
                 dv(c0 + 1), dv(c1 + 1), dv(c0 + 2), dv(c1 + 2), dv(2 * (n[0] + 2) + 2 * n[1]),
                 dv(2 * (c0 + 2) + 2 * c1)};
 }

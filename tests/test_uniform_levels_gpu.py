@@ -115,3 +115,30 @@ def test_mixed_cluster_equals_launches(pkg, ctx, case):
         h.close()
     assert out[0][0] == out[1][0]
     assert np.max(np.abs(out[0][1] - out[1][1])) <= 1e-9 * max(1.0, np.max(np.abs(out[1][1])))
+
+
+# (extents, minlevel): rows dealt unevenly, one shared level, none, pairs of
+# two cells a row, one level only, levels too large for the cluster above it
+BOXES = [((16, 96), -3), ((200, 56), -2), ((4, 64), -1), ((2, 2), 0), ((20, 20), 0), ((34, 50), 0), ((128, 128), -6),
+         ((256, 192), -5), ((16, 24, 40), -2), ((32, 32, 32), -4), ((4, 4, 64), -1), ((6, 10, 2), 0), ((64, 48, 32), -3)]
+
+
+@pytest.mark.parametrize("n,mn", BOXES)
+def test_box_solve_reaches_the_fp64_solution(pkg, ctx, n, mn):
+    """Mixed steps on periodic boxes, converged tightly, against the FP64
+    path: the residual 1e-11 bounds the difference by about 1e-11 over the
+    operator's smallest eigenvalue (one), 1e-9 is a hundred times that."""
+    nd = len(n)
+    q = {}
+    for mode in ("fp64", "mixed"):
+        h = pkg.Hierarchy(ctx, nd, 2, "ch", [1e-5, 0.05])
+        h.build_uniform(list(n) + [1] * (3 - nd), mn, [2] * (2 * nd) + [10] * (6 - 2 * nd), [0, 0, 0],
+                        [v / n[0] for v in n] + [1] * (3 - nd))
+        h.commit()
+        h.seed_spinodal(0, 3)
+        for s in range(3):
+            _, res = h.time_step(s == 0, 0, mn, tol=1e-11, maxvcycles=40, mode=mode)
+            assert res[-1] < 1e-11
+        q[mode] = h.get(0, "q")
+        h.close()
+    assert np.max(np.abs(q["mixed"] - q["fp64"])) <= 1e-9
