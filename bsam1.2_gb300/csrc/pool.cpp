@@ -10,6 +10,7 @@
 #include <atomic>
 #include <condition_variable>
 #include <functional>
+#include <memory>
 #include <mutex>
 #include <thread>
 #include <vector>
@@ -40,52 +41,60 @@ class Pool {
       for (int x = 0; x < n; x++) f(x);
       return;
     }
+    auto b = std::make_shared<Batch>(f, n);
     {
       std::lock_guard<std::mutex> g(mu_);
-      fn_ = &f;
-      n_ = n;
-      next_.store(0);
-      left_ = n;
+      batch_ = b;
       gen_++;
     }
     cv_.notify_all();
-    work();
+    work(*b);
     std::unique_lock<std::mutex> g(mu_);
-    done_.wait(g, [&] { return left_ == 0; });
-    fn_ = nullptr;
+    done_.wait(g, [&] { return b->left.load() == 0; });
+    batch_.reset();
   }
 
  private:
-  void work() {
+  // One call's items.  Every call has its own counters: a worker that is
+  // still leaving an earlier call draws its last number from that call's
+  // (with counters shared by all calls it could draw an item of the next one
+  // that another thread draws again, and the count of what is left missed
+  // zero).  f outlives every item, not the batch.
+  struct Batch {
+    const std::function<void(int)>& f;
+    const int n;
+    std::atomic<int> next{0}, left;
+    Batch(const std::function<void(int)>& fn, int items) : f(fn), n(items), left(items) {}
+  };
+  void work(Batch& b) {
     int done = 0;
-    for (int x; (x = next_.fetch_add(1)) < n_;) {
-      (*fn_)(x);
+    for (int x; (x = b.next.fetch_add(1)) < b.n;) {
+      b.f(x);
       done++;
     }
-    if (done) {
+    if (done && b.left.fetch_sub(done) == done) {
       std::lock_guard<std::mutex> g(mu_);
-      left_ -= done;
-      if (left_ == 0) done_.notify_all();
+      done_.notify_all();
     }
   }
   void loop() {
     unsigned long long seen = 0;
     for (;;) {
+      std::shared_ptr<Batch> b;
       {
         std::unique_lock<std::mutex> g(mu_);
-        cv_.wait(g, [&] { return quit_ || (gen_ != seen && fn_); });
+        cv_.wait(g, [&] { return quit_ || (gen_ != seen && batch_); });
         if (quit_) return;
         seen = gen_;
+        b = batch_;
       }
-      work();
+      work(*b);
     }
   }
   std::vector<std::thread> workers_;
   std::mutex mu_, run_mu_;
   std::condition_variable cv_, done_;
-  const std::function<void(int)>* fn_ = nullptr;
-  int n_ = 0, left_ = 0;
-  std::atomic<int> next_{0};
+  std::shared_ptr<Batch> batch_;
   unsigned long long gen_ = 0;
   bool quit_ = false;
 };
