@@ -1873,14 +1873,8 @@ int bx_vcycle(Hier& H, int level, int minlevel, int nsmooth, bool fresh) {
 }
 
 int bx_finish(Hier& H, int finest, long long nparts, int errortype, bool to_host = true) {
-  int r = after_launch(H, launch_norm_finish(H.s, H.d_partial, (int)nparts, H.nrvars, H.L(finest).count, errortype,
-                                             H.d_norm, H.d_nonfinite));
-  if (r || !to_host) return r;
-  cudaError_t ce = cudaMemcpyAsync(H.h_norm, H.d_norm, 2 * sizeof(double), cudaMemcpyDeviceToHost, H.s);
-  if (ce != cudaSuccess) return cuda_fail(ce, "cudaMemcpyAsync(norm)");
-  ce = cudaMemcpyAsync(H.h_nonfinite, H.d_nonfinite, sizeof(int), cudaMemcpyDeviceToHost, H.s);
-  if (ce != cudaSuccess) return cuda_fail(ce, "cudaMemcpyAsync(nonfinite)");
-  return BSAMG_OK;
+  return after_launch(H, launch_norm_finish(H.s, H.d_partial, (int)nparts, H.nrvars, H.L(finest).count, errortype,
+                                            H.d_norm, H.d_nonfinite, to_host ? H.h_norm : nullptr));
 }
 
 int bx_resid(Hier& H, int finest, int errortype, bool to_host = true) {

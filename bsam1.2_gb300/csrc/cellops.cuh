@@ -1,6 +1,7 @@
 // Cell addressing and the undivided Laplacian, shared by the kernels of both
 // paths and by the plugins' device code.
 #pragma once
+#include "fp64int.cuh"
 #include "internal.h"
 
 namespace bsamg {
@@ -20,8 +21,14 @@ __device__ __forceinline__ long long iofs(const int* mx, int i, int j, int k) {
 }
 
 // ULap2D / ULap3D, LIBRARY/gridutilities.f90:50-72, :372-399
+// In the FP64 part of a plugin (the reference's rounding) the 3D sum runs on
+// the integer pipe: the FP64 unit bounds every kernel that evaluates it.
 template <int DIM, typename T>
 __device__ __forceinline__ T ulap(const T* a, long long c, long long sy, long long sz) {
+#ifdef BSAMG_PART_FP64
+  if constexpr (DIM == 3 && sizeof(T) == sizeof(double))
+    return fxp::lap6({a[c + 1], a[c - 1], a[c + sy], a[c - sy], a[c + sz], a[c - sz]}, a[c]);
+#endif
   if (DIM == 2) return a[c + 1] + a[c - 1] + a[c + sy] + a[c - sy] - T(4) * a[c];
   return a[c + 1] + a[c - 1] + a[c + sy] + a[c - sy] + a[c + sz] + a[c - sz] - T(6) * a[c];
 }

@@ -97,38 +97,54 @@ __global__ void __launch_bounds__(kBlock) k_norm_stage(const double* __restrict_
 // One CTA of 1024 threads; each thread keeps eight independent partial sums
 // per variable so that eight loads are in flight, then a fixed-shape tree.
 // The order of the additions depends only on nblk, so the result is
-// deterministic.  Partials hold NV values per block.
+// deterministic.  Partials hold NV values per block.  Additions of the zeros
+// of threads without a partial change nothing and are left out: on GB300 an
+// FP64 instruction holds a scheduler for 64 cycles or more, and the whole
+// tree took 10.4 us whatever nblk, 4 us now for up to 64 partials.
 constexpr int kFinishThreads = 1024;
 template <int NV>
 __global__ void __launch_bounds__(kFinishThreads) k_norm_finish(const double* __restrict__ partial, int nblk,
                                                                 double count, int errortype, double* out,
-                                                                int* nonfinite) {
+                                                                int* nonfinite, double* host, double* one) {
   __shared__ double red[NV][kFinishThreads / 32];
-  double a[NV][8];
-  for (int v = 0; v < NV; v++)
-    for (int u = 0; u < 8; u++) a[v][u] = 0.0;
-  int n = threadIdx.x;
-  for (; n + 7 * kFinishThreads < nblk; n += 8 * kFinishThreads)
-    for (int u = 0; u < 8; u++)
-      for (int v = 0; v < NV; v++) a[v][u] = a[v][u] + partial[NV * (n + u * kFinishThreads) + v];
-  // the remaining (at most seven) partials of this thread; a constant index
-  // keeps a[][] in registers
-  for (; n < nblk; n += kFinishThreads)
-    for (int v = 0; v < NV; v++) a[v][0] = a[v][0] + partial[NV * n + v];
-  double t[NV];
-  for (int v = 0; v < NV; v++)
-    t[v] = ((a[v][0] + a[v][1]) + (a[v][2] + a[v][3])) + ((a[v][4] + a[v][5]) + (a[v][6] + a[v][7]));
-  for (int o = 16; o > 0; o >>= 1)
-    for (int v = 0; v < NV; v++) t[v] = t[v] + __shfl_down_sync(0xffffffffu, t[v], o);
-  int w = threadIdx.x >> 5;
-  if ((threadIdx.x & 31) == 0)
-    for (int v = 0; v < NV; v++) red[v][w] = t[v];
-  __syncthreads();
-  if (w == 0) {
-    for (int v = 0; v < NV; v++) t[v] = red[v][threadIdx.x];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int warps = min(kFinishThreads / 32, (nblk + 31) / 32);  // warps that hold a partial
+  if (w < warps) {
+    double t[NV];
+    if (nblk > 7 * kFinishThreads) {
+      double a[NV][8];
+      for (int v = 0; v < NV; v++)
+        for (int u = 0; u < 8; u++) a[v][u] = 0.0;
+      int n = threadIdx.x;
+      for (; n + 7 * kFinishThreads < nblk; n += 8 * kFinishThreads)
+        for (int u = 0; u < 8; u++)
+          for (int v = 0; v < NV; v++) a[v][u] = a[v][u] + partial[NV * (n + u * kFinishThreads) + v];
+      // the remaining (at most seven) partials of this thread; a constant index
+      // keeps a[][] in registers
+      for (; n < nblk; n += kFinishThreads)
+        for (int v = 0; v < NV; v++) a[v][0] = a[v][0] + partial[NV * n + v];
+      for (int v = 0; v < NV; v++)
+        t[v] = ((a[v][0] + a[v][1]) + (a[v][2] + a[v][3])) + ((a[v][4] + a[v][5]) + (a[v][6] + a[v][7]));
+    } else {  // fewer than eight a thread: one sum
+      for (int v = 0; v < NV; v++) t[v] = threadIdx.x < nblk ? partial[NV * threadIdx.x + v] : 0.0;
+      for (int n = threadIdx.x + kFinishThreads; n < nblk; n += kFinishThreads)
+        for (int v = 0; v < NV; v++) t[v] = t[v] + partial[NV * n + v];
+    }
+    const int lanes = nblk - (w << 5);  // lanes of the warp that hold one (the last warp's; the others all)
     for (int o = 16; o > 0; o >>= 1)
-      for (int v = 0; v < NV; v++) t[v] = t[v] + __shfl_down_sync(0xffffffffu, t[v], o);
-    if (threadIdx.x == 0)
+      if (o < lanes)
+        for (int v = 0; v < NV; v++) t[v] = t[v] + __shfl_down_sync(0xffffffffu, t[v], o);
+    if (lane == 0)
+      for (int v = 0; v < NV; v++) red[v][w] = t[v];
+  }
+  __syncthreads();
+  if (w == 0 && warps > 1) {
+    double t[NV];
+    for (int v = 0; v < NV; v++) t[v] = lane < warps ? red[v][lane] : 0.0;
+    for (int o = 16; o > 0; o >>= 1)
+      if (o < warps)
+        for (int v = 0; v < NV; v++) t[v] = t[v] + __shfl_down_sync(0xffffffffu, t[v], o);
+    if (lane == 0)
       for (int v = 0; v < NV; v++) red[v][0] = t[v];
   }
   __syncthreads();
@@ -148,7 +164,14 @@ __global__ void __launch_bounds__(kFinishThreads) k_norm_finish(const double* __
     }
     out[0] = r;
     out[1] = sum;
-    if (nonfinite) nonfinite[0] = isfinite(r) ? 0 : 1;
+    const int bad = isfinite(r) ? 0 : 1;
+    if (nonfinite) nonfinite[0] = bad;
+    if (host) {
+      host[0] = r;
+      host[1] = sum;
+      *reinterpret_cast<int*>(host + 8) = bad;
+    }
+    if (one) *one = r;
   }
 }
 
@@ -234,7 +257,7 @@ int launch_norm_partial(const LaunchCtx& c, const Blk* blk, int nblk, double* pa
   return ops_of(c).norm_partial(c, blk, nblk, partial, store_rf);
 }
 int launch_norm_finish(cudaStream_t s, const double* partial, int nblk, int nrvars, double count, int errortype,
-                       double* out, int* nonfinite) {
+                       double* out, int* nonfinite, double* host, double* one) {
   int n = 1;
   if (nblk > 2048) {
     // two stages; out[8 ..] holds the stage sums
@@ -247,8 +270,9 @@ int launch_norm_finish(cudaStream_t s, const double* partial, int nblk, int nrva
     nblk = g;
     n = 2;
   }
-  if (nrvars == 3) k_norm_finish<3><<<1, kFinishThreads, 0, s>>>(partial, nblk, count, errortype, out, nonfinite);
-  else k_norm_finish<2><<<1, kFinishThreads, 0, s>>>(partial, nblk, count, errortype, out, nonfinite);
+  if (nrvars == 3) k_norm_finish<3><<<1, kFinishThreads, 0, s>>>(partial, nblk, count, errortype, out, nonfinite, host, one);
+  else
+    k_norm_finish<2><<<1, kFinishThreads, 0, s>>>(partial, nblk, count, errortype, out, nonfinite, host, one);
   return n;
 }
 int launch_ghost_stage(const LaunchCtx& c, const GhostOp* ops, int n) {

@@ -272,13 +272,18 @@ int enq_update_source(Hier& H, int finest) {
   return BSAMG_OK;
 }
 
-// ErrorAFAS on `level` -> H.d_norm[0] (device)
-int enq_norm(Hier& H, int level, int errortype) {
+// ErrorAFAS on `level` -> H.d_norm[0] (device) and the pinned record; update:
+// UpdateSourceFunction on the (uniform) level in the same pass
+int enq_norm(Hier& H, int level, int errortype, bool update) {
   LevelT& L = H.L(level);
-  RET(after_launch(H, launch_norm_partial(H.lc(), L.d_blk[kKindInterior], L.nblk[kKindInterior], H.d_partial, 1)));
+  if (uni_level(H, level)) {
+    const int p = uni_patch(H, level);
+    RET(after_launch(H, find_plugin(H.problem)->fp64->uni_norm(H.lc(), p, H.hP[p], H.d_partial, 1, update)));
+  } else {
+    RET(after_launch(H, launch_norm_partial(H.lc(), L.d_blk[kKindInterior], L.nblk[kKindInterior], H.d_partial, 1)));
+  }
   return after_launch(H, launch_norm_finish(H.s, H.d_partial, norm_partials(L.nblk[kKindInterior]), H.nrvars, L.count,
-                                            errortype,
-                                            H.d_norm, H.d_nonfinite));
+                                            errortype, H.d_norm, H.d_nonfinite, H.h_norm));
 }
 
 int enq_copy_q_to_qold(Hier& H, int minlevel, int finest) {
@@ -305,7 +310,7 @@ int finish_fill_down(Hier& H, int finest, int minlevel) {
 }
 
 // One V-cycle iteration body of MultigridIterations (afasroutines.f90:81-104)
-// followed by a copy of the norm to pinned host memory.
+// followed by the norm, which the host reads in pinned memory.
 int enq_iteration(Hier& H, int finest, int minlevel, int nsmooth, int errortype) {
   RET(enq_vcycle(H, finest, minlevel, nsmooth));
   // With uniform levels <= 0 the next V-cycle writes q and f below level 0,
@@ -313,12 +318,10 @@ int enq_iteration(Hier& H, int finest, int minlevel, int nsmooth, int errortype)
   // CoarseLoadingFunction cover them whole), so FillDown of those is done
   // once, after the last cycle (finish_fill_down).
   RET(enq_fill_down(H, 2, finest, H.uni ? std::max(0, minlevel) : minlevel));
-  RET(enq_update_source(H, finest));
+  const bool fused = uni_level(H, finest);  // one level to update: in the norm's pass
+  if (!fused) RET(enq_update_source(H, finest));
   if (!H.uni) RET(enq_fill_down(H, 1, finest, minlevel));
-  RET(enq_norm(H, finest, errortype));
-  CK(cudaMemcpyAsync(H.h_norm, H.d_norm, 2 * sizeof(double), cudaMemcpyDeviceToHost, H.s));
-  CK(cudaMemcpyAsync(H.h_nonfinite, H.d_nonfinite, sizeof(int), cudaMemcpyDeviceToHost, H.s));
-  return BSAMG_OK;
+  return enq_norm(H, finest, errortype, fused);
 }
 
 int capture_graph(Hier& H, const GraphKey& key, const std::function<int()>& body, Hier::GraphRec** out) {
@@ -1207,8 +1210,7 @@ int bsamg_residual_norm(bsamg_hier* h, int level, int errortype, double* out) {
   if (!h || !h->committed || !level_ok(*h, level) || !out || (errortype != 1 && errortype != 2))
     return BSAMG_ERR_ARG;
   RET(set_device(*h));
-  RET(enq_norm(*h, level, errortype));
-  CK(cudaMemcpyAsync(h->h_norm, h->d_norm, 2 * sizeof(double), cudaMemcpyDeviceToHost, h->s));
+  RET(enq_norm(*h, level, errortype, false));
   CK(cudaStreamSynchronize(h->s));
   *out = h->h_norm[0];
   return BSAMG_OK;

@@ -221,7 +221,7 @@ int set_device(const Hier& H);
 int enq_set_ghost(Hier& H, int level, int ipass);
 int enq_fill_down(Hier& H, int field, int finest, int minlevel);
 int enq_update_source(Hier& H, int finest);
-int enq_norm(Hier& H, int level, int errortype);
+int enq_norm(Hier& H, int level, int errortype, bool update);
 int enq_relax(Hier& H, int level, int ipass);
 // plugin coefficients for a spacing h (PatchDev::c)
 void coefficients(const Hier& H, double h, double* c);

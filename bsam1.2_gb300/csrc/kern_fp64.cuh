@@ -323,20 +323,38 @@ __global__ void __launch_bounds__(kBlock) k_update_source(const PatchDev* __rest
   for (int v = 0; v < NV; v++) pool[p.of + v * p.sf + fc] = pool[p.oftmp + v * p.sf + fc] + su[v];
 }
 
+// the sums of a block's NV values a thread -> partial[NV blockIdx.x + v], in a
+// fixed order
+template <int NV>
+__device__ __forceinline__ void block_sum(double (&s)[NV], double (*red)[kBlock / 32], double* __restrict__ partial) {
+  for (int o = 16; o > 0; o >>= 1)
+    for (int v = 0; v < NV; v++) s[v] = s[v] + __shfl_down_sync(0xffffffffu, s[v], o);
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  if (l == 0)
+    for (int v = 0; v < NV; v++) red[v][w] = s[v];
+  __syncthreads();
+  if (threadIdx.x < NV) {  // a thread a variable
+    const int v = threadIdx.x;
+    double t = 0.0;
+    for (int n = 0; n < kBlock / 32; n++) t = t + red[v][n];
+    partial[NV * blockIdx.x + v] = t;
+  }
+}
+
 // ErrorAFAS partial sums (afasroutines.f90:113-233): rf = f - Op(q) on the
-// level's patches, sums of rf^2 per variable over kNormGroup consecutive
+// level's patches, sums of rf^2 per variable over `group` consecutive
 // blocks of the work list per CTA (each thread adds its cells in block
 // order, then one fixed reduction tree).
 template <class PL, int DIM>
-__global__ void __launch_bounds__(kBlock) k_norm_partial(const PatchDev* __restrict__ P, double* __restrict__ pool,
-                                                         const Blk* __restrict__ blk, int nblk, ProbParams pp,
-                                                         double* __restrict__ partial, int store_rf) {
+__global__ void __launch_bounds__(kBlock, 4) k_norm_partial(const PatchDev* __restrict__ P, double* __restrict__ pool,
+                                                         const Blk* __restrict__ blk, int nblk, int group,
+                                                         ProbParams pp, double* __restrict__ partial, int store_rf) {
   constexpr int NV = PL::kNV;
   __shared__ double red[NV][kBlock / 32];
   double s[NV];
   for (int v = 0; v < NV; v++) s[v] = 0.0;
-  for (int sub = 0; sub < kNormGroup; sub++) {
-    int bi = blockIdx.x * kNormGroup + sub;
+  for (int sub = 0; sub < group; sub++) {
+    int bi = blockIdx.x * group + sub;
     if (bi >= nblk) break;
     const Blk b = blk[bi];
     const PatchDev& p = P[b.patch];
@@ -351,21 +369,55 @@ __global__ void __launch_bounds__(kBlock) k_norm_partial(const PatchDev* __restr
     for (int v = 0; v < NV; v++) {
       double e = pool[p.of + v * p.sf + fc] - r[v];
       if (store_rf) pool[p.orf + v * p.sf + fc] = e;
-      s[v] = s[v] + e * e;
+      s[v] = fma(e, e, s[v]);
     }
   }
-  for (int o = 16; o > 0; o >>= 1)
-    for (int v = 0; v < NV; v++) s[v] = s[v] + __shfl_down_sync(0xffffffffu, s[v], o);
-  int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  if (l == 0)
-    for (int v = 0; v < NV; v++) red[v][w] = s[v];
-  __syncthreads();
-  if (threadIdx.x == 0)
-    for (int v = 0; v < NV; v++) {
-      double t = 0.0;
-      for (int n = 0; n < kBlock / 32; n++) t = t + red[v][n];
-      partial[NV * blockIdx.x + v] = t;
+  block_sum<NV>(s, red, partial);
+}
+
+// The same on a uniform level, without a work list, and with
+// UpdateSourceFunction (afasroutines.f90:438-492) first when `update`:
+// f = ftmp + SourceUpdate.  The block decomposition and the order of the
+// sums are k_norm_partial's.
+template <class PL, int DIM>
+__global__ void __launch_bounds__(kBlock, 4) k_uni_norm(const PatchDev* __restrict__ P, double* __restrict__ pool,
+                                                     int patch, const __grid_constant__ UniPatch u, int group,
+                                                     ProbParams pp, double* __restrict__ partial, int store_rf,
+                                                     int update) {
+  constexpr int NV = PL::kNV;
+  __shared__ double red[NV][kBlock / 32];
+  const PatchDev& p = u.p;
+  const int cells = (int)p.sf;
+  const long long sy = p.qn[0], sz = (long long)p.qn[0] * p.qn[1];
+  const double* q = pool + p.oq;
+  double s[NV];
+  for (int v = 0; v < NV; v++) s[v] = 0.0;
+  for (int sub = 0; sub < group; sub++) {
+    const int fc = (blockIdx.x * group + sub) * kBlock + (int)threadIdx.x;
+    if (fc >= cells) break;
+    int i, j, k;
+    uni::inner_unit<DIM>(u.d.n0, u.d.n1, fc, i, j, k);
+    const long long c = gofs<DIM>(p.qn, i, j, k);
+    const QoldView qo{pool + p.oqold + c, sy, sz, p.sq};
+    double f[NV], r[NV];
+    if (update) {
+      double su[NV];
+      PL::template source_update<DIM>(q, c, sy, sz, p.sq, qo, P[patch].c, pp, su);
+      for (int v = 0; v < NV; v++) {
+        f[v] = pool[p.oftmp + v * p.sf + fc] + su[v];
+        pool[p.of + v * p.sf + fc] = f[v];
+      }
+    } else {
+      for (int v = 0; v < NV; v++) f[v] = pool[p.of + v * p.sf + fc];
     }
+    PL::template op<DIM>(q, c, sy, sz, p.sq, qo, P[patch].c, pp, r);
+    for (int v = 0; v < NV; v++) {
+      const double e = f[v] - r[v];
+      if (store_rf) pool[p.orf + v * p.sf + fc] = e;
+      s[v] = fma(e, e, s[v]);
+    }
+  }
+  block_sum<NV>(s, red, partial);
 }
 
 // The coarse tail of the V-cycle in one block (see TailPhase): the
@@ -543,9 +595,18 @@ struct Fp64Launchers {
   }
   static int norm_partial(const LaunchCtx& c, const Blk* blk, int nblk, double* partial, int store_rf) {
     if (nblk <= 0) return 0;
-    int g = norm_partials(nblk);
-    if (c.ndims == 2) k_norm_partial<PL, 2><<<g, kBlock, 0, c.s>>>(c.P, c.pool, blk, nblk, c.pp, partial, store_rf);
-    else k_norm_partial<PL, 3><<<g, kBlock, 0, c.s>>>(c.P, c.pool, blk, nblk, c.pp, partial, store_rf);
+    const int g = norm_partials(nblk), n = norm_group(nblk);
+    if (c.ndims == 2) k_norm_partial<PL, 2><<<g, kBlock, 0, c.s>>>(c.P, c.pool, blk, nblk, n, c.pp, partial, store_rf);
+    else k_norm_partial<PL, 3><<<g, kBlock, 0, c.s>>>(c.P, c.pool, blk, nblk, n, c.pp, partial, store_rf);
+    return 1;
+  }
+  static int uni_norm(const LaunchCtx& c, int patch, const PatchDev& hp, double* partial, int store_rf, int update) {
+    const int nblk = (int)((hp.sf + kBlock - 1) / kBlock), g = norm_partials(nblk), n = norm_group(nblk);
+    const UniPatch u = uni_patch_of(hp);
+    if (c.ndims == 2)
+      k_uni_norm<PL, 2><<<g, kBlock, 0, c.s>>>(c.P, c.pool, patch, u, n, c.pp, partial, store_rf, update);
+    else
+      k_uni_norm<PL, 3><<<g, kBlock, 0, c.s>>>(c.P, c.pool, patch, u, n, c.pp, partial, store_rf, update);
     return 1;
   }
   static int get_source(const LaunchCtx& c, const Blk* blk, int nblk) {
@@ -583,7 +644,7 @@ const PluginFp64* fp64_ops() {
                                  &Fp64Launchers<PL>::norm_partial, &Fp64Launchers<PL>::get_source,
                                  &Fp64Launchers<PL>::update_source, &Fp64Launchers<PL>::tail,
                                  &Fp64Launchers<PL>::tail_smem,    &Fp64Launchers<PL>::tail_smem_attributes,
-                                 uni::UniLaunchers<Uni64<PL>>::table()};
+                                 uni::UniLaunchers<Uni64<PL>>::table(), &Fp64Launchers<PL>::uni_norm};
   return &ops;
 }
 

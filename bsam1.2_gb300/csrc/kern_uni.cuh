@@ -182,13 +182,33 @@ __device__ __forceinline__ void relax(const View<typename TR::T>& V, int ipass, 
   }
 }
 
+// x 2^K and, in 3D, 3 x: FP64 on the integer pipe (fp64int.cuh; a chain of
+// FP64 instructions bounds the small levels, their number the large ones)
+template <int K>
+__device__ __forceinline__ double scaled(double x) {
+  return fxp::scaled<K>(x);
+}
+template <int K>
+__device__ __forceinline__ float scaled(float x) {
+  return x * (K < 0 ? 1.0f / (1 << (K < 0 ? -K : 0)) : 1.0f * (1 << (K > 0 ? K : 0)));
+}
+template <int DIM>
+__device__ __forceinline__ double triple(double x) {
+  if constexpr (DIM == 3) return fxp::triple(x);
+  return 3.0 * x;
+}
+template <int DIM>
+__device__ __forceinline__ float triple(float x) {
+  return 3.0f * x;
+}
+
 // mean of the 4 (8) fine values whose highest cell is a[0], summed in the
 // order of Restriction2D/3D (gridutilities.f90:103-126, :437-466)
 template <int DIM, typename T>
 __device__ __forceinline__ T mean(const T* a, int sy, int sz) {
   T s = a[0] + a[-1] + a[-sy] + a[-sy - 1];
   if (DIM == 3) s = s + a[-sz] + a[-sz - 1] + a[-sz - sy] + a[-sz - sy - 1];
-  return (DIM == 2 ? T(0.25) : T(0.125)) * s;
+  return scaled<DIM == 2 ? -2 : -3>(s);
 }
 
 // RestrictSolution (afasroutines.f90:610-652): the coarse image and the
@@ -251,7 +271,7 @@ __device__ __forceinline__ void coarse_load(const View<typename TR::T>& V, const
     const int fu = icell<DIM>(U.g, ci, cj, ck);
     TR::template op<DIM>(V.c, gcell<DIM>(gc, ci, cj, ck), gc, U, gcell<DIM>(U.g, ci, cj, ck), fu, PU, par, cr);
 #pragma unroll
-    for (int v = 0; v < TR::NV; v++) U.f[v * U.sf + fu] = (DIM == 2 ? T(0.25) : T(0.125)) * R[v] + cr[v];
+    for (int v = 0; v < TR::NV; v++) U.f[v * U.sf + fu] = scaled<DIM == 2 ? -2 : -3>(R[v]) + cr[v];
   }
 }
 
@@ -339,21 +359,21 @@ __device__ __forceinline__ void correct_b(const View<typename TR::T>& V, const V
 #pragma unroll
         for (int dy = 0; dy < 2; dy++) {
           const T lo = at(ci, cj + dy, ck + dz), hi = at(ci + 1, cj + dy, ck + dz);
-          b[dz][dy][0] = T(3) * lo + hi;
-          b[dz][dy][1] = lo + T(3) * hi;
+          b[dz][dy][0] = triple<DIM>(lo) + hi;
+          b[dz][dy][1] = lo + triple<DIM>(hi);
         }
 #pragma unroll
       for (int fy = 0; fy < 2; fy++)
 #pragma unroll
         for (int fx = 0; fx < 2; fx++) {
-          const T c0 = fy == 0 ? T(3) * b[0][0][fx] + b[0][1][fx] : b[0][0][fx] + T(3) * b[0][1][fx];
+          const T c0 = fy == 0 ? triple<DIM>(b[0][0][fx]) + b[0][1][fx] : b[0][0][fx] + triple<DIM>(b[0][1][fx]);
           if (DIM == 2) {
-            out[fy * 2 + fx][v] = c0 * T(1.0 / 16.0);
+            out[fy * 2 + fx][v] = scaled<-4>(c0);
           } else {
-            const T c1 =
-                fy == 0 ? T(3) * b[NZ - 1][0][fx] + b[NZ - 1][1][fx] : b[NZ - 1][0][fx] + T(3) * b[NZ - 1][1][fx];
-            out[fy * 2 + fx][v] = (T(3) * c0 + c1) * T(1.0 / 64.0);
-            out[(NZ - 1) * 4 + fy * 2 + fx][v] = (c0 + T(3) * c1) * T(1.0 / 64.0);
+            const T c1 = fy == 0 ? triple<DIM>(b[NZ - 1][0][fx]) + b[NZ - 1][1][fx]
+                                 : b[NZ - 1][0][fx] + triple<DIM>(b[NZ - 1][1][fx]);
+            out[fy * 2 + fx][v] = scaled<-6>(triple<DIM>(c0) + c1);
+            out[(NZ - 1) * 4 + fy * 2 + fx][v] = scaled<-6>(c0 + triple<DIM>(c1));
           }
         }
     }
@@ -902,18 +922,18 @@ __device__ __forceinline__ void correct_slab(const View<typename TR::T>& V, cons
       };
       auto row = [&](int jj, int kk) -> T {  // the x stage at coarse row (jj, kk)
         const T lo = at(ci, jj, kk), hi = at(ci + 1, jj, kk);
-        return fx ? lo + T(3) * hi : T(3) * lo + hi;
+        return fx ? lo + triple<DIM>(hi) : triple<DIM>(lo) + hi;
       };
       auto plane = [&](int kk) -> T {
         const T lo = row(cj, kk), hi = row(cj + 1, kk);
-        return fy ? lo + T(3) * hi : T(3) * lo + hi;
+        return fy ? lo + triple<DIM>(hi) : triple<DIM>(lo) + hi;
       };
       T add;
       if (DIM == 2) {
-        add = plane(0) * T(1.0 / 16.0);
+        add = scaled<-4>(plane(0));
       } else {
         const T lo = plane(ck), hi = plane(ck + 1);
-        add = (fz ? lo + T(3) * hi : T(3) * lo + hi) * T(1.0 / 64.0);
+        add = scaled<-6>(fz ? lo + triple<DIM>(hi) : triple<DIM>(lo) + hi);
       }
       w[v] = V.q[v * g.sq + c] + add;
       V.q[v * g.sq + c] = w[v];

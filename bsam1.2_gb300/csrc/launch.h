@@ -196,20 +196,27 @@ int launch_fill_down(const LaunchCtx& c, const Blk* blk, int nblk, int field);
 int launch_get_source(const LaunchCtx& c, const Blk* blk, int nblk);
 int launch_update_source(const LaunchCtx& c, const Blk* blk, int nblk);
 // partial sums of rf^2 (nrvars per CTA) -> partial[norm_partials(nblk)*nrvars]:
-// one CTA per kNormGroup consecutive blocks of the work list, so the FP64
-// shuffle reduction is paid once per kNormGroup * 256 cells
-constexpr int kNormGroup = 4;
-inline int norm_partials(int nblk) { return (nblk + kNormGroup - 1) / kNormGroup; }
+// one CTA per norm_group(nblk) consecutive blocks of the work list, as many
+// CTAs as are resident at once (four an SM), so that the last wave is a full
+// one and the FP64 shuffle reduction (10 additions a thread for two
+// variables, beside about 14 FP64 instructions a cell) is paid once a group;
+// a small level takes one block a CTA to reach every SM (a 128^2 level in 16
+// CTAs of four blocks: 17 us, in 64: 6 us).
+constexpr int kNormPartialsMax = 608;
+inline int norm_group(int nblk) { return nblk <= kNormPartialsMax ? 1 : (nblk + kNormPartialsMax - 1) / kNormPartialsMax; }
+inline int norm_partials(int nblk) { return (nblk + norm_group(nblk) - 1) / norm_group(nblk); }
 int launch_norm_partial(const LaunchCtx& c, const Blk* blk, int nblk,
                         double* partial, int store_rf);
 // deterministic final sum; writes out[0] = norm, out[1] = raw sum,
 // and nonfinite[0] = 0 when the norm is finite, 1 otherwise (nothing when
-// nonfinite is null).  out must hold
+// nonfinite is null).  With `host` (pinned memory) the record a host reads
+// goes there too: host[0] and host[1] as out, the flag as an int at host + 8;
+// with `one` the norm also goes to *one.  out must hold
 // kNormOutLen doubles (out[8 ..] is scratch of the two-stage sum); the
 // partials hold nrvars values per block.
 int launch_norm_finish(cudaStream_t s, const double* partial, int nblk,
                        int nrvars, double count, int errortype, double* out,
-                       int* nonfinite);
+                       int* nonfinite, double* host = nullptr, double* one = nullptr);
 int launch_ghost_stage(const LaunchCtx& c, const GhostOp* ops, int n);
 
 // ---- after-step statistics and uniform-mesh output (io.cu, --fmad=false) ----

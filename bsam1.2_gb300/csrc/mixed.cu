@@ -342,15 +342,7 @@ int mx_norm(Hier& H, int level, int errortype) {
   int r = after_launch(H, mxp(H).norm(mxl(H), H.mx_norm_blk[level + kMaxDepth], nb, H.d_partial));
   if (r) return r;
   return after_launch(H, launch_norm_finish(H.s, H.d_partial, nb, H.nrvars, L.count, errortype, H.d_norm,
-                                            H.d_nonfinite));
-}
-
-int to_host(Hier& H) {
-  cudaError_t ce = cudaMemcpyAsync(H.h_norm, H.d_norm, 2 * sizeof(double), cudaMemcpyDeviceToHost, H.s);
-  if (ce != cudaSuccess) return cuda_fail(ce, "cudaMemcpyAsync(norm)");
-  ce = cudaMemcpyAsync(H.h_nonfinite, H.d_nonfinite, sizeof(int), cudaMemcpyDeviceToHost, H.s);
-  if (ce != cudaSuccess) return cuda_fail(ce, "cudaMemcpyAsync(nonfinite)");
-  return BSAMG_OK;
+                                            H.d_nonfinite, H.h_norm));
 }
 
 // FillDown of q in FP64 (restriction to the parents, with their ghosts)
@@ -388,7 +380,7 @@ int mx_iteration(Hier& H, int finest, int minlevel, int nsmooth, int errortype, 
     if ((r = after_launch(H, mxp(H).track(mxl(H), L.d_blk[kKindInterior], L.nblk[kKindInterior], H.d_partial))))
       return r;
     if ((r = after_launch(H, launch_norm_finish(H.s, H.d_partial, L.nblk[kKindInterior], H.nrvars, L.count,
-                                                 errortype, H.d_norm, H.d_nonfinite))))
+                                                 errortype, H.d_norm, H.d_nonfinite, H.h_norm))))
       return r;
   }
   for (int level = finest; level >= 0; level--) {
@@ -401,14 +393,10 @@ int mx_iteration(Hier& H, int finest, int minlevel, int nsmooth, int errortype, 
   // interpolation reads the parent values FillDown just restricted)
   for (int level = 1; level <= finest; level++)
     if ((r = enq_set_ghost(H, level, 0))) return r;
-  return to_host(H);
+  return BSAMG_OK;
 }
 
-int mx_verify(Hier& H, int finest, int errortype) {
-  int r = mx_norm(H, finest, errortype);
-  if (r) return r;
-  return to_host(H);
-}
+int mx_verify(Hier& H, int finest, int errortype) { return mx_norm(H, finest, errortype); }
 
 // ---------------------------------------------------------------------------
 // The whole solve of a hierarchy with refinement levels in one launch of one
@@ -1158,7 +1146,6 @@ int mixed_iterations(Hier& H, int finest, int minlevel, int nsmooth, int maxvcyc
   // residual of the finest level
   int r = mx_norm(H, finest, errortype);
   if (r) return r;
-  if ((r = to_host(H))) return r;
   if (int rw = stream_wait(H)) return rw;
   double r_sync = H.h_norm[0];  // FP64 residual the current g was taken from
   if (!H.uni && (r = mx_prepare_tail(H, finest, minlevel, nsmooth))) return r;

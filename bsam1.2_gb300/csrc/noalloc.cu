@@ -24,7 +24,7 @@
 // that resets a device must not call this entry point on it afterwards.
 //
 // Same arithmetic, block decomposition and final reduction as the
-// hierarchy's norm (the partial kernel below is k_norm_partial's for one CH
+// hierarchy's norm (the partial kernel below is k_uni_norm's for one CH
 // patch, built with --fmad=false like it, and the final sum is
 // launch_norm_finish itself), so the two agree bit for bit.
 #include <cuda_runtime.h>
@@ -34,13 +34,14 @@
 #include "../../include/bsamg.h"
 #include "hier.h"
 #include "internal.h"
+#include "kern_fp64.cuh"
 #include "launch.h"
 
 namespace {
 
 using namespace bsamg;
 
-constexpr int kMaxBlocks = BSAMG_NOALLOC_MAX_CELLS / (kBlock * kNormGroup);
+constexpr int kMaxBlocks = kNormPartialsMax;
 
 // [0, 2*kMaxBlocks): per-CTA partial sums of rf^2 (two variables);
 // [2*kMaxBlocks, 2*kMaxBlocks + kNormOutLen): the final reduction's output
@@ -68,68 +69,43 @@ int scratch_on_current_device(double** out) {
 }
 
 template <int DIM>
-__device__ __forceinline__ double ulap(const double* a, long long c, long long sy, long long sz) {
+__device__ __forceinline__ double lap(const double* a, int c, int sy, int sz) {
   if (DIM == 2) return a[c + 1] + a[c - 1] + a[c + sy] + a[c - sy] - 4.0 * a[c];
-  return a[c + 1] + a[c - 1] + a[c + sy] + a[c - sy] + a[c + sz] + a[c - sz] - 6.0 * a[c];
+  return fxp::lap6({a[c + 1], a[c - 1], a[c + sy], a[c - sy], a[c + sz], a[c - sz]}, a[c]);
 }
 
 // rf = f - Operator(q) (CH/problem.f90:393-422, :638-669) per interior cell,
-// sums of rf^2 over kNormGroup consecutive runs of kBlock cells per CTA, in
-// the order of the hierarchy's k_norm_partial on a one-patch level (whose
-// work-list blocks are the same runs of cells)
+// sums of rf^2 over `group` consecutive runs of kBlock cells per CTA, in the
+// order of the hierarchy's norm on a one-patch level (whose blocks are the
+// same runs of cells).  Bound by the FP64 unit: about 12 of its instructions
+// a cell, the two Laplacians on the integer pipe beside them (31 with all of
+// them on it: 119 us for 160 x 96 x 128, now 82).
 template <int DIM>
-__global__ void __launch_bounds__(kBlock) k_norm_single(const double* __restrict__ q, const double* __restrict__ f,
-                                                        int mx0, int mx1, int mx2, double c0, double c1,
+__global__ void __launch_bounds__(kBlock, 4) k_norm_single(const double* __restrict__ q, const double* __restrict__ f,
+                                                        int mx0, int mx1, int mx2, const __grid_constant__ UniDim d,
+                                                        int group, double c0, double c1,
                                                         double* __restrict__ partial) {
   __shared__ double red[2][kBlock / 32];
-  double s0 = 0.0, s1 = 0.0;
-  for (int sub = 0; sub < kNormGroup; sub++) {
-    long long t = ((long long)blockIdx.x * kNormGroup + sub) * kBlock + threadIdx.x;
-    int i = (int)(t % mx0) + 1, j, k;
-    long long r = t / mx0;
-    if (DIM == 2) {
-      j = (int)r + 1;
-      k = 1;
-      if (j > mx1) break;
-    } else {
-      j = (int)(r % mx1) + 1;
-      k = (int)(r / mx1) + 1;
-      if (k > mx2) break;
-    }
-    long long n0 = mx0 + 2, n1 = mx1 + 2;
-    long long sy = n0, sz = n0 * n1;
-    long long sq = DIM == 2 ? n0 * n1 : n0 * n1 * (mx2 + 2);
-    long long sf = (long long)mx0 * mx1 * (DIM == 2 ? 1 : mx2);
-    long long c = DIM == 2 ? (long long)j * n0 + i : ((long long)k * n1 + j) * n0 + i;
-    long long fc = DIM == 2 ? (long long)(j - 1) * mx0 + (i - 1) : ((long long)(k - 1) * mx1 + (j - 1)) * mx0 + (i - 1);
+  double s[2] = {0.0, 0.0};
+  const int cells = mx0 * mx1 * (DIM == 2 ? 1 : mx2);
+  const int n0 = mx0 + 2, n1 = mx1 + 2, sy = n0, sz = n0 * n1;
+  const int sq = DIM == 2 ? sz : sz * (mx2 + 2);
+  for (int sub = 0; sub < group; sub++) {
+    const int fc = (blockIdx.x * group + sub) * kBlock + (int)threadIdx.x;
+    if (fc >= cells) break;
+    int i, j, k;
+    uni::inner_unit<DIM>(d.n0, d.n1, fc, i, j, k);
+    const int c = DIM == 2 ? j * n0 + i : (k * n1 + j) * n0 + i;
     const double* a0 = q;
     const double* a1 = q + sq;
-    double r0 = a0[c] - c0 * ulap<DIM>(a1, c, sy, sz);
-    double r1 = a1[c] - a0[c] * a0[c] * a0[c] + c1 * ulap<DIM>(a0, c, sy, sz);
+    double r0 = a0[c] - c0 * lap<DIM>(a1, c, sy, sz);
+    double r1 = a1[c] - a0[c] * a0[c] * a0[c] + c1 * lap<DIM>(a0, c, sy, sz);
     double e0 = f[fc] - r0;
-    double e1 = f[sf + fc] - r1;
-    s0 = s0 + e0 * e0;
-    s1 = s1 + e1 * e1;
+    double e1 = f[cells + fc] - r1;
+    s[0] = fma(e0, e0, s[0]);
+    s[1] = fma(e1, e1, s[1]);
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    s0 = s0 + __shfl_down_sync(0xffffffffu, s0, o);
-    s1 = s1 + __shfl_down_sync(0xffffffffu, s1, o);
-  }
-  int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  if (l == 0) {
-    red[0][w] = s0;
-    red[1][w] = s1;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t0 = 0.0, t1 = 0.0;
-    for (int n = 0; n < kBlock / 32; n++) {
-      t0 = t0 + red[0][n];
-      t1 = t1 + red[1][n];
-    }
-    partial[2 * blockIdx.x] = t0;
-    partial[2 * blockIdx.x + 1] = t1;
-  }
+  block_sum<2>(s, red, partial);
 }
 
 }  // namespace
@@ -156,19 +132,19 @@ extern "C" int bsamg_ch_residual_norm_noalloc(const double* q, const double* f, 
   double h2 = h * h;
   double eps2 = eps * eps;
   double c0 = dt / h2, c1 = eps2 / h2;
-  int nblk = norm_partials((int)((cells + kBlock - 1) / kBlock));
+  const int runs = (int)((cells + kBlock - 1) / kBlock), nblk = norm_partials(runs), group = norm_group(runs);
+  const int n[3] = {mx[0], mx[1], ndims == 2 ? 1 : mx[2]};
+  const UniDim d = uni_dim(n);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (ndims == 2)
-    k_norm_single<2><<<nblk, kBlock, 0, s>>>(q, f, mx[0], mx[1], 1, c0, c1, scratch);
+    k_norm_single<2><<<nblk, kBlock, 0, s>>>(q, f, n[0], n[1], 1, d, group, c0, c1, scratch);
   else
-    k_norm_single<3><<<nblk, kBlock, 0, s>>>(q, f, mx[0], mx[1], mx[2], c0, c1, scratch);
+    k_norm_single<3><<<nblk, kBlock, 0, s>>>(q, f, n[0], n[1], n[2], d, group, c0, c1, scratch);
   // the hierarchy's own final reduction (two stages above 2048 blocks);
   // no non-finite flag: a NaN or Inf input shows as a NaN or Inf norm
   double* out = scratch + 2 * kMaxBlocks;
-  launch_norm_finish(s, scratch, nblk, 2, 2.0 * (double)cells, errortype, out, nullptr);
+  launch_norm_finish(s, scratch, nblk, 2, 2.0 * (double)cells, errortype, out, nullptr, nullptr, norm_out);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "bsamg_ch_residual_norm_noalloc launch");
-  e = cudaMemcpyAsync(norm_out, out, sizeof(double), cudaMemcpyDeviceToDevice, s);
-  if (e != cudaSuccess) return cuda_fail(e, "bsamg_ch_residual_norm_noalloc copy");
   return BSAMG_OK;
 }

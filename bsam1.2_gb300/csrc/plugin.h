@@ -128,6 +128,8 @@ struct PluginFp64 {
                    int smem_bytes);
   int (*tail_smem_attributes)();
   PluginUni uni;
+  // norm_partial of a uniform level; update: f = ftmp + SourceUpdate first
+  int (*uni_norm)(const LaunchCtx&, int patch, const PatchDev& p, double* partial, int store_rf, int update);
 };
 
 // Launchers of the mixed path's plugin-dependent kernels (the correction

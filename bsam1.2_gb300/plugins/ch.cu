@@ -51,15 +51,19 @@ struct CH {
     const double* f1 = f0 + x.sf;
     const long long c = x.c, fc = x.fc, sy = x.sy, sz = x.sz;
     double phi = q0[c];
-    double a21 = -3.0 * sqr(phi) - cf[2];
-    double b1, b2;
+    double b1, b2, a21;
     if (DIM == 2) {
+      a21 = -3.0 * sqr(phi) - cf[2];
       b1 = f0[fc] + cf[0] * (q1[c - 1] + q1[c + 1] + q1[c - sy] + q1[c + sy]);
       b2 = f1[fc] - cf[1] * (q0[c + 1] + q0[c - 1] + q0[c + sy] + q0[c - sy]) - 2.0 * cube(phi);
     } else {
-      b1 = f0[fc] + cf[0] * (q1[c - 1] + q1[c + 1] + q1[c - sy] + q1[c + sy] + q1[c - sz] + q1[c + sz]);
-      b2 = f1[fc] - cf[1] * (q0[c + 1] + q0[c - 1] + q0[c + sy] + q0[c - sy] + q0[c + sz] + q0[c - sz]) -
-           2.0 * cube(phi);
+      // the FP64 unit bounds the 3D sweep: the neighbour sums and the products
+      // with 3 and 2 run on the integer pipe, to the same bits
+      const double p2 = sqr(phi);
+      a21 = -fxp::triple(p2) - cf[2];
+      b1 = f0[fc] + cf[0] * fxp::sum<6>({q1[c - 1], q1[c + 1], q1[c - sy], q1[c + sy], q1[c - sz], q1[c + sz]});
+      b2 = f1[fc] - cf[1] * fxp::sum<6>({q0[c + 1], q0[c - 1], q0[c + sy], q0[c - sy], q0[c + sz], q0[c - sz]}) -
+           fxp::scaled<1>(p2 * phi);
     }
     double det = 1.0 - cf[3] * a21;  // >= 1: a21 <= -tmp3 < 0
     // the reference's two divisions by det, :365-366 (:609-610), each
