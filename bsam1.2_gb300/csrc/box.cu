@@ -37,6 +37,8 @@
 #include <algorithm>
 #include <cstddef>
 #include <functional>
+#include <memory>
+#include <vector>
 
 #include "box.h"
 #include "kern_uni.cuh"
@@ -1279,6 +1281,37 @@ __device__ __forceinline__ void cyc_coarsest(const Cyc& A, int x, const Slab& S,
   }
 }
 
+// the levels of A once down and up, from the top level's e, g and pb in
+// shared memory; the top level's e is final, and every CTA of it past its
+// last barrier, at the end
+template <int DIM>
+__device__ __forceinline__ void cyc_vcycle(const Cyc& A, int rank, int t, int nt) {
+  auto smooth = [&](int x, int begin, bool restrict_, bool emit) {
+    const Slab S = slab<DIM, false>(A, x, rank);
+    const Slab C = x + 1 < A.nl ? slab<DIM, true>(A, x + 1, rank) : S;
+    auto sync = [&] {
+      if (S.shared) uni::cluster_sync();
+      else __syncthreads();
+    };
+    const int units = (S.n0 >> 1) * (DIM == 3 ? S.n1 : 1) * A.L[x].maxr;
+    if (x == A.nl - 1) cyc_coarsest<DIM>(A, x, S, begin == kDown, emit, t, sync);
+    else if (units <= nt) cyc_smooth<DIM, 1>(A, x, S, C, begin, restrict_, emit, t, nt, sync);
+    else cyc_smooth<DIM, kCycPairs>(A, x, S, C, begin, restrict_, emit, t, nt, sync);
+    // what the next level reads has been written
+    if (S.shared) uni::cluster_sync();
+    else __syncthreads();
+  };
+  for (int x = 0; x < A.nl; x++) {
+    if (!A.L[x].mul && rank) break;
+    smooth(x, x ? kDown : kTop, x + 1 < A.nl, x && x + 1 == A.nl);
+  }
+  for (int x = A.nl - 2; x >= 0; x--) {
+    if (!A.L[x].mul && rank) continue;
+    if (A.L[x].mul && !A.L[x + 1].mul) uni::cluster_sync();  // CTA 0 has finished the levels it holds
+    smooth(x, kUp, false, x > 0);
+  }
+}
+
 template <int DIM>
 __global__ void __launch_bounds__(kCycThreads, 1) k_bx_cycle(float* __restrict__ fp, const __grid_constant__ Cyc A,
                                                              BoxLev T, int fresh) {
@@ -1318,30 +1351,7 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_bx_cycle(float* __restrict__
       }
   }
   all();
-  auto smooth = [&](int x, int begin, bool restrict_, bool emit) {
-    const Slab S = slab<DIM, false>(A, x, rank);
-    const Slab C = x + 1 < A.nl ? slab<DIM, true>(A, x + 1, rank) : S;
-    auto sync = [&] {
-      if (S.shared) uni::cluster_sync();
-      else __syncthreads();
-    };
-    const int units = (S.n0 >> 1) * (DIM == 3 ? S.n1 : 1) * A.L[x].maxr;
-    if (x == A.nl - 1) cyc_coarsest<DIM>(A, x, S, begin == kDown, emit, t, sync);
-    else if (units <= nt) cyc_smooth<DIM, 1>(A, x, S, C, begin, restrict_, emit, t, nt, sync);
-    else cyc_smooth<DIM, kCycPairs>(A, x, S, C, begin, restrict_, emit, t, nt, sync);
-    // what the next level reads has been written
-    if (S.shared) uni::cluster_sync();
-    else __syncthreads();
-  };
-  for (int x = 0; x < A.nl; x++) {
-    if (!A.L[x].mul && rank) break;
-    smooth(x, x ? kDown : kTop, x + 1 < A.nl, x && x + 1 == A.nl);
-  }
-  for (int x = A.nl - 2; x >= 0; x--) {
-    if (!A.L[x].mul && rank) continue;
-    if (A.L[x].mul && !A.L[x + 1].mul) all();  // CTA 0 has finished the levels it holds
-    smooth(x, kUp, false, x > 0);
-  }
+  cyc_vcycle<DIM>(A, rank, t, nt);
   const Slab S = slab<DIM, false>(A, 0, rank);
   const CycLev& L = A.L[0];
   const V2 E = var2(fp, T.oe, T.half);
@@ -1412,9 +1422,34 @@ __global__ void __launch_bounds__(256, R == 1 ? 6 : 5) k_bx_track_update(float* 
   cta_sum2(s0, s1, partial);
 }
 
-// The true residual r = f - N(qbar) of the finest level in double-float
-// (ErrorAFAS, afasroutines.f90:113-233, with f = (phi_old, -phi_old)); g is
-// set to r and the per-CTA sums of r^2 go to partial.
+// The true residual r = f - N(qbar) at a cell of the finest level in
+// double-float (ErrorAFAS, afasroutines.f90:113-233, with f = (phi_old,
+// -phi_old))
+template <int DIM>
+__device__ __forceinline__ void resid_at(const float* fp, const BoxLev& L, long long oqlo, long long ofhi,
+                                         long long oflo, const Loc<DIM>& l, float& a0, float& a1) {
+  const DF c0 = {L.c0h, L.c0l}, c1 = {L.c1h, L.c1l};
+  const float* QH[2] = {fp + L.opb, fp + L.opb + 2 * L.half};
+  const float* QL[2] = {fp + oqlo, fp + oqlo + 2 * L.half};
+  const unsigned nbi[6] = {l.xm, l.xp, l.ym, l.yp, l.zm, l.zp};
+  DF v[2], nb[2][6];
+  for (int q = 0; q < 2; q++) {
+    v[q] = {QH[q][l.own], QL[q][l.own]};
+    for (int m = 0; m < 2 * DIM; m++) nb[q][m] = {QH[q][nbi[m]], QL[q][nbi[m]]};
+  }
+  DF f1 = {fp[ofhi + l.own], fp[oflo + l.own]};
+  DF lphi = df_lap<DIM>(nb[0], v[0]);
+  DF lmu = df_lap<DIM>(nb[1], v[1]);
+  // r1 = f1 - (phi - c0 lap(mu)); r2 = -f1 - (mu - phi^3 + c1 lap(phi))
+  DF r1 = df_add(df_add(f1, df_neg(v[0])), df_mul(c0, lmu));
+  DF p3 = df_mul(df_mul(v[0], v[0]), v[0]);
+  DF r2 = df_add(df_add(df_neg(df_add(f1, v[1])), p3), df_neg(df_mul(c1, lphi)));
+  a0 = r1.h + r1.l;
+  a1 = r2.h + r2.l;
+}
+
+// the residual over the level: g is set to it, the per-CTA sums of its
+// squares go to partial
 template <int DIM>
 __global__ void __launch_bounds__(256) k_bx_resid(float* __restrict__ fp, BoxLev L, long long oqlo, long long ofhi,
                                                   long long oflo, double* __restrict__ partial) {
@@ -1423,25 +1458,10 @@ __global__ void __launch_bounds__(256) k_bx_resid(float* __restrict__ fp, BoxLev
   int z = blockIdx.z;
   float s0 = 0.f, s1 = 0.f;
   if (x < L.n[0] && y < L.n[1]) {
-    const DF c0 = {L.c0h, L.c0l}, c1 = {L.c1h, L.c1l};
-    V2 QH = var2(fp, L.opb, L.half), QL = var2(fp, oqlo, L.half), G = var2(fp, L.og, L.half);
+    V2 G = var2(fp, L.og, L.half);
     Loc<DIM> l(L, x, y, z);
-    const unsigned nbi[6] = {l.xm, l.xp, l.ym, l.yp, l.zm, l.zp};
-    DF v[2], nb[2][6];
-    for (int q = 0; q < 2; q++) {
-      const float* hi = q ? QH.v1 : QH.v0;
-      const float* lo = q ? QL.v1 : QL.v0;
-      v[q] = {hi[l.own], lo[l.own]};
-      for (int m = 0; m < 2 * DIM; m++) nb[q][m] = {hi[nbi[m]], lo[nbi[m]]};
-    }
-    DF f1 = {fp[ofhi + l.own], fp[oflo + l.own]};
-    DF lphi = df_lap<DIM>(nb[0], v[0]);
-    DF lmu = df_lap<DIM>(nb[1], v[1]);
-    // r1 = f1 - (phi - c0 lap(mu)); r2 = -f1 - (mu - phi^3 + c1 lap(phi))
-    DF r1 = df_add(df_add(f1, df_neg(v[0])), df_mul(c0, lmu));
-    DF p3 = df_mul(df_mul(v[0], v[0]), v[0]);
-    DF r2 = df_add(df_add(df_neg(df_add(f1, v[1])), p3), df_neg(df_mul(c1, lphi)));
-    float a0 = r1.h + r1.l, a1 = r2.h + r2.l;
+    float a0, a1;
+    resid_at<DIM>(fp, L, oqlo, ofhi, oflo, l, a0, a1);
     G.v0[l.own] = a0;
     G.v1[l.own] = a1;
     s0 = a0 * a0;
@@ -1553,6 +1573,267 @@ __global__ void __launch_bounds__(256) k_bx_merge(double* __restrict__ pool, lon
   }
   for (int b = 0; b < 2; b++)
     for (int v = 0; v < 2; v++) pool[oq + v * sq + g + b] = f2d(hi[b][v]) + f2d(lo[b][v]);
+}
+
+// ---------------------------------------------------------------------------
+// The whole solve of a box whose finest level fits the cluster (k_bx_cycle)
+// as one launch: the split of q, the starting residual, the V-cycles, the
+// tracked residual and qbar += e after each, the confirming residuals, the
+// exit test of box_iterations and the write-back of q with its periodic
+// images.  e, g and pb stay in shared memory from cycle to cycle; qhi, qlo
+// and f stay where the other kernels keep them (a cluster barrier makes one
+// CTA's writes visible to the others).  Per cell it computes what the
+// separate kernels compute; the norms add the same squares in another order.
+//
+// A step of such a box was some 14 launches and a graph with a conditional
+// loop of six launches a V-cycle; now it is this one, the fill of the coarse
+// levels and one wait.  A step of five V-cycles at 32^2: 285 -> 206 us; of
+// seven at 128^2: 510 -> 460 us.  What bounds it is the chain of sweeps.
+constexpr int kSolveMaxCycles = 64;
+struct BoxSolve {
+  long long oqlo, ofhi, oflo;      // float offsets
+  long long oq, oqold, sq;         // FP64 pool: q, qold (cell (0,0,0) of variable 1), variable stride
+  int qn0, qn1;
+  double tol, count;               // exit tolerance, ErrorAFAS denominator
+  int maxv, errortype, warm;
+};
+// what the host reads (pinned memory)
+struct BoxSolveOut {
+  int it, conv, status, nconfirm;
+  double res[kSolveMaxCycles];
+};
+
+template <int DIM>
+__global__ void __launch_bounds__(kCycThreads, 1) k_bx_solve(float* __restrict__ fp, double* __restrict__ pool,
+                                                             const __grid_constant__ Cyc A, BoxLev T, BoxSolve B,
+                                                             BoxSolveOut* __restrict__ out) {
+  const int rank = A.ctas > 1 ? uni::my_rank() : 0;
+  const int t = threadIdx.x, nt = blockDim.x;
+  __shared__ float wsum[2][kCycThreads / 32];
+  __shared__ double part[2][32];  // two norms' worth: a CTA may start the next while another still adds up this one
+  __shared__ double norm_now;
+  int turn = 0;
+  auto all = [&] {
+    if (A.ctas > 1) uni::cluster_sync();
+    else __syncthreads();
+  };
+  const Slab S = slab<DIM, false>(A, 0, rank);
+  const CycLev& L = A.L[0];
+  const int n1 = DIM == 3 ? S.n1 : 1;
+  // a top level that CTA 0 holds alone leaves the others without cells
+  const int units = S.shared || rank == 0 ? (S.n0 >> 1) * n1 * S.nr : 0;
+  const V2 G = var2(fp, T.og, T.half), QH = var2(fp, T.opb, T.half), QL = var2(fp, B.oqlo, T.half);
+  // pair u's global y, z and the element of its cell b in a colour-split array
+  struct At {
+    int x, y, z;
+    unsigned i[2];
+  };
+  auto at = [&](int u, const Pair& p) {
+    At a;
+    int r, h;
+    uni::fdivmod(u, L.hx, r, h);
+    a.x = 2 * h;
+    if (DIM == 3) {
+      int k;
+      uni::fdivmod(r, L.d1, k, a.y);
+      a.z = k + S.r0;
+    } else {
+      a.y = r + S.r0;
+      a.z = 0;
+    }
+    const unsigned q = ((unsigned)S.r0 * n1 + r) * T.hh + h;
+    for (int b = 0; b < 2; b++) a.i[b] = q + ((b ^ p.b0) ? (unsigned)T.half : 0u);
+    return a;
+  };
+  auto fp64_at = [&](const At& a) {  // offset of cell (x, y, z) in a ghosted plane of q
+    return (long long)(a.x + 1) + (long long)(a.y + 1) * B.qn0 +
+           (DIM == 3 ? (long long)(a.z + 1) * B.qn0 * B.qn1 : 0);
+  };
+  // ErrorAFAS of the squares each thread summed, in every CTA
+  auto norm = [&](float s0, float s1) {
+    for (int o = 16; o > 0; o >>= 1) {
+      s0 += __shfl_down_sync(0xffffffffu, s0, o);
+      s1 += __shfl_down_sync(0xffffffffu, s1, o);
+    }
+    if ((t & 31) == 0) wsum[0][t >> 5] = s0, wsum[1][t >> 5] = s1;
+    double* const sums = part[turn];
+    turn ^= 1;
+    __syncthreads();
+    if (t < 32) {
+      float a = t < nt / 32 ? wsum[0][t] : 0.f, b = t < nt / 32 ? wsum[1][t] : 0.f;
+      for (int o = 8; o > 0; o >>= 1) {
+        a += __shfl_down_sync(0xffffffffu, a, o);
+        b += __shfl_down_sync(0xffffffffu, b, o);
+      }
+      a = __shfl_sync(0xffffffffu, a, 0);
+      b = __shfl_sync(0xffffffffu, b, 0);
+      if (t < A.ctas) {  // to every CTA
+        double* p = A.ctas > 1 ? uni::on_rank(sums, t) : sums;
+        p[rank] = f2d(a);
+        p[16 + rank] = f2d(b);
+      }
+    }
+    all();
+    if (t < 32) {
+      double a = t < A.ctas ? sums[t] : 0.0, b = t < A.ctas ? sums[16 + t] : 0.0;
+      for (int o = 8; o > 0; o >>= 1)
+        if (o < A.ctas) {
+          a += __shfl_down_sync(0xffffffffu, a, o);
+          b += __shfl_down_sync(0xffffffffu, b, o);
+        }
+      if (t == 0) {
+        if (B.errortype == 1) {
+          norm_now = sqrt((a + b) / B.count);
+        } else {
+          const double r0 = sqrt(a / (0.5 * B.count)), r1 = sqrt(b / (0.5 * B.count));
+          norm_now = r1 > r0 ? r1 : r0;
+        }
+      }
+    }
+    __syncthreads();
+    return norm_now;
+  };
+  // the true residual to g; its norm
+  auto confirm = [&] {
+    float s0 = 0.f, s1 = 0.f;
+    for (int u = t; u < units; u += nt) {
+      const Pair p = pair_of<DIM>(S, L, u);
+      const At a = at(u, p);
+#pragma unroll 1
+      for (int b = 0; b < 2; b++) {
+        const Loc<DIM> l(T, a.x + b, a.y, a.z);
+        float r0, r1;
+        resid_at<DIM>(fp, T, B.oqlo, B.ofhi, B.oflo, l, r0, r1);
+        S.g[p.in + b] = r0;
+        S.g[S.ivar + p.in + b] = r1;
+        s0 += r0 * r0;
+        s1 += r1 * r1;
+      }
+    }
+    return norm(s0, s1);
+  };
+  // q and qold split into float pairs (k_bx_split, k_bx_split_warm)
+  float w0 = 0.f, w1 = 0.f;
+  for (int u = t; u < units; u += nt) {
+    const Pair p = pair_of<DIM>(S, L, u);
+    const At a = at(u, p);
+    const long long g = fp64_at(a);
+#pragma unroll
+    for (int b = 0; b < 2; b++) {
+      const unsigned i = a.i[b];
+      const DF s0 = split64(pool[B.oq + g + b]), s1 = split64(pool[B.oq + B.sq + g + b]);
+      const DF f = split64(pool[B.oqold + g + b]);
+      if (B.warm) {
+        const DF d = df_add(f, df_neg(DF{fp[B.ofhi + i], fp[B.oflo + i]}));
+        const DF r1 = df_add(DF{G.v0[i], 0.f}, d), r2 = df_add(DF{G.v1[i], 0.f}, df_neg(d));
+        const float a0 = r1.h + r1.l, a1 = r2.h + r2.l;
+        S.g[p.in + b] = a0;
+        S.g[S.ivar + p.in + b] = a1;
+        w0 += a0 * a0;
+        w1 += a1 * a1;
+      }
+      QH.v0[i] = s0.h;
+      QL.v0[i] = s0.l;
+      QH.v1[i] = s1.h;
+      QL.v1[i] = s1.l;
+      fp[B.ofhi + i] = f.h;
+      fp[B.oflo + i] = f.l;
+      S.pb[p.in + b] = s0.h;
+    }
+  }
+  auto clear = [&] {  // e = 0, halo rows too
+    if (units)
+      for (int q = t; q < 2 * S.var; q += nt) S.e[q] = 0.f;
+  };
+  clear();
+  all();
+  double r_sync = B.warm ? norm(w0, w1) : confirm();
+  int status = !isfinite(r_sync), conv = 0, it = 0, nconfirm = 0;
+  while (!status && it < B.maxv) {
+    it++;
+    cyc_vcycle<DIM>(A, rank, t, nt);
+    // g -= M(e), then qbar += e (k_bx_track_update)
+    float s0 = 0.f, s1 = 0.f;
+    for (int u = t; u < units; u += nt) {
+      const Pair p = pair_of<DIM>(S, L, u);
+      const At a = at(u, p);
+#pragma unroll
+      for (int b = 0; b < 2; b++) {
+        const float *E0 = S.e + p.at + b, *E1 = E0 + S.var;
+        const float x = E0[0], y = E1[0], pb = S.pb[p.in + b];
+        auto diff = [&](const float* c, float v) {  // ndiff
+          const float q = (c[b ? -1 : p.xl] - v) + (c[b ? p.xr : 1] - v);
+          if (DIM == 2) return q + ((c[p.rm] - v) + (c[p.rp] - v));
+          float z = q + ((c[p.ym] - v) + (c[p.yp] - v));
+          z += (c[p.rm] - v) + (c[p.rp] - v);
+          return z;
+        };
+        const float m0 = x - L.c0 * diff(E1, y);
+        const float m1 = y - x * (3.0f * pb * (pb + x) + x * x) + L.c1 * diff(E0, x);
+        const float a0 = S.g[p.in + b] - m0, a1 = S.g[S.ivar + p.in + b] - m1;
+        const unsigned i = a.i[b];
+        DF t0 = two_sum(pb, x);
+        t0 = fast_two_sum(t0.h, t0.l + QL.v0[i]);
+        DF t1 = two_sum(QH.v1[i], y);
+        t1 = fast_two_sum(t1.h, t1.l + QL.v1[i]);
+        S.g[p.in + b] = a0;
+        S.g[S.ivar + p.in + b] = a1;
+        S.pb[p.in + b] = t0.h;
+        QH.v0[i] = t0.h;
+        QL.v0[i] = t0.l;
+        QH.v1[i] = t1.h;
+        QL.v1[i] = t1.l;
+        s0 += a0 * a0;
+        s1 += a1 * a1;
+      }
+    }
+    double res = norm(s0, s1);
+    clear();  // after norm's barrier: every read of e is done
+    if (!isfinite(res)) {
+      status = 1;
+    } else if (res < B.tol || res < 1e-5 * r_sync || it >= B.maxv) {
+      res = confirm();
+      nconfirm++;
+      if (!isfinite(res)) status = 1;
+      r_sync = res;
+      conv = !status && res < B.tol;
+    }
+    if (rank == 0 && t == 0 && !status) out->res[it - 1] = res;
+    if (conv) break;
+    all();  // e is zero in every CTA
+  }
+  // q, its periodic images, and the residual the next step starts from
+  for (int u = t; u < units; u += nt) {
+    const Pair p = pair_of<DIM>(S, L, u);
+    const At a = at(u, p);
+    const long long g = fp64_at(a);
+#pragma unroll
+    for (int b = 0; b < 2; b++) {
+      const unsigned i = a.i[b];
+      G.v0[i] = S.g[p.in + b];
+      G.v1[i] = S.g[S.ivar + p.in + b];
+      const double v[2] = {f2d(QH.v0[i]) + f2d(QL.v0[i]), f2d(QH.v1[i]) + f2d(QL.v1[i])};
+      const int x = a.x + b;
+      const long long dx = x == 0 ? T.n[0] : (x == T.n[0] - 1 ? -T.n[0] : 0);
+      const long long dy = (a.y == 0 ? T.n[1] : (a.y == T.n[1] - 1 ? -T.n[1] : 0)) * (long long)B.qn0;
+      const long long dz =
+          DIM == 3 ? (a.z == 0 ? T.n[2] : (a.z == T.n[2] - 1 ? -T.n[2] : 0)) * (long long)B.qn0 * B.qn1 : 0;
+#pragma unroll
+      for (int m = 0; m < (1 << DIM); m++) {
+        if (((m & 1) && !dx) || ((m & 2) && !dy) || ((m & 4) && !dz)) continue;
+        const long long o = g + b + (m & 1 ? dx : 0) + (m & 2 ? dy : 0) + (m & 4 ? dz : 0);
+        pool[B.oq + o] = v[0];
+        pool[B.oq + B.sq + o] = v[1];
+      }
+    }
+  }
+  if (rank == 0 && t == 0) {
+    out->it = it;
+    out->conv = conv;
+    out->status = status;
+    out->nconfirm = nconfirm;
+  }
+  all();  // a CTA's shared memory stays while another may still address it
 }
 
 // ---------------------------------------------------------------------------
@@ -1726,9 +2007,27 @@ int cycle_fit(int ndims, int ctas, int smem) {
     if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess) return 0;
     return n;
   };
-  const int n = ndims == 2 ? fit(k_bx_cycle<2>) : fit(k_bx_cycle<3>);
+  const int n = ndims == 2 ? std::min(fit(k_bx_cycle<2>), fit(k_bx_solve<2>))
+                           : std::min(fit(k_bx_cycle<3>), fit(k_bx_solve<3>));
   cudaGetLastError();  // a shape that does not fit is an answer, not an error
   return n;
+}
+
+template <typename K, typename... Args>
+cudaError_t launch_cluster(K k, int ctas, int threads, int smem, cudaStream_t s, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = ctas;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k, args...);
 }
 
 // The cluster's plan for the levels top .. minlevel with the first `share`
@@ -1794,23 +2093,29 @@ bool cycle_layout(Hier& H, int top, int minlevel, int nsmooth, int share, Cyc& A
 // about 70 instructions a pair.
 bool cycle_plan(Hier& H, int level, int minlevel, int nsmooth, Cyc& best, int* smem, int* at) {
   for (int top = level; top >= minlevel; top--) {
-    double best_us = 0.0;
-    for (int share = 0; share <= top - minlevel + 1; share++) {
+    struct Form {
+      double us;
+      int smem;
       Cyc A;
-      int sm = 0;
-      if (!cycle_layout(H, top, minlevel, nsmooth, share, A, &sm) || cycle_fit(H.ndims, A.ctas, sm) < 1) continue;
-      double us = 0.0;
-      for (int x = 0; x < A.nl; x++) {
-        const double pairs = (double)B(H, top - x).half / (x < share ? A.ctas : 1);
-        us += (x < share ? 0.75 : 0.3) + pairs * 70 / 32 / 4 / 2000.0 * 1.5;
+    };
+    std::vector<Form> forms;
+    for (int share = 0; share <= top - minlevel + 1; share++) {
+      Form f{0.0, 0, {}};
+      if (!cycle_layout(H, top, minlevel, nsmooth, share, f.A, &f.smem)) continue;
+      for (int x = 0; x < f.A.nl; x++) {
+        const double pairs = (double)B(H, top - x).half / (x < share ? f.A.ctas : 1);
+        f.us += (x < share ? 0.75 : 0.3) + pairs * 70 / 32 / 4 / 2000.0 * 1.5;
       }
-      if (best_us > 0.0 && us >= best_us) continue;
-      best_us = us;
-      best = A;
-      *smem = sm;
-      *at = top;
+      forms.push_back(f);
     }
-    if (best_us > 0.0) return true;
+    std::stable_sort(forms.begin(), forms.end(), [](const Form& a, const Form& b) { return a.us < b.us; });
+    for (const Form& f : forms)  // the cheapest that fits: asking the runtime costs tens of microseconds
+      if (cycle_fit(H.ndims, f.A.ctas, f.smem) >= 1) {
+        best = f.A;
+        *smem = f.smem;
+        *at = top;
+        return true;
+      }
   }
   return false;
 }
@@ -1818,21 +2123,9 @@ bool cycle_plan(Hier& H, int level, int minlevel, int nsmooth, Cyc& best, int* s
 // AFASVcycle (afasroutines.f90:495-529) on the correction
 int bx_vcycle_from(Hier& H, int level, int minlevel, int nsmooth, bool fresh, const Cyc& cyc, int cyc_smem, int cyc_at) {
   if (level <= cyc_at) {  // the rest of the V-cycle in one cluster launch
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(cyc.ctas);
-    cfg.blockDim = dim3(kCycThreads);
-    cfg.dynamicSmemBytes = cyc_smem;
-    cfg.stream = H.s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = cyc.ctas;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
     const BoxLev& T = B(H, level);
-    cudaError_t e = H.ndims == 2 ? cudaLaunchKernelEx(&cfg, k_bx_cycle<2>, H.fpool, cyc, T, fresh ? 1 : 0)
-                                 : cudaLaunchKernelEx(&cfg, k_bx_cycle<3>, H.fpool, cyc, T, fresh ? 1 : 0);
+    auto k = H.ndims == 2 ? k_bx_cycle<2> : k_bx_cycle<3>;
+    cudaError_t e = launch_cluster(k, cyc.ctas, kCycThreads, cyc_smem, H.s, H.fpool, cyc, T, fresh ? 1 : 0);
     if (e != cudaSuccess) return cuda_fail(e, "coarse V-cycle launch");
     return after_launch(H, 1);
   }
@@ -1863,6 +2156,24 @@ int bx_vcycle_from(Hier& H, int level, int minlevel, int nsmooth, bool fresh, co
     if ((r = bx_level_relax(H, level, nsmooth, false))) return r;
   }
   return BSAMG_OK;
+}
+
+// the plan of the whole V-cycle from the finest level, where that fits: made
+// once per (finest, minlevel, nsmooth) and coefficients
+bool solve_plan(Hier& H, int finest, int minlevel, int nsmooth, Cyc& cyc, int* smem) {
+  auto key = std::make_tuple(finest, minlevel, nsmooth);
+  if (!H.box_plan || H.box_plan_key != key) {
+    auto pl = std::make_shared<std::pair<Cyc, int>>();
+    int at = finest - 1;
+    if (!cycle_plan(H, finest, minlevel, nsmooth, pl->first, &pl->second, &at) || at != finest) pl->second = -1;
+    H.box_plan = pl;
+    H.box_plan_key = key;
+  }
+  const auto& pl = *std::static_pointer_cast<std::pair<Cyc, int>>(H.box_plan);
+  if (pl.second < 0) return false;
+  cyc = pl.first;
+  *smem = pl.second;
+  return true;
 }
 
 int bx_vcycle(Hier& H, int level, int minlevel, int nsmooth, bool fresh) {
@@ -1914,7 +2225,9 @@ struct BoxCtl {
   double res[kLoopMaxCycles];
 };
 constexpr int kCtlSlotOffset = 16;  // doubles into the hierarchy's pinned slot
-static_assert(sizeof(BoxCtl) <= (128 - kCtlSlotOffset) * sizeof(double), "pinned slot too small");
+static_assert(sizeof(BoxCtl) <= (128 - kCtlSlotOffset) * sizeof(double) &&
+                  sizeof(BoxSolveOut) <= (128 - kCtlSlotOffset) * sizeof(double),
+              "pinned slot too small");
 
 // after a cycle: the tracked norm decides whether to confirm on the true
 // residual (the host loop's test: below the tolerance, 1e5 below the last
@@ -2065,6 +2378,7 @@ bool box_eligible(const Hier& H, bool periodic_single) {
 // where pb is qhi(phi)), ec (below the finest); on the finest level qhi,
 // qlo, fhi, flo
 void box_coefficients(Hier& H) {
+  H.box_plan.reset();  // it holds them
   for (int l = H.maxlevel; l >= H.minlevel; l--) {
     const HostPatch& P = H.patches[H.L(l).patches[0]];
     BoxLev& L = H.blev[l + kMaxDepth];
@@ -2137,6 +2451,28 @@ int box_iterations(Hier& H, int finest, int minlevel, int nsmooth, int maxvcycle
   Launch sh = shape(L.hh, L.n[1], L.n[2]);
   bool warm = H.box_g_valid;  // g is the residual at this q: update it for the new f
   H.box_g_valid = false;
+  if (maxvcycles >= 1 && maxvcycles <= kSolveMaxCycles) {  // one launch where the finest level fits the cluster
+    Cyc cyc;
+    int smem = 0;
+    if (solve_plan(H, finest, minlevel, nsmooth, cyc, &smem)) {
+      const BoxSolve bs{H.b_oqlo, H.b_ofhi, H.b_oflo, P.oq, P.oqold, P.sq, P.qn[0], P.qn[1], tol,
+                        H.L(finest).count, maxvcycles, errortype, warm ? 1 : 0};
+      BoxSolveOut* out = reinterpret_cast<BoxSolveOut*>(H.h_norm + kCtlSlotOffset);
+      auto k = H.ndims == 2 ? k_bx_solve<2> : k_bx_solve<3>;
+      cudaError_t ce = launch_cluster(k, cyc.ctas, kCycThreads, smem, H.s, H.fpool, H.pool, cyc, L, bs, out);
+      if (ce != cudaSuccess) return cuda_fail(ce, "box solve launch");
+      int r = after_launch(H, 1);
+      if (r || (r = enq_fill_down(H, 2, finest, minlevel))) return r;
+      if ((r = stream_wait(H))) return r;
+      if (out->status) return BSAMG_ERR_NONFINITE;
+      if (residuals)
+        for (int n = 0; n < out->it; n++) residuals[n] = out->res[n];
+      const bool conv = out->conv != 0;
+      if (ncycles) *ncycles = conv ? out->it : maxvcycles;
+      H.box_g_valid = true;
+      return !conv && strict ? BSAMG_ERR_NOT_CONVERGED : BSAMG_OK;
+    }
+  }
   // the whole solve as one graph launch when the loop fits its control block
   bool loop = maxvcycles >= 1 && maxvcycles <= kLoopMaxCycles && !H.box_loop_off;
   if (loop) {

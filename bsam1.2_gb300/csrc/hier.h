@@ -5,6 +5,7 @@
 #include <atomic>
 #include <functional>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <tuple>
 #include <unordered_map>
@@ -172,6 +173,9 @@ struct Hier {
   long long box_loop_n1 = 0, box_loop_n2 = 0;  // launches per cycle, per confirming residual
   bool box_loop_off = false;                   // the loop graph could not be built: host loop
   void* box_ctl = nullptr;                     // device control block of the loop
+  // the box solve's cluster plan (box.cu solve_plan) of (finest, minlevel, nsmooth)
+  std::shared_ptr<void> box_plan;
+  std::tuple<int, int, int> box_plan_key{};
   size_t bytes = 0;
   size_t reserved = 0;  // bytes counted against the context budget
 

@@ -142,3 +142,29 @@ def test_box_solve_reaches_the_fp64_solution(pkg, ctx, n, mn):
         q[mode] = h.get(0, "q")
         h.close()
     assert np.max(np.abs(q["mixed"] - q["fp64"])) <= 1e-9
+
+
+@pytest.mark.parametrize("errortype", [1, 2])
+@pytest.mark.parametrize("n,mn", BOXES)
+def test_box_solve_in_one_launch_equals_the_host_loop(pkg, ctx, n, mn, errortype):
+    """A V-cycle limit above 64 takes the loop of separate launches; up to 64
+    a box that fits is one launch.  Both compute each cell alike (1e-9 of the
+    solution's size, as above), ghosts included; their norms add in another
+    order, in single precision over a thread's and a warp's cells."""
+    nd = len(n)
+    out = []
+    for most in (64, 65):
+        h = pkg.Hierarchy(ctx, nd, 2, "ch", [1e-5, 0.05])
+        h.build_uniform(list(n) + [1] * (3 - nd), mn, [2] * (2 * nd) + [10] * (6 - 2 * nd), [0, 0, 0],
+                        [v / n[0] for v in n] + [1] * (3 - nd))
+        h.commit()
+        h.seed_spinodal(0, 3)
+        steps = [h.time_step(s == 0, 0, mn, tol=1e-9, maxvcycles=most, errortype=errortype, mode="mixed")
+                 for s in range(3)]
+        out.append((steps, [h.get(p, "q") for p in range(-mn + 1)]))
+        h.close()
+    for (na, ra), (nb, rb) in zip(out[0][0], out[1][0]):
+        assert na == nb
+        assert np.allclose(ra, rb, rtol=1e-4, atol=0)
+    for a, b in zip(out[0][1], out[1][1]):
+        assert np.max(np.abs(a - b)) <= 1e-9 * max(1.0, np.max(np.abs(b)))
