@@ -201,16 +201,24 @@ __device__ __forceinline__ DF split64(double x) {
   float hi = (float)x;
   return {hi, (float)(x - (double)hi)};
 }
-// float -> double by bit operations for normal floats and zeros
+// float -> double by integer operations, every case of it: a conversion held
+// back by a predicate still takes the FP64 unit's 64 cycles
 __device__ __forceinline__ double f2d(float f) {
-  unsigned int u = __float_as_uint(f);
-  unsigned int ex = (u >> 23) & 0xFFu;
-  if (ex != 0 && ex != 0xFFu)
-    return __longlong_as_double((long long)(((unsigned long long)(u & 0x80000000u) << 32) |
-                                            ((unsigned long long)(ex + 896u) << 52) |
-                                            ((unsigned long long)(u & 0x7FFFFFu) << 29)));
-  if ((u << 1) == 0) return __longlong_as_double((long long)((unsigned long long)u << 32));
-  return (double)f;
+  const unsigned u = __float_as_uint(f), a = u & 0x7FFFFFFFu;
+  unsigned hi = (a >> 3) + 0x38000000u, lo = u << 29;
+  if (a - 0x00800000u >= 0x7F000000u) {  // zero, subnormal, infinite or NaN
+    if (a >= 0x7F800000u) {
+      hi = (a >> 3) + 0x70000000u;
+    } else if (a == 0) {
+      hi = 0;
+    } else {  // the leading bit to the implicit place
+      const int s = __clz(a) - 8;
+      const unsigned m = a << s;
+      hi = (m >> 3) + 0x38000000u - ((unsigned)s << 20);
+      lo = m << 29;
+    }
+  }
+  return __hiloint2double((int)(hi | (u & 0x80000000u)), (int)lo);
 }
 
 // deterministic per-CTA sums of two values -> partial[2*cta], [2*cta+1]:
@@ -1004,39 +1012,57 @@ __device__ __forceinline__ T pair_sum(const float* a, const Pair& p, int b, T ot
 enum CycBegin { kTop = 0, kDown = 1, kUp = 2 };
 
 // One smoothing of this CTA's slab of level x (see above), K pairs a thread.
-// sync: the level's barrier.  C: the parent level's slab.  The caller's
+// sync: the level's barrier; local: that of this CTA's nt threads on it.  C: the
+// parent level's slab.  The caller's
 // barrier follows the call.
-template <int DIM, int K, typename F>
+template <int DIM, int K, typename F, typename G>
 __device__ __forceinline__ void cyc_smooth(const Cyc& A, int x, const Slab& S, const Slab& C, int begin, bool restrict_,
-                                           bool emit, int t, int nt, F&& sync) {
+                                           bool emit, int t, int nt, F&& sync, G&& local) {
   const CycLev& L = A.L[x];
   const int units = (S.n0 >> 1) * (DIM == 3 ? S.n1 : 1) * S.nr;
   float *E0 = S.e, *E1 = S.e + S.var;
   const HaloOut H0 = halo_out(S, E0), H1 = halo_out(S, E1);
+  // the pair's cells by colour, so that a sweep selects nothing: their places,
+  // the step to the x-neighbour beyond the pair, e, g, pb ([..][variable])
   Pair p[K];
   bool on[K];
-  float e[K][2][2], g[K][2][2], pb[K][2];  // [cell of the pair][variable]
+  int at[K][2], xo[K][2];
+  float e[K][2][2], g[K][2][2], pb[K][2];
 #pragma unroll
   for (int q = 0; q < K; q++) {
     on[q] = t + q * nt < units;
     if (!on[q]) continue;
     p[q] = pair_of<DIM>(S, L, t + q * nt);
 #pragma unroll
-    for (int b = 0; b < 2; b++) {
-      e[q][b][0] = E0[p[q].at + b];
-      e[q][b][1] = E1[p[q].at + b];
-      g[q][b][0] = S.g[p[q].in + b];
-      g[q][b][1] = S.g[S.ivar + p[q].in + b];
-      pb[q][b] = S.pb[p[q].in + b];
+    for (int c = 0; c < 2; c++) {
+      const int b = p[q].b0 ^ c, in = p[q].in + b;
+      at[q][c] = p[q].at + b;
+      xo[q][c] = b ? p[q].xr : p[q].xl;
+      e[q][c][0] = E0[at[q][c]];
+      e[q][c][1] = E1[at[q][c]];
+      g[q][c][0] = S.g[in];
+      g[q][c][1] = S.g[S.ivar + in];
+      pb[q][c] = S.pb[in];
     }
   }
+  auto sum = [&](const float* a, int q, int c, float other) {  // pair_sum
+    const float* w = a + at[q][c];
+    float s = w[xo[q][c]] + other;
+    if (DIM == 3) {
+      s = s + w[p[q].ym] + w[p[q].yp];
+      s += w[p[q].rm] + w[p[q].rp];
+    } else {
+      s = s + w[p[q].rm] + w[p[q].rp];
+    }
+    return s;
+  };
   const float kc = DIM == 2 ? 4.0f : 6.0f;
-  auto mop_pair = [&](int q, int b, float& m0, float& m1) {  // M(e) at a cell (mop)
-    const float xx = e[q][b][0], y = e[q][b][1];
-    const float s0 = pair_sum<DIM, float>(E0, p[q], b, e[q][1 - b][0]);
-    const float s1 = pair_sum<DIM, float>(E1, p[q], b, e[q][1 - b][1]);
+  auto mop_cell = [&](int q, int c, float& m0, float& m1) {  // M(e) (mop)
+    const float xx = e[q][c][0], y = e[q][c][1];
+    const float s0 = sum(E0, q, c, e[q][1 - c][0]);
+    const float s1 = sum(E1, q, c, e[q][1 - c][1]);
     m0 = xx - L.c0 * (s1 - kc * y);
-    m1 = y - xx * (3.0f * pb[q][b] * (pb[q][b] + xx) + xx * xx) + L.c1 * (s0 - kc * xx);
+    m1 = y - xx * (3.0f * pb[q][c] * (pb[q][c] + xx) + xx * xx) + L.c1 * (s0 - kc * xx);
   };
   if (begin == kDown) {  // g = R(g - M(e)) (left by the finer level) + M_c(ec); e is ec here
 #pragma unroll
@@ -1044,13 +1070,13 @@ __device__ __forceinline__ void cyc_smooth(const Cyc& A, int x, const Slab& S, c
       if (on[q]) {
         float m[2][2];
 #pragma unroll
-        for (int b = 0; b < 2; b++) mop_pair(q, b, m[b][0], m[b][1]);
+        for (int c = 0; c < 2; c++) mop_cell(q, c, m[c][0], m[c][1]);
 #pragma unroll
-        for (int b = 0; b < 2; b++)
+        for (int c = 0; c < 2; c++)
 #pragma unroll
           for (int v = 0; v < 2; v++) {
-            g[q][b][v] += m[b][v];
-            S.g[v * S.ivar + p[q].in + b] = g[q][b][v];
+            g[q][c][v] += m[c][v];
+            S.g[v * S.ivar + at[q][c] - S.plane] = g[q][c][v];
           }
       }
     sync();
@@ -1095,50 +1121,48 @@ __device__ __forceinline__ void cyc_smooth(const Cyc& A, int x, const Slab& S, c
             xstage(a, 0, zf, l2, h2);
           }
           const float w = DIM == 3 ? 1.0f / 64.0f : 1.0f / 16.0f;
-          e[q][0][v] += (3.0f * lo + l2) * w;
-          e[q][1][v] += (3.0f * hi + h2) * w;
+          const float elo = p[q].b0 ? e[q][1][v] : e[q][0][v], ehi = p[q].b0 ? e[q][0][v] : e[q][1][v];
+          const float nlo = elo + (3.0f * lo + l2) * w, nhi = ehi + (3.0f * hi + h2) * w;
+          e[q][0][v] = p[q].b0 ? nhi : nlo;
+          e[q][1][v] = p[q].b0 ? nlo : nhi;
 #pragma unroll
-          for (int b = 0; b < 2; b++) {
-            (v ? E1 : E0)[p[q].at + b] = e[q][b][v];
-            halo_put(S, v ? H1 : H0, p[q].row, p[q].at + b, e[q][b][v]);
+          for (int c = 0; c < 2; c++) {
+            (v ? E1 : E0)[at[q][c]] = e[q][c][v];
+            halo_put(S, v ? H1 : H0, p[q].row, at[q][c], e[q][c][v]);
           }
         }
       }
     sync();
   }
-  for (int s = 0; s < 2 * A.nsmooth; s++) {
-    const int c = s & 1;
+  for (int s = 0; s < A.nsmooth; s++)
 #pragma unroll
-    for (int q = 0; q < K; q++)
-      if (on[q]) {
-        const int b = p[q].b0 ^ c;
-        const float o0 = b ? e[q][0][0] : e[q][1][0], o1 = b ? e[q][0][1] : e[q][1][1];
-        const float s0 = pair_sum<DIM, float>(E0, p[q], b, o0), s1 = pair_sum<DIM, float>(E1, p[q], b, o1);
-        float r0, r1;
-        newton_cell(L.c0, L.c1, L.tmp3, L.a12, b ? pb[q][1] : pb[q][0], b ? e[q][1][0] : e[q][0][0], s0, s1,
-                    b ? g[q][1][0] : g[q][0][0], b ? g[q][1][1] : g[q][0][1], r0, r1);
-        if (b) e[q][1][0] = r0, e[q][1][1] = r1;
-        else e[q][0][0] = r0, e[q][0][1] = r1;
-        E0[p[q].at + b] = r0;
-        E1[p[q].at + b] = r1;
-        halo_put(S, H0, p[q].row, p[q].at + b, r0);
-        halo_put(S, H1, p[q].row, p[q].at + b, r1);
-      }
-    if (s + 1 < 2 * A.nsmooth || restrict_) sync();
-  }
+    for (int c = 0; c < 2; c++) {
+#pragma unroll
+      for (int q = 0; q < K; q++)
+        if (on[q]) {
+          const float s0 = sum(E0, q, c, e[q][1 - c][0]), s1 = sum(E1, q, c, e[q][1 - c][1]);
+          newton_cell(L.c0, L.c1, L.tmp3, L.a12, pb[q][c], e[q][c][0], s0, s1, g[q][c][0], g[q][c][1], e[q][c][0],
+                      e[q][c][1]);
+          E0[at[q][c]] = e[q][c][0];
+          E1[at[q][c]] = e[q][c][1];
+          halo_put(S, H0, p[q].row, at[q][c], e[q][c][0]);
+          halo_put(S, H1, p[q].row, at[q][c], e[q][c][1]);
+        }
+      if (c == 0 || s + 1 < A.nsmooth || restrict_) sync();
+    }
   if (emit) {  // ec = e - ec, for the finer level's prolongation
     const HaloOut C0 = halo_out(S, S.ec), C1 = halo_out(S, S.ec + S.var);
 #pragma unroll
     for (int q = 0; q < K; q++)
       if (on[q])
 #pragma unroll
-        for (int b = 0; b < 2; b++)
+        for (int c = 0; c < 2; c++)
 #pragma unroll
           for (int v = 0; v < 2; v++) {
-            float* d = S.ec + v * S.var + p[q].at + b;
-            const float w = e[q][b][v] - *d;
+            float* d = S.ec + v * S.var + at[q][c];
+            const float w = e[q][c][v] - *d;
             *d = w;
-            halo_put(S, v ? C1 : C0, p[q].row, p[q].at + b, w);
+            halo_put(S, v ? C1 : C0, p[q].row, at[q][c], w);
           }
   }
   if (!restrict_) return;
@@ -1148,14 +1172,14 @@ __device__ __forceinline__ void cyc_smooth(const Cyc& A, int x, const Slab& S, c
   for (int q = 0; q < K; q++)
     if (on[q]) {
 #pragma unroll
-      for (int b = 0; b < 2; b++) {
+      for (int c = 0; c < 2; c++) {
         float m0, m1;
-        mop_pair(q, b, m0, m1);
-        sc[p[q].in + b] = g[q][b][0] - m0;
-        sc[S.ivar + p[q].in + b] = g[q][b][1] - m1;
+        mop_cell(q, c, m0, m1);
+        sc[at[q][c] - S.plane] = g[q][c][0] - m0;
+        sc[S.ivar + at[q][c] - S.plane] = g[q][c][1] - m1;
       }
     }
-  __syncthreads();
+  local();
   // RestrictSolution and the fine half of CoarseLoadingFunction
   const int cu = units >> (DIM == 3 ? 2 : 1);
   const float w = DIM == 3 ? 0.125f : 0.25f;
@@ -1204,112 +1228,181 @@ __device__ __forceinline__ void cyc_smooth(const Cyc& A, int x, const Slab& S, c
   }
 }
 
-// The coarsest level, smoothed in FP64 arithmetic (FP32 storage): one pair a
-// thread.  Values are widened by bit operations, which leave the FP64 unit
-// to the arithmetic.
-template <int DIM, typename F>
+// The coarsest level, smoothed in FP64 arithmetic (FP32 storage).  Values are
+// widened by bit operations, which leave the FP64 unit to the arithmetic: a
+// warp's FP64 instruction takes 64 cycles and more, however few of its lanes
+// work.  LANES = 2 gives the two variables of a pair to two lanes, so that
+// each instruction does both variables' half of the 2x2 system: 19
+// instructions a sweep for 30 (2 x 2 cells: 3300 -> 2000 cycles a sweep),
+// while all the pairs' lanes fit one warp per scheduler (kCoarsePairs2 pairs);
+// more pairs than that take a lane each.
+constexpr int kCoarsePairs2 = 64;
+template <int DIM, int LANES, typename F>
 __device__ __forceinline__ void cyc_coarsest(const Cyc& A, int x, const Slab& S, bool down, bool emit, int t,
                                              F&& sync) {
   const CycLev& L = A.L[x];
   const int units = (S.n0 >> 1) * (DIM == 3 ? S.n1 : 1) * S.nr;
-  float *E0 = S.e, *E1 = S.e + S.var;
-  const bool on = t < units;
+  const int u = LANES == 2 ? t >> 1 : t;
+  const int v = LANES == 2 ? t & 1 : 0;  // this lane's variable
+  const bool on = u < units;
+  constexpr int NV = 3 - LANES;  // variables a lane holds
+  float* const E0 = S.e + v * S.var;
   Pair p;
-  float e[2][2], g[2][2], pb[2];
-  const HaloOut H0 = halo_out(S, E0), H1 = halo_out(S, E1);
-  if (on) {
-    p = pair_of<DIM>(S, L, t);
-    const float kc = DIM == 2 ? 4.0f : 6.0f;
+  float e[2][NV], pb[2];
+  float g[2][NV];  // LANES 2: the other variable's right-hand side, which takes this variable's neighbours
+  HaloOut H[NV];
+#pragma unroll
+  for (int w = 0; w < NV; w++) H[w] = halo_out(S, E0 + w * S.var);
+  p = pair_of<DIM>(S, L, on ? u : 0);
+  const float kc = DIM == 2 ? 4.0f : 6.0f;
+#pragma unroll
+  for (int b = 0; b < 2; b++) {
+#pragma unroll
+    for (int w = 0; w < NV; w++) {
+      e[b][w] = E0[w * S.var + p.at + b];
+      g[b][w] = S.g[(LANES == 2 ? 1 - v : w) * S.ivar + p.in + b];
+    }
+    pb[b] = S.pb[p.in + b];
+  }
+  auto partner = [](float q) { return __shfl_xor_sync(0xffffffffu, q, 1); };
+  if (down) {
 #pragma unroll
     for (int b = 0; b < 2; b++) {
-      e[b][0] = E0[p.at + b];
-      e[b][1] = E1[p.at + b];
-      g[b][0] = S.g[p.in + b];
-      g[b][1] = S.g[S.ivar + p.in + b];
-      pb[b] = S.pb[p.in + b];
-    }
-    if (down) {
-#pragma unroll
-      for (int b = 0; b < 2; b++) {
-        const float xx = e[b][0], y = e[b][1];
+      if (LANES == 1) {
+        const float xx = e[b][0], y = e[b][NV - 1];
         const float s0 = pair_sum<DIM, float>(E0, p, b, e[1 - b][0]);
-        const float s1 = pair_sum<DIM, float>(E1, p, b, e[1 - b][1]);
+        const float s1 = pair_sum<DIM, float>(E0 + S.var, p, b, e[1 - b][NV - 1]);
         g[b][0] += xx - L.c0 * (s1 - kc * y);
-        g[b][1] += y - xx * (3.0f * pb[b] * (pb[b] + xx) + xx * xx) + L.c1 * (s0 - kc * xx);
+        g[b][NV - 1] += y - xx * (3.0f * pb[b] * (pb[b] + xx) + xx * xx) + L.c1 * (s0 - kc * xx);
+      } else {
+        const float other = partner(e[b][0]), xx = v ? other : e[b][0], y = v ? e[b][0] : other;
+        const float s = pair_sum<DIM, float>(E0, p, b, e[1 - b][0]);
+        if (v) g[b][0] += xx - L.c0 * (s - kc * y);
+        else g[b][0] += y - xx * (3.0f * pb[b] * (pb[b] + xx) + xx * xx) + L.c1 * (s - kc * xx);
       }
     }
+    sync();
   }
-  if (down) sync();
   for (int s = 0; s < 2 * A.nsmooth; s++) {
-    if (on) {
-      const int b = p.b0 ^ (s & 1);
-      auto dsum = [&](const float* a, float other) {
-        const float* c = a + p.at + b;
-        double q = f2d(b ? c[p.xr] : c[p.xl]) + f2d(other);
-        if (DIM == 2) return q + f2d(c[p.rm]) + f2d(c[p.rp]);
-        q = q + f2d(c[p.ym]) + f2d(c[p.yp]);
-        return q + (f2d(c[p.rm]) + f2d(c[p.rp]));
-      };
-      const double s0 = dsum(E0, b ? e[0][0] : e[1][0]), s1 = dsum(E1, b ? e[0][1] : e[1][1]);
-      const double pbd = f2d(b ? pb[1] : pb[0]), xv = f2d(b ? e[1][0] : e[0][0]);
+    const int b = p.b0 ^ (s & 1);
+    auto dsum = [&](const float* a, float other) {
+      const float* c = a + p.at + b;
+      double q = f2d(b ? c[p.xr] : c[p.xl]) + f2d(other);
+      if (DIM == 2) return q + f2d(c[p.rm]) + f2d(c[p.rp]);
+      q = q + f2d(c[p.ym]) + f2d(c[p.yp]);
+      return q + (f2d(c[p.rm]) + f2d(c[p.rp]));
+    };
+    const double pbd = f2d(b ? pb[1] : pb[0]);
+    float r[NV];
+    if (LANES == 1) {
+      const double s0 = dsum(E0, b ? e[0][0] : e[1][0]), s1 = dsum(E0 + S.var, b ? e[0][NV - 1] : e[1][NV - 1]);
+      const double xv = f2d(b ? e[1][0] : e[0][0]);
       const double w = pbd + xv;
       const double a21 = -3.0 * w * w - A.cd[2];
       const double b1 = f2d(b ? g[1][0] : g[0][0]) + A.cd[0] * s1;
-      const double b2 = f2d(b ? g[1][1] : g[0][1]) - A.cd[1] * s0 - xv * xv * (3.0 * pbd + 2.0 * xv);
+      const double b2 = f2d(b ? g[1][NV - 1] : g[0][NV - 1]) - A.cd[1] * s0 - xv * xv * (3.0 * pbd + 2.0 * xv);
       const double rdet = __drcp_rn(1.0 - A.cd[3] * a21);
-      const float r0 = (float)((b1 - A.cd[3] * b2) * rdet), r1 = (float)((b2 - a21 * b1) * rdet);
-      if (b) e[1][0] = r0, e[1][1] = r1;
-      else e[0][0] = r0, e[0][1] = r1;
-      E0[p.at + b] = r0;
-      E1[p.at + b] = r1;
-      halo_put(S, H0, p.row, p.at + b, r0);
-      halo_put(S, H1, p.row, p.at + b, r1);
+      r[0] = (float)((b1 - A.cd[3] * b2) * rdet);
+      r[NV - 1] = (float)((b2 - a21 * b1) * rdet);
+    } else {  // the same values, lane 0 | lane 1
+      auto swap = [](double q) { return __shfl_xor_sync(0xffffffffu, q, 1); };
+      const float own = b ? e[1][0] : e[0][0];
+      const float other = partner(own);
+      const double xv = f2d(v ? other : own);
+      const double sum = dsum(E0, b ? e[0][0] : e[1][0]);
+      const double f = __fma_rn(v ? A.cd[0] : -A.cd[1], sum, f2d(b ? g[1][0] : g[0][0]));  // g1 - c1 s0 | b1
+      const double f_ = swap(f);
+      const double w = (v ? xv : pbd) + xv;                                  // pb + x | 2 x
+      const double h = __fma_rn(v ? 3.0 : -3.0, v ? pbd : w, v ? w : 0.0);    // -3 w | 3 pb + 2 x
+      const double k = __fma_rn(v ? xv : h, v ? xv : w, v ? 0.0 : -A.cd[2]);  // a21 | x^2
+      const double k_ = swap(k);
+      const double m = __fma_rn(v ? -k : -A.cd[3], v ? h : k, v ? f_ : 1.0);  // det | b2
+      const double m_ = swap(m);
+      const double rdet = __drcp_rn(v ? m_ : m);
+      // b1 - a12 b2 | b2 - a21 b1
+      r[0] = (float)(__fma_rn(v ? -k_ : -A.cd[3], v ? f : m_, v ? m : f_) * rdet);
     }
+    if (on)
+#pragma unroll
+      for (int w = 0; w < NV; w++) {
+        if (b) e[1][w] = r[w];
+        else e[0][w] = r[w];
+        E0[w * S.var + p.at + b] = r[w];
+        halo_put(S, H[w], p.row, p.at + b, r[w]);
+      }
     if (s + 1 < 2 * A.nsmooth) sync();
   }
-  if (emit && on) {
-    const HaloOut C0 = halo_out(S, S.ec), C1 = halo_out(S, S.ec + S.var);
+  if (emit && on)
 #pragma unroll
-    for (int b = 0; b < 2; b++)
+    for (int w = 0; w < NV; w++) {
+      float* const C0 = S.ec + (v + w) * S.var;
+      const HaloOut C = halo_out(S, C0);
 #pragma unroll
-      for (int v = 0; v < 2; v++) {
-        float* d = S.ec + v * S.var + p.at + b;
-        const float w = e[b][v] - *d;
-        *d = w;
-        halo_put(S, v ? C1 : C0, p.row, p.at + b, w);
+      for (int b = 0; b < 2; b++) {
+        const float d = e[b][w] - C0[p.at + b];
+        C0[p.at + b] = d;
+        halo_put(S, C, p.row, p.at + b, d);
       }
-  }
+    }
 }
 
-// the levels of A once down and up, from the top level's e, g and pb in
+// The levels of A once down and up, from the top level's e, g and pb in
 // shared memory; the top level's e is final, and every CTA of it past its
-// last barrier, at the end
+// last barrier, at the end.  A level is worked on by as many warps as its
+// pairs fill: the others wait for the next level that needs them, so that the
+// chain of sweeps through the small levels has the schedulers to itself.
 template <int DIM>
 __device__ __forceinline__ void cyc_vcycle(const Cyc& A, int rank, int t, int nt) {
+  auto workers = [&](int x) {  // threads; coarser levels have no more than finer ones
+    const CycLev& L = A.L[x];
+    int units = (L.n0 >> 1) * (DIM == 3 ? L.n1 : 1) * L.maxr;
+    if (x == A.nl - 1 && units <= kCoarsePairs2) units *= 2;
+    return min(nt, (units + 31) & ~31);
+  };
   auto smooth = [&](int x, int begin, bool restrict_, bool emit) {
-    const Slab S = slab<DIM, false>(A, x, rank);
-    const Slab C = x + 1 < A.nl ? slab<DIM, true>(A, x + 1, rank) : S;
+    const bool shared = A.L[x].mul != 0;
+    const int nw = workers(x);
+    // barriers of the level's warps, an id a level; shared levels meet across the cluster
+    auto local = [&] { asm volatile("bar.sync %0, %1;" ::"r"(1 + x), "r"(nw) : "memory"); };
     auto sync = [&] {
-      if (S.shared) uni::cluster_sync();
-      else __syncthreads();
+      if (shared) uni::cluster_sync();
+      else local();
     };
-    const int units = (S.n0 >> 1) * (DIM == 3 ? S.n1 : 1) * A.L[x].maxr;
-    if (x == A.nl - 1) cyc_coarsest<DIM>(A, x, S, begin == kDown, emit, t, sync);
-    else if (units <= nt) cyc_smooth<DIM, 1>(A, x, S, C, begin, restrict_, emit, t, nt, sync);
-    else cyc_smooth<DIM, kCycPairs>(A, x, S, C, begin, restrict_, emit, t, nt, sync);
-    // what the next level reads has been written
-    if (S.shared) uni::cluster_sync();
-    else __syncthreads();
+    if (t >= nw) {  // (a shared level) the cluster's barriers count every warp
+      const int n = (begin != kTop) + max(0, 2 * A.nsmooth - (restrict_ ? 0 : 1));
+      for (int k = 0; k < n; k++) uni::cluster_sync();
+    } else {
+      const Slab S = slab<DIM, false>(A, x, rank);
+      const Slab C = x + 1 < A.nl ? slab<DIM, true>(A, x + 1, rank) : S;
+      const int units = (S.n0 >> 1) * (DIM == 3 ? S.n1 : 1) * A.L[x].maxr;
+      if (x == A.nl - 1) {
+        if (units <= kCoarsePairs2 && nw >= 2 * units) cyc_coarsest<DIM, 2>(A, x, S, begin == kDown, emit, t, sync);
+        else cyc_coarsest<DIM, 1>(A, x, S, begin == kDown, emit, t, sync);
+      } else if (units <= nw) {
+        cyc_smooth<DIM, 1>(A, x, S, C, begin, restrict_, emit, t, nw, sync, local);
+      } else {
+        cyc_smooth<DIM, kCycPairs>(A, x, S, C, begin, restrict_, emit, t, nw, sync, local);
+      }
+    }
+    if (shared) uni::cluster_sync();  // what the next level reads has been written
+  };
+  auto meet = [&](int x) {  // the warps of a level that CTA 0 holds alone
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + x), "r"(workers(x)) : "memory");
   };
   for (int x = 0; x < A.nl; x++) {
-    if (!A.L[x].mul && rank) break;
+    const bool shared = A.L[x].mul != 0;
+    if (!shared && (rank || t >= workers(x))) break;
     smooth(x, x ? kDown : kTop, x + 1 < A.nl, x && x + 1 == A.nl);
+    if (!shared) meet(x);
   }
   for (int x = A.nl - 2; x >= 0; x--) {
-    if (!A.L[x].mul && rank) continue;
-    if (A.L[x].mul && !A.L[x + 1].mul) uni::cluster_sync();  // CTA 0 has finished the levels it holds
+    const bool shared = A.L[x].mul != 0;
+    if (!shared && (rank || t >= workers(x))) continue;
+    if (!shared) meet(x);  // the next coarser level is finished
+    else if (!A.L[x + 1].mul) uni::cluster_sync();
     smooth(x, kUp, false, x > 0);
   }
+  if (!A.L[0].mul) __syncthreads();
 }
 
 template <int DIM>
@@ -1587,8 +1680,8 @@ __global__ void __launch_bounds__(256) k_bx_merge(double* __restrict__ pool, lon
 //
 // A step of such a box was some 14 launches and a graph with a conditional
 // loop of six launches a V-cycle; now it is this one, the fill of the coarse
-// levels and one wait.  A step of five V-cycles at 32^2: 285 -> 206 us; of
-// seven at 128^2: 510 -> 460 us.  What bounds it is the chain of sweeps.
+// levels and one wait.  A step of five V-cycles at 32^2: 285 -> 200 us; of
+// seven at 128^2: 510 -> 440 us.  What bounds it is the chain of sweeps.
 constexpr int kSolveMaxCycles = 64;
 struct BoxSolve {
   long long oqlo, ofhi, oflo;      // float offsets
@@ -1612,6 +1705,7 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_bx_solve(float* __restrict__
   __shared__ float wsum[2][kCycThreads / 32];
   __shared__ double part[2][32];  // two norms' worth: a CTA may start the next while another still adds up this one
   __shared__ double norm_now;
+  __shared__ int verdict;
   int turn = 0;
   auto all = [&] {
     if (A.ctas > 1) uni::cluster_sync();
@@ -1649,8 +1743,10 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_bx_solve(float* __restrict__
     return (long long)(a.x + 1) + (long long)(a.y + 1) * B.qn0 +
            (DIM == 3 ? (long long)(a.z + 1) * B.qn0 * B.qn1 : 0);
   };
-  // ErrorAFAS of the squares each thread summed, in every CTA
-  auto norm = [&](float s0, float s1) {
+  // ErrorAFAS of the squares each thread summed, in every CTA, and what
+  // judge(it) makes of it: by one thread, an FP64 comparison of every warp
+  // would take the FP64 unit longer than the norm itself
+  auto norm = [&](float s0, float s1, auto&& judge) {
     for (int o = 16; o > 0; o >>= 1) {
       s0 += __shfl_down_sync(0xffffffffu, s0, o);
       s1 += __shfl_down_sync(0xffffffffu, s1, o);
@@ -1688,13 +1784,14 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_bx_solve(float* __restrict__
           const double r0 = sqrt(a / (0.5 * B.count)), r1 = sqrt(b / (0.5 * B.count));
           norm_now = r1 > r0 ? r1 : r0;
         }
+        verdict = judge(norm_now);
       }
     }
     __syncthreads();
-    return norm_now;
+    return verdict;
   };
   // the true residual to g; its norm
-  auto confirm = [&] {
+  auto confirm = [&](auto&& judge) {
     float s0 = 0.f, s1 = 0.f;
     for (int u = t; u < units; u += nt) {
       const Pair p = pair_of<DIM>(S, L, u);
@@ -1710,7 +1807,7 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_bx_solve(float* __restrict__
         s1 += r1 * r1;
       }
     }
-    return norm(s0, s1);
+    return norm(s0, s1, judge);
   };
   // q and qold split into float pairs (k_bx_split, k_bx_split_warm)
   float w0 = 0.f, w1 = 0.f;
@@ -1747,8 +1844,13 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_bx_solve(float* __restrict__
   };
   clear();
   all();
-  double r_sync = B.warm ? norm(w0, w1) : confirm();
-  int status = !isfinite(r_sync), conv = 0, it = 0, nconfirm = 0;
+  double r_sync = 0.0;  // the last true residual (thread 0)
+  enum { kNonfinite = 1, kConfirm = 2, kConverged = 4 };
+  auto judge_true = [&](double r) {
+    r_sync = r;
+    return !isfinite(r) ? kNonfinite : (r < B.tol ? kConverged : 0);
+  };
+  int status = (B.warm ? norm(w0, w1, judge_true) : confirm(judge_true)) & kNonfinite, conv = 0, it = 0, nconfirm = 0;
   while (!status && it < B.maxv) {
     it++;
     cyc_vcycle<DIM>(A, rank, t, nt);
@@ -1787,18 +1889,17 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_bx_solve(float* __restrict__
         s1 += a1 * a1;
       }
     }
-    double res = norm(s0, s1);
+    int v = norm(s0, s1, [&](double r) {
+      return !isfinite(r) ? kNonfinite : (r < B.tol || r < 1e-5 * r_sync || it >= B.maxv ? kConfirm : 0);
+    });
     clear();  // after norm's barrier: every read of e is done
-    if (!isfinite(res)) {
-      status = 1;
-    } else if (res < B.tol || res < 1e-5 * r_sync || it >= B.maxv) {
-      res = confirm();
+    if (v & kConfirm) {
+      v = confirm(judge_true);
       nconfirm++;
-      if (!isfinite(res)) status = 1;
-      r_sync = res;
-      conv = !status && res < B.tol;
     }
-    if (rank == 0 && t == 0 && !status) out->res[it - 1] = res;
+    status = v & kNonfinite;
+    conv = v & kConverged;
+    if (rank == 0 && t == 0 && !status) out->res[it - 1] = norm_now;
     if (conv) break;
     all();  // e is zero in every CTA
   }
@@ -1829,8 +1930,8 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_bx_solve(float* __restrict__
   }
   if (rank == 0 && t == 0) {
     out->it = it;
-    out->conv = conv;
-    out->status = status;
+    out->conv = conv != 0;
+    out->status = status != 0;
     out->nconfirm = nconfirm;
   }
   all();  // a CTA's shared memory stays while another may still address it
@@ -2079,7 +2180,7 @@ bool cycle_layout(Hier& H, int top, int minlevel, int nsmooth, int share, Cyc& A
     // levels colour by colour, the others as k_bx_restrict_load
     L.by_colour = 2 * P.half <= 8192;
     if (x + 1 < A.nl) scratch = std::max(scratch, 4 * pairs);
-    if (o * 4 > kUniSmemMax) return false;
+    if (o * 4 > kUniSmemMax || A.nl > 15) return false;  // (a named barrier a level)
   }
   A.scratch = add(scratch);
   for (int v = 0; v < 4; v++) A.cd[v] = B(H, minlevel).cd[v];
