@@ -126,4 +126,41 @@ __device__ __forceinline__ bool ghosted_cell(const int* n, int gs, int t, int& i
   return ok;
 }
 
+// The sums of a warp's NV FP64 values a lane -> red[v][w], each the tree of
+// shfl_down(16, 8, 4, 2, 1) bit for bit.  An FP64 add takes the unit 64
+// cycles for however many lanes: two to four variables share the adds, each
+// half (quarter) of the warp holding one of them after the first steps (5
+// adds for 2 variables instead of 10, 6 for 3 instead of 15).  A warp whose
+// lanes all hold zero adds nothing.
+template <int NV, int W>
+__device__ __forceinline__ void warp_sums(const double (&s)[NV], double (*red)[W], int w, int lane, bool any) {
+  if (!any) {
+    if (lane < NV) red[lane][w] = 0.0;
+    return;
+  }
+  auto peer = [](double x, int o) { return __shfl_xor_sync(0xffffffffu, x, o); };
+  if constexpr (NV < 2 || NV > 4) {
+    for (int v = 0; v < NV; v++) {
+      double t = s[v];
+      for (int o = 16; o > 0; o >>= 1) t = __dadd_rn(t, peer(t, o));
+      if (lane == 0) red[v][w] = t;
+    }
+  } else {
+    const bool h = lane & 16, q = lane & 8;
+    double r = __dadd_rn(h ? s[1] : s[0], peer(h ? s[0] : s[1], 16));  // variable 0 | 1
+    if constexpr (NV == 2) {
+      r = __dadd_rn(r, peer(r, 8));
+    } else {
+      double r2;  // variable 2 (| 3)
+      if constexpr (NV == 4) r2 = __dadd_rn(h ? s[3] : s[2], peer(h ? s[2] : s[3], 16));
+      else r2 = __dadd_rn(s[2], peer(s[2], 16));
+      const double send = q ? r : r2;
+      r = __dadd_rn(q ? r2 : r, peer(send, 8));
+    }
+    for (int o = 4; o > 0; o >>= 1) r = __dadd_rn(r, peer(r, o));
+    const int v = (h ? 1 : 0) + (NV > 2 && q ? 2 : 0);
+    if ((lane & 7) == 0 && (NV > 2 || !q) && v < NV && !(NV == 3 && h && q)) red[v][w] = r;
+  }
+}
+
 }  // namespace bsamg

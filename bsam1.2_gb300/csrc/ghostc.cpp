@@ -692,15 +692,20 @@ std::vector<GhostOp> stage_ops(const Hier& H, std::vector<Em>& ops, std::vector<
     rst[d] = -1;
     nst = std::max(nst, st + 1);
   }
+  // within a stage by type, in the order they came: a warp whose lanes run
+  // different types runs each in turn, its loads' latencies and (FP64) the
+  // unit's 64 cycles an instruction included
+  constexpr int kTypes = kGCfAC + 1;
   std::vector<GhostOp> res;
-  stage_off.assign(nst + 1, 0);
+  std::vector<int> fill(nst * kTypes + 1, 0);
   for (int x = 0; x < m; x++)
-    if (!dead[x]) stage_off[stage[x] + 1]++;
-  for (int s = 0; s < nst; s++) stage_off[s + 1] += stage_off[s];
+    if (!dead[x]) fill[stage[x] * kTypes + ops[x].op.type + 1]++;
+  for (int s = 0; s < nst * kTypes; s++) fill[s + 1] += fill[s];
+  stage_off.resize(nst + 1);
+  for (int s = 0; s <= nst; s++) stage_off[s] = fill[s * kTypes];
   res.resize(stage_off[nst]);
-  std::vector<int> fill(stage_off.begin(), stage_off.end() - 1);
   for (int x = 0; x < m; x++)
-    if (!dead[x]) res[fill[stage[x]]++] = ops[x].op;
+    if (!dead[x]) res[fill[stage[x] * kTypes + ops[x].op.type]++] = ops[x].op;
   return res;
 }
 

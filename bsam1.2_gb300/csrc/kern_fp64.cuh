@@ -327,11 +327,7 @@ __global__ void __launch_bounds__(kBlock) k_update_source(const PatchDev* __rest
 // fixed order
 template <int NV>
 __device__ __forceinline__ void block_sum(double (&s)[NV], double (*red)[kBlock / 32], double* __restrict__ partial) {
-  for (int o = 16; o > 0; o >>= 1)
-    for (int v = 0; v < NV; v++) s[v] = s[v] + __shfl_down_sync(0xffffffffu, s[v], o);
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  if (l == 0)
-    for (int v = 0; v < NV; v++) red[v][w] = s[v];
+  warp_sums<NV>(s, red, threadIdx.x >> 5, threadIdx.x & 31, true);
   __syncthreads();
   if (threadIdx.x < NV) {  // a thread a variable
     const int v = threadIdx.x;

@@ -334,6 +334,7 @@ __global__ void __launch_bounds__(kBlock) k_mx_norm(const PatchDev* __restrict__
   constexpr int NV = PL::kNV;
   __shared__ double red[NV][kBlock / 32];
   double s[NV];
+  bool any = false;
   for (int v = 0; v < NV; v++) s[v] = 0.0;
   for (int sub = 0; sub < kNormCells; sub++) {
     const Blk b = blk[blockIdx.x * kNormCells + sub];
@@ -341,6 +342,7 @@ __global__ void __launch_bounds__(kBlock) k_mx_norm(const PatchDev* __restrict__
     const PatchDev& p = P[b.patch];
     int i, j, k;
     if (!interior_cell<DIM>(p.mx, b.start + threadIdx.x, i, j, k)) continue;
+    any = true;
     const double* q = pool + p.oq;
     long long sy = p.qn[0], sz = (long long)p.qn[0] * p.qn[1];
     long long c = gofs<DIM>(p.qn, i, j, k);
@@ -353,18 +355,13 @@ __global__ void __launch_bounds__(kBlock) k_mx_norm(const PatchDev* __restrict__
       s[v] = fma(e, e, s[v]);
     }
   }
-  for (int o = 16; o > 0; o >>= 1)
-    for (int v = 0; v < NV; v++) s[v] += __shfl_down_sync(0xffffffffu, s[v], o);
-  int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  if (l == 0)
-    for (int v = 0; v < NV; v++) red[v][w] = s[v];
+  warp_sums<NV>(s, red, threadIdx.x >> 5, threadIdx.x & 31, __any_sync(0xffffffffu, any));
   __syncthreads();
-  if (threadIdx.x == 0)
-    for (int v = 0; v < NV; v++) {
-      double t = 0.0;
-      for (int m = 0; m < kBlock / 32; m++) t += red[v][m];
-      partial[NV * blockIdx.x + v] = t;
-    }
+  if (threadIdx.x < NV) {  // a thread a variable
+    double t = 0.0;
+    for (int m = 0; m < kBlock / 32; m++) t += red[threadIdx.x][m];
+    partial[NV * blockIdx.x + threadIdx.x] = t;
+  }
 }
 
 // Residual tracked in FP32 between FP64 evaluations: after qbar += e the

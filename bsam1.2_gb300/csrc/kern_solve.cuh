@@ -139,6 +139,7 @@ __device__ __forceinline__ void s_norm(const PatchDev* __restrict__ P, double* p
                                        double (*red)[kBlock / 32]) {
   constexpr int NV = PL::kNV;
   double s[NV];
+  bool any = false;
   for (int v = 0; v < NV; v++) s[v] = 0.0;
   for (int sub = 0; sub < kNormCells; sub++) {
     const Blk bb = blk[b * kNormCells + sub];
@@ -146,6 +147,7 @@ __device__ __forceinline__ void s_norm(const PatchDev* __restrict__ P, double* p
     const PatchDev& p = P[bb.patch];
     int i, j, k;
     if (!interior_cell<DIM>(p.mx, bb.start + u, i, j, k)) continue;
+    any = true;
     const double* q = pool + p.oq;
     long long sy = p.qn[0], sz = (long long)p.qn[0] * p.qn[1];
     long long c = gofs<DIM>(p.qn, i, j, k);
@@ -158,65 +160,42 @@ __device__ __forceinline__ void s_norm(const PatchDev* __restrict__ P, double* p
       s[v] = fma(e, e, s[v]);
     }
   }
-  for (int o = 16; o > 0; o >>= 1)
-    for (int v = 0; v < NV; v++) s[v] += __shfl_down_sync(0xffffffffu, s[v], o);
-  int w = u >> 5, l = u & 31;
-  if (l == 0)
-    for (int v = 0; v < NV; v++) red[v][w] = s[v];
+  warp_sums<NV>(s, red, u >> 5, u & 31, __any_sync(0xffffffffu, any));
   group_barrier(g);
-  if (u == 0)
-    for (int v = 0; v < NV; v++) {
-      double t = 0.0;
-      for (int m = 0; m < kBlock / 32; m++) t += red[v][m];
-      partial[NV * b + v] = t;
-    }
+  if (u < NV) {  // a thread a variable
+    double t = 0.0;
+    for (int m = 0; m < kBlock / 32; m++) t += red[u][m];
+    partial[NV * b + u] = t;
+  }
   group_barrier(g);
 }
 
 // The final sum of launch_norm_finish (one stage: nb <= 2048 partials) by
-// the T threads of one CTA: the 1024 threads of k_norm_finish are emulated,
-// their shuffle trees replayed in shared memory on the lanes that reach
-// lane 0, so the sum is the same bit for bit.  Thread 0 returns the norm.
+// the T threads of one CTA: the sums of its 1024 threads and their trees,
+// bit for bit.  Sums of nothing are left out, as there: with 129 partials 5
+// warps add instead of 32.  Thread 0 returns the variables' sums.
 template <int NV, int T>
-__device__ __forceinline__ void s_finish(const double* partial, int nb, double (*tv)[1024], double (*r2)[32],
-                                         double* sum_out, double* red0) {
+__device__ __forceinline__ void s_finish(const double* partial, int nb, double (*r2)[32], double* red0) {
   constexpr int kF = 1024;
-  for (int vt = threadIdx.x; vt < kF; vt += T) {
-    double a[NV][8];
-    for (int v = 0; v < NV; v++)
-      for (int u = 0; u < 8; u++) a[v][u] = 0.0;
-    int n = vt;
-    for (; n + 7 * kF < nb; n += 8 * kF)
-      for (int u = 0; u < 8; u++)
-        for (int v = 0; v < NV; v++) a[v][u] = a[v][u] + partial[NV * (n + u * kF) + v];
-    for (; n < nb; n += kF)
-      for (int v = 0; v < NV; v++) a[v][0] = a[v][0] + partial[NV * n + v];
-    for (int v = 0; v < NV; v++)
-      tv[v][vt] = ((a[v][0] + a[v][1]) + (a[v][2] + a[v][3])) + ((a[v][4] + a[v][5]) + (a[v][6] + a[v][7]));
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warps = min(32, (nb + 31) / 32);  // emulated warps that hold a partial
+  for (int x = w; x < warps; x += T / 32) {
+    double t[NV];
+    const int n = x * 32 + lane;
+    for (int v = 0; v < NV; v++) t[v] = n < nb ? partial[NV * n + v] : 0.0;
+    if (x * 32 + kF < nb)
+      for (int v = 0; v < NV; v++) t[v] += n + kF < nb ? partial[NV * (n + kF) + v] : 0.0;
+    warp_sums<NV>(t, r2, x, lane, true);
   }
   __syncthreads();
-  // t = t + shfl_down(t, o) within each warp of 32 emulated lanes: lanes
-  // l < o are the ones whose values reach lane 0
-  for (int o = 16; o > 0; o >>= 1) {
-    for (int x = threadIdx.x; x < 32 * o; x += T) {
-      int w = x / o, l = x - w * o;
-      for (int v = 0; v < NV; v++) tv[v][w * 32 + l] = tv[v][w * 32 + l] + tv[v][w * 32 + l + o];
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x < 32)
-    for (int v = 0; v < NV; v++) r2[v][threadIdx.x] = tv[v][threadIdx.x * 32];
-  __syncthreads();
-  for (int o = 16; o > 0; o >>= 1) {
-    if (threadIdx.x < o)
-      for (int v = 0; v < NV; v++) r2[v][threadIdx.x] = r2[v][threadIdx.x] + r2[v][threadIdx.x + o];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    double sum = r2[0][0];
-    for (int v = 1; v < NV; v++) sum = sum + r2[v][0];
-    *sum_out = sum;
-    for (int v = 0; v < NV; v++) red0[v] = r2[v][0];
+  if (w == 0) {
+    double t[NV];
+    for (int v = 0; v < NV; v++) t[v] = lane < warps ? r2[v][lane] : 0.0;
+    for (int o = 16; o > 0; o >>= 1)
+      if (o < warps)
+        for (int v = 0; v < NV; v++) t[v] += __shfl_down_sync(0xffffffffu, t[v], o);
+    if (lane == 0)
+      for (int v = 0; v < NV; v++) red0[v] = t[v];
   }
 }
 
@@ -337,7 +316,6 @@ __global__ void __launch_bounds__(T, 1)
                double* res, double* partial, ProbParams pp, MxParams mp) {
   constexpr int NV = PL::kNV;
   __shared__ double red[T / 256][NV][kBlock / 32];
-  __shared__ double tv[NV][1024];
   __shared__ double r2[NV][32];
   // every CTA stages the read-only program image after its data area and
   // its ghost operations: phases, patch table, block, stage and part pools
@@ -398,9 +376,11 @@ __global__ void __launch_bounds__(T, 1)
       if (f.op == kSFinish) {
         // every CTA sums the partials in the same order and takes the same
         // decision; CTA 0 records it
-        double sum, comp[NV];
-        s_finish<NV, T>(partial, f.n, tv, r2, &sum, comp);
+        double comp[NV];  // thread 0's
+        s_finish<NV, T>(partial, f.n, r2, comp);
         if (threadIdx.x == 0) {
+          double sum = comp[0];
+          for (int v = 1; v < NV; v++) sum = sum + comp[v];
           double r;
           if (errortype == 1) {
             r = sqrt(sum / count);  // ErrorAFAS, afasroutines.f90:135
