@@ -121,6 +121,7 @@ struct Hier {
   // while a solve program is recorded: the V-cycle level from which CTA 0
   // runs the coarse end alone (a kTSolo marker precedes those phases)
   int rec_solo = -kMaxDepth - 2;
+  bool rec_push = false;  // recording a solve whose levels <= 0 write their own ghosts
   // the mixed solve of a hierarchy with refinement levels as one cluster
   // launch (kern_solve.cuh): mode 1 uses it where it applies, 0 keeps the
   // per-launch graphs; its launch shape and the cells of the coarse end run

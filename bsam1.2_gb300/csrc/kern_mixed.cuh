@@ -154,30 +154,36 @@ __device__ __forceinline__ void u_prolong(const PatchDev* __restrict__ P, float*
 }
 
 // ghost programs on e: homogeneous boundary conditions
-template <bool CL = false>
+__device__ __forceinline__ float ghost32_value(const GhostOp& g, const float* dq, const float* sq, int v) {
+  switch (g.type) {
+    case kGCopy:
+    case kGCopyAdd:
+    case kGCopySub: return sq[g.s0];  // the qpo offset cancels in a correction
+    case kGBC: return ((g.mask >> v) & 0x101) ? -sq[g.s0] : sq[g.s0];  // 2 - q, -q -> -e
+    case kGCfA: return fA1 * dq[g.s0] + fA2 * dq[g.s1] + fA3 * sq[g.c0];
+    case kGCfAB: return fA1 * dq[g.s0] + fA2 * dq[g.s1] + fA3 * (fB1 * sq[g.c0] + fB2 * sq[g.c1] + fB3 * sq[g.c2]);
+    default:
+      return fA1 * dq[g.s0] + fA2 * dq[g.s1] +
+             fA3 * (fC1 * sq[g.c0] + fC2 * sq[g.c1] + fC3 * sq[g.c2] + fC4 * sq[g.c3]);
+  }
+}
+// NV > 0: the number of variables, all of whose loads come before the first
+// store (a load cannot pass a store, and each costs a trip to another CTA)
+template <bool CL = false, int NV = 0>
 __device__ __forceinline__ void ghost32_apply(const PatchDev* __restrict__ P, float* __restrict__ fpool,
                                               const GhostOp& g, int nrvars) {
   const PatchDev& d = P[g.dp];
   const PatchDev& s = P[g.sp];
-  float* fd = fbase<CL>(fpool, d);
-  const float* fs = fbase<CL>(fpool, s);
-  for (int v = 0; v < nrvars; v++) {
-    float* dq = fd + d.eq + v * d.sq;
-    const float* sq = fs + s.eq + v * s.sq;
-    float val;
-    switch (g.type) {
-      case kGCopy:
-      case kGCopyAdd:
-      case kGCopySub: val = sq[g.s0]; break;  // the qpo offset cancels in a correction
-      case kGBC: val = ((g.mask >> v) & 0x101) ? -sq[g.s0] : sq[g.s0]; break;  // 2 - q, -q -> -e
-      case kGCfA: val = fA1 * dq[g.s0] + fA2 * dq[g.s1] + fA3 * sq[g.c0]; break;
-      case kGCfAB: val = fA1 * dq[g.s0] + fA2 * dq[g.s1] + fA3 * (fB1 * sq[g.c0] + fB2 * sq[g.c1] + fB3 * sq[g.c2]); break;
-      default:
-        val = fA1 * dq[g.s0] + fA2 * dq[g.s1] +
-              fA3 * (fC1 * sq[g.c0] + fC2 * sq[g.c1] + fC3 * sq[g.c2] + fC4 * sq[g.c3]);
-        break;
-    }
-    dq[g.dcell] = val;
+  float* fd = fbase<CL>(fpool, d) + d.eq;
+  const float* fs = fbase<CL>(fpool, s) + s.eq;
+  if constexpr (NV > 0) {
+    float val[NV];
+#pragma unroll
+    for (int v = 0; v < NV; v++) val[v] = ghost32_value(g, fd + v * d.sq, fs + v * s.sq, v);
+#pragma unroll
+    for (int v = 0; v < NV; v++) fd[v * d.sq + g.dcell] = val[v];
+  } else {
+    for (int v = 0; v < nrvars; v++) fd[v * d.sq + g.dcell] = ghost32_value(g, fd + v * d.sq, fs + v * s.sq, v);
   }
 }
 

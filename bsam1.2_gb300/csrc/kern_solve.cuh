@@ -65,50 +65,127 @@ __device__ __forceinline__ void s_ghost64(const PatchDev* __restrict__ P, double
                                           const ProbParams& pp) {
   const PatchDev& d = P[g.dp];
   const PatchDev& s = P[g.sp];
+  double val[NV];  // every variable's loads before the first store
 #pragma unroll
   for (int v = 0; v < NV; v++) {
-    double* dq = pool + d.oq + v * d.sq;
+    const double* dq = pool + d.oq + v * d.sq;
     const double* sq = pool + s.oq + v * s.sq;
-    double val;
     switch (g.type) {
-      case kGCopy: val = sq[g.s0]; break;
-      case kGCopyAdd: val = __dadd_rn(sq[g.s0], pp.qpo[v]); break;
-      case kGCopySub: val = __dsub_rn(sq[g.s0], pp.qpo[v]); break;
+      case kGCopy: val[v] = sq[g.s0]; break;
+      case kGCopyAdd: val[v] = __dadd_rn(sq[g.s0], pp.qpo[v]); break;
+      case kGCopySub: val[v] = __dsub_rn(sq[g.s0], pp.qpo[v]); break;
       case kGBC:
-        val = ((g.mask >> v) & 1) ? __dsub_rn(2.0, sq[g.s0]) : (((g.mask >> (8 + v)) & 1) ? -sq[g.s0] : sq[g.s0]);
+        val[v] = ((g.mask >> v) & 1) ? __dsub_rn(2.0, sq[g.s0]) : (((g.mask >> (8 + v)) & 1) ? -sq[g.s0] : sq[g.s0]);
         break;
       case kGCfA:
-        val = __dadd_rn(__dadd_rn(__dmul_rn(dA1, dq[g.s0]), __dmul_rn(dA2, dq[g.s1])), __dmul_rn(dA3, sq[g.c0]));
+        val[v] = __dadd_rn(__dadd_rn(__dmul_rn(dA1, dq[g.s0]), __dmul_rn(dA2, dq[g.s1])), __dmul_rn(dA3, sq[g.c0]));
         break;
       case kGCfAB: {
         double c = __dadd_rn(__dadd_rn(__dmul_rn(dB1, sq[g.c0]), __dmul_rn(dB2, sq[g.c1])), __dmul_rn(dB3, sq[g.c2]));
-        val = __dadd_rn(__dadd_rn(__dmul_rn(dA1, dq[g.s0]), __dmul_rn(dA2, dq[g.s1])), __dmul_rn(dA3, c));
+        val[v] = __dadd_rn(__dadd_rn(__dmul_rn(dA1, dq[g.s0]), __dmul_rn(dA2, dq[g.s1])), __dmul_rn(dA3, c));
         break;
       }
       default: {
         double c = __dadd_rn(__dadd_rn(__dadd_rn(__dmul_rn(dC1, sq[g.c0]), __dmul_rn(dC2, sq[g.c1])),
                                        __dmul_rn(dC3, sq[g.c2])),
                              __dmul_rn(dC4, sq[g.c3]));
-        val = __dadd_rn(__dadd_rn(__dmul_rn(dA1, dq[g.s0]), __dmul_rn(dA2, dq[g.s1])), __dmul_rn(dA3, c));
+        val[v] = __dadd_rn(__dadd_rn(__dmul_rn(dA1, dq[g.s0]), __dmul_rn(dA2, dq[g.s1])), __dmul_rn(dA3, c));
         break;
       }
     }
-    dq[g.dcell] = val;
   }
+#pragma unroll
+  for (int v = 0; v < NV; v++) pool[d.oq + v * d.sq + g.dcell] = val[v];
+}
+
+// Ghost images on a uniform level (kern_uni.cuh push): the FP64 solution's
+// values, each rounding explicit as in s_ghost64; the correction's with the
+// homogeneous conditions
+template <int NVARS>
+struct Push64 {
+  using T = double;
+  using Par = ProbParams;
+  static constexpr int NV = NVARS;
+  __device__ __forceinline__ static double shift(double w, int s, int v, const Par& pp) {
+    return s == 0 ? w : (s == 1 ? __dadd_rn(w, pp.qpo[v]) : __dsub_rn(w, pp.qpo[v]));
+  }
+  __device__ __forceinline__ static double wall(double u, int mask, int v) {
+    return ((mask >> v) & 1) ? __dsub_rn(2.0, u) : (((mask >> (8 + v)) & 1) ? -u : u);
+  }
+};
+template <int NVARS>
+struct Push32 {
+  using T = float;
+  using Par = int;
+  static constexpr int NV = NVARS;
+  __device__ __forceinline__ static float shift(float w, int, int, int) { return w; }
+  __device__ __forceinline__ static float wall(float u, int mask, int v) { return ((mask >> v) & 0x101) ? -u : u; }
+};
+template <class TR, int DIM>
+__device__ __forceinline__ void s_push(typename TR::T* base, const PatchDev& p, int i, int j, int k,
+                                       const typename TR::T* w, const UniBC& bc, const typename TR::Par& par) {
+  const int N = DIM == 3 ? p.mx[2] : p.mx[1];
+  const uni::Geo g{p.mx[0], p.mx[1], N, 0, N, p.qn[0], p.qn[0] * p.qn[1], (int)p.sq};
+  uni::push<TR, DIM>(base, g, i, j, k, w, true, bc, par);
+}
+
+// The operations of a uniform level that write their cells' images
+// (kPushGhosts).  Its ghost program is two stages of a few hundred cells, on
+// the critical path of every sweep: 6700 cycles on a 64^2 level, 3000 in the
+// CTA that runs the coarse end alone.  (The prolongation sets four to eight
+// cells a thread: its images are a phase of their own, kSUniGhost.)
+template <class PL, int DIM>
+__device__ __forceinline__ void s_relax_push(const PatchDev* __restrict__ P, float* fpool, const Blk b, int tid,
+                                             int arg, const MxParams& mp, const UniBC& bc) {
+  constexpr int NV = PL::kNV;
+  const PatchDev& p = P[b.patch];
+  int i, j, k;
+  if (!color_cell<DIM>(p, b.start + tid, arg & 3, i, j, k)) return;
+  const Cell32 x = cell32<PL, DIM, true>(p, fpool, i, j, k);
+  if (arg & kRelax64) PL::template mx_relax<DIM, double>(x, p.c, mp);
+  else PL::template mx_relax<DIM, float>(x, p.cf, mp);
+  float w[NV];
+  for (int v = 0; v < NV; v++) w[v] = x.e[v * x.sq + x.c];
+  s_push<Push32<NV>, DIM>(x.e, p, i, j, k, w, bc, 0);
+}
+// u_restrict onto a uniform parent
+template <int NV, int DIM>
+__device__ __forceinline__ void s_restrict_push(const PatchDev* __restrict__ P, float* fpool, const Blk b, int tid,
+                                                const UniBC& bc) {
+  const PatchDev& p = P[b.patch];
+  int ci, cj, ck;
+  if (!interior_cell<DIM>(p.cmx, b.start + tid, ci, cj, ck)) return;
+  const PatchDev& par = P[p.parent];
+  float* fp = fbase<true>(fpool, p);
+  float* fq = fbase<true>(fpool, par);
+  const int pi = p.mb[0] + ci - 1, pj = p.mb[1] + cj - 1, pk = DIM == 3 ? p.mb[2] + ck - 1 : 1;
+  float w[NV];
+  for (int v = 0; v < NV; v++) {
+    const float* e = fp + p.eq + v * p.sq;
+    auto at = [&](int i, int j, int k) { return e[gofs<DIM>(p.qn, i, j, k)]; };
+    w[v] = restrict_at32<DIM>(at, ci, cj, ck);
+  }
+  for (int v = 0; v < NV; v++) {
+    fp[p.ecq + v * p.sc + gofs<DIM>(p.cn, ci, cj, ck)] = w[v];
+    fq[par.eq + v * par.sq + gofs<DIM>(par.qn, pi, pj, DIM == 3 ? pk : 0)] = w[v];
+  }
+  s_push<Push32<NV>, DIM>(fq + par.eq, par, pi, pj, pk, w, bc, 0);
 }
 
 // FillDownLevel of q (afasroutines.f90:257-327, field 2): parent q(mb) =
 // Restriction2D/3D (gridutilities.f90:103-126, :437-466) of the child's q,
 // the sum left to right and then the product, as the FP64 path's kernel.
-template <int DIM>
-__device__ __forceinline__ void s_fill64(const PatchDev* __restrict__ P, double* pool, const Blk b, int tid,
-                                         int nrvars) {
+template <int NV, int DIM>
+__device__ __forceinline__ void s_fill64(const PatchDev* __restrict__ P, double* pool, const Blk b, int tid, int push,
+                                         const UniBC& bc, const ProbParams& pp) {
   const PatchDev& p = P[b.patch];
   int ci, cj, ck;
   if (!interior_cell<DIM>(p.cmx, b.start + tid, ci, cj, ck)) return;
   const PatchDev& par = P[p.parent];
   const int i = 2 * ci, j = 2 * cj, k = DIM == 3 ? 2 * ck : 0;
-  for (int v = 0; v < nrvars; v++) {
+  double w[NV];
+#pragma unroll
+  for (int v = 0; v < NV; v++) {
     const double* q = pool + p.oq + v * p.sq;
     auto at = [&](int a, int b2, int c) { return q[gofs<DIM>(p.qn, a, b2, c)]; };
     double val;
@@ -126,9 +203,11 @@ __device__ __forceinline__ void s_fill64(const PatchDev* __restrict__ P, double*
       s = __dadd_rn(s, at(i - 1, j - 1, k - 1));
       val = __dmul_rn(0.125, s);
     }
-    pool[par.oq + v * par.sq + gofs<DIM>(par.qn, p.mb[0] + ci - 1, p.mb[1] + cj - 1, DIM == 3 ? p.mb[2] + ck - 1 : 0)] =
-        val;
+    w[v] = val;
   }
+  const int pi = p.mb[0] + ci - 1, pj = p.mb[1] + cj - 1, pk = DIM == 3 ? p.mb[2] + ck - 1 : 0;
+  for (int v = 0; v < NV; v++) pool[par.oq + v * par.sq + gofs<DIM>(par.qn, pi, pj, pk)] = w[v];
+  if (push) s_push<Push64<NV>, DIM>(pool + par.oq, par, pi, pj, DIM == 3 ? pk : 1, w, bc, pp);
 }
 
 // the FP64 residual partial sums of k_mx_norm, by one group of 256 threads
@@ -212,6 +291,8 @@ struct SolveRun {
   const int* ppool;   // the image's part pool
   float* sdata;       // this CTA's FP32 data area (shared memory)
   int lg;             // log2 of the units per tile of the FP32 work lists
+  UniBC ubc;
+  const UniDim* dims;  // of the uniform levels (shared memory)
   const GhostOp* sops;  // this CTA's FP32 ghost operations in shared memory, or null
   const GhostOp* gops;  // the same in global memory, from this CTA's segment on
   int rank, ctas;
@@ -236,12 +317,21 @@ struct SolveRun {
   __device__ __forceinline__ void exec(const SolvePhase& f, int t0, int nt, bool cluster,
                                        double (*red)[PL::kNV][kBlock / 32]) const {
     constexpr int nr = PL::kNV;
+    // FP64 work is dealt a warp to each CTA in turn: its instructions take
+    // their SM's FP64 unit 64 cycles each
+    const int d0 = cluster ? (((int)threadIdx.x >> 5) * ctas + rank) * 32 + ((int)threadIdx.x & 31) : t0;
     switch (f.op) {
       case kTRelax:
-        owned(f, cluster, [&](const Blk& b, int u) { u_relax_any<PL, DIM, true>(P, fpool, b, u, f.arg, mp); });
+        if (f.arg & kPushGhosts)
+          owned(f, cluster, [&](const Blk& b, int u) { s_relax_push<PL, DIM>(P, fpool, b, u, f.arg, mp, ubc); });
+        else
+          owned(f, cluster, [&](const Blk& b, int u) { u_relax_any<PL, DIM, true>(P, fpool, b, u, f.arg, mp); });
         break;
       case kTRestrict:
-        owned(f, cluster, [&](const Blk& b, int u) { u_restrict<DIM, true>(P, fpool, b, u, nr); });
+        if (f.arg & kPushGhosts)
+          owned(f, cluster, [&](const Blk& b, int u) { s_restrict_push<nr, DIM>(P, fpool, b, u, ubc); });
+        else
+          owned(f, cluster, [&](const Blk& b, int u) { u_restrict<DIM, true>(P, fpool, b, u, nr); });
         break;
       case kTRing:
         owned(f, cluster, [&](const Blk& b, int u) { u_coarse_ring<DIM, true>(P, fpool, b, u, nr, f.arg); });
@@ -266,7 +356,7 @@ struct SolveRun {
           const int lo = st[2 * (s * ctas + rank)], hi = st[2 * (s * ctas + rank) + 1];
           for (int t = lo + (int)threadIdx.x; t < hi; t += T) {
             const GhostOp g = sops ? sops[t] : gops[t];
-            ghost32_apply<true>(P, fpool, g, nr);
+            ghost32_apply<true, nr>(P, fpool, g, nr);
           }
           if (s + 1 < f.nstages) sync(cluster);
         }
@@ -275,12 +365,19 @@ struct SolveRun {
       case kSGhost64: {
         const int* st = spool + f.stage;
         for (int s = 0; s < f.nstages; s++) {
-          for (int t = st[s] + t0; t < st[s + 1]; t += nt) {
+          for (int t = st[s] + d0; t < st[s + 1]; t += nt) {
             const GhostOp g = f.ops[t];
             s_ghost64<PL::kNV>(P, pool, g, pp);
           }
           if (s + 1 < f.nstages) sync(cluster);
         }
+        break;
+      }
+      case kSUniGhost: {
+        const PatchDev& p = P[f.n];
+        const int N = DIM == 3 ? p.mx[2] : p.mx[1];
+        const uni::Geo g{p.mx[0], p.mx[1], N, 0, N, p.qn[0], p.qn[0] * p.qn[1], (int)p.sq};
+        uni::set_ghost<Push32<nr>, DIM>(fbase<true>(fpool, p) + p.eq, g, dims[f.arg], t0, nt, ubc, 0);
         break;
       }
       case kSClear: {
@@ -295,7 +392,8 @@ struct SolveRun {
       }
       case kSFill64: {
         const Blk* blk = bpool + f.blk;
-        for (int b = t0 >> 8; b < f.n; b += nt >> 8) s_fill64<DIM>(P, pool, blk[b], t0 & 255, nr);
+        for (int b = d0 >> 5; b < f.n; b += nt >> 5)
+          s_fill64<nr, DIM>(P, pool, blk[b], d0 & 31, f.arg & kPushGhosts, ubc, pp);
         break;
       }
       case kSNorm: {
@@ -347,6 +445,8 @@ __global__ void __launch_bounds__(T, 1)
                                reinterpret_cast<const int*>(simg + im.off_part),
                                reinterpret_cast<float*>(solve_smem),
                                im.tile_log2,
+                               im.ubc,
+                               reinterpret_cast<const UniDim*>(simg + im.off_dims),
                                sops,
                                gops,
                                rank,

@@ -39,6 +39,10 @@ enum TailOp : int { kTRelax = 0, kTRestrict = 1, kTRing = 2, kTLoad = 3, kTProlo
 // smoother computes in FP64 (FP32 storage), the coarse solve of the
 // V-cycle at the reference's precision.
 constexpr int kRelax64 = 4;
+// recorded for the one-launch solve: the operation writes the ghost images of
+// the cells of a uniform level that it sets (restriction: of the parent's), and
+// no ghost program follows
+constexpr int kPushGhosts = 16;
 struct TailPhase {
   int op, arg, nblk, nstages;
   const Blk* blk;
@@ -62,6 +66,7 @@ enum SolveOp : int {
   kSGhost64 = 12,  // an FP64 ghost program
   kSNorm = 13,     // FP64 residual of the finest level: rf and n partial sums (padded interior list)
   kSFinish = 14,   // one CTA: the deterministic final sum, the residual record and the exit decision
+  kSUniGhost = 16, // the ghosts of the correction on a uniform level (arg = -level, n = its patch)
   kSSolo = 15      // the next n phases run in CTA 0 alone (barriers of that CTA between them)
 };
 // FP32 operations (0-5, kSClear, kSPrep, kSUpdate) take their work by
@@ -79,6 +84,12 @@ struct SolvePhase {
   const GhostOp* ops;  // a ghost program's operations (global memory)
   long long a, len;    // kSClear: the range of the FP32 pool
 };
+// Uniform levels (kern_uni.cuh).  UniBC: per dimension 0 periodic, 1
+// physical faces (UserBC with the plugin's mask).
+struct UniBC {
+  int phys[3];
+  int mask;
+};
 // The program image every CTA of a solve copies into its shared memory at
 // the start, after a data area of `data` bytes that holds the FP32 arrays
 // of the patches it owns in distributed shared memory: the phases at
@@ -88,11 +99,13 @@ struct SolvePhase {
 // discards what the L1 cache holds.
 struct SolveImage {
   int bytes, data, off_patches, off_blk, off_stage, off_part;
+  int off_dims;   // the UniDim of level -l at index l (uniform levels)
   // the FP32 ghost operations are ordered by CTA: CTA r's are [seg[r],
   // seg[r+1]) of the program's operation array (seg: ctas+1 entries of the
   // part pool at off_seg); when ops_smem, each CTA stages its own after its
   // data area (ops bytes reserved per CTA)
   int seg, ops_smem, ops;
+  UniBC ubc;      // boundary conditions of the uniform levels (kPushGhosts)
   int tile_log2;  // FP32 work lists are split into tiles of 2^tile_log2 units (at most 256)
 };
 constexpr int kSolveSmemMax = 192 * 1024;  // largest image a solve stages
@@ -118,12 +131,6 @@ struct SolveShape {
   int tile;  // units per tile of the FP32 work lists (32, 64, 128 or 256)
 };
 
-// Uniform levels (kern_uni.cuh).  UniBC: per dimension 0 periodic, 1
-// physical faces (UserBC with the plugin's mask).
-struct UniBC {
-  int phys[3];
-  int mask;
-};
 // Division by d as a multiplication by m = ceil(2^32 / d) (0: d = 1)
 struct UniDiv {
   int d;

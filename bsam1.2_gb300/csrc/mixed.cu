@@ -170,6 +170,9 @@ int mx_op(Hier& H, int level, int kind, int op, int arg) {
   return BSAMG_OK;
 }
 
+// a level whose operations write their own ghosts in a recorded solve
+bool rec_push(const Hier& H, int level) { return H.rec_push && level <= 0; }
+
 // the smoothing of one level; on the V-cycle's coarsest level (coarse) in
 // FP64 arithmetic
 int mx_level_relax(Hier& H, int level, int nsmooth, bool coarse) {
@@ -181,8 +184,9 @@ int mx_level_relax(Hier& H, int level, int nsmooth, bool coarse) {
         if (ru) return ru;
         continue;
       }
-      int r = mx_op(H, level, kKindColor, kTRelax, coarse ? rb | kRelax64 : rb);
-      if (!r) r = mx_set_ghost(H, level, rb);
+      const bool push = rec_push(H, level);
+      int r = mx_op(H, level, kKindColor, kTRelax, (coarse ? rb | kRelax64 : rb) | (push ? kPushGhosts : 0));
+      if (!r && !push) r = mx_set_ghost(H, level, rb);
       if (r) return r;
     }
   return BSAMG_OK;
@@ -229,14 +233,16 @@ int mx_vcycle(Hier& H, int level, int minlevel, int nsmooth) {
   int r = mx_level_relax(H, level, nsmooth, level == minlevel);
   if (r) return r;
   if (level > minlevel) {
-    if ((r = mx_op(H, level, kKindCoarse, kTRestrict, 0))) return r;
-    if ((r = mx_set_ghost(H, level - 1, 0))) return r;
+    const bool pp = rec_push(H, level - 1), pl = rec_push(H, level);
+    if ((r = mx_op(H, level, kKindCoarse, kTRestrict, pp ? kPushGhosts : 0))) return r;
+    if (!pp && (r = mx_set_ghost(H, level - 1, 0))) return r;
     if ((r = mx_op(H, level, kKindCGhost, kTRing, 0))) return r;
     if ((r = mx_op(H, level, kKindCoarse, kTLoad, 0))) return r;
     if ((r = mx_vcycle(H, level - 1, minlevel, nsmooth))) return r;
     if ((r = mx_op(H, level, kKindCGhost, kTRing, 1))) return r;
     if ((r = mx_op(H, level, kKindProl, kTProlong, 0))) return r;
-    if ((r = mx_set_ghost(H, level, 0))) return r;
+    if (pl) rec_of(H)->push_back(TailPhase{kSUniGhost, -level, uni_patch(H, level), 0, nullptr, nullptr, nullptr});
+    else if ((r = mx_set_ghost(H, level, 0))) return r;
     if ((r = mx_level_relax(H, level, nsmooth, false))) return r;
   }
   return BSAMG_OK;
@@ -614,6 +620,17 @@ int solve_record(Hier& H, int finest, int minlevel, int nsmooth, int solo, int C
     f.blk = blk_at(blk);
     B.prog.push_back(f);
   };
+  auto push_fill = [&](int arg, const Blk* blk) {  // FillDown in tiles of a warp
+    SolvePhase f = phase(kSFill64, arg, 1);
+    f.blk = (int)B.bpool.size();
+    if (const std::vector<Blk>* v = host_list(blk))
+      for (const Blk& b : *v) {
+        const long long end = std::min<long long>(b.start + kBlock, kind_units(H, H.patches[b.patch], kKindCoarse));
+        for (long long t = b.start; t < end; t += 32) B.bpool.push_back(Blk{b.patch, (int)t});
+      }
+    f.n = (int)B.bpool.size() - f.blk;
+    B.prog.push_back(f);
+  };
   auto push_owned = [&](int op, int arg, int n, const Blk* blk, int bar) {
     SolvePhase f = phase(op, arg, bar);
     f.n = n;
@@ -649,6 +666,8 @@ int solve_record(Hier& H, int finest, int minlevel, int nsmooth, int solo, int C
         f.op = kSGhost64;
         f.ops = t.ops;
         f.stage = stage_at(t.stage_off);
+      } else if (t.op == kSUniGhost) {
+        // its patch in n, -level in arg
       } else if (t.op == kTGhost) {
         f.stage = ghost_at(t.ops);  // f.ops: the operations by CTA, set after their upload
       } else {
@@ -679,7 +698,9 @@ int solve_record(Hier& H, int finest, int minlevel, int nsmooth, int solo, int C
   }
   B.prog.back().bar = 1;
   H.rec_solo = solo;
+  H.rec_push = H.uni;
   int r = record([&] { return mx_vcycle(H, finest, minlevel, nsmooth); }, false);
+  H.rec_push = false;
   H.rec_solo = -kMaxDepth - 2;
   if (r) return r;
   for (int level = finest; level >= 0; level--) {
@@ -696,8 +717,9 @@ int solve_record(Hier& H, int finest, int minlevel, int nsmooth, int solo, int C
       B.prog.push_back(phase(kSSolo, 0, 0));
     }
     LevelT& L = H.L(level);
-    if (L.nblk[kKindCoarse] > 0) push_fp64(kSFill64, 2, L.nblk[kKindCoarse], L.d_blk[kKindCoarse], 1);
-    if ((r = record([&] { return enq_set_ghost(H, level - 1, 0); }, true))) return r;
+    const bool push = H.uni && level <= 0;  // the parent is set whole: its ghosts with it
+    if (L.nblk[kKindCoarse] > 0) push_fill(push ? 2 | kPushGhosts : 2, L.d_blk[kKindCoarse]);
+    if (!push && (r = record([&] { return enq_set_ghost(H, level - 1, 0); }, true))) return r;
   }
   if (solo_at != (size_t)-1) B.prog[solo_at].n = (int)(B.prog.size() - solo_at - 1);
   for (int level = 1; level <= finest; level++)
@@ -773,6 +795,8 @@ int solve_build(Hier& H, int finest, int minlevel, int nsmooth) {
   o = al16(o + sizeof(int) * B.spool.size());
   im.off_part = (int)o;
   o = al16(o + sizeof(int) * (B.ppool.size() + C + 1));  // + the CTAs' operation segments
+  im.off_dims = (int)o;
+  if (H.uni) o = al16(o + sizeof(UniDim) * (1 - H.minlevel));
   im.bytes = (int)o;
   if (o > (size_t)kSolveSmemMax) return no_fit();  // too large to stage
   const long long budget = ((long long)kSolveSmemMax - (long long)o) / 4;
@@ -783,6 +807,13 @@ int solve_build(Hier& H, int finest, int minlevel, int nsmooth) {
     for (int p : H.L(l).patches) add[owner[p]] += floats(p);
     bool fits = true;
     for (int q = 0; q < C; q++) fits = fits && mem[q] + add[q] <= budget;
+    // a level whose patches leave one CTA more than four times its share (the
+    // base level's single patch) stays in the pool, where every CTA works on
+    // it: its sweep on one SM took 6300 cycles of 64^2 cells, its FP64 base
+    // fields 36000, against 2400 and 3300
+    long long most = 0, all = 0;
+    for (int q = 0; q < C; q++) most = std::max(most, add[q]), all += add[q];
+    if (l > solo && most * C > 4 * all) fits = false;
     if (!fits) continue;
     for (int q = 0; q < C; q++) mem[q] += add[q];
     for (int p : H.L(l).patches) dsm[p] = 1;
@@ -841,6 +872,7 @@ int solve_build(Hier& H, int finest, int minlevel, int nsmooth) {
   B.ppool.push_back((int)perm.size());
   im.ops = (int)al16(sizeof(GhostOp) * opmax);
   im.tile_log2 = 0;
+  if (H.uni) im.ubc = H.ubc;
   while ((1 << im.tile_log2) < H.solve_shape.tile) im.tile_log2++;
   im.ops_smem = (size_t)im.data + im.ops + o <= (size_t)kSolveSmemMax ? 1 : 0;
   if (!im.ops_smem) im.ops = 0;
@@ -874,6 +906,11 @@ int solve_build(Hier& H, int finest, int minlevel, int nsmooth) {
   if (!B.bpool.empty()) std::memcpy(img.data() + im.off_blk, B.bpool.data(), sizeof(Blk) * B.bpool.size());
   if (!B.spool.empty()) std::memcpy(img.data() + im.off_stage, B.spool.data(), sizeof(int) * B.spool.size());
   std::memcpy(img.data() + im.off_part, B.ppool.data(), sizeof(int) * B.ppool.size());
+  if (H.uni)
+    for (int l = 0; l >= H.minlevel; l--) {
+      const UniDim ud = uni_dim(H.hP[uni_patch(H, l)].mx);
+      std::memcpy(img.data() + im.off_dims + sizeof(UniDim) * -l, &ud, sizeof(ud));
+    }
   if (H.solve_img) cudaFreeAsync(H.solve_img, H.s);
   H.solve_img = nullptr;
   cudaError_t e = dev_alloc(H, &H.solve_img, img.size());

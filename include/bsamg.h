@@ -337,9 +337,9 @@ int bsamg_get_solve(const bsamg_hier* h, int* mode, int* ctas, int* threads, int
  * at the end of every phase of the program's prologue and first outer
  * iteration; bsamg_solve_trace_read returns, for each of the `count` phases
  * of the last traced solve (up to cap), its operation code (0-5 the FP32
- * V-cycle's relax, restrict, ring, load, prolong, ghost; 8-15 clear, prep,
- * update, FP64 FillDown, FP64 ghost, norm, finish, solo block), its work
- * size (blocks, or ghost stages) and the cycles since the previous phase
+ * V-cycle's relax, restrict, ring, load, prolong, ghost; 8-16 clear, prep,
+ * update, FP64 FillDown, FP64 ghost, norm, finish, solo block, ghosts of a
+ * uniform level), its work size (blocks, or ghost stages; 16: its patch) and the cycles since the previous phase
  * ended (a solo block's time is given on its last phase, 0 on the others). */
 int bsamg_solve_trace(bsamg_hier* h, int enable);
 /* The last one-launch solve program of the hierarchy: info[0] phases,
