@@ -138,7 +138,7 @@ struct Hier {
   double solve_ms[3] = {};    // last solve, host clock: program build, launch to finish, read-back
   int solve_nph = 0, solve_body = 0, solve_nb = 0;
   std::tuple<int, int, int, int, int> solve_key{kMaxDepth + 1, 0, 0, 0, 0};
-  GhostOp* solve_ops = nullptr;  // the program's FP32 ghost operations, each stage in owner order
+  PackedGhost* solve_ops = nullptr;  // the program's FP32 ghost operations, each stage in owner order
   int solve_dsm_levels = 0;      // levels whose FP32 arrays the program keeps in distributed shared memory
   void* solve_ctl = nullptr;
   int solve_ctl_cap = 0;  // residual slots of solve_ctl

@@ -293,8 +293,8 @@ struct SolveRun {
   int lg;             // log2 of the units per tile of the FP32 work lists
   UniBC ubc;
   const UniDim* dims;  // of the uniform levels (shared memory)
-  const GhostOp* sops;  // this CTA's FP32 ghost operations in shared memory, or null
-  const GhostOp* gops;  // the same in global memory, from this CTA's segment on
+  const PackedGhost* sops;  // this CTA's FP32 ghost operations in shared memory, or null
+  const PackedGhost* gops;  // the same in global memory, from this CTA's segment on
   int rank, ctas;
 
   __device__ __forceinline__ void sync(bool cluster) const {
@@ -355,7 +355,7 @@ struct SolveRun {
         for (int s = 0; s < f.nstages; s++) {
           const int lo = st[2 * (s * ctas + rank)], hi = st[2 * (s * ctas + rank) + 1];
           for (int t = lo + (int)threadIdx.x; t < hi; t += T) {
-            const GhostOp g = sops ? sops[t] : gops[t];
+            const GhostOp g = ghost_op(sops ? sops[t] : gops[t]);
             ghost32_apply<true, nr>(P, fpool, g, nr);
           }
           if (s + 1 < f.nstages) sync(cluster);
@@ -423,11 +423,11 @@ __global__ void __launch_bounds__(T, 1)
   __syncthreads();
   const int rank = (int)cluster_rank(), ctas = (int)cluster_ctas();
   const int* seg = reinterpret_cast<const int*>(simg + im.off_part) + im.seg;
-  const GhostOp* gops = ctl->ops + seg[rank];
-  GhostOp* sops = nullptr;
+  const PackedGhost* gops = ctl->ops + seg[rank];
+  PackedGhost* sops = nullptr;
   if (im.ops_smem) {  // this CTA's FP32 ghost operations, as words
-    sops = reinterpret_cast<GhostOp*>(solve_smem + im.data);
-    const int nw = (seg[rank + 1] - seg[rank]) * (int)(sizeof(GhostOp) / 4);
+    sops = reinterpret_cast<PackedGhost*>(solve_smem + im.data);
+    const int nw = (seg[rank + 1] - seg[rank]) * (int)(sizeof(PackedGhost) / 4);
     for (int x = threadIdx.x; x < nw; x += T) reinterpret_cast<int*>(sops)[x] = reinterpret_cast<const int*>(gops)[x];
   }
   // the data areas of the other CTAs are written from the first phase on:

@@ -108,7 +108,35 @@ struct SolveImage {
   UniBC ubc;      // boundary conditions of the uniform levels (kPushGhosts)
   int tile_log2;  // FP32 work lists are split into tiles of 2^tile_log2 units (at most 256)
 };
-constexpr int kSolveSmemMax = 192 * 1024;  // largest image a solve stages
+constexpr int kSolveSmemMax = 222 * 1024;  // shared memory of a CTA: data area, image, ghost operations
+// An FP32 ghost operation of a solve in seven words (GhostOp takes eleven):
+// an adaptive level's operations then fit beside the data area and the image,
+// where each cost a trip to the L2 cache in every ghost stage.  The cells an
+// interpolation reads lie within two rows (planes) of the first; the patches
+// are 16-bit indices (solve_build checks both).
+struct PackedGhost {
+  unsigned type_mask;  // type | mask << 3
+  unsigned short dp, sp;
+  int dcell, s0, c0;
+  short s1, c1, c2, c3;  // relative to s0 and c0
+};
+__host__ __device__ inline PackedGhost solve_op(const GhostOp& g) {
+  PackedGhost o;
+  o.type_mask = (unsigned)g.type | (unsigned)g.mask << 3;
+  o.dp = (unsigned short)g.dp, o.sp = (unsigned short)g.sp;
+  o.dcell = g.dcell, o.s0 = g.s0, o.c0 = g.c0;
+  o.s1 = (short)(g.s1 - g.s0);
+  o.c1 = (short)(g.c1 - g.c0), o.c2 = (short)(g.c2 - g.c0), o.c3 = (short)(g.c3 - g.c0);
+  return o;
+}
+__host__ __device__ inline GhostOp ghost_op(const PackedGhost& o) {
+  GhostOp g;
+  g.type = (int)(o.type_mask & 7u), g.mask = (int)(o.type_mask >> 3);
+  g.dp = o.dp, g.sp = o.sp;
+  g.dcell = o.dcell, g.s0 = o.s0, g.s1 = o.s0 + o.s1;
+  g.c0 = o.c0, g.c1 = o.c0 + o.c1, g.c2 = o.c0 + o.c2, g.c3 = o.c0 + o.c3;
+  return g;
+}
 // Control block of a solve launch (device memory); the residual of V-cycle
 // it (1-based) follows it at res[it-1].
 struct SolveCtl {
@@ -119,7 +147,7 @@ struct SolveCtl {
   // results
   int ncycles, converged, nonfinite, stop;
   double norm[2];     // the last norm and its raw sum
-  const GhostOp* ops;  // the program's FP32 ghost operations, CTA after CTA
+  const PackedGhost* ops;  // the program's FP32 ghost operations, CTA after CTA
   // when set: CTA 0's clock at the end of every phase of the prologue and
   // the first outer iteration (trace[x], cycles of the SM it runs on), and
   // at the start (trace[nph])

@@ -92,11 +92,11 @@ __global__ void __launch_bounds__(kBlock) k_ghost32_program(const PatchDev* __re
 // operation (ref & 0xfffff) of program (ref >> 20)
 __global__ void __launch_bounds__(kBlock) k_gather_ops(const GhostOp* const* __restrict__ base,
                                                        const unsigned* __restrict__ ref, int n,
-                                                       GhostOp* __restrict__ out) {
+                                                       PackedGhost* __restrict__ out) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   unsigned r = ref[i];
-  out[i] = base[r >> 20][r & 0xfffffu];
+  out[i] = solve_op(base[r >> 20][r & 0xfffffu]);
 }
 
 // ---------------------------------------------------------------------------
@@ -669,7 +669,7 @@ int solve_record(Hier& H, int finest, int minlevel, int nsmooth, int solo, int C
       } else if (t.op == kSUniGhost) {
         // its patch in n, -level in arg
       } else if (t.op == kTGhost) {
-        f.stage = ghost_at(t.ops);  // f.ops: the operations by CTA, set after their upload
+        f.stage = ghost_at(t.ops);
       } else {
         auto pr = part_at(t.blk);
         f.blk = pr.first;
@@ -775,13 +775,27 @@ int solve_build(Hier& H, int finest, int minlevel, int nsmooth) {
   // image), then record the final program
   std::vector<char> dsm(np, 0);
   SolveBuild B;
-  int r = solve_record(H, finest, minlevel, nsmooth, solo, C, owner, dsm, true, B);
   auto no_fit = [&] {  // the per-launch path runs this hierarchy
     solve_invalidate(H);
     H.solve_key = key;
     H.solve_nofit = true;
     return BSAMG_ERR_UNSUPPORTED;
   };
+  // the ghost operations' 16-bit fields (PackedGhost): by the patches' strides, or
+  // operation by operation where those are long
+  bool near = np <= 65535, strides = true;
+  for (const HostPatch& P : H.patches)
+    strides = strides && 2 * ((long long)P.qn[0] * (H.ndims == 3 ? P.qn[1] + 1 : 1) + 1) <= 32767;
+  if (near && !strides)
+    for (int l = minlevel; l <= finest; l++)
+      for (const GhostProg& g : H.L(l).gp)
+        for (const GhostOp& o : g.ops) {
+          const GhostOp u = ghost_op(solve_op(o));
+          near = near && (o.type < kGCfA || (u.s1 == o.s1 && (o.type < kGCfAB || (u.c1 == o.c1 && u.c2 == o.c2)) &&
+                                             (o.type < kGCfAC || u.c3 == o.c3)));
+        }
+  if (!near) return no_fit();
+  int r = solve_record(H, finest, minlevel, nsmooth, solo, C, owner, dsm, true, B);
   if (r == BSAMG_ERR_UNSUPPORTED) return no_fit();
   if (r) return r;
   auto al16 = [](size_t x) { return (x + 15) & ~(size_t)15; };
@@ -870,7 +884,7 @@ int solve_build(Hier& H, int finest, int minlevel, int nsmooth) {
     opmax = std::max(opmax, B.ops[q].size());
   }
   B.ppool.push_back((int)perm.size());
-  im.ops = (int)al16(sizeof(GhostOp) * opmax);
+  im.ops = (int)al16(sizeof(PackedGhost) * opmax);
   im.tile_log2 = 0;
   if (H.uni) im.ubc = H.ubc;
   while ((1 << im.tile_log2) < H.solve_shape.tile) im.tile_log2++;
@@ -881,7 +895,7 @@ int solve_build(Hier& H, int finest, int minlevel, int nsmooth) {
   if (!perm.empty()) {  // gathered on the device from the programs' own arrays
     size_t nperm = perm.size(), np8 = B.progs.size();
     void* tmp = nullptr;
-    cudaError_t e = dev_alloc(H, (void**)&H.solve_ops, sizeof(GhostOp) * nperm);
+    cudaError_t e = dev_alloc(H, (void**)&H.solve_ops, sizeof(PackedGhost) * nperm);
     // the programs' base pointers first (8-byte aligned), then the references
     if (e == cudaSuccess) e = dev_alloc(H, &tmp, sizeof(void*) * np8 + sizeof(unsigned) * nperm);
     const GhostOp** dbase = static_cast<const GhostOp**>(tmp);
@@ -898,8 +912,6 @@ int solve_build(Hier& H, int finest, int minlevel, int nsmooth) {
     if (tmp) cudaFreeAsync(tmp, H.s);
     if (e != cudaSuccess) return cuda_fail(e, "solve ghost operations");
   }
-  for (SolvePhase& f : B.prog)
-    if (f.op == kTGhost) f.ops = H.solve_ops;
   std::vector<unsigned char> img(o, 0);
   std::memcpy(img.data(), B.prog.data(), sizeof(SolvePhase) * B.prog.size());
   std::memcpy(img.data() + im.off_patches, table.data(), sizeof(PatchDev) * table.size());
