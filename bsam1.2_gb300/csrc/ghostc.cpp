@@ -14,11 +14,18 @@
 // them, and groups the rest into stages such that no two operations of a
 // stage touch the same cell in a conflicting way.  Executing the stages in
 // order on the device gives exactly the state the sequential sequence gives.
+//
+// Operations conflict only where they touch cells that some operation writes:
+// ghost cells, which only operations of their own patch read -- unless the
+// interiors of two patches of the level overlap.  So the sequence is emitted
+// and analysed a patch at a time, on all host threads and in arrays the size of
+// a patch; the general analysis of the whole level (stage_ops) remains for
+// overlapping patches.  124 patches of 101 cells, three passes: 0.72 -> 0.2 ms.
 #include <algorithm>
+#include <atomic>
 #include <cstdint>
 #include <iterator>
 #include <memory>
-#include <unordered_map>
 
 #include "hier.h"
 
@@ -359,50 +366,35 @@ struct Emitter {
   // only).  Ghost cells of g1 that lie in the interior of g2 (shifted by
   // off) take g2's values, then the converse.
   void ghost_overlap(int g1, int g2, const int* off) {
-    const HostPatch& A = H.patches[g1];
-    const HostPatch& B = H.patches[g2];
-    int nd = H.ndims, mbc = H.mbc;
-    int mg1[3][2], mg2[3][2], ovg[3][2], ovg1[3][2], ovg2[3][2];
-    for (int n = 0; n < 3; n++)
-      for (int s = 0; s < 2; s++) mg1[n][s] = mg2[n][s] = ovg[n][s] = ovg1[n][s] = ovg2[n][s] = 1;
+    overlap_onto(g1, g2, nullptr, off);
+    overlap_onto(g2, g1, off, nullptr);
+  }
+  // one direction of it: the cells of dst (shifted by offd) in the interior
+  // of src (shifted by offs).  False when the two interiors meet: dst's own
+  // cells are then written too.
+  bool overlap_onto(int dst, int src, const int* offd, const int* offs) {
+    const HostPatch& D = H.patches[dst];
+    const HostPatch& S = H.patches[src];
+    const int nd = H.ndims, mbc = H.mbc;
+    int lo[3] = {1, 1, 1}, ls[3] = {1, 1, 1}, ext[3] = {0, 0, 0};
+    bool meet = true;
     for (int n = 0; n < nd; n++) {
-      mg1[n][0] = A.mglobal[n][0];
-      mg1[n][1] = A.mglobal[n][1];
-      mg2[n][0] = B.mglobal[n][0] + (off ? off[n] : 0);
-      mg2[n][1] = B.mglobal[n][1] + (off ? off[n] : 0);
+      const int od = offd ? offd[n] : 0, os = offs ? offs[n] : 0;
+      const int d0 = D.mglobal[n][0] + od, d1 = D.mglobal[n][1] + od;
+      const int s0 = S.mglobal[n][0] + os, s1 = S.mglobal[n][1] + os;
+      const int v0 = std::max(d0 - mbc, s0), v1 = std::min(d1 + mbc, s1);
+      if (v1 < v0) return true;
+      meet = meet && std::max(d0, s0) <= std::min(d1, s1);
+      lo[n] = v0 - d0 + 1;
+      ls[n] = v0 - s0 + 1;
+      ext[n] = v1 - v0;
     }
-    for (int n = 0; n < nd; n++) {
-      ovg[n][0] = std::max(mg1[n][0] - mbc, mg2[n][0] - mbc);
-      ovg[n][1] = std::min(mg1[n][1] + mbc, mg2[n][1] + mbc);
-    }
-    for (int n = 0; n < nd; n++)
-      if (ovg[n][1] - ovg[n][0] < 0) return;
-    for (int n = 0; n < nd; n++) {
-      ovg1[n][0] = std::max(ovg[n][0], mg2[n][0]);
-      ovg1[n][1] = std::min(ovg[n][1], mg2[n][1]);
-      ovg2[n][0] = std::max(ovg[n][0], mg1[n][0]);
-      ovg2[n][1] = std::min(ovg[n][1], mg1[n][1]);
-    }
-    auto xfer = [&](int dst, int src, int ov[3][2], int mgd[3][2], int mgs[3][2]) {
-      int lo[3], ls[3], ext[3];
-      for (int n = 0; n < 3; n++) {
-        if (n < nd) {
-          lo[n] = ov[n][0] - mgd[n][0] + 1;
-          ls[n] = ov[n][0] - mgs[n][0] + 1;
-          ext[n] = ov[n][1] - ov[n][0];
-        } else {
-          lo[n] = ls[n] = 1;
-          ext[n] = 0;
-        }
-      }
-      for (int k = 0; k <= ext[2]; k++)
-        for (int j = 0; j <= ext[1]; j++)
-          for (int i = 0; i <= ext[0]; i++)
-            copy(kGCopy, dst, cell(dst, lo[0] + i, lo[1] + j, nd == 3 ? lo[2] + k : 0), src,
-                 cell(src, ls[0] + i, ls[1] + j, nd == 3 ? ls[2] + k : 0));
-    };
-    xfer(g1, g2, ovg1, mg1, mg2);
-    xfer(g2, g1, ovg2, mg2, mg1);
+    for (int k = 0; k <= ext[2]; k++)
+      for (int j = 0; j <= ext[1]; j++)
+        for (int i = 0; i <= ext[0]; i++)
+          copy(kGCopy, dst, cell(dst, lo[0] + i, lo[1] + j, nd == 3 ? lo[2] + k : 0), src,
+               cell(src, ls[0] + i, ls[1] + j, nd == 3 ? ls[2] + k : 0));
+    return !meet;
   }
 
   // SelfPeriodicBC, boundary.f90:480-577
@@ -575,6 +567,44 @@ struct LevelEmit {
   }
 };
 
+// The operations of the sequence that write patch ps[a], in its order (a pair
+// (x, y) of patches, x before y, is met in the order of x, then y), with the
+// interpolation of each pass of `passes` at the front: heads[i] for pass
+// passes[i], the rest in `tail`.  False when another patch's interior meets
+// this one's: its operations then touch cells that other patches' read.
+// Otherwise the operations read this patch, interiors of the level's other
+// patches and the parents -- cells that only this patch's operations write, or
+// none -- so that the sequence may be analysed and executed a patch at a time.
+bool emit_patch(const LevelEmit& L, int a, const int* passes, int npasses, std::vector<Em>* heads,
+                std::vector<Em>& tail) {
+  const Hier& H = L.H;
+  const int n = L.n, p = L.ps[a];
+  bool alone = true;
+  Emitter E(H, L.org);
+  for (int i = 0; i < npasses && L.level > 0; i++) {
+    E.out.swap(heads[i]);
+    if (H.ndims == 2) E.interpolate2d(p, passes[i]);
+    else E.interpolate3d(p, passes[i]);
+    E.out.swap(heads[i]);
+  }
+  E.out.swap(tail);
+  if (L.level > 0)
+    for (int b = 0; b < n; b++)
+      if (b != a) alone = E.overlap_onto(p, L.ps[b], nullptr, nullptr) && alone;
+  if (H.periodic) E.self_periodic(p);
+  if (H.periodic && L.level > 0 && L.edge[a])
+    for (int b = 0; b < n; b++)
+      if (b != a && L.edge[b])
+        for (int pol = -1; pol <= 1; pol += 2)
+          for (int o = 0; o < H.nperoff; o++) {  // the offset moves the later patch of the pair
+            const int off[3] = {pol * L.poff[o][0], pol * L.poff[o][1], pol * L.poff[o][2]};
+            alone = E.overlap_onto(p, L.ps[b], b < a ? off : nullptr, b < a ? nullptr : off) && alone;
+          }
+  E.physical_bc(p);
+  E.out.swap(tail);
+  return alone;
+}
+
 std::vector<Em> concat(std::vector<std::vector<Em>>& parts) {
   size_t m = 0;
   for (auto& v : parts) m += v.size();
@@ -595,15 +625,28 @@ std::vector<Em> emit_set_ghost(const Hier& H, int level, int ipass) {
   return concat(parts);
 }
 
+constexpr int kTypes = kGCfAC + 1;
+
 // Dead writes and stages of one emitted sequence (see the file comment).
 std::vector<GhostOp> stage_ops(const Hier& H, std::vector<Em>& ops, std::vector<int>& stage_off);
 
 }  // namespace
 
-std::vector<GhostOp> set_ghost_sequence(const Hier& H, int level, int ipass) {
+std::vector<std::vector<GhostOp>> set_ghost_sequences(const Hier& H, int level, int ipass) {
+  LevelEmit L(H, level, ipass);
+  std::vector<std::vector<GhostOp>> res(L.n);
+  std::atomic<bool> alone{true};
+  parallel_for(L.n, [&](int a) {
+    std::vector<Em> head, tail;
+    if (!emit_patch(L, a, &ipass, 1, &head, tail)) alone = false;
+    res[a].reserve(head.size() + tail.size());
+    for (const std::vector<Em>* v : {&head, &tail})
+      for (const Em& e : *v) res[a].push_back(e.op);
+  });
+  if (alone) return res;
   std::vector<Em> em = emit_set_ghost(H, level, ipass);
-  std::vector<GhostOp> res(em.size());
-  for (size_t x = 0; x < em.size(); x++) res[x] = em[x].op;
+  res.assign(1, std::vector<GhostOp>(em.size()));
+  for (size_t x = 0; x < em.size(); x++) res[0][x] = em[x].op;
   return res;
 }
 
@@ -612,25 +655,146 @@ std::vector<GhostOp> compile_set_ghost(const Hier& H, int level, int ipass, std:
   return stage_ops(H, em, stage_off);
 }
 
+namespace {
+
+// The live operations of one patch, by (stage, type) in emission order:
+// run[s * kTypes + t] is the first of stage s, type t.
+struct PatchProg {
+  std::vector<GhostOp> ops;
+  std::vector<int> run;
+};
+// stage_ops of the operations that write one patch, which only conflict among
+// themselves (emit_patch); three arrays over its cells, kept between calls
+void stage_patch(const HostPatch& P, int p, const std::vector<Em>& head, const std::vector<Em>& tail, PatchProg& out) {
+  const int cells = P.qn[0] * P.qn[1] * P.qn[2], nh = (int)head.size(), m = nh + (int)tail.size();
+  thread_local std::vector<int> last, wst, rst, stage;
+  thread_local std::vector<char> dead, readf;
+  last.assign(cells, -1);
+  wst.assign(cells, -1);
+  rst.assign(cells, -1);
+  stage.assign(m, -1);
+  dead.assign(m, 0);
+  readf.assign(m, 0);
+  auto op = [&](int x) -> const Em& { return x < nh ? head[x] : tail[x - nh]; };
+  auto own = [&](int64_t key) { return (int)(key >> 32) == p; };
+  for (int x = 0; x < m; x++) {  // drop writes overwritten before any read
+    const Em& e = op(x);
+    for (int s = 0; s < e.nsrc; s++)
+      if (own(e.src[s])) {
+        const int w = last[(uint32_t)e.src[s]];
+        if (w >= 0) readf[w] = 1;
+      }
+    int& l = last[(uint32_t)e.dst];
+    if (l >= 0 && !readf[l]) dead[l] = 1;
+    l = x;
+  }
+  int nst = 0;
+  for (int x = 0; x < m; x++) {  // stage = 1 + latest conflicting live predecessor
+    if (dead[x]) continue;
+    const Em& e = op(x);
+    int st = 0;
+    for (int s = 0; s < e.nsrc; s++)
+      if (own(e.src[s])) st = std::max(st, wst[(uint32_t)e.src[s]] + 1);
+    const uint32_t d = (uint32_t)e.dst;
+    st = std::max(st, std::max(rst[d], wst[d]) + 1);
+    stage[x] = st;
+    for (int s = 0; s < e.nsrc; s++)
+      if (own(e.src[s])) {
+        int& r = rst[(uint32_t)e.src[s]];
+        r = std::max(r, st);
+      }
+    wst[d] = st;
+    rst[d] = -1;
+    nst = std::max(nst, st + 1);
+  }
+  out.run.assign(nst * kTypes + 1, 0);
+  for (int x = 0; x < m; x++)
+    if (!dead[x]) out.run[stage[x] * kTypes + op(x).op.type + 1]++;
+  for (int s = 0; s < nst * kTypes; s++) out.run[s + 1] += out.run[s];
+  out.ops.resize(out.run.back());
+  std::vector<int> fill(out.run.begin(), out.run.end() - 1);
+  for (int x = 0; x < m; x++)
+    if (!dead[x]) out.ops[fill[stage[x] * kTypes + op(x).op.type]++] = op(x).op;
+}
+
+}  // namespace
+
 void compile_set_ghost_all(const Hier& H, const std::vector<std::pair<int, int>>& jobs,
                            std::vector<std::vector<GhostOp>*> out, std::vector<std::vector<int>*> stage_off) {
-  // every item of every job in one parallel pass, then the jobs' staging
-  std::vector<std::unique_ptr<LevelEmit>> le;
-  std::vector<int> first(jobs.size() + 1, 0);
+  // a patch at a time in one parallel pass: each patch's operations for every
+  // pass of its level, whose overlaps and boundary copies they share
+  struct Level {
+    std::unique_ptr<LevelEmit> L;
+    std::vector<int> job, pass;
+    std::vector<PatchProg> prog;  // [pass * n + patch]
+    std::atomic<bool> alone{true};
+    int first = 0;
+  };
+  std::vector<std::unique_ptr<Level>> lev;
   for (size_t j = 0; j < jobs.size(); j++) {
-    le.emplace_back(new LevelEmit(H, jobs[j].first, jobs[j].second));
-    first[j + 1] = first[j] + le.back()->items();
+    Level* g = nullptr;
+    for (auto& l : lev)
+      if (l->L->level == jobs[j].first) g = l.get();
+    if (!g) {
+      lev.emplace_back(new Level);
+      g = lev.back().get();
+      g->L.reset(new LevelEmit(H, jobs[j].first, jobs[j].second));
+    }
+    g->job.push_back((int)j);
+    g->pass.push_back(jobs[j].second);
   }
-  std::vector<std::vector<Em>> parts(first.back());
-  parallel_for(first.back(), [&](int x) {
-    size_t j = std::upper_bound(first.begin(), first.end(), x) - first.begin() - 1;
-    le[j]->item(x - first[j], parts[x]);
+  int items = 0;
+  for (auto& g : lev) {
+    g->first = items;
+    items += g->L->n;
+    g->prog.resize(g->pass.size() * g->L->n);
+  }
+  parallel_for(items, [&](int x) {
+    size_t l = lev.size() - 1;
+    while (lev[l]->first > x) l--;
+    Level& g = *lev[l];
+    const int a = x - g.first, np = (int)g.pass.size();
+    thread_local std::vector<Em> tail, heads[3];
+    tail.clear();
+    for (auto& h : heads) h.clear();
+    if (!emit_patch(*g.L, a, g.pass.data(), np, heads, tail)) {
+      g.alone = false;
+      return;
+    }
+    for (int i = 0; i < np; i++)
+      stage_patch(H.patches[g.L->ps[a]], g.L->ps[a], heads[i], tail, g.prog[i * g.L->n + a]);
   });
-  parallel_for((int)jobs.size(), [&](int j) {
-    std::vector<std::vector<Em>> mine(std::make_move_iterator(parts.begin() + first[j]),
-                                      std::make_move_iterator(parts.begin() + first[j + 1]));
-    std::vector<Em> em = concat(mine);
-    *out[j] = stage_ops(H, em, *stage_off[j]);
+  // a program: its patches' operations by (stage, type), then patch
+  std::vector<std::pair<Level*, int>> progs;
+  for (auto& g : lev)
+    for (size_t i = 0; i < g->pass.size(); i++) progs.emplace_back(g.get(), (int)i);
+  parallel_for((int)progs.size(), [&](int x) {
+    Level& g = *progs[x].first;
+    const int i = progs[x].second, j = g.job[i], n = g.L->n;
+    if (!g.alone) {
+      *out[j] = compile_set_ghost(H, g.L->level, g.pass[i], *stage_off[j]);
+      return;
+    }
+    int nst = 0;
+    size_t total = 0;
+    for (int a = 0; a < n; a++) {
+      const PatchProg& q = g.prog[i * n + a];
+      nst = std::max(nst, (int)(q.run.size() - 1) / kTypes);
+      total += q.ops.size();
+    }
+    std::vector<int>& so = *stage_off[j];
+    std::vector<GhostOp>& res = *out[j];
+    so.assign(nst + 1, 0);
+    res.clear();
+    res.reserve(total);
+    for (int s = 0; s < nst; s++) {
+      for (int t = s * kTypes; t < (s + 1) * kTypes; t++)
+        for (int a = 0; a < n; a++) {
+          const PatchProg& q = g.prog[i * n + a];
+          if (t + 1 < (int)q.run.size()) res.insert(res.end(), q.ops.begin() + q.run[t], q.ops.begin() + q.run[t + 1]);
+        }
+      so[s + 1] = (int)res.size();
+    }
   });
 }
 
@@ -695,7 +859,6 @@ std::vector<GhostOp> stage_ops(const Hier& H, std::vector<Em>& ops, std::vector<
   // within a stage by type, in the order they came: a warp whose lanes run
   // different types runs each in turn, its loads' latencies and (FP64) the
   // unit's 64 cycles an instruction included
-  constexpr int kTypes = kGCfAC + 1;
   std::vector<GhostOp> res;
   std::vector<int> fill(nst * kTypes + 1, 0);
   for (int x = 0; x < m; x++)

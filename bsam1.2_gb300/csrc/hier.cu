@@ -653,21 +653,14 @@ long long kind_units(const Hier& H, const HostPatch& P, int kind) {
 
 namespace {
 
-int upload_blocks(Hier& H, LevelT& L, int kind) {
-  std::vector<Blk> v;
+void add_blocks(Hier& H, LevelT& L, int kind, TableUpload& up) {
+  std::vector<Blk>& v = L.h_blk[kind];
   for (int p : L.patches) {
     long long units = kind_units(H, H.patches[p], kind);
     for (long long s = 0; s < units; s += kBlock) v.push_back(Blk{p, (int)s});
   }
   L.nblk[kind] = (int)v.size();
-  if (v.empty()) return BSAMG_OK;
-  CK(dev_alloc(H, (void**)&L.d_blk[kind], sizeof(Blk) * v.size()));
-  H.bytes += sizeof(Blk) * v.size();
-  // a copy from pageable memory returns once the source has been staged, so
-  // v may be freed on return
-  CK(cudaMemcpyAsync(L.d_blk[kind], v.data(), sizeof(Blk) * v.size(), cudaMemcpyHostToDevice, H.s));
-  L.h_blk[kind] = std::move(v);
-  return BSAMG_OK;
+  up.add(&L.d_blk[kind], v);
 }
 
 // every cell an operation touches must lie inside its patch's ghosted
@@ -696,15 +689,27 @@ bool ghost_ops_in_bounds(const Hier& H, const GhostProg& g) {
   return true;
 }
 
-int upload_ghost(Hier& H, GhostProg& g) {
-  if (g.ops.empty()) return BSAMG_OK;
-  if (!ghost_ops_in_bounds(H, g)) return BSAMG_ERR_ARG;
-  CK(dev_alloc(H, (void**)&g.d_ops, sizeof(GhostOp) * g.ops.size()));
-  CK(dev_alloc(H, (void**)&g.d_stage_off, sizeof(int) * g.stage_off.size()));
-  H.bytes += sizeof(GhostOp) * g.ops.size() + sizeof(int) * g.stage_off.size();
-  CK(cudaMemcpyAsync(g.d_ops, g.ops.data(), sizeof(GhostOp) * g.ops.size(), cudaMemcpyHostToDevice, H.s));
-  CK(cudaMemcpyAsync(g.d_stage_off, g.stage_off.data(), sizeof(int) * g.stage_off.size(), cudaMemcpyHostToDevice,
-                     H.s));
+int upload_tables(Hier& H, const TableUpload& up) {
+  auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
+  size_t small = 0, total = 0;
+  for (const auto& p : up.pieces) (p.bytes < TableUpload::kDirect ? small : total) += al(p.bytes);
+  total += small;
+  if (!total) return BSAMG_OK;
+  CK(dev_alloc(H, &H.tables, total));
+  H.bytes += total;
+  std::vector<unsigned char> image(small);
+  unsigned char* const base = static_cast<unsigned char*>(H.tables);
+  size_t at = 0, far = small;
+  for (const auto& p : up.pieces) {
+    const bool direct = p.bytes >= TableUpload::kDirect;
+    size_t& o = direct ? far : at;
+    *p.slot = base + o;
+    // a copy from pageable memory returns once the source has been staged
+    if (direct) CK(cudaMemcpyAsync(base + o, p.data, p.bytes, cudaMemcpyHostToDevice, H.s));
+    else std::memcpy(image.data() + o, p.data, p.bytes);
+    o += al(p.bytes);
+  }
+  if (small) CK(cudaMemcpyAsync(base, image.data(), small, cudaMemcpyHostToDevice, H.s));
   return BSAMG_OK;
 }
 
@@ -815,9 +820,10 @@ int commit(Hier& H) {
   H.hP = std::move(pd);
 
   int maxblk = 1;
+  TableUpload up;
   for (int l = H.minlevel; l <= H.maxlevel; l++) {
     LevelT& L = H.L(l);
-    for (int k = 0; k < kNKind; k++) RET(upload_blocks(H, L, k));
+    for (int k = 0; k < kNKind; k++) add_blocks(H, L, k, up);
     maxblk = std::max(maxblk, L.nblk[kKindInterior]);
     L.count = 0.0;
     for (int p : L.patches) {
@@ -840,21 +846,26 @@ int commit(Hier& H) {
     compile_set_ghost_all(H, jobs, out, so);
   }
   H.regrid_ms[4] = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - tg0).count();
-  for (int l = H.minlevel; l <= H.maxlevel; l++) {
-    LevelT& L = H.L(l);
-    for (int ip = 0; ip < 3; ip++) {
-      // below and at the root the program does not depend on the colour
-      if (l <= 0 && ip > 0) {
-        L.gp[ip].ops = L.gp[0].ops;
-        L.gp[ip].stage_off = L.gp[0].stage_off;
-        L.gp[ip].d_ops = L.gp[0].d_ops;
-        L.gp[ip].d_stage_off = L.gp[0].d_stage_off;
-        continue;
+  {
+    std::vector<GhostProg*> gs;
+    for (int l = H.minlevel; l <= H.maxlevel; l++)
+      for (int ip = 0; ip < (l <= 0 ? 1 : 3); ip++) gs.push_back(&H.L(l).gp[ip]);
+    std::atomic<bool> bad{false};
+    parallel_for((int)gs.size(), [&](int x) {
+      if (!ghost_ops_in_bounds(H, *gs[x])) bad = true;
+    });
+    if (bad) return BSAMG_ERR_ARG;
+    for (GhostProg* g : gs)
+      if (!g->ops.empty()) {
+        up.add(&g->d_ops, g->ops);
+        up.add(&g->d_stage_off, g->stage_off);
       }
-      RET(upload_ghost(H, L.gp[ip]));
-    }
   }
-  RET(mixed_tables(H));
+  mixed_tables(H, up);
+  RET(upload_tables(H, up));
+  // below and at the root the program does not depend on the colour
+  for (int l = H.minlevel; l <= std::min(0, H.maxlevel); l++)
+    for (int ip = 1; ip < 3; ip++) H.L(l).gp[ip] = H.L(l).gp[0];
   set_tail(H, H.tail_cells);
   maxblk = std::max(maxblk, (int)H.b_partials);
   H.partial_cap = maxblk;
@@ -879,18 +890,7 @@ void release(Hier& H) {
     for (auto& kv : *gm)
       if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
   H.graphs.clear();
-  for (int l = 0; l < kNLev; l++) {
-    LevelT& L = H.lev[l];
-    for (int k = 0; k < kNKind; k++)
-      if (L.d_blk[k]) cudaFreeAsync(L.d_blk[k], H.s);
-    for (int ip = 0; ip < 3; ip++) {
-      bool shared = ip > 0 && L.gp[ip].d_ops == L.gp[0].d_ops;
-      if (!shared) {
-        if (L.gp[ip].d_ops) cudaFreeAsync(L.gp[ip].d_ops, H.s);
-        if (L.gp[ip].d_stage_off) cudaFreeAsync(L.gp[ip].d_stage_off, H.s);
-      }
-    }
-  }
+  if (H.tables) cudaFreeAsync(H.tables, H.s);
   mixed_free(H);
   for (auto& kv : H.fp_tail_progs) free_tail(H, kv.second);
   H.fp_tail_progs.clear();

@@ -4,6 +4,7 @@
 
 #include <atomic>
 #include <functional>
+#include <cstring>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -52,13 +53,32 @@ struct Hier;
 void parallel_for(int n, const std::function<void(int)>& f);
 // Inputs of the ghost compiler.
 std::vector<GhostOp> compile_set_ghost(const Hier& H, int level, int ipass, std::vector<int>& stage_off);
-// the programs of several (level, ipass) jobs at once, every emission item
-// of every job on the thread pool
+// the programs of several (level, ipass) jobs at once (at most three passes a
+// level), a patch at a time on the thread pool
 void compile_set_ghost_all(const Hier& H, const std::vector<std::pair<int, int>>& jobs,
                            std::vector<std::vector<GhostOp>*> out, std::vector<std::vector<int>*> stage_off);
-// the same writes unprocessed, in the reference's order (for sequential
-// execution on the host)
-std::vector<GhostOp> set_ghost_sequence(const Hier& H, int level, int ipass);
+// the same writes unprocessed, for execution on the host: sequences that may
+// run side by side, each in the reference's order (one a patch; a single one
+// where patches of the level overlap)
+std::vector<std::vector<GhostOp>> set_ghost_sequences(const Hier& H, int level, int ipass);
+
+// The read-only tables of a commit (work lists, ghost programs) as one
+// allocation: an adaptive hierarchy has some eighty.  Small ones are gathered
+// and copied together, large ones copied from their vector, which stays in
+// place until upload_tables.
+struct TableUpload {
+  static constexpr size_t kDirect = 64 * 1024;
+  struct Piece {
+    void** slot;  // where the table's device address goes
+    const void* data;
+    size_t bytes;
+  };
+  std::vector<Piece> pieces;
+  template <typename T>
+  void add(T** slot, const std::vector<T>& v) {
+    if (!v.empty()) pieces.push_back(Piece{reinterpret_cast<void**>(slot), v.data(), sizeof(T) * v.size()});
+  }
+};
 
 struct Hier {
   bsamg_ctx* ctx = nullptr;
@@ -83,6 +103,7 @@ struct Hier {
   size_t fpool_elems = 0;
   size_t e_len = 0;  // leading FP32 elements holding every patch's correction e
   size_t e_coarse_off = 0, e_coarse_len = 0;  // the part of it on levels < 0
+  void* tables = nullptr;                     // every work list and ghost program of the commit
   Blk* mx_norm_blk[kNLev] = {};               // padded interior lists (mixed norm)
   Blk* mx_prep_coarse = nullptr;              // interior lists of all levels < 0
   int mx_prep_coarse_n = 0;

@@ -1075,8 +1075,6 @@ void mixed_free(Hier& H) {
   H.box_loop = nullptr;
   if (H.box_ctl) cudaFreeAsync(H.box_ctl, H.s);
   H.box_ctl = nullptr;
-  if (H.mx_prep_coarse) cudaFreeAsync(H.mx_prep_coarse, H.s);
-  H.mx_prep_coarse = nullptr;
   for (auto& kv : H.mx_tail_progs) free_tail(H, kv.second);
   H.mx_tail_progs.clear();
   for (void** p : {&H.solve_img, &H.solve_ctl, (void**)&H.solve_trace, (void**)&H.solve_ops}) {
@@ -1084,51 +1082,28 @@ void mixed_free(Hier& H) {
     *p = nullptr;
   }
   H.solve_ctl_cap = 0;
-  for (int l = 0; l < kNLev; l++) {
-    if (H.mx_norm_blk[l]) cudaFreeAsync(H.mx_norm_blk[l], H.s);
-    H.mx_norm_blk[l] = nullptr;
-  }
 }
 
-int mixed_tables(Hier& H) {
-  if (!has_mixed(H) || !H.fpool || H.box) return BSAMG_OK;
+void mixed_tables(Hier& H, TableUpload& up) {
+  if (!has_mixed(H) || !H.fpool || H.box) return;
+  auto interior = [&](int l, std::vector<Blk>& v) {
+    for (int p : H.L(l).patches) {
+      const HostPatch& P = H.patches[p];
+      long long units = (long long)P.mx[0] * P.mx[1] * P.mx[2];
+      for (long long s = 0; s < units; s += kBlock) v.push_back(Blk{p, (int)s});
+    }
+  };
   for (int l = H.minlevel; l <= H.maxlevel; l++) {
     // interior work list padded with patch = -1 to a multiple of kNormCells
-    std::vector<Blk> v;
-    for (int p : H.L(l).patches) {
-      const HostPatch& P = H.patches[p];
-      long long units = (long long)P.mx[0] * P.mx[1] * P.mx[2];
-      for (long long s = 0; s < units; s += kBlock) v.push_back(Blk{p, (int)s});
-    }
+    std::vector<Blk>& v = H.h_mx_norm_blk[l + kMaxDepth];
+    interior(l, v);
     while (v.size() % kNormCells) v.push_back(Blk{-1, 0});
-    Blk* d = nullptr;
-    cudaError_t e = dev_alloc(H, (void**)&d, sizeof(Blk) * v.size());
-    if (e != cudaSuccess) return cuda_fail(e, "device allocation (norm list)");
-    // staged from pageable memory before the call returns: v may go
-    e = cudaMemcpyAsync(d, v.data(), sizeof(Blk) * v.size(), cudaMemcpyHostToDevice, H.s);
-    if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpyAsync(norm list)");
-    H.mx_norm_blk[l + kMaxDepth] = d;
-    H.bytes += sizeof(Blk) * v.size();
-    H.h_mx_norm_blk[l + kMaxDepth] = v;
+    up.add(&H.mx_norm_blk[l + kMaxDepth], v);
   }
   // the interior lists of all levels below the root, concatenated
-  std::vector<Blk> v;
-  for (int l = H.minlevel; l < 0; l++)
-    for (int p : H.L(l).patches) {
-      const HostPatch& P = H.patches[p];
-      long long units = (long long)P.mx[0] * P.mx[1] * P.mx[2];
-      for (long long s = 0; s < units; s += kBlock) v.push_back(Blk{p, (int)s});
-    }
-  if (!v.empty()) {
-    cudaError_t e = dev_alloc(H, (void**)&H.mx_prep_coarse, sizeof(Blk) * v.size());
-    if (e == cudaSuccess)  // staged from pageable memory before it returns
-      e = cudaMemcpyAsync(H.mx_prep_coarse, v.data(), sizeof(Blk) * v.size(), cudaMemcpyHostToDevice, H.s);
-    if (e != cudaSuccess) return cuda_fail(e, "coarse prep list");
-    H.mx_prep_coarse_n = (int)v.size();
-    H.bytes += sizeof(Blk) * v.size();
-    H.h_mx_prep_coarse = v;
-  }
-  return BSAMG_OK;
+  for (int l = H.minlevel; l < 0; l++) interior(l, H.h_mx_prep_coarse);
+  H.mx_prep_coarse_n = (int)H.h_mx_prep_coarse.size();
+  up.add(&H.mx_prep_coarse, H.h_mx_prep_coarse);
 }
 
 void set_tail(Hier& H, long long cells) {

@@ -11,7 +11,7 @@ size_t mixed_pool_bytes(const Hier& H);
 int mixed_alloc(Hier& H);
 void mixed_free(Hier& H);
 // work lists of the mixed path, after the level tables exist
-int mixed_tables(Hier& H);
+void mixed_tables(Hier& H, TableUpload& up);
 // MultigridIterations in the mixed mode (after the common prologue:
 // FillDown(q), sources, FillDown(f)); same contract as the FP64 loop
 int mixed_iterations(Hier& H, int finest, int minlevel, int nsmooth, int maxvcycles, double tol, int errortype,

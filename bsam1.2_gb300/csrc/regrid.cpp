@@ -17,6 +17,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstring>
@@ -65,12 +66,12 @@ int host_tables(const Model& M, Hier& T) {
 }
 
 // SetGhost(level, 0) on the model's host arrays: the level's writer
-// sequence executed in order
+// sequences executed in order, side by side
 int host_set_ghost(Model& M, int level) {
   Hier T;
   int r = host_tables(M, T);
   if (r) return r;
-  std::vector<GhostOp> ops = set_ghost_sequence(T, level, 0);
+  const std::vector<std::vector<GhostOp>> seqs = set_ghost_sequences(T, level, 0);
   const double a1 = -01.0 / 05.0, a2 = 02.0 / 03.0, a3 = 08.0 / 15.0;   // boundary.f90:54-63
   const double b1 = 05.0 / 32.0, b2 = 15.0 / 16.0, b3 = -03.0 / 32.0;
   const double c1 = 09.0 / 16.0, c2 = 03.0 / 16.0, c3 = 03.0 / 16.0, c4 = 01.0 / 16.0;
@@ -81,26 +82,33 @@ int host_set_ghost(Model& M, int level) {
     plane[p] = M.nq(M.g[p]);
     if (!M.q[p].empty()) base[p] = M.q[p].data() + origin_of(M.src, M.g[p].qn);
   }
-  for (const GhostOp& o : ops) {
-    if (!base[o.dp] || !base[o.sp]) return BSAMG_ERR_ARG;  // below-root data is not on the host
-    for (int v = 0; v < M.src.nrvars; v++) {
-      double* dq = base[o.dp] + v * plane[o.dp];
-      const double* sq = base[o.sp] + v * plane[o.sp];
-      double val;
-      switch (o.type) {
-        case kGCopy: val = sq[o.s0]; break;
-        case kGCopyAdd: val = sq[o.s0] + M.src.pp.qpo[v]; break;
-        case kGCopySub: val = sq[o.s0] - M.src.pp.qpo[v]; break;
-        case kGBC: val = ((o.mask >> v) & 1) ? 2.0 - sq[o.s0] : (((o.mask >> (8 + v)) & 1) ? -sq[o.s0] : sq[o.s0]); break;
-        case kGCfA: val = a1 * dq[o.s0] + a2 * dq[o.s1] + a3 * sq[o.c0]; break;
-        case kGCfAB: val = a1 * dq[o.s0] + a2 * dq[o.s1] + a3 * (b1 * sq[o.c0] + b2 * sq[o.c1] + b3 * sq[o.c2]); break;
-        default:
-          val = a1 * dq[o.s0] + a2 * dq[o.s1] + a3 * (c1 * sq[o.c0] + c2 * sq[o.c1] + c3 * sq[o.c2] + c4 * sq[o.c3]);
-          break;
+  std::atomic<bool> bad{false};
+  parallel_for((int)seqs.size(), [&](int x) {
+    for (const GhostOp& o : seqs[x]) {
+      if (!base[o.dp] || !base[o.sp]) {  // below-root data is not on the host
+        bad = true;
+        return;
       }
-      dq[o.dcell] = val;
+      for (int v = 0; v < M.src.nrvars; v++) {
+        double* dq = base[o.dp] + v * plane[o.dp];
+        const double* sq = base[o.sp] + v * plane[o.sp];
+        double val;
+        switch (o.type) {
+          case kGCopy: val = sq[o.s0]; break;
+          case kGCopyAdd: val = sq[o.s0] + M.src.pp.qpo[v]; break;
+          case kGCopySub: val = sq[o.s0] - M.src.pp.qpo[v]; break;
+          case kGBC: val = ((o.mask >> v) & 1) ? 2.0 - sq[o.s0] : (((o.mask >> (8 + v)) & 1) ? -sq[o.s0] : sq[o.s0]); break;
+          case kGCfA: val = a1 * dq[o.s0] + a2 * dq[o.s1] + a3 * sq[o.c0]; break;
+          case kGCfAB: val = a1 * dq[o.s0] + a2 * dq[o.s1] + a3 * (b1 * sq[o.c0] + b2 * sq[o.c1] + b3 * sq[o.c2]); break;
+          default:
+            val = a1 * dq[o.s0] + a2 * dq[o.s1] + a3 * (c1 * sq[o.c0] + c2 * sq[o.c1] + c3 * sq[o.c2] + c4 * sq[o.c3]);
+            break;
+        }
+        dq[o.dcell] = val;
+      }
     }
-  }
+  });
+  if (bad) return BSAMG_ERR_ARG;
   return BSAMG_OK;
 }
 
