@@ -876,7 +876,9 @@ __global__ void __launch_bounds__(256) k_bx_prolong(float* __restrict__ fp, BoxL
 // shared memory, in natural order with one halo row at each side of e and ec;
 // a CTA writes its boundary rows into its neighbours' halos as it computes
 // them (distributed shared memory), so all reads are local and a sweep costs
-// one cluster barrier.  Levels too small to share out are CTA 0's.
+// one cluster barrier.  Levels too small to share out are CTA 0's, or every
+// second, fourth, .. CTA's (fold) where a CTA 0 would have more pairs than
+// threads to hold them.
 //
 // A thread owns pairs of x-neighbours (2h, 2h+1), one cell of each colour,
 // and keeps their e, g and pb in registers through a smoothing: a sweep reads
@@ -896,7 +898,9 @@ __global__ void __launch_bounds__(256) k_bx_prolong(float* __restrict__ fp, BoxL
 // bits.
 struct CycLev {
   int n0, n1, N;       // extents (n1: 3D), rows
-  int maxr, mul;       // rows a CTA holds at most, rows per row of the partition (0: CTA 0 alone)
+  int maxr;            // rows a CTA holds at most
+  int mul, down;       // rows per row of the partition: mul / 2^down (mul 0: CTA 0 alone)
+  int fold;            // every 2^fold-th CTA holds the level
   int e, ec, g, pb;    // starts in shared memory (floats)
   int by_colour;       // order of the restriction's sums (see cyc_smooth)
   float c0, c1, tmp3, a12;
@@ -904,7 +908,7 @@ struct CycLev {
 };
 struct Cyc {
   CycLev L[kNLev];     // finest first
-  UniRank R[16];
+  int row0[17];        // CTA r's first row of the level with mul = 1, down = 0 (the last: its rows)
   int nl, ctas, nsmooth, scratch;
   double cd[4];        // the coarsest level's coefficients in FP64
 };
@@ -918,28 +922,56 @@ struct Slab {
   bool shared;
   int lo, hi, lo_rows;   // neighbours (around the domain) and the rows of the one below
   float *e, *ec, *g, *pb;
+  float* base;           // the start of its CTA's shared memory
 };
-template <int DIM, bool REMOTE>
-__device__ __forceinline__ Slab slab(const Cyc& A, int x, int rank) {
-  const CycLev& L = A.L[x];
-  Slab S;
-  float* sm = csm;
+// A level's geometry as this CTA sees it, worked out once a launch and kept in
+// shared memory: each smoothing starts from it.
+struct __align__(16) SlabInfo {
+  int n0, n1, N, r0;
+  int nr, lo, hi, lo_rows;
+  int e, ec, g, pb;
+  int own, shared, maxr, workers;  // own: the CTA that holds this one's rows
+};
+constexpr int kCoarsePairs2 = 64;  // cyc_coarsest: most pairs that get two lanes each
+template <int DIM>
+__device__ __forceinline__ void slab_info(const Cyc& A, SlabInfo* info, int rank, int t, int nt) {
+  if (t >= A.nl) return;
+  const CycLev& L = A.L[t];
+  SlabInfo S;
   S.n0 = L.n0, S.n1 = L.n1, S.N = L.N, S.r0 = 0, S.nr = L.N;
-  S.shared = L.mul != 0;
   S.lo = S.hi = 0, S.lo_rows = L.N;
+  S.own = 0, S.shared = L.mul != 0, S.maxr = L.maxr;
   if (S.shared) {
-    S.r0 = A.R[rank].row0 * L.mul;
-    S.nr = A.R[rank].rows * L.mul;
-    S.lo = rank ? rank - 1 : A.ctas - 1;
-    S.hi = rank + 1 < A.ctas ? rank + 1 : 0;
-    S.lo_rows = A.R[S.lo].rows * L.mul;
-  } else if (REMOTE && rank) {
-    sm = uni::on_rank(sm, 0);
+    const int st = 1 << L.fold;  // CTAs st apart hold the level
+    S.own = rank & -st;
+    auto row = [&](int r) { return (A.row0[r] * L.mul) >> L.down; };
+    S.r0 = row(S.own);
+    S.nr = row(S.own + st) - S.r0;
+    S.lo = S.own ? S.own - st : A.ctas - st;
+    S.hi = S.own + st < A.ctas ? S.own + st : 0;
+    S.lo_rows = row(S.lo + st) - row(S.lo);
   }
-  S.plane = DIM == 3 ? L.n0 * L.n1 : L.n0;
-  S.var = S.plane * (L.maxr + 2);
-  S.ivar = S.plane * L.maxr;
-  S.e = sm + L.e, S.ec = sm + L.ec, S.g = sm + L.g, S.pb = sm + L.pb;
+  S.e = L.e, S.ec = L.ec, S.g = L.g, S.pb = L.pb;
+  // threads that work on it; coarser levels have no more than finer ones
+  int units = (L.n0 >> 1) * (DIM == 3 ? L.n1 : 1) * L.maxr;
+  if (t == A.nl - 1 && units <= kCoarsePairs2) units *= 2;
+  S.workers = min(nt, (units + 31) & ~31);
+  info[t] = S;
+}
+template <int DIM, bool REMOTE>
+__device__ __forceinline__ Slab slab(const SlabInfo* info, int x, int rank) {
+  const SlabInfo I = info[x];
+  Slab S;
+  S.n0 = I.n0, S.n1 = I.n1, S.N = I.N, S.r0 = I.r0, S.nr = I.nr;
+  S.lo = I.lo, S.hi = I.hi, S.lo_rows = I.lo_rows;
+  S.shared = I.shared != 0;
+  S.plane = DIM == 3 ? I.n0 * I.n1 : I.n0;
+  S.var = S.plane * (I.maxr + 2);
+  S.ivar = S.plane * I.maxr;
+  float* sm = csm;
+  if (REMOTE && I.own != rank) sm = uni::on_rank(sm, I.own);
+  S.base = sm;
+  S.e = sm + I.e, S.ec = sm + I.ec, S.g = sm + I.g, S.pb = sm + I.pb;
   return S;
 }
 
@@ -953,8 +985,9 @@ struct HaloOut {
 __device__ __forceinline__ HaloOut halo_out(const Slab& S, float* a) {
   HaloOut h{nullptr, nullptr, 0, 0};
   if (S.shared) {
-    h.lo = uni::on_rank(a, S.lo);
-    h.hi = uni::on_rank(a, S.hi);
+    float* const mine = csm + (a - S.base);  // the array's place in every CTA
+    h.lo = uni::on_rank(mine, S.lo);
+    h.hi = uni::on_rank(mine, S.hi);
     h.dlo = S.lo_rows * S.plane;
     h.dhi = -S.nr * S.plane;
   }
@@ -1236,7 +1269,6 @@ __device__ __forceinline__ void cyc_smooth(const Cyc& A, int x, const Slab& S, c
 // instructions a sweep for 30 (2 x 2 cells: 3300 -> 2000 cycles a sweep),
 // while all the pairs' lanes fit one warp per scheduler (kCoarsePairs2 pairs);
 // more pairs than that take a lane each.
-constexpr int kCoarsePairs2 = 64;
 template <int DIM, int LANES, typename F>
 __device__ __forceinline__ void cyc_coarsest(const Cyc& A, int x, const Slab& S, bool down, bool emit, int t,
                                              F&& sync) {
@@ -1352,15 +1384,10 @@ __device__ __forceinline__ void cyc_coarsest(const Cyc& A, int x, const Slab& S,
 // pairs fill: the others wait for the next level that needs them, so that the
 // chain of sweeps through the small levels has the schedulers to itself.
 template <int DIM>
-__device__ __forceinline__ void cyc_vcycle(const Cyc& A, int rank, int t, int nt) {
-  auto workers = [&](int x) {  // threads; coarser levels have no more than finer ones
-    const CycLev& L = A.L[x];
-    int units = (L.n0 >> 1) * (DIM == 3 ? L.n1 : 1) * L.maxr;
-    if (x == A.nl - 1 && units <= kCoarsePairs2) units *= 2;
-    return min(nt, (units + 31) & ~31);
-  };
+__device__ __forceinline__ void cyc_vcycle(const Cyc& A, const SlabInfo* info, int rank, int t, int nt) {
+  auto workers = [&](int x) { return info[x].workers; };
   auto smooth = [&](int x, int begin, bool restrict_, bool emit) {
-    const bool shared = A.L[x].mul != 0;
+    const bool shared = info[x].shared != 0;
     const int nw = workers(x);
     // barriers of the level's warps, an id a level; shared levels meet across the cluster
     auto local = [&] { asm volatile("bar.sync %0, %1;" ::"r"(1 + x), "r"(nw) : "memory"); };
@@ -1368,13 +1395,14 @@ __device__ __forceinline__ void cyc_vcycle(const Cyc& A, int rank, int t, int nt
       if (shared) uni::cluster_sync();
       else local();
     };
-    if (t >= nw) {  // (a shared level) the cluster's barriers count every warp
+    // (a shared level) the cluster's barriers count every warp of every CTA
+    if (t >= nw || (shared && info[x].own != rank)) {
       const int n = (begin != kTop) + max(0, 2 * A.nsmooth - (restrict_ ? 0 : 1));
       for (int k = 0; k < n; k++) uni::cluster_sync();
     } else {
-      const Slab S = slab<DIM, false>(A, x, rank);
-      const Slab C = x + 1 < A.nl ? slab<DIM, true>(A, x + 1, rank) : S;
-      const int units = (S.n0 >> 1) * (DIM == 3 ? S.n1 : 1) * A.L[x].maxr;
+      const Slab S = slab<DIM, false>(info, x, rank);
+      const Slab C = x + 1 < A.nl ? slab<DIM, true>(info, x + 1, rank) : S;
+      const int units = (S.n0 >> 1) * (DIM == 3 ? S.n1 : 1) * info[x].maxr;
       if (x == A.nl - 1) {
         if (units <= kCoarsePairs2 && nw >= 2 * units) cyc_coarsest<DIM, 2>(A, x, S, begin == kDown, emit, t, sync);
         else cyc_coarsest<DIM, 1>(A, x, S, begin == kDown, emit, t, sync);
@@ -1390,19 +1418,19 @@ __device__ __forceinline__ void cyc_vcycle(const Cyc& A, int rank, int t, int nt
     asm volatile("bar.sync %0, %1;" ::"r"(1 + x), "r"(workers(x)) : "memory");
   };
   for (int x = 0; x < A.nl; x++) {
-    const bool shared = A.L[x].mul != 0;
+    const bool shared = info[x].shared != 0;
     if (!shared && (rank || t >= workers(x))) break;
     smooth(x, x ? kDown : kTop, x + 1 < A.nl, x && x + 1 == A.nl);
     if (!shared) meet(x);
   }
   for (int x = A.nl - 2; x >= 0; x--) {
-    const bool shared = A.L[x].mul != 0;
+    const bool shared = info[x].shared != 0;
     if (!shared && (rank || t >= workers(x))) continue;
     if (!shared) meet(x);  // the next coarser level is finished
-    else if (!A.L[x + 1].mul) uni::cluster_sync();
+    else if (!info[x + 1].shared) uni::cluster_sync();
     smooth(x, kUp, false, x > 0);
   }
-  if (!A.L[0].mul) __syncthreads();
+  if (!info[0].shared) __syncthreads();
 }
 
 template <int DIM>
@@ -1414,8 +1442,11 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_bx_cycle(float* __restrict__
     if (A.ctas > 1) uni::cluster_sync();
     else __syncthreads();
   };
+  __shared__ SlabInfo info[16];
+  slab_info<DIM>(A, info, rank, t, nt);
+  __syncthreads();
   {  // the top level: e (halo rows too; zero when fresh), g and pb from the colour-split arrays, a pair a thread
-    const Slab S = slab<DIM, false>(A, 0, rank);
+    const Slab S = slab<DIM, false>(info, 0, rank);
     const CycLev& L = A.L[0];
     const V2 E = var2(fp, T.oe, T.half), G = var2(fp, T.og, T.half);
     const int pr = (S.n0 >> 1) * (DIM == 3 ? S.n1 : 1);
@@ -1444,8 +1475,8 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_bx_cycle(float* __restrict__
       }
   }
   all();
-  cyc_vcycle<DIM>(A, rank, t, nt);
-  const Slab S = slab<DIM, false>(A, 0, rank);
+  cyc_vcycle<DIM>(A, info, rank, t, nt);
+  const Slab S = slab<DIM, false>(info, 0, rank);
   const CycLev& L = A.L[0];
   const V2 E = var2(fp, T.oe, T.half);
   if (S.shared || rank == 0)
@@ -1711,7 +1742,10 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_bx_solve(float* __restrict__
     if (A.ctas > 1) uni::cluster_sync();
     else __syncthreads();
   };
-  const Slab S = slab<DIM, false>(A, 0, rank);
+  __shared__ SlabInfo info[16];
+  slab_info<DIM>(A, info, rank, t, nt);
+  __syncthreads();
+  const Slab S = slab<DIM, false>(info, 0, rank);
   const CycLev& L = A.L[0];
   const int n1 = DIM == 3 ? S.n1 : 1;
   // a top level that CTA 0 holds alone leaves the others without cells
@@ -1853,7 +1887,7 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_bx_solve(float* __restrict__
   int status = (B.warm ? norm(w0, w1, judge_true) : confirm(judge_true)) & kNonfinite, conv = 0, it = 0, nconfirm = 0;
   while (!status && it < B.maxv) {
     it++;
-    cyc_vcycle<DIM>(A, rank, t, nt);
+    cyc_vcycle<DIM>(A, info, rank, t, nt);
     // g -= M(e), then qbar += e (k_bx_track_update)
     float s0 = 0.f, s1 = 0.f;
     for (int u = t; u < units; u += nt) {
@@ -2134,7 +2168,7 @@ cudaError_t launch_cluster(K k, int ctas, int threads, int smem, cudaStream_t s,
 // The cluster's plan for the levels top .. minlevel with the first `share`
 // of them shared out; false when it does not fit (shared memory, pairs a
 // thread, the coarsest level's one pair a thread)
-bool cycle_layout(Hier& H, int top, int minlevel, int nsmooth, int share, Cyc& A, int* smem) {
+bool cycle_layout(Hier& H, int top, int minlevel, int nsmooth, int share, int base, Cyc& A, int* smem) {
   const int D = H.ndims;
   A = Cyc{};
   A.nl = top - minlevel + 1;
@@ -2142,18 +2176,16 @@ bool cycle_layout(Hier& H, int top, int minlevel, int nsmooth, int share, Cyc& A
   A.ctas = 1;
   int nc = 1;
   if (share) {
-    // whole rows of the first level CTA 0 holds (each CTA restricts whole
-    // coarse rows), or of the last level when all are shared
-    nc = B(H, top - std::min(share, A.nl - 1)).n[D - 1];
+    // every CTA's rows are whole rows of level `base`: the first level CTA 0
+    // holds alone (each CTA restricts whole coarse rows), or the last one when
+    // all are shared.  A base above that has one row a CTA, and the shared
+    // levels from it down are held by every 2nd, 4th, .. CTA, two rows each.
+    nc = B(H, top - base).n[D - 1];
     A.ctas = std::min(16, nc);
-    if (A.ctas < 2) return false;
+    const int folds = std::min(share, A.nl) - base;  // levels held by some CTAs only
+    if (A.ctas < 2 || (base < std::min(share, A.nl - 1) && (A.ctas != nc || (A.ctas >> folds) < 2))) return false;
   }
-  int most = 0;
-  for (int r = 0; r < A.ctas; r++) {
-    const int a = r * nc / A.ctas, b = (r + 1) * nc / A.ctas;
-    A.R[r] = UniRank{(short)a, (short)(b - a)};
-    most = std::max(most, b - a);
-  }
+  for (int r = 0; r <= A.ctas; r++) A.row0[r] = r * nc / A.ctas;
   long long o = 0, scratch = 0;
   auto add = [&](long long n) {
     const long long at = o;
@@ -2165,8 +2197,18 @@ bool cycle_layout(Hier& H, int top, int minlevel, int nsmooth, int share, Cyc& A
     const BoxLev& P = B(H, top - x);
     CycLev& L = A.L[x];
     L.n0 = P.n[0], L.n1 = P.n[1], L.N = P.n[D - 1];
-    L.mul = x < share ? 1 << (std::min(share, A.nl - 1) - x) : 0;
-    L.maxr = L.mul ? most * L.mul : L.N;
+    L.mul = x < share ? 1 << std::max(0, base - x) : 0;
+    L.down = std::max(0, x - base);
+    L.fold = base < std::min(share, A.nl - 1) && x >= base ? 1 + x - base : 0;
+    L.maxr = L.N;
+    if (L.mul) {
+      const int st = 1 << L.fold;
+      if (A.ctas % st) return false;
+      L.maxr = 0;
+      for (int r = 0; r < A.ctas; r += st)
+        L.maxr = std::max(L.maxr, ((A.row0[r + st] * L.mul) >> L.down) - ((A.row0[r] * L.mul) >> L.down));
+      if (L.maxr < 1) return false;
+    }
     const long long plane = (long long)P.n[0] * (D == 3 ? P.n[1] : 1);
     const long long pairs = plane / 2 * L.maxr;
     if (pairs > kCycThreads * (x + 1 < A.nl ? kCycPairs : 1)) return false;
@@ -2200,15 +2242,17 @@ bool cycle_plan(Hier& H, int level, int minlevel, int nsmooth, Cyc& best, int* s
       Cyc A;
     };
     std::vector<Form> forms;
-    for (int share = 0; share <= top - minlevel + 1; share++) {
-      Form f{0.0, 0, {}};
-      if (!cycle_layout(H, top, minlevel, nsmooth, share, f.A, &f.smem)) continue;
-      for (int x = 0; x < f.A.nl; x++) {
-        const double pairs = (double)B(H, top - x).half / (x < share ? f.A.ctas : 1);
-        f.us += (x < share ? 0.75 : 0.3) + pairs * 70 / 32 / 4 / 2000.0 * 1.5;
+    const int nl = top - minlevel + 1;
+    for (int share = 0; share <= nl; share++)
+      for (int base = std::min(share, nl - 1); base >= std::min(std::min(share, 1), nl - 1); base--) {
+        Form f{0.0, 0, {}};
+        if (!cycle_layout(H, top, minlevel, nsmooth, share, base, f.A, &f.smem)) continue;
+        for (int x = 0; x < f.A.nl; x++) {
+          const double pairs = (double)B(H, top - x).half / (x < share ? f.A.ctas >> f.A.L[x].fold : 1);
+          f.us += (x < share ? 0.75 : 0.3) + pairs * 70 / 32 / 4 / 2000.0 * 1.5;
+        }
+        forms.push_back(f);
       }
-      forms.push_back(f);
-    }
     std::stable_sort(forms.begin(), forms.end(), [](const Form& a, const Form& b) { return a.us < b.us; });
     for (const Form& f : forms)  // the cheapest that fits: asking the runtime costs tens of microseconds
       if (cycle_fit(H.ndims, f.A.ctas, f.smem) >= 1) {
