@@ -115,7 +115,7 @@ int enq_set_ghost(Hier& H, int level, int ipass) {
   }
   int nops = g.stage_off[nst];
   LaunchCtx c = H.lc();
-  if (nops <= 2048) return after_launch(H, launch_ghost_program_1cta(c, g.d_ops, g.d_stage_off, nst));
+  if (ghost_in_one_cta(nst, nops)) return after_launch(H, launch_ghost_program_1cta(c, g.d_ops, g.d_stage_off, nst));
   for (int s = 0; s < nst; s++)
     RET(after_launch(H, launch_ghost_stage(c, g.d_ops + g.stage_off[s], g.stage_off[s + 1] - g.stage_off[s])));
   return BSAMG_OK;

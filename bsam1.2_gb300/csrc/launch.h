@@ -269,6 +269,12 @@ int launch_seed_spinodal(cudaStream_t s, int ndims, int mbc, double* q, long lon
 // into the uniform block U (extents un)
 int launch_uniform_scatter(cudaStream_t s, int ndims, const double* pool, long long oq, long long sq, const int qn[3],
                            const int mx[3], const int g[3], double* U, const int un[3], int nv);
+// A ghost program of several stages and few operations runs in one CTA, its
+// stages apart by CTA barriers; otherwise a launch a stage.  One CTA takes a
+// round of 256 operations (FP64: some 20 dependent instructions of 64 cycles)
+// after the other: a program of one stage and 1000 operations 14 us, its stage
+// over the GPU 6.5.
+inline bool ghost_in_one_cta(int nstages, int nops) { return nstages > 1 && nops <= 512; }
 int launch_ghost_program_1cta(const LaunchCtx& c, const GhostOp* ops,
                               const int* stage_off, int nstages);
 // the recorded coarse tail of an FP64 V-cycle, one block

@@ -137,7 +137,7 @@ int mx_set_ghost(Hier& H, int level, int ipass) {
     return BSAMG_OK;
   }
   int nops = g.stage_off[nst];
-  if (nops <= 2048) {
+  if (ghost_in_one_cta(nst, nops)) {
     k_ghost32_program<<<1, kBlock, 0, H.s>>>(H.dP, H.fpool, g.d_ops, g.d_stage_off, nst, H.nrvars);
     return after_launch(H, 1);
   }
