@@ -318,6 +318,7 @@ __device__ __forceinline__ void relax64_at(float* __restrict__ fp, const BoxLev&
 // that no small-level cycle covers): one cell of the colour per thread
 template <int DIM>
 __global__ void __launch_bounds__(256) k_bx_relax64(float* __restrict__ fp, BoxLev L, int c, int first) {
+  after_previous();
   int h = blockIdx.x * blockDim.x + threadIdx.x;
   int y = blockIdx.y * blockDim.y + threadIdx.y;
   if (h < L.hh && y < L.n[1]) relax64_at<DIM>(fp, L, c, first, h, y, blockIdx.z);
@@ -328,6 +329,7 @@ __global__ void __launch_bounds__(256) k_bx_relax64(float* __restrict__ fp, BoxL
 // so that R times the loads are in flight per thread.
 template <int DIM, int R = 2, int MINB = 8>
 __global__ void __launch_bounds__(256, MINB) k_bx_relax(float* __restrict__ fp, BoxLev L, int c, int first) {
+  after_previous();
   int h = blockIdx.x * blockDim.x + threadIdx.x;
   int yp = blockIdx.y * blockDim.y + threadIdx.y;
   int z = blockIdx.z;
@@ -396,6 +398,7 @@ __host__ __device__ __forceinline__ int tile_stage_floats(int T, int hh) { retur
 // T rows per tile, NS stages (NS - 1 tiles in flight ahead of the one computed)
 template <int T, int NS>
 __global__ void __launch_bounds__(kTileThreads) k_bx_relax_tiled(float* __restrict__ fp, BoxLev L, int c, int first) {
+  after_previous();
   extern __shared__ __align__(128) float tsm[];
   __shared__ __align__(8) unsigned long long bar[NS];
   const int hh = L.hh, n1 = L.n[1], n2 = L.n[2];
@@ -559,6 +562,7 @@ __device__ __forceinline__ void stv(float* p, const float* v) {
 template <int TY, int HH, bool FRESH, int NS = kSmStages, int CPT = 4, int NT = kSmThreads>
 __global__ void __launch_bounds__(NT, 1) k_bx_smooth(float* __restrict__ fp, BoxLev L, long long oe_out, int nz,
                                                    const __grid_constant__ CUtensorMap emap) {
+  after_previous();
   extern __shared__ __align__(128) float ssm[];
   constexpr int NSL = smooth_slots(NS);
   constexpr int R = TY + 2 * NS, AR = R * HH, SL = 4 * AR, LG = ilog2(HH);
@@ -783,6 +787,7 @@ __device__ __forceinline__ void restrict_load_at(float* __restrict__ fp, const B
 }
 template <int DIM>
 __global__ void __launch_bounds__(256, 6) k_bx_restrict_load(float* __restrict__ fp, BoxLev F, BoxLev C) {
+  after_previous();
   int X = blockIdx.x * blockDim.x + threadIdx.x;
   int Y = blockIdx.y * blockDim.y + threadIdx.y;
   if (X < C.n[0] && Y < C.n[1]) restrict_load_at<DIM>(fp, F, C, X, Y, blockIdx.z);
@@ -790,6 +795,7 @@ __global__ void __launch_bounds__(256, 6) k_bx_restrict_load(float* __restrict__
 // coarse g += M_c(ec), the coarse operator on the restricted correction
 template <int DIM>
 __global__ void __launch_bounds__(256) k_bx_coarse_op(float* __restrict__ fp, BoxLev C) {
+  after_previous();
   int X = blockIdx.x * blockDim.x + threadIdx.x;
   int Y = blockIdx.y * blockDim.y + threadIdx.y;
   if (X >= C.n[0] || Y >= C.n[1]) return;
@@ -865,6 +871,7 @@ __device__ __forceinline__ void prolong_at(float* __restrict__ fp, const BoxLev&
 }
 template <int DIM>
 __global__ void __launch_bounds__(256) k_bx_prolong(float* __restrict__ fp, BoxLev F, BoxLev C) {
+  after_previous();
   int X = blockIdx.x * blockDim.x + threadIdx.x;
   int Y = blockIdx.y * blockDim.y + threadIdx.y;
   if (X < C.n[0] && Y < C.n[1]) prolong_at<DIM>(fp, F, C, X, Y, blockIdx.z);
@@ -1436,6 +1443,7 @@ __device__ __forceinline__ void cyc_vcycle(const Cyc& A, const SlabInfo* info, i
 template <int DIM>
 __global__ void __launch_bounds__(kCycThreads, 1) k_bx_cycle(float* __restrict__ fp, const __grid_constant__ Cyc A,
                                                              BoxLev T, int fresh) {
+  after_previous();
   const int rank = A.ctas > 1 ? uni::my_rank() : 0;
   const int t = threadIdx.x, nt = blockDim.x;
   auto all = [&] {
@@ -1504,6 +1512,7 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_bx_cycle(float* __restrict__
 template <int DIM, int R = 1>
 __global__ void __launch_bounds__(256, R == 1 ? 6 : 5) k_bx_track_update(float* __restrict__ fp, BoxLev L,
                                                                        long long oqlo, double* __restrict__ partial) {
+  after_previous();
   // R rows per thread (y = R yp .. R yp + R - 1): every load of the R cells
   // is issued before the first store, R times the loads in flight
   int x = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1577,6 +1586,7 @@ __device__ __forceinline__ void resid_at(const float* fp, const BoxLev& L, long 
 template <int DIM>
 __global__ void __launch_bounds__(256) k_bx_resid(float* __restrict__ fp, BoxLev L, long long oqlo, long long ofhi,
                                                   long long oflo, double* __restrict__ partial) {
+  after_previous();
   int x = blockIdx.x * blockDim.x + threadIdx.x;
   int y = blockIdx.y * blockDim.y + threadIdx.y;
   int z = blockIdx.z;
@@ -1600,6 +1610,7 @@ template <int DIM>
 __global__ void __launch_bounds__(256) k_bx_split(const double* __restrict__ pool, long long oq, long long oqold,
                                                   long long sq, int qn0, int qn1, float* __restrict__ fp, BoxLev L,
                                                   long long oqlo, long long ofhi, long long oflo) {
+  after_previous();
   int h = blockIdx.x * blockDim.x + threadIdx.x;
   int y = blockIdx.y * blockDim.y + threadIdx.y;
   int z = blockIdx.z;
@@ -1635,6 +1646,7 @@ __global__ void __launch_bounds__(256) k_bx_split_warm(const double* __restrict_
                                                        long long sq, int qn0, int qn1, float* __restrict__ fp,
                                                        BoxLev L, long long oqlo, long long ofhi, long long oflo,
                                                        double* __restrict__ partial) {
+  after_previous();
   int h = blockIdx.x * blockDim.x + threadIdx.x;
   int y = blockIdx.y * blockDim.y + threadIdx.y;
   int z = blockIdx.z;
@@ -1681,6 +1693,7 @@ __global__ void __launch_bounds__(256) k_bx_split_warm(const double* __restrict_
 template <int DIM>
 __global__ void __launch_bounds__(256) k_bx_merge(double* __restrict__ pool, long long oq, long long sq, int qn0,
                                                   int qn1, float* __restrict__ fp, BoxLev L, long long oqlo) {
+  after_previous();
   int h = blockIdx.x * blockDim.x + threadIdx.x;
   int y = blockIdx.y * blockDim.y + threadIdx.y;
   int z = blockIdx.z;
@@ -1731,6 +1744,7 @@ template <int DIM>
 __global__ void __launch_bounds__(kCycThreads, 1) k_bx_solve(float* __restrict__ fp, double* __restrict__ pool,
                                                              const __grid_constant__ Cyc A, BoxLev T, BoxSolve B,
                                                              BoxSolveOut* __restrict__ out) {
+  after_previous();
   const int rank = A.ctas > 1 ? uni::my_rank() : 0;
   const int t = threadIdx.x, nt = blockDim.x;
   __shared__ float wsum[2][kCycThreads / 32];
@@ -1988,8 +2002,8 @@ long long ctas(const Launch& s) { return (long long)s.g.x * s.g.y * s.g.z; }
 
 #define BX_LAUNCH(H, SH, KER, ...)                                            \
   do {                                                                        \
-    if ((H).ndims == 2) KER<2><<<(SH).g, (SH).b, 0, (H).s>>>(__VA_ARGS__);    \
-    else KER<3><<<(SH).g, (SH).b, 0, (H).s>>>(__VA_ARGS__);                   \
+    if ((H).ndims == 2) launch_after(KER<2>, (SH).g, (SH).b, 0, (H).s, __VA_ARGS__);    \
+    else launch_after(KER<3>, (SH).g, (SH).b, 0, (H).s, __VA_ARGS__);                   \
     int r__ = after_launch(H, 1);                                             \
     if (r__) return r__;                                                      \
   } while (0)
@@ -2017,7 +2031,7 @@ int launch_staged(Hier& H, const BoxLev& L, int c, int first) {
   if (e != cudaSuccess || occ < 1) return cuda_fail(e, "occupancy(k_bx_relax_tiled)");
   int ntiles = (L.n[1] / kTileT) * L.n[2];
   int grid = std::min(ntiles, occ * H.box_sms);
-  ker<<<grid, kTileThreads, smem, H.s>>>(H.fpool, L, c, first);
+  launch_after(ker, grid, kTileThreads, smem, H.s, H.fpool, L, c, first);
   return after_launch(H, 1);
 }
 
@@ -2082,7 +2096,7 @@ int bx_smooth(Hier& H, const BoxLev& in, long long out_oe, bool fresh) {
   int r = e_tensor_map(H, in, in.oe, &emap);
   if (r) return r;
   auto ker = fresh ? k_bx_smooth<8, 128, true> : k_bx_smooth<8, 128, false>;
-  ker<<<ytiles * nz, kSmThreads, smem, H.s>>>(H.fpool, in, out_oe, nz, emap);
+  launch_after(ker, ytiles * nz, kSmThreads, smem, H.s, H.fpool, in, out_oe, nz, emap);
   return after_launch(H, 1);
 }
 bool smooth_applies(const Hier& H, const BoxLev& L, int nsmooth) {
@@ -2096,7 +2110,7 @@ int bx_relax(Hier& H, int level, int c, int first) {
     // four rows per thread at five blocks per SM (40 registers): four
     // cells' loads in flight per thread
     Launch sh = shape(L.hh, L.n[1] / 4, L.n[2]);
-    k_bx_relax<3, 4, 5><<<sh.g, sh.b, 0, H.s>>>(H.fpool, L, c, first);
+    launch_after(k_bx_relax<3, 4, 5>, sh.g, sh.b, 0, H.s, H.fpool, L, c, first);
     return after_launch(H, 1);
   }
   Launch sh = shape(L.hh, L.n[1] / 2, L.n[2]);
@@ -2155,13 +2169,15 @@ cudaError_t launch_cluster(K k, int ctas, int threads, int smem, cudaStream_t s,
   cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = ctas;
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.numAttrs = 2;
   return cudaLaunchKernelEx(&cfg, k, args...);
 }
 
@@ -2346,7 +2362,7 @@ int bx_cycle(Hier& H, int finest, int minlevel, int nsmooth, int errortype, bool
   BoxLev& L = B(H, finest);
   if (H.ndims == 3 && L.n[1] % 2 == 0) {  // two rows per thread
     Launch sh = shape(L.n[0], L.n[1] / 2, L.n[2]);
-    k_bx_track_update<3, 2><<<sh.g, sh.b, 0, H.s>>>(H.fpool, L, H.b_oqlo, H.d_partial);
+    launch_after(k_bx_track_update<3, 2>, sh.g, sh.b, 0, H.s, H.fpool, L, H.b_oqlo, H.d_partial);
     if ((r = after_launch(H, 1))) return r;
     return bx_finish(H, finest, ctas(sh), errortype, to_host);
   }
@@ -2379,6 +2395,7 @@ static_assert(sizeof(BoxCtl) <= (128 - kCtlSlotOffset) * sizeof(double) &&
 // true residual, or the last cycle)
 __global__ void k_bx_decide_cycle(BoxCtl* c, const double* __restrict__ norm, const int* __restrict__ nonfinite,
                                   cudaGraphConditionalHandle hw, cudaGraphConditionalHandle hi) {
+  after_previous();
   int it = ++c->it;
   if (c->status || nonfinite[0]) {
     c->status = 1;
@@ -2395,6 +2412,7 @@ __global__ void k_bx_decide_cycle(BoxCtl* c, const double* __restrict__ norm, co
 // after a true residual: converged or the last cycle ends the loop
 __global__ void k_bx_decide_true(BoxCtl* c, const double* __restrict__ norm, const int* __restrict__ nonfinite,
                                  cudaGraphConditionalHandle hw) {
+  after_previous();
   int it = c->it;
   c->nconfirm++;
   if (nonfinite[0]) {
@@ -2459,7 +2477,7 @@ int box_loop_graph(Hier& H, int finest, int minlevel, int nsmooth, int errortype
     r = capture_into(H, body, [&]() -> int {
       int rr = bx_cycle(H, finest, minlevel, nsmooth, errortype, false);
       if (rr) return rr;
-      k_bx_decide_cycle<<<1, 1, 0, H.s>>>(ctl, H.d_norm, H.d_nonfinite, hw, hi);
+      launch_after(k_bx_decide_cycle, 1, 1, 0, H.s, ctl, H.d_norm, H.d_nonfinite, hw, hi);
       if ((rr = after_launch(H, 1))) return rr;
       cudaStreamCaptureStatus st;
       cudaGraph_t cg = nullptr;
@@ -2482,7 +2500,7 @@ int box_loop_graph(Hier& H, int finest, int minlevel, int nsmooth, int errortype
     r = capture_into(H, ip.conditional.phGraph_out[0], [&]() -> int {
       int rr = bx_resid(H, finest, errortype, false);
       if (rr) return rr;
-      k_bx_decide_true<<<1, 1, 0, H.s>>>(ctl, H.d_norm, H.d_nonfinite, hw);
+      launch_after(k_bx_decide_true, 1, 1, 0, H.s, ctl, H.d_norm, H.d_nonfinite, hw);
       return after_launch(H, 1);
     }, &H.box_loop_n2);
     if (r) break;

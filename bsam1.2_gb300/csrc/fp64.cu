@@ -22,6 +22,7 @@ namespace bsamg {
 template <int DIM>
 __global__ void __launch_bounds__(kBlock) k_restrict_q(const PatchDev* __restrict__ P, double* __restrict__ pool,
                                                        const Blk* __restrict__ blk, int nrvars) {
+  after_previous();
   u_restrict_q<DIM>(P, pool, blk[blockIdx.x], threadIdx.x, nrvars);
 }
 
@@ -29,6 +30,7 @@ __global__ void __launch_bounds__(kBlock) k_restrict_q(const PatchDev* __restric
 template <int DIM>
 __global__ void __launch_bounds__(kBlock) k_coarse_ghost(const PatchDev* __restrict__ P, double* __restrict__ pool,
                                                          const Blk* __restrict__ blk, int nrvars) {
+  after_previous();
   u_coarse_ghost<DIM>(P, pool, blk[blockIdx.x], threadIdx.x, nrvars);
 }
 
@@ -36,6 +38,7 @@ __global__ void __launch_bounds__(kBlock) k_coarse_ghost(const PatchDev* __restr
 template <int DIM>
 __global__ void __launch_bounds__(kBlock) k_correct_a(const PatchDev* __restrict__ P, double* __restrict__ pool,
                                                       const Blk* __restrict__ blk, int nrvars) {
+  after_previous();
   u_correct_a<DIM>(P, pool, blk[blockIdx.x], threadIdx.x, nrvars);
 }
 
@@ -44,6 +47,7 @@ __global__ void __launch_bounds__(kBlock) k_correct_a(const PatchDev* __restrict
 template <int DIM>
 __global__ void __launch_bounds__(kBlock) k_qc_from_parent(const PatchDev* __restrict__ P, double* __restrict__ pool,
                                                            const Blk* __restrict__ blk, int nrvars) {
+  after_previous();
   const Blk b = blk[blockIdx.x];
   const PatchDev& p = P[b.patch];
   int i, j, k;
@@ -58,12 +62,14 @@ __global__ void __launch_bounds__(kBlock) k_qc_from_parent(const PatchDev* __res
 template <int DIM>
 __global__ void __launch_bounds__(kBlock) k_correct_b(const PatchDev* __restrict__ P, double* __restrict__ pool,
                                                       const Blk* __restrict__ blk, int nrvars) {
+  after_previous();
   u_correct_b<DIM>(P, pool, blk[blockIdx.x], threadIdx.x, nrvars);
 }
 
 template <int DIM>
 __global__ void __launch_bounds__(kBlock) k_fill_down(const PatchDev* __restrict__ P, double* __restrict__ pool,
                                                       const Blk* __restrict__ blk, int nrvars, int field) {
+  after_previous();
   u_fill_down<DIM>(P, pool, blk[blockIdx.x], threadIdx.x, nrvars, field);
 }
 
@@ -77,6 +83,7 @@ constexpr int kStageBlocks = (kNormOutLen - 8) / 3;
 template <int NV>
 __global__ void __launch_bounds__(kBlock) k_norm_stage(const double* __restrict__ partial, int nblk, int chunk,
                                                        double* __restrict__ stage) {
+  after_previous();
   __shared__ double red[NV][kBlock];
   int lo = blockIdx.x * chunk, hi = min(lo + chunk, nblk);
   double a[NV];
@@ -106,6 +113,7 @@ template <int NV>
 __global__ void __launch_bounds__(kFinishThreads) k_norm_finish(const double* __restrict__ partial, int nblk,
                                                                 double count, int errortype, double* out,
                                                                 int* nonfinite, double* host, double* one) {
+  after_previous();
   __shared__ double red[NV][kFinishThreads / 32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int warps = min(kFinishThreads / 32, (nblk + 31) / 32);  // warps that hold a partial
@@ -177,6 +185,7 @@ __global__ void __launch_bounds__(kFinishThreads) k_norm_finish(const double* __
 
 __global__ void __launch_bounds__(kBlock) k_ghost_stage(const PatchDev* __restrict__ P, double* __restrict__ pool,
                                                         const GhostOp* __restrict__ ops, int n, ProbParams pp) {
+  after_previous();
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
   GhostOp g = ops[t];
@@ -188,6 +197,7 @@ __global__ void __launch_bounds__(kBlock) k_ghost_program(const PatchDev* __rest
                                                           const GhostOp* __restrict__ ops,
                                                           const int* __restrict__ stage_off, int nstages,
                                                           ProbParams pp) {
+  after_previous();
   for (int s = 0; s < nstages; s++) {
     int lo = stage_off[s], hi = stage_off[s + 1];
     for (int t = lo + threadIdx.x; t < hi; t += blockDim.x) {
@@ -207,8 +217,8 @@ __global__ void __launch_bounds__(kBlock) k_ghost_program(const PatchDev* __rest
 
 #define DISPATCH_DIM(c, KER, ...)                            \
   do {                                                       \
-    if ((c).ndims == 2) KER<2><<<nblk, kBlock, 0, (c).s>>>(__VA_ARGS__); \
-    else KER<3><<<nblk, kBlock, 0, (c).s>>>(__VA_ARGS__);    \
+    if ((c).ndims == 2) launch_after(KER<2>, nblk, kBlock, 0, (c).s, __VA_ARGS__); \
+    else launch_after(KER<3>, nblk, kBlock, 0, (c).s, __VA_ARGS__);    \
   } while (0)
 
 // the plugin's FP64 launchers; a hierarchy is created only for a registered
@@ -264,26 +274,26 @@ int launch_norm_finish(cudaStream_t s, const double* partial, int nblk, int nrva
     int g = std::min(kStageBlocks, (nblk + 511) / 512);
     int chunk = (nblk + g - 1) / g;
     g = (nblk + chunk - 1) / chunk;
-    if (nrvars == 3) k_norm_stage<3><<<g, kBlock, 0, s>>>(partial, nblk, chunk, out + 8);
-    else k_norm_stage<2><<<g, kBlock, 0, s>>>(partial, nblk, chunk, out + 8);
+    if (nrvars == 3) launch_after(k_norm_stage<3>, g, kBlock, 0, s, partial, nblk, chunk, out + 8);
+    else launch_after(k_norm_stage<2>, g, kBlock, 0, s, partial, nblk, chunk, out + 8);
     partial = out + 8;
     nblk = g;
     n = 2;
   }
-  if (nrvars == 3) k_norm_finish<3><<<1, kFinishThreads, 0, s>>>(partial, nblk, count, errortype, out, nonfinite, host, one);
+  if (nrvars == 3) launch_after(k_norm_finish<3>, 1, kFinishThreads, 0, s, partial, nblk, count, errortype, out, nonfinite, host, one);
   else
-    k_norm_finish<2><<<1, kFinishThreads, 0, s>>>(partial, nblk, count, errortype, out, nonfinite, host, one);
+    launch_after(k_norm_finish<2>, 1, kFinishThreads, 0, s, partial, nblk, count, errortype, out, nonfinite, host, one);
   return n;
 }
 int launch_ghost_stage(const LaunchCtx& c, const GhostOp* ops, int n) {
   if (n <= 0) return 0;
   int nb = (n + kBlock - 1) / kBlock;
-  k_ghost_stage<<<nb, kBlock, 0, c.s>>>(c.P, c.pool, ops, n, c.pp);
+  launch_after(k_ghost_stage, nb, kBlock, 0, c.s, c.P, c.pool, ops, n, c.pp);
   return 1;
 }
 int launch_ghost_program_1cta(const LaunchCtx& c, const GhostOp* ops, const int* stage_off, int nstages) {
   if (nstages <= 0) return 0;
-  k_ghost_program<<<1, kBlock, 0, c.s>>>(c.P, c.pool, ops, stage_off, nstages, c.pp);
+  launch_after(k_ghost_program, 1, kBlock, 0, c.s, c.P, c.pool, ops, stage_off, nstages, c.pp);
   return 1;
 }
 int launch_tail(const LaunchCtx& c, const TailPhase* ph, int nph) { return ops_of(c).tail(c, ph, nph); }

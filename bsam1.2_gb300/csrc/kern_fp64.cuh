@@ -235,6 +235,7 @@ __device__ __forceinline__ void u_relax(const PatchDev* __restrict__ P, double* 
 template <class PL, int DIM>
 __global__ void __launch_bounds__(kBlock) k_relax(const PatchDev* __restrict__ P, double* __restrict__ pool,
                                                   const Blk* __restrict__ blk, int ipass, ProbParams pp) {
+  after_previous();
   u_relax<PL, DIM>(P, pool, blk[blockIdx.x], threadIdx.x, ipass, pp);
 }
 
@@ -287,6 +288,7 @@ __device__ __forceinline__ void u_coarse_load(const PatchDev* __restrict__ P, do
 template <class PL, int DIM>
 __global__ void __launch_bounds__(kBlock) k_coarse_load(const PatchDev* __restrict__ P, double* __restrict__ pool,
                                                         const Blk* __restrict__ blk, ProbParams pp) {
+  after_previous();
   u_coarse_load<PL, DIM>(P, pool, blk[blockIdx.x], threadIdx.x, pp);
 }
 
@@ -294,6 +296,7 @@ __global__ void __launch_bounds__(kBlock) k_coarse_load(const PatchDev* __restri
 template <class PL, int DIM>
 __global__ void __launch_bounds__(kBlock) k_get_source(const PatchDev* __restrict__ P, double* __restrict__ pool,
                                                        const Blk* __restrict__ blk, ProbParams pp) {
+  after_previous();
   const Blk b = blk[blockIdx.x];
   const PatchDev& p = P[b.patch];
   int i, j, k;
@@ -310,6 +313,7 @@ __global__ void __launch_bounds__(kBlock) k_get_source(const PatchDev* __restric
 template <class PL, int DIM>
 __global__ void __launch_bounds__(kBlock) k_update_source(const PatchDev* __restrict__ P, double* __restrict__ pool,
                                                           const Blk* __restrict__ blk, ProbParams pp) {
+  after_previous();
   const Blk b = blk[blockIdx.x];
   const PatchDev& p = P[b.patch];
   int i, j, k;
@@ -345,6 +349,7 @@ template <class PL, int DIM>
 __global__ void __launch_bounds__(kBlock, 4) k_norm_partial(const PatchDev* __restrict__ P, double* __restrict__ pool,
                                                          const Blk* __restrict__ blk, int nblk, int group,
                                                          ProbParams pp, double* __restrict__ partial, int store_rf) {
+  after_previous();
   constexpr int NV = PL::kNV;
   __shared__ double red[NV][kBlock / 32];
   double s[NV];
@@ -380,6 +385,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_uni_norm(const PatchDev* __restri
                                                      int patch, const __grid_constant__ UniPatch u, int group,
                                                      ProbParams pp, double* __restrict__ partial, int store_rf,
                                                      int update) {
+  after_previous();
   constexpr int NV = PL::kNV;
   __shared__ double red[NV][kBlock / 32];
   const PatchDev& p = u.p;
@@ -457,6 +463,7 @@ __device__ __forceinline__ void run_tail(const PatchDev* __restrict__ P, double*
 template <class PL, int DIM>
 __global__ void __launch_bounds__(kBlock) k_tail(const PatchDev* __restrict__ P, double* __restrict__ pool,
                                                  const TailPhase* __restrict__ ph, int nph, ProbParams pp) {
+  after_previous();
   run_tail<PL, DIM>(P, pool, ph, nph, pp);
 }
 
@@ -466,6 +473,7 @@ template <class PL, int DIM>
 __global__ void __launch_bounds__(kBlock) k_tail_smem(const PatchDev* __restrict__ P, double* __restrict__ pool,
                                                       const TailPhase* __restrict__ ph, int nph, ProbParams pp,
                                                       const StageSeg* __restrict__ segs, int nsegs) {
+  after_previous();
   extern __shared__ double smd[];
   for (int x = 0; x < nsegs; x++) {
     const StageSeg sg = segs[x];
@@ -573,57 +581,57 @@ template <class PL>
 struct Fp64Launchers {
   static int relax(const LaunchCtx& c, const Blk* blk, int nblk, int ipass) {
     if (nblk <= 0) return 0;
-    if (c.ndims == 2) k_relax<PL, 2><<<nblk, kBlock, 0, c.s>>>(c.P, c.pool, blk, ipass, c.pp);
-    else k_relax<PL, 3><<<nblk, kBlock, 0, c.s>>>(c.P, c.pool, blk, ipass, c.pp);
+    if (c.ndims == 2) launch_after(k_relax<PL, 2>, nblk, kBlock, 0, c.s, c.P, c.pool, blk, ipass, c.pp);
+    else launch_after(k_relax<PL, 3>, nblk, kBlock, 0, c.s, c.P, c.pool, blk, ipass, c.pp);
     return 1;
   }
   static int coarse_load(const LaunchCtx& c, const Blk* blk, int nblk) {
     if (nblk <= 0) return 0;
-    if (c.ndims == 2) k_coarse_load<PL, 2><<<nblk, kBlock, 0, c.s>>>(c.P, c.pool, blk, c.pp);
-    else k_coarse_load<PL, 3><<<nblk, kBlock, 0, c.s>>>(c.P, c.pool, blk, c.pp);
+    if (c.ndims == 2) launch_after(k_coarse_load<PL, 2>, nblk, kBlock, 0, c.s, c.P, c.pool, blk, c.pp);
+    else launch_after(k_coarse_load<PL, 3>, nblk, kBlock, 0, c.s, c.P, c.pool, blk, c.pp);
     return 1;
   }
   static int update_source(const LaunchCtx& c, const Blk* blk, int nblk) {
     if (nblk <= 0) return 0;
-    if (c.ndims == 2) k_update_source<PL, 2><<<nblk, kBlock, 0, c.s>>>(c.P, c.pool, blk, c.pp);
-    else k_update_source<PL, 3><<<nblk, kBlock, 0, c.s>>>(c.P, c.pool, blk, c.pp);
+    if (c.ndims == 2) launch_after(k_update_source<PL, 2>, nblk, kBlock, 0, c.s, c.P, c.pool, blk, c.pp);
+    else launch_after(k_update_source<PL, 3>, nblk, kBlock, 0, c.s, c.P, c.pool, blk, c.pp);
     return 1;
   }
   static int norm_partial(const LaunchCtx& c, const Blk* blk, int nblk, double* partial, int store_rf) {
     if (nblk <= 0) return 0;
     const int g = norm_partials(nblk), n = norm_group(nblk);
-    if (c.ndims == 2) k_norm_partial<PL, 2><<<g, kBlock, 0, c.s>>>(c.P, c.pool, blk, nblk, n, c.pp, partial, store_rf);
-    else k_norm_partial<PL, 3><<<g, kBlock, 0, c.s>>>(c.P, c.pool, blk, nblk, n, c.pp, partial, store_rf);
+    if (c.ndims == 2) launch_after(k_norm_partial<PL, 2>, g, kBlock, 0, c.s, c.P, c.pool, blk, nblk, n, c.pp, partial, store_rf);
+    else launch_after(k_norm_partial<PL, 3>, g, kBlock, 0, c.s, c.P, c.pool, blk, nblk, n, c.pp, partial, store_rf);
     return 1;
   }
   static int uni_norm(const LaunchCtx& c, int patch, const PatchDev& hp, double* partial, int store_rf, int update) {
     const int nblk = (int)((hp.sf + kBlock - 1) / kBlock), g = norm_partials(nblk), n = norm_group(nblk);
     const UniPatch u = uni_patch_of(hp);
     if (c.ndims == 2)
-      k_uni_norm<PL, 2><<<g, kBlock, 0, c.s>>>(c.P, c.pool, patch, u, n, c.pp, partial, store_rf, update);
+      launch_after(k_uni_norm<PL, 2>, g, kBlock, 0, c.s, c.P, c.pool, patch, u, n, c.pp, partial, store_rf, update);
     else
-      k_uni_norm<PL, 3><<<g, kBlock, 0, c.s>>>(c.P, c.pool, patch, u, n, c.pp, partial, store_rf, update);
+      launch_after(k_uni_norm<PL, 3>, g, kBlock, 0, c.s, c.P, c.pool, patch, u, n, c.pp, partial, store_rf, update);
     return 1;
   }
   static int get_source(const LaunchCtx& c, const Blk* blk, int nblk) {
     if (nblk <= 0) return 0;
-    if (c.ndims == 2) k_get_source<PL, 2><<<nblk, kBlock, 0, c.s>>>(c.P, c.pool, blk, c.pp);
-    else k_get_source<PL, 3><<<nblk, kBlock, 0, c.s>>>(c.P, c.pool, blk, c.pp);
+    if (c.ndims == 2) launch_after(k_get_source<PL, 2>, nblk, kBlock, 0, c.s, c.P, c.pool, blk, c.pp);
+    else launch_after(k_get_source<PL, 3>, nblk, kBlock, 0, c.s, c.P, c.pool, blk, c.pp);
     return 1;
   }
   static int tail(const LaunchCtx& c, const TailPhase* ph, int nph) {
     if (nph <= 0) return 0;
-    if (c.ndims == 2) k_tail<PL, 2><<<1, kBlock, 0, c.s>>>(c.P, c.pool, ph, nph, c.pp);
-    else k_tail<PL, 3><<<1, kBlock, 0, c.s>>>(c.P, c.pool, ph, nph, c.pp);
+    if (c.ndims == 2) launch_after(k_tail<PL, 2>, 1, kBlock, 0, c.s, c.P, c.pool, ph, nph, c.pp);
+    else launch_after(k_tail<PL, 3>, 1, kBlock, 0, c.s, c.P, c.pool, ph, nph, c.pp);
     return 1;
   }
   static int tail_smem(const LaunchCtx& c, const PatchDev* shadow, const TailPhase* ph, int nph,
                        const StageSeg* segs, int nsegs, int smem_bytes) {
     if (nph <= 0) return 0;
     if (c.ndims == 2)
-      k_tail_smem<PL, 2><<<1, kBlock, smem_bytes, c.s>>>(shadow, c.pool, ph, nph, c.pp, segs, nsegs);
+      launch_after(k_tail_smem<PL, 2>, 1, kBlock, smem_bytes, c.s, shadow, c.pool, ph, nph, c.pp, segs, nsegs);
     else
-      k_tail_smem<PL, 3><<<1, kBlock, smem_bytes, c.s>>>(shadow, c.pool, ph, nph, c.pp, segs, nsegs);
+      launch_after(k_tail_smem<PL, 3>, 1, kBlock, smem_bytes, c.s, shadow, c.pool, ph, nph, c.pp, segs, nsegs);
     return 1;
   }
   static int tail_smem_attributes() {

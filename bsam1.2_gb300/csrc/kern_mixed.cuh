@@ -217,6 +217,7 @@ __device__ __forceinline__ void u_prep(const PatchDev* __restrict__ P, double* p
 template <class PL, int DIM>
 __global__ void __launch_bounds__(kBlock) k_mx_prep(const PatchDev* __restrict__ P, double* pool, float* fpool,
                                                     const Blk* __restrict__ blk, int mode, ProbParams pp) {
+  after_previous();
   u_prep<PL, DIM>(P, pool, fpool, blk[blockIdx.x], threadIdx.x, mode, pp);
 }
 
@@ -280,6 +281,7 @@ __device__ __forceinline__ void u_relax_any(const PatchDev* __restrict__ P, floa
 template <class PL, int DIM, typename T>
 __global__ void __launch_bounds__(kBlock) k_mx_relax(const PatchDev* __restrict__ P, float* __restrict__ fpool,
                                                      const Blk* __restrict__ blk, int ipass, MxParams mp) {
+  after_previous();
   u_relax<PL, DIM, false, T>(P, fpool, blk[blockIdx.x], threadIdx.x, ipass, mp);
 }
 
@@ -323,6 +325,7 @@ __device__ __forceinline__ void u_coarse_load(const PatchDev* __restrict__ P, fl
 template <class PL, int DIM>
 __global__ void __launch_bounds__(kBlock) k_mx_coarse_load(const PatchDev* __restrict__ P, float* __restrict__ fpool,
                                                            const Blk* __restrict__ blk, MxParams mp) {
+  after_previous();
   u_coarse_load<PL, DIM>(P, fpool, blk[blockIdx.x], threadIdx.x, mp);
 }
 
@@ -337,6 +340,7 @@ template <class PL, int DIM>
 __global__ void __launch_bounds__(kBlock) k_mx_norm(const PatchDev* __restrict__ P, double* __restrict__ pool,
                                                     const Blk* __restrict__ blk, ProbParams pp,
                                                     double* __restrict__ partial) {
+  after_previous();
   constexpr int NV = PL::kNV;
   __shared__ double red[NV][kBlock / 32];
   double s[NV];
@@ -379,6 +383,7 @@ template <class PL, int DIM>
 __global__ void __launch_bounds__(kBlock) k_mx_track(const PatchDev* __restrict__ P, float* __restrict__ fpool,
                                                      const Blk* __restrict__ blk, double* __restrict__ partial,
                                                      MxParams mp) {
+  after_previous();
   constexpr int NV = PL::kNV;
   __shared__ float red[NV][kBlock / 32];
   const Blk b = blk[blockIdx.x];
@@ -452,6 +457,7 @@ __device__ __forceinline__ void run_tail(const PatchDev* __restrict__ P, float* 
 template <class PL, int DIM>
 __global__ void __launch_bounds__(kBlock) k_mx_tail(const PatchDev* __restrict__ P, float* __restrict__ fpool,
                                                    const TailPhase* __restrict__ ph, int nph, int nrvars, MxParams mp) {
+  after_previous();
   run_tail<PL, DIM>(P, fpool, ph, nph, nrvars, mp);
 }
 
@@ -463,6 +469,7 @@ template <class PL, int DIM>
 __global__ void __launch_bounds__(kBlock) k_mx_tail_smem(const PatchDev* __restrict__ P, float* __restrict__ fpool,
                                                         const TailPhase* __restrict__ ph, int nph, int nrvars,
                                                         MxParams mp, const StageSeg* __restrict__ segs, int nsegs) {
+  after_previous();
   extern __shared__ float sm[];
   for (int x = 0; x < nsegs; x++) {
     const StageSeg sg = segs[x];
@@ -567,8 +574,8 @@ template <class PL>
 struct Launchers {
   static int prep(const MxLaunch& L, const Blk* blk, int nblk, int mode) {
     if (nblk <= 0) return 0;
-    if (L.ndims == 2) k_mx_prep<PL, 2><<<nblk, kBlock, 0, L.s>>>(L.P, L.pool, L.fpool, blk, mode, L.pp);
-    else k_mx_prep<PL, 3><<<nblk, kBlock, 0, L.s>>>(L.P, L.pool, L.fpool, blk, mode, L.pp);
+    if (L.ndims == 2) launch_after(k_mx_prep<PL, 2>, nblk, kBlock, 0, L.s, L.P, L.pool, L.fpool, blk, mode, L.pp);
+    else launch_after(k_mx_prep<PL, 3>, nblk, kBlock, 0, L.s, L.P, L.pool, L.fpool, blk, mode, L.pp);
     return 1;
   }
   static int relax(const MxLaunch& L, const Blk* blk, int nblk, int ipass) {
@@ -576,32 +583,32 @@ struct Launchers {
     MxParams mp = PL::mx_params(L.pp);
     const int ip = ipass & 3;
     if (ipass & kRelax64) {
-      if (L.ndims == 2) k_mx_relax<PL, 2, double><<<nblk, kBlock, 0, L.s>>>(L.P, L.fpool, blk, ip, mp);
-      else k_mx_relax<PL, 3, double><<<nblk, kBlock, 0, L.s>>>(L.P, L.fpool, blk, ip, mp);
+      if (L.ndims == 2) launch_after(k_mx_relax<PL, 2, double>, nblk, kBlock, 0, L.s, L.P, L.fpool, blk, ip, mp);
+      else launch_after(k_mx_relax<PL, 3, double>, nblk, kBlock, 0, L.s, L.P, L.fpool, blk, ip, mp);
     } else {
-      if (L.ndims == 2) k_mx_relax<PL, 2, float><<<nblk, kBlock, 0, L.s>>>(L.P, L.fpool, blk, ip, mp);
-      else k_mx_relax<PL, 3, float><<<nblk, kBlock, 0, L.s>>>(L.P, L.fpool, blk, ip, mp);
+      if (L.ndims == 2) launch_after(k_mx_relax<PL, 2, float>, nblk, kBlock, 0, L.s, L.P, L.fpool, blk, ip, mp);
+      else launch_after(k_mx_relax<PL, 3, float>, nblk, kBlock, 0, L.s, L.P, L.fpool, blk, ip, mp);
     }
     return 1;
   }
   static int coarse_load(const MxLaunch& L, const Blk* blk, int nblk) {
     if (nblk <= 0) return 0;
     MxParams mp = PL::mx_params(L.pp);
-    if (L.ndims == 2) k_mx_coarse_load<PL, 2><<<nblk, kBlock, 0, L.s>>>(L.P, L.fpool, blk, mp);
-    else k_mx_coarse_load<PL, 3><<<nblk, kBlock, 0, L.s>>>(L.P, L.fpool, blk, mp);
+    if (L.ndims == 2) launch_after(k_mx_coarse_load<PL, 2>, nblk, kBlock, 0, L.s, L.P, L.fpool, blk, mp);
+    else launch_after(k_mx_coarse_load<PL, 3>, nblk, kBlock, 0, L.s, L.P, L.fpool, blk, mp);
     return 1;
   }
   static int track(const MxLaunch& L, const Blk* blk, int nblk, double* partial) {
     if (nblk <= 0) return 0;
     MxParams mp = PL::mx_params(L.pp);
-    if (L.ndims == 2) k_mx_track<PL, 2><<<nblk, kBlock, 0, L.s>>>(L.P, L.fpool, blk, partial, mp);
-    else k_mx_track<PL, 3><<<nblk, kBlock, 0, L.s>>>(L.P, L.fpool, blk, partial, mp);
+    if (L.ndims == 2) launch_after(k_mx_track<PL, 2>, nblk, kBlock, 0, L.s, L.P, L.fpool, blk, partial, mp);
+    else launch_after(k_mx_track<PL, 3>, nblk, kBlock, 0, L.s, L.P, L.fpool, blk, partial, mp);
     return 1;
   }
   static int norm(const MxLaunch& L, const Blk* padded, int nb, double* partial) {
     if (nb <= 0) return 0;
-    if (L.ndims == 2) k_mx_norm<PL, 2><<<nb, kBlock, 0, L.s>>>(L.P, L.pool, padded, L.pp, partial);
-    else k_mx_norm<PL, 3><<<nb, kBlock, 0, L.s>>>(L.P, L.pool, padded, L.pp, partial);
+    if (L.ndims == 2) launch_after(k_mx_norm<PL, 2>, nb, kBlock, 0, L.s, L.P, L.pool, padded, L.pp, partial);
+    else launch_after(k_mx_norm<PL, 3>, nb, kBlock, 0, L.s, L.P, L.pool, padded, L.pp, partial);
     return 1;
   }
   static int tail(const MxLaunch& L, const PatchDev* table, const TailPhase* ph, int nph, const StageSeg* segs,
@@ -611,12 +618,12 @@ struct Launchers {
     int nr = L.pp.nrvars;
     if (smem_bytes) {
       if (L.ndims == 2)
-        k_mx_tail_smem<PL, 2><<<1, kBlock, smem_bytes, L.s>>>(table, L.fpool, ph, nph, nr, mp, segs, nsegs);
+        launch_after(k_mx_tail_smem<PL, 2>, 1, kBlock, smem_bytes, L.s, table, L.fpool, ph, nph, nr, mp, segs, nsegs);
       else
-        k_mx_tail_smem<PL, 3><<<1, kBlock, smem_bytes, L.s>>>(table, L.fpool, ph, nph, nr, mp, segs, nsegs);
+        launch_after(k_mx_tail_smem<PL, 3>, 1, kBlock, smem_bytes, L.s, table, L.fpool, ph, nph, nr, mp, segs, nsegs);
     } else {
-      if (L.ndims == 2) k_mx_tail<PL, 2><<<1, kBlock, 0, L.s>>>(table, L.fpool, ph, nph, nr, mp);
-      else k_mx_tail<PL, 3><<<1, kBlock, 0, L.s>>>(table, L.fpool, ph, nph, nr, mp);
+      if (L.ndims == 2) launch_after(k_mx_tail<PL, 2>, 1, kBlock, 0, L.s, table, L.fpool, ph, nph, nr, mp);
+      else launch_after(k_mx_tail<PL, 3>, 1, kBlock, 0, L.s, table, L.fpool, ph, nph, nr, mp);
     }
     return 1;
   }

@@ -492,18 +492,21 @@ template <class TR, int DIM>
 __global__ void __launch_bounds__(kBlock) k_uni_relax(const PatchDev* __restrict__ P, typename TR::Mem m, int patch,
                                                       const __grid_constant__ UniPatch p, int ipass, int full, UniBC bc,
                                                       typename TR::Par par) {
+  after_previous();
   relax<TR, DIM>(global_view<TR, DIM>(p.p, p.d, m), ipass, full, UNI_T0, P[patch], bc, par);
 }
 template <class TR, int DIM>
 __global__ void __launch_bounds__(kBlock) k_uni_restrict(typename TR::Mem m, const __grid_constant__ UniPatch p,
                                                          const __grid_constant__ UniPatch u, UniBC bc,
                                                          typename TR::Par par) {
+  after_previous();
   restrict_q<TR, DIM>(global_view<TR, DIM>(p.p, p.d, m), global_view<TR, DIM>(u.p, u.d, m), UNI_T0, bc, par);
 }
 template <class TR, int DIM>
 __global__ void __launch_bounds__(kBlock) k_uni_load(const PatchDev* __restrict__ P, typename TR::Mem m, int patch,
                                                      const __grid_constant__ UniPatch p, int parent,
                                                      const __grid_constant__ UniPatch u, typename TR::Par par) {
+  after_previous();
   coarse_load<TR, DIM>(global_view<TR, DIM>(p.p, p.d, m), global_view<TR, DIM>(u.p, u.d, m), TR::rf(p.p, m), UNI_T0,
                        P[patch], P[parent], par);
 }
@@ -511,18 +514,21 @@ template <class TR, int DIM>
 __global__ void __launch_bounds__(kBlock) k_uni_correct_a(typename TR::Mem m, const __grid_constant__ UniPatch p,
                                                           const __grid_constant__ UniPatch u, UniBC bc,
                                                           typename TR::Par par) {
+  after_previous();
   correct_a<TR, DIM, true>(global_view<TR, DIM>(p.p, p.d, m), global_view<TR, DIM>(u.p, u.d, m), UNI_T0, bc, par);
 }
 template <class TR, int DIM>
 __global__ void __launch_bounds__(kBlock) k_uni_correct_b(typename TR::Mem m, const __grid_constant__ UniPatch p,
                                                           const __grid_constant__ UniPatch u, UniBC bc,
                                                           typename TR::Par par) {
+  after_previous();
   correct_b<TR, DIM, !TR::kStoreRf>(global_view<TR, DIM>(p.p, p.d, m), global_view<TR, DIM>(u.p, u.d, m), UNI_T0, bc,
                                     par);
 }
 template <class TR, int DIM>
 __global__ void __launch_bounds__(kBlock) k_uni_ghost(typename TR::Mem m, const __grid_constant__ UniPatch p, UniBC bc,
                                                       typename TR::Par par) {
+  after_previous();
   const View<typename TR::T> V = global_view<TR, DIM>(p.p, p.d, m);
   set_ghost<TR, DIM>(V.q, V.g, p.d, UNI_T0, bc, par);
 }
@@ -530,6 +536,7 @@ template <class TR, int DIM>
 __global__ void __launch_bounds__(kBlock) k_uni_fill(typename TR::Mem m, const __grid_constant__ UniPatch p,
                                                      const __grid_constant__ UniPatch u, int fields, UniBC bc,
                                                      typename TR::Par par) {
+  after_previous();
   fill_down<TR, DIM>(global_view<TR, DIM>(p.p, p.d, m), global_view<TR, DIM>(u.p, u.d, m), fields, UNI_T0, bc, par);
 }
 
@@ -550,6 +557,7 @@ template <class TR, int DIM>
 __global__ void __launch_bounds__(kUniFillThreads) k_uni_fill_small(const PatchDev* __restrict__ P, typename TR::Mem m,
                                                                     const __grid_constant__ UniCycle A, int fields,
                                                                     typename TR::Par par) {
+  after_previous();
   __shared__ __align__(16) PatchDev sp[kNLev];
   stage_table(sp, P, A);
   for (int x = 0; x + 1 < A.nl; x++) {
@@ -976,6 +984,7 @@ template <class TR, int DIM>
 __global__ void __launch_bounds__(kUniThreads, 1) k_uni_cycle(const PatchDev* __restrict__ P, typename TR::Mem m,
                                                               const __grid_constant__ UniCycle A,
                                                               typename TR::Par par) {
+  after_previous();
   using T = typename TR::T;
   const int rank = A.ctas > 1 ? my_rank() : 0;
   const int t = threadIdx.x, nt = blockDim.x;
@@ -1056,20 +1065,20 @@ struct UniLaunchers {
     const UniPatch p = uni_patch_of(hp);
     const int nb = blocks((long long)((hp.mx[0] + 1) / 2) * hp.mx[1] * hp.mx[2]);
     if (c.ndims == 2)
-      k_uni_relax<TR, 2><<<nb, kBlock, 0, c.s>>>(c.P, TR::mem(c), patch, p, ipass, full, bc, TR::par(c));
+      launch_after(k_uni_relax<TR, 2>, nb, kBlock, 0, c.s, c.P, TR::mem(c), patch, p, ipass, full, bc, TR::par(c));
     else
-      k_uni_relax<TR, 3><<<nb, kBlock, 0, c.s>>>(c.P, TR::mem(c), patch, p, ipass, full, bc, TR::par(c));
+      launch_after(k_uni_relax<TR, 3>, nb, kBlock, 0, c.s, c.P, TR::mem(c), patch, p, ipass, full, bc, TR::par(c));
     return 1;
   }
   static int restrict_load(const LaunchCtx& c, const UniBC& bc, int patch, const PatchDev& hp, const PatchDev& hu) {
     const UniPatch p = uni_patch_of(hp), u = uni_patch_of(hu);
     const int nb = blocks(cells(hp.cmx));
     if (c.ndims == 2) {
-      k_uni_restrict<TR, 2><<<nb, kBlock, 0, c.s>>>(TR::mem(c), p, u, bc, TR::par(c));
-      k_uni_load<TR, 2><<<nb, kBlock, 0, c.s>>>(c.P, TR::mem(c), patch, p, hp.parent, u, TR::par(c));
+      launch_after(k_uni_restrict<TR, 2>, nb, kBlock, 0, c.s, TR::mem(c), p, u, bc, TR::par(c));
+      launch_after(k_uni_load<TR, 2>, nb, kBlock, 0, c.s, c.P, TR::mem(c), patch, p, hp.parent, u, TR::par(c));
     } else {
-      k_uni_restrict<TR, 3><<<nb, kBlock, 0, c.s>>>(TR::mem(c), p, u, bc, TR::par(c));
-      k_uni_load<TR, 3><<<nb, kBlock, 0, c.s>>>(c.P, TR::mem(c), patch, p, hp.parent, u, TR::par(c));
+      launch_after(k_uni_restrict<TR, 3>, nb, kBlock, 0, c.s, TR::mem(c), p, u, bc, TR::par(c));
+      launch_after(k_uni_load<TR, 3>, nb, kBlock, 0, c.s, c.P, TR::mem(c), patch, p, hp.parent, u, TR::par(c));
     }
     return 2;
   }
@@ -1078,34 +1087,34 @@ struct UniLaunchers {
     int n = 1;
     if (TR::kStoreRf) {
       const int na = blocks(cells(hp.cn));
-      if (c.ndims == 2) k_uni_correct_a<TR, 2><<<na, kBlock, 0, c.s>>>(TR::mem(c), p, u, bc, TR::par(c));
-      else k_uni_correct_a<TR, 3><<<na, kBlock, 0, c.s>>>(TR::mem(c), p, u, bc, TR::par(c));
+      if (c.ndims == 2) launch_after(k_uni_correct_a<TR, 2>, na, kBlock, 0, c.s, TR::mem(c), p, u, bc, TR::par(c));
+      else launch_after(k_uni_correct_a<TR, 3>, na, kBlock, 0, c.s, TR::mem(c), p, u, bc, TR::par(c));
       n++;
     }
     const int nb = blocks((long long)(hp.cmx[0] + 1) * (hp.cmx[1] + 1) * (c.ndims == 3 ? hp.cmx[2] + 1 : 1));
-    if (c.ndims == 2) k_uni_correct_b<TR, 2><<<nb, kBlock, 0, c.s>>>(TR::mem(c), p, u, bc, TR::par(c));
-    else k_uni_correct_b<TR, 3><<<nb, kBlock, 0, c.s>>>(TR::mem(c), p, u, bc, TR::par(c));
+    if (c.ndims == 2) launch_after(k_uni_correct_b<TR, 2>, nb, kBlock, 0, c.s, TR::mem(c), p, u, bc, TR::par(c));
+    else launch_after(k_uni_correct_b<TR, 3>, nb, kBlock, 0, c.s, TR::mem(c), p, u, bc, TR::par(c));
     return n;
   }
   static int ghost(const LaunchCtx& c, const UniBC& bc, const PatchDev& hp) {
     const UniPatch p = uni_patch_of(hp);
     const int nb = blocks(cells(hp.qn) - cells(hp.mx));
-    if (c.ndims == 2) k_uni_ghost<TR, 2><<<nb, kBlock, 0, c.s>>>(TR::mem(c), p, bc, TR::par(c));
-    else k_uni_ghost<TR, 3><<<nb, kBlock, 0, c.s>>>(TR::mem(c), p, bc, TR::par(c));
+    if (c.ndims == 2) launch_after(k_uni_ghost<TR, 2>, nb, kBlock, 0, c.s, TR::mem(c), p, bc, TR::par(c));
+    else launch_after(k_uni_ghost<TR, 3>, nb, kBlock, 0, c.s, TR::mem(c), p, bc, TR::par(c));
     return 1;
   }
   static int fill(const LaunchCtx& c, const UniBC& bc, const PatchDev& hp, const PatchDev& hu, int fields) {
     const UniPatch p = uni_patch_of(hp), u = uni_patch_of(hu);
     const int nb = blocks(cells(hp.cmx));
-    if (c.ndims == 2) k_uni_fill<TR, 2><<<nb, kBlock, 0, c.s>>>(TR::mem(c), p, u, fields, bc, TR::par(c));
-    else k_uni_fill<TR, 3><<<nb, kBlock, 0, c.s>>>(TR::mem(c), p, u, fields, bc, TR::par(c));
+    if (c.ndims == 2) launch_after(k_uni_fill<TR, 2>, nb, kBlock, 0, c.s, TR::mem(c), p, u, fields, bc, TR::par(c));
+    else launch_after(k_uni_fill<TR, 3>, nb, kBlock, 0, c.s, TR::mem(c), p, u, fields, bc, TR::par(c));
     return 1;
   }
   static int fill_small(const LaunchCtx& c, const UniCycle& A, int fields) {
     if (c.ndims == 2)
-      k_uni_fill_small<TR, 2><<<1, kUniFillThreads, 0, c.s>>>(c.P, TR::mem(c), A, fields, TR::par(c));
+      launch_after(k_uni_fill_small<TR, 2>, 1, kUniFillThreads, 0, c.s, c.P, TR::mem(c), A, fields, TR::par(c));
     else
-      k_uni_fill_small<TR, 3><<<1, kUniFillThreads, 0, c.s>>>(c.P, TR::mem(c), A, fields, TR::par(c));
+      launch_after(k_uni_fill_small<TR, 3>, 1, kUniFillThreads, 0, c.s, c.P, TR::mem(c), A, fields, TR::par(c));
     return 1;
   }
   static int cycle(const LaunchCtx& c, const UniCycle& A, int smem) {
@@ -1114,13 +1123,15 @@ struct UniLaunchers {
     cfg.blockDim = dim3(A.threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = c.s;
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = A.ctas;
     at[0].val.clusterDim.y = 1;
     at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     cudaError_t e = c.ndims == 2 ? cudaLaunchKernelEx(&cfg, k_uni_cycle<TR, 2>, c.P, TR::mem(c), A, TR::par(c))
                                  : cudaLaunchKernelEx(&cfg, k_uni_cycle<TR, 3>, c.P, TR::mem(c), A, TR::par(c));
     return e == cudaSuccess ? 1 : -1;

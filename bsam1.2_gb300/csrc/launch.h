@@ -4,6 +4,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <utility>
+
 #include "internal.h"
 
 namespace bsamg {
@@ -285,5 +287,34 @@ int launch_tail(const LaunchCtx& c, const TailPhase* ph, int nph);
 int launch_tail_smem(const LaunchCtx& c, const PatchDev* shadow, const TailPhase* ph, int nph, const StageSeg* segs,
                      int nsegs, int smem_bytes);
 int tail_smem_attributes(int problem);
+
+#ifdef __CUDACC__
+// Programmatic dependent launch: a kernel launched by launch_after may be set
+// up, its CTAs resident, while the kernel before it in the stream still runs,
+// which takes part of the launch latency off chains of small kernels (a V-cycle
+// of 30 to 110 launches: 2 to 5 % of it).  Its first statement is
+// after_previous(): it lets the next kernel do the same and waits until the
+// one before has finished and its writes are visible.  Grids of many waves are
+// launched in the plain order: their early CTAs wait in the slots of the
+// running kernel's last wave (a step at 256^3 5.43 -> 5.56 ms).
+constexpr unsigned kEarlyCtas = 1024;
+__device__ __forceinline__ void after_previous() {
+  asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory");
+}
+template <typename... P, typename... A>
+inline void launch_after(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... a) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = (unsigned long long)grid.x * grid.y * grid.z <= kEarlyCtas ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, k, std::forward<A>(a)...);
+}
+#endif
 
 }  // namespace bsamg

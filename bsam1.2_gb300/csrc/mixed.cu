@@ -44,18 +44,21 @@ using namespace mx;
 template <int DIM>
 __global__ void __launch_bounds__(kBlock) k_mx_restrict(const PatchDev* __restrict__ P, float* __restrict__ fpool,
                                                         const Blk* __restrict__ blk, int nrvars) {
+  after_previous();
   u_restrict<DIM>(P, fpool, blk[blockIdx.x], threadIdx.x, nrvars);
 }
 
 template <int DIM>
 __global__ void __launch_bounds__(kBlock) k_mx_coarse_ring(const PatchDev* __restrict__ P, float* __restrict__ fpool,
                                                            const Blk* __restrict__ blk, int nrvars, int corr) {
+  after_previous();
   u_coarse_ring<DIM>(P, fpool, blk[blockIdx.x], threadIdx.x, nrvars, corr);
 }
 
 template <int DIM>
 __global__ void __launch_bounds__(kBlock) k_mx_prolong(const PatchDev* __restrict__ P, float* __restrict__ fpool,
                                                        const Blk* __restrict__ blk, int nrvars) {
+  after_previous();
   u_prolong<DIM>(P, fpool, blk[blockIdx.x], threadIdx.x, nrvars);
 }
 
@@ -64,11 +67,13 @@ template <int DIM>
 __global__ void __launch_bounds__(kBlock) k_mx_update(const PatchDev* __restrict__ P, double* __restrict__ pool,
                                                       float* __restrict__ fpool, const Blk* __restrict__ blk,
                                                       int nrvars, int nbase) {
+  after_previous();
   u_update<DIM>(P, pool, fpool, blk[blockIdx.x], threadIdx.x, nrvars, nbase);
 }
 
 __global__ void __launch_bounds__(kBlock) k_ghost32_stage(const PatchDev* __restrict__ P, float* __restrict__ fpool,
                                                           const GhostOp* __restrict__ ops, int n, int nrvars) {
+  after_previous();
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
   GhostOp g = ops[t];
@@ -79,6 +84,7 @@ __global__ void __launch_bounds__(kBlock) k_ghost32_program(const PatchDev* __re
                                                             const GhostOp* __restrict__ ops,
                                                             const int* __restrict__ stage_off, int nstages,
                                                             int nrvars) {
+  after_previous();
   for (int s = 0; s < nstages; s++) {
     for (int t = stage_off[s] + threadIdx.x; t < stage_off[s + 1]; t += blockDim.x) {
       GhostOp g = ops[t];
@@ -106,8 +112,8 @@ __global__ void __launch_bounds__(kBlock) k_gather_ops(const GhostOp* const* __r
   do {                                                                                      \
     int nb__ = L.nblk[kind];                                                                \
     if (nb__ > 0) {                                                                         \
-      if ((H).ndims == 2) KER<2><<<nb__, kBlock, 0, (H).s>>>(__VA_ARGS__);                  \
-      else KER<3><<<nb__, kBlock, 0, (H).s>>>(__VA_ARGS__);                                 \
+      if ((H).ndims == 2) launch_after(KER<2>, nb__, kBlock, 0, (H).s, __VA_ARGS__);                  \
+      else launch_after(KER<3>, nb__, kBlock, 0, (H).s, __VA_ARGS__);                                 \
       int r__ = after_launch(H, 1);                                                         \
       if (r__) return r__;                                                                  \
     }                                                                                       \
@@ -138,13 +144,13 @@ int mx_set_ghost(Hier& H, int level, int ipass) {
   }
   int nops = g.stage_off[nst];
   if (ghost_in_one_cta(nst, nops)) {
-    k_ghost32_program<<<1, kBlock, 0, H.s>>>(H.dP, H.fpool, g.d_ops, g.d_stage_off, nst, H.nrvars);
+    launch_after(k_ghost32_program, 1, kBlock, 0, H.s, H.dP, H.fpool, g.d_ops, g.d_stage_off, nst, H.nrvars);
     return after_launch(H, 1);
   }
   for (int s = 0; s < nst; s++) {
     int n = g.stage_off[s + 1] - g.stage_off[s];
     if (n <= 0) continue;
-    k_ghost32_stage<<<(n + kBlock - 1) / kBlock, kBlock, 0, H.s>>>(H.dP, H.fpool, g.d_ops + g.stage_off[s], n,
+    launch_after(k_ghost32_stage, (n + kBlock - 1) / kBlock, kBlock, 0, H.s, H.dP, H.fpool, g.d_ops + g.stage_off[s], n,
                                                                     H.nrvars);
     int r = after_launch(H, 1);
     if (r) return r;
