@@ -1,4 +1,4 @@
-// IEEE double sums on the integer pipe.
+// IEEE double sums and quotients on the integer pipe.
 //
 // GB300 issues one FP64 warp instruction per scheduler every 77 cycles (64
 // when a warp is alone on its SM), against about one integer instruction a
@@ -12,9 +12,10 @@
 // cancels to less than 2^-26 of the largest operand, the additions are done
 // as additions.
 //
-// Measured (GB300): a 3D CH sweep has 27 FP64 instructions a cell instead of
-// 38 and 500 integer ones, 256^3: 612 -> 440 us a colour; the residual norm
-// 12 instead of 32, 1143 -> 660 us.
+// Measured (GB300), a 3D CH sweep of 256^3, a colour: 38 FP64 instructions a
+// cell, 612 us; 27 with the sums and about 500 integer ones, 440 us; 14 with
+// the two quotients, 344 us.  The residual norm 12 instead of 32, 1143 -> 660
+// us.
 #pragma once
 #ifndef FXP_CPU  // a test compiles this file for the host, with the intrinsics it spells out
 #include <cuda_runtime.h>
@@ -208,6 +209,107 @@ __device__ __forceinline__ double scaled(double x) {
   double y = __hiloint2double(hi + K * (1 << 20), __double2loint(x));
   if ((unsigned)(e - 8) >= 2030u) y = plain_mul(x, K < 0 ? 1.0 / (1 << (K < 0 ? -K : 0)) : 1.0 * (1 << (K > 0 ? K : 0)));
   return y;
+}
+
+// ---- quotients ----
+//
+// RN(a / b) needs seven FP64 instructions for a correctly rounded reciprocal
+// and three for each quotient; on the integer pipe it is a reciprocal of 60
+// bits (35 instructions) and, for each quotient, a product, a remainder and
+// one comparison (40).  Two quotients of one divisor share the reciprocal.
+//
+// The significand of b as D in [2^63, 2^64); x = 2^63 / D in (0.5, 1].  A
+// single-precision reciprocal of D's leading 24 bits is x to 2^-21.7, a
+// Newton step x (2 - x / x_true) to 2^-42.9 and another to 2^-59.8, where
+// the steps' truncations are kept on one side: the result never exceeds x,
+// so that neither does the quotient T with ten bits below its last place,
+// and T, rounded, is the correctly rounded quotient or the value below it.
+// The remainder, exact modulo 2^64, tells which; there are no ties.
+FXP_CALL double plain_div(double a, double b) { return a / b; }
+
+#ifdef FXP_CPU
+#ifndef FXP_SEED_ULPS
+#define FXP_SEED_ULPS 0
+#endif
+static inline unsigned seed_bits(unsigned d) {  // the device's approximation is within one unit of this
+  float f, r;
+  memcpy(&f, &d, 4);
+  r = 1.0f / f;
+  unsigned u;
+  memcpy(&u, &r, 4);
+  return u + FXP_SEED_ULPS;
+}
+#else
+__device__ __forceinline__ unsigned seed_bits(unsigned d) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(__uint_as_float(d)));
+  return __float_as_uint(r);
+}
+#endif
+
+// a divisor: its significand m in [2^52, 2^53), its exponent and y = x 2^64,
+// at most 10 units low
+struct Divisor {
+  unsigned long long m, y;
+  int e;
+};
+__device__ __forceinline__ Divisor divisor(double b) {
+  Divisor r;
+  const unsigned hi = (unsigned)__double2hiint(b), lo = (unsigned)__double2loint(b);
+  r.e = (int)(hi >> 20);  // b > 0
+  const unsigned mh = (hi & 0xfffffu) | 0x100000u;
+  r.m = ((unsigned long long)mh << 32) | lo;
+  const unsigned dh = __funnelshift_l(lo, mh, 11), dl = lo << 11;
+  // y0 = x 2^32: the seed's 24 bits (a seed of 1 counts as the value below it)
+  const unsigned s = seed_bits(0x3f800000u | ((dh >> 8) & 0x7fffffu));
+  const unsigned y0 = (min((int)s, 0x3f7fffff) << 8) | 0x80000000u;
+  // 1 - x^-1 y0 in units of 2^-52, below 2^31
+  const unsigned long long p = (unsigned long long)dh * y0 + (((unsigned long long)dl * y0) >> 32);
+  const int e1 = (int)((long long)(0x8000000000000000ull - p) >> 11);
+  const unsigned long long y1 = ((unsigned long long)y0 << 32) + (unsigned long long)(((long long)e1 * (int)(y0 >> 1)) >> 19);
+  // 1 - x^-1 y1 in units of 2^-63, below 2^21: its low 32 bits are all of it
+  const unsigned yh = (unsigned)(y1 >> 32), yl = (unsigned)y1;
+  const unsigned long long c1 = (unsigned long long)dl * yh, c2 = (unsigned long long)dh * yl;
+  const unsigned long long mid = (c1 & 0xffffffffull) + (c2 & 0xffffffffull);
+  const unsigned low = dh * yh + (unsigned)(c1 >> 32) + (unsigned)(c2 >> 32) + (unsigned)(mid >> 32);
+  const int e2 = -(int)low - 4;  // four units to stay below x, whatever was cut off
+  r.y = y1 + (unsigned long long)(((long long)e2 * (int)(yh >> 1)) >> 30);
+  return r;
+}
+// 1 <= b < 2^400 and 2^-400 <= |a| < 2^400: quotients in the normal range
+__device__ __forceinline__ bool divides(double b) { return ((unsigned)__double2hiint(b) >> 20) - 1023u < 400u; }
+__device__ __forceinline__ bool divisible(double a) { return (unsigned)(exponent(a) - (1023 - 400)) <= 799u; }
+__device__ __forceinline__ double quotient(double a, const Divisor& b) {
+  const unsigned hi = (unsigned)__double2hiint(a), lo = (unsigned)__double2loint(a);
+  unsigned long long A = ((unsigned long long)((hi & 0xfffffu) | 0x100000u) << 32) | lo;
+  const int half = A < b.m;  // a quotient of significands in [1, 2)
+  A <<= half;
+#ifdef FXP_CPU
+  const unsigned long long T = (unsigned long long)(((unsigned __int128)(A << 10) * b.y) >> 64);
+#else
+  const unsigned long long T = __umul64hi(A << 10, b.y);
+#endif
+  unsigned long long q = (T + 512u) >> 10;
+  const long long rem = (long long)((A << 52) - q * b.m);
+  q += 2 * rem > (long long)b.m;
+  const int e = (int)((hi >> 20) & 0x7ff) - b.e + 1023 - half;
+  return __hiloint2double((int)(((hi & 0x80000000u) | ((unsigned)(e - 1) << 20)) + (unsigned)(q >> 32)), (int)q);
+}
+// RN(a / b)
+__device__ __forceinline__ double quot(double a, double b) {
+  double q = quotient(a, divisor(b));
+  if (!(divides(b) && divisible(a))) q = plain_div(a, b);
+  return q;
+}
+// RN(a0 / b), RN(a1 / b)
+__device__ __forceinline__ void quot2(double a0, double a1, double b, double& q0, double& q1) {
+  const Divisor d = divisor(b);
+  q0 = quotient(a0, d);
+  q1 = quotient(a1, d);
+  if (!(divides(b) && divisible(a0) && divisible(a1))) {
+    q0 = plain_div(a0, b);
+    q1 = plain_div(a1, b);
+  }
 }
 
 }  // namespace fxp

@@ -54,10 +54,11 @@ struct BioGrowth {
       double phi = q0[c];
       double ol = x.qold[c];
       double tmp2 = cf[2] + dt * sqr(phi);
-      q0[c] = (f0[fc] + dt * (pp.gamma * 0.5 * (ol + 1.0)) * (q1[c] - pp.czero) +
-               cf[0] * (q0[c - 1] + q0[c + 1] + q0[c - sy] + q0[c + sy])) / tmp2;
+      // the divisions on the integer pipe, to the same bits
+      q0[c] = fxp::quot(f0[fc] + dt * (pp.gamma * 0.5 * (ol + 1.0)) * (q1[c] - pp.czero) +
+                        cf[0] * (q0[c - 1] + q0[c + 1] + q0[c - sy] + q0[c + sy]), tmp2);
       double tmp4 = cf[3] + (pp.lambda * 0.5 * (ol + 1.0));
-      q1[c] = (f1[fc] + cf[1] * (q1[c + 1] + q1[c - 1] + q1[c + sy] + q1[c - sy])) / tmp4;
+      q1[c] = fxp::quot(f1[fc] + cf[1] * (q1[c + 1] + q1[c - 1] + q1[c + sy] + q1[c - sy]), tmp4);
     } else {
       q0[c] = 0.0;
       q1[c] = 0.0;

@@ -67,7 +67,7 @@ struct CH {
     }
     double det = 1.0 - cf[3] * a21;  // >= 1: a21 <= -tmp3 < 0
     // the reference's two divisions by det, :365-366 (:609-610), each
-    // correctly rounded as `/` is, from one reciprocal
+    // correctly rounded as `/` is, from one reciprocal on the integer pipe
     double n0, n1;
     div2_rn(b1 - cf[3] * b2, b2 - a21 * b1, det, n0, n1);
     q0[c] = n0;

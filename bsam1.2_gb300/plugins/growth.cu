@@ -55,20 +55,23 @@ struct Growth {
     double phi = q0[c];
     double ol = x.qold[c];
     double tmp2 = cf[2] + dt * sqr(phi);
-    double s0 = q0[c - 1] + q0[c + 1] + q0[c - sy] + q0[c + sy];
-    double s1 = q1[c + 1] + q1[c - 1] + q1[c + sy] + q1[c - sy];
-    double s2 = q2[c + 1] + q2[c - 1] + q2[c + sy] + q2[c - sy];
-    if (DIM == 3) {
-      s0 = s0 + q0[c - sz] + q0[c + sz];
-      s1 = s1 + q1[c + sz] + q1[c - sz];
-      s2 = s2 + q2[c + sz] + q2[c - sz];
+    // neighbour sums (3D) and divisions on the integer pipe, to the same bits
+    double s0, s1, s2;
+    if (DIM == 2) {
+      s0 = q0[c - 1] + q0[c + 1] + q0[c - sy] + q0[c + sy];
+      s1 = q1[c + 1] + q1[c - 1] + q1[c + sy] + q1[c - sy];
+      s2 = q2[c + 1] + q2[c - 1] + q2[c + sy] + q2[c - sy];
+    } else {
+      s0 = fxp::sum<6>({q0[c - 1], q0[c + 1], q0[c - sy], q0[c + sy], q0[c - sz], q0[c + sz]});
+      s1 = fxp::sum<6>({q1[c + 1], q1[c - 1], q1[c + sy], q1[c - sy], q1[c + sz], q1[c - sz]});
+      s2 = fxp::sum<6>({q2[c + 1], q2[c - 1], q2[c + sy], q2[c - sy], q2[c + sz], q2[c - sz]});
     }
-    double np = (f0[fc] + dt * (pp.gamma * 0.5 * (ol + 1.0)) * (q1[c] - pp.czero) + cf[0] * s0) / tmp2;
+    double np = fxp::quot(f0[fc] + dt * (pp.gamma * 0.5 * (ol + 1.0)) * (q1[c] - pp.czero) + cf[0] * s0, tmp2);
     double tmp4 = cf[3] + (pp.lambda * 0.5 * (ol + 1.0));
-    double nn = (f1[fc] + cf[1] * s1) / tmp4;
+    double nn = fxp::quot(f1[fc] + cf[1] * s1, tmp4);
     q0[c] = np;
     q1[c] = nn;
-    q2[c] = (f2[fc] + cf[1] * s2 + pp.cpress * np * nn) / cf[3];
+    q2[c] = fxp::quot(f2[fc] + cf[1] * s2 + pp.cpress * np * nn, cf[3]);
   }
 
   template <int DIM>
