@@ -13,9 +13,8 @@
 // as additions.
 //
 // Measured (GB300), a 3D CH sweep of 256^3, a colour: 38 FP64 instructions a
-// cell, 612 us; 27 with the sums and about 500 integer ones, 440 us; 14 with
-// the two quotients, 344 us.  The residual norm 12 instead of 32, 1143 -> 660
-// us.
+// cell, 612 us; 27 with the sums and about 500 integer ones, 440 us; 16 with
+// the two quotients, 321 us.  The residual norm: 16 instead of 32.
 #pragma once
 #ifndef FXP_CPU  // a test compiles this file for the host, with the intrinsics it spells out
 #include <cuda_runtime.h>
@@ -156,37 +155,19 @@ __device__ __forceinline__ double sum(const double (&a)[N]) {
   return r;
 }
 
-// RN(sum(a) - RN(6 c)): the undivided Laplacian of the six neighbours
+// RN(.. + a[5]) with the first five terms on the integer pipe: an addition is
+// about 40 instructions there, as long as the FP64 unit takes for one, and
+// with one or two of them left to it both pipes are busy alike (256^3 sweep:
+// six terms 344 us, five 321, four 329)
+__device__ __forceinline__ double sum6(const double (&a)[6]) {
+  return __dadd_rn(sum<5>({a[0], a[1], a[2], a[3], a[4]}), a[5]);
+}
+
+// RN(sum(a) - RN(6 c)): the undivided Laplacian of the six neighbours (the
+// norm of 160x96x128 with the centre in the frame too 88 us, so 82, with five
+// terms 85)
 __device__ __forceinline__ double lap6(const double (&a)[6], double c) {
-  Range R{0, 0x7ff, 0u};
-  widen(R, c);
-#pragma unroll
-  for (int i = 0; i < 6; i++) widen(R, a[i]);
-  const int E = R.E, ec = exponent(c);
-  Acc A{0, 0u, 0u};
-#pragma unroll
-  for (int i = 0; i < 6; i++) {
-    add_value<6>(A, a[i], E);
-    if (i) round53(A);
-  }
-  {  // 6 c = 2 (3 m): 3 m has 54 or 55 bits and is rounded to 53
-    const int hi = __double2hiint(c);
-    const unsigned long long m =
-        ((unsigned long long)(((unsigned)hi & 0xfffffu) | (ec ? 0x100000u : 0u)) << 32) | (unsigned)__double2loint(c);
-    unsigned long long m3 = m + (m << 1);
-    const int r = 1 + ((int)(m3 >> 54) & 1);
-    const unsigned mask = (1u << r) - 1u;
-    m3 += (mask >> 1) + (((unsigned)m3 >> r) & 1u);
-    m3 &= ~(unsigned long long)mask;
-    m3 <<= 7;  // 2 (3 m), six bits above its place
-    add_shifted(A, (unsigned)(m3 >> 32), (unsigned)m3, (E - ec) & 31, ~(hi >> 31));
-  }
-  round53(A);
-  bool ok;
-  double r = pack<6>(A, E, ok);
-  if (!(ok && serves(R)))
-    r = plain_add(plain_sum6(a[0], a[1], a[2], a[3], a[4], a[5]), -plain_mul(6.0, c));
-  return r;
+  return __dadd_rn(sum<6>(a), -__dmul_rn(6.0, c));
 }
 
 // RN(3 x): a significand times three has 54 or 55 bits

@@ -61,8 +61,8 @@ struct CH {
       // with 3 and 2 run on the integer pipe, to the same bits
       const double p2 = sqr(phi);
       a21 = -fxp::triple(p2) - cf[2];
-      b1 = f0[fc] + cf[0] * fxp::sum<6>({q1[c - 1], q1[c + 1], q1[c - sy], q1[c + sy], q1[c - sz], q1[c + sz]});
-      b2 = f1[fc] - cf[1] * fxp::sum<6>({q0[c + 1], q0[c - 1], q0[c + sy], q0[c - sy], q0[c + sz], q0[c - sz]}) -
+      b1 = f0[fc] + cf[0] * fxp::sum6({q1[c - 1], q1[c + 1], q1[c - sy], q1[c + sy], q1[c - sz], q1[c + sz]});
+      b2 = f1[fc] - cf[1] * fxp::sum6({q0[c + 1], q0[c - 1], q0[c + sy], q0[c - sy], q0[c + sz], q0[c - sz]}) -
            fxp::scaled<1>(p2 * phi);
     }
     double det = 1.0 - cf[3] * a21;  // >= 1: a21 <= -tmp3 < 0

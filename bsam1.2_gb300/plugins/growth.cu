@@ -62,9 +62,9 @@ struct Growth {
       s1 = q1[c + 1] + q1[c - 1] + q1[c + sy] + q1[c - sy];
       s2 = q2[c + 1] + q2[c - 1] + q2[c + sy] + q2[c - sy];
     } else {
-      s0 = fxp::sum<6>({q0[c - 1], q0[c + 1], q0[c - sy], q0[c + sy], q0[c - sz], q0[c + sz]});
-      s1 = fxp::sum<6>({q1[c + 1], q1[c - 1], q1[c + sy], q1[c - sy], q1[c + sz], q1[c - sz]});
-      s2 = fxp::sum<6>({q2[c + 1], q2[c - 1], q2[c + sy], q2[c - sy], q2[c + sz], q2[c - sz]});
+      s0 = fxp::sum6({q0[c - 1], q0[c + 1], q0[c - sy], q0[c + sy], q0[c - sz], q0[c + sz]});
+      s1 = fxp::sum6({q1[c + 1], q1[c - 1], q1[c + sy], q1[c - sy], q1[c + sz], q1[c - sz]});
+      s2 = fxp::sum6({q2[c + 1], q2[c - 1], q2[c + sy], q2[c - sy], q2[c + sz], q2[c - sz]});
     }
     double np = fxp::quot(f0[fc] + dt * (pp.gamma * 0.5 * (ol + 1.0)) * (q1[c] - pp.czero) + cf[0] * s0, tmp2);
     double tmp4 = cf[3] + (pp.lambda * 0.5 * (ol + 1.0));
