@@ -508,8 +508,10 @@ __global__ void __launch_bounds__(kTileThreads) k_bx_relax_tiled(float* __restri
 
 // ---------------------------------------------------------------------------
 // One smoothing of a 3D level's V-cycle visit (nsmooth = 2: colour
-// half-sweeps 0, 1, 0, 1) in one pass over memory.  A CTA owns TY rows y0 ..
-// y0+TY-1 of the planes z0 .. z1-1 and streams the planes z0-NS .. z1+NS-1
+// half-sweeps 0, 1, 0, 1) in one pass over memory.  A CTA owns a run of the
+// planes of the y-tiles laid end to end (see SmoothSplit): for every tile of
+// its run, the TY rows y0 .. y0+TY-1 of the planes z0 .. z1-1, for which it
+// streams the planes z0-NS .. z1+NS-1
 // through a ring of NS+3 shared-memory slots, each holding the four
 // colour-split e arrays of rows y0-NS .. y0+TY+NS-1 of one plane (TMA tensor
 // copies of four rows of one array, at row chunks wrapped around the plane).
@@ -528,7 +530,13 @@ __global__ void __launch_bounds__(kTileThreads) k_bx_relax_tiled(float* __restri
 // separate half-sweeps.
 constexpr int kSmStages = 4;      // half-sweeps per pass
 constexpr int kSmThreads = 512;
-constexpr int kSmMinPlanes = 16;  // smallest z range of a CTA (the halo costs 2 NS planes)
+constexpr int kSmMinPlanes = 16;  // fewest planes a CTA is made for (the halo costs 2 NS more)
+constexpr int kSmMaxCtas = 256;
+// CTA b smooths the planes start[b] .. start[b+1]-1 of the line in which plane
+// z of y-tile t is t * n2 + z
+struct SmoothSplit {
+  int start[kSmMaxCtas + 1];
+};
 
 __host__ __device__ constexpr int smooth_slots(int ns) { return ns + 3; }  // planes i-ns-1 .. i, i+1 in flight
 __host__ __device__ constexpr long long smooth_slot_floats(int ty, int hh, int ns = kSmStages) {
@@ -560,7 +568,8 @@ __device__ __forceinline__ void stv(float* p, const float* v) {
 // cells a thread at 1024 threads measured no faster: the kernel is bound by
 // its instructions, not by the warps it has to hide latency).
 template <int TY, int HH, bool FRESH, int NS = kSmStages, int CPT = 4, int NT = kSmThreads>
-__global__ void __launch_bounds__(NT, 1) k_bx_smooth(float* __restrict__ fp, BoxLev L, long long oe_out, int nz,
+__global__ void __launch_bounds__(NT, 1) k_bx_smooth(float* __restrict__ fp, BoxLev L, long long oe_out,
+                                                   const __grid_constant__ SmoothSplit split,
                                                    const __grid_constant__ CUtensorMap emap) {
   after_previous();
   extern __shared__ __align__(128) float ssm[];
@@ -575,10 +584,7 @@ __global__ void __launch_bounds__(NT, 1) k_bx_smooth(float* __restrict__ fp, Box
   __shared__ __align__(8) unsigned long long bar[NSL];
   const int n1 = L.n[1], n2 = L.n[2];
   const unsigned half = (unsigned)L.half;  // a level's cells are fewer than 2^31
-  const int ytiles = n1 / TY;
-  const int y0 = (blockIdx.x % ytiles) * TY, zc = blockIdx.x / ytiles;
-  const int z0 = (int)((long long)zc * n2 / nz), z1 = (int)((long long)(zc + 1) * n2 / nz);
-  const int P = z1 - z0 + 2 * NS;  // local plane j is z0 - NS + j
+  int y0 = 0, z0 = 0, P = 0;  // the segment of one tile: local plane j is z0 - NS + j
   const float* G = fp + L.og;
   const float* PB = fp + L.opb;
   float* EO = fp + oe_out;
@@ -591,8 +597,6 @@ __global__ void __launch_bounds__(NT, 1) k_bx_smooth(float* __restrict__ fp, Box
   const int li = threadIdx.x % W, rb = threadIdx.x / W, hc = CPT * li;
   const int hm = (hc - 1) & (HH - 1), hp = (hc + CPT) & (HH - 1);  // the row's periodic wrap
   unsigned goff[KQ];  // the cells' offset within a plane of a colour-split array
-#pragma unroll
-  for (int k = 0; k < KQ; k++) goff[k] = (unsigned)(wrap(y0 - NS + rb + k * RK, n1) * HH + hc);
   if (threadIdx.x == 0) {
     for (int b = 0; b < NSL; b++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&bar[b])));
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -645,106 +649,116 @@ __global__ void __launch_bounds__(NT, 1) k_bx_smooth(float* __restrict__ fp, Box
   // per stage, the other colour of the thread's cells in the plane after the
   // one last passed
   float cz[NS][CARRY ? KQ : 1][2][CPT];
-  issue(0, 0);
-  issue(1, 1);
   bool ok = true;
-  int si = 0;               // the slot of plane i: i mod NSL
-  unsigned phase = 0;       // its barrier's phase parity: (i / NSL) & 1
+  int si = 0;               // the slot of plane i: the planes passed before it, of all segments, mod NSL
+  unsigned phase = 0;       // its barrier's phase parity: those planes / NSL, & 1
   auto slot = [&](int d) {  // the slot of plane i - d (0 <= d < NSL)
     const int t = si - d;
     return t < 0 ? t + NSL : t;
   };
-  for (int i = 0; i < P; i++) {
-    if (!FRESH) ok = mbar_wait(smem_addr(&bar[si]), phase) && ok;
-    float fw[KQ][2][CPT];  // the last stage's new values: the z+1 values of the next stage
+  const int end = split.start[blockIdx.x + 1];
+  for (int p = split.start[blockIdx.x]; p < end; p += P - 2 * NS) {
+    const int tile = p / n2;
+    y0 = tile * TY, z0 = p - tile * n2;
+    P = min(n2 - z0, end - p) + 2 * NS;
 #pragma unroll
-    for (int s = 1; s <= NS; s++) {
-      const int j = i - s;
-      if (j >= s && j <= P - 1 - s) {  // uniform over the CTA
-        const int c = (s - 1) & 1, o = 1 - c;
-        const int first = FRESH ? (s <= 2 ? s : 0) : 0;
-        // x = 2h + bb: the parity is the same for all of the thread's rows (RK is even)
-        const int bb = (c + y0 - NS + rb + z0 - NS + j + 1) & 1;
-        float* S = ssm + slot(s) * SL + (rb << LG);
-        const float* Sm = ssm + slot(s + 1) * SL + (rb << LG);
-        const float* Sp = ssm + slot(s - 1) * SL + (rb << LG);
+    for (int k = 0; k < KQ; k++) goff[k] = (unsigned)(wrap(y0 - NS + rb + k * RK, n1) * HH + hc);
+    // the last barrier of the segment before lies behind the last reads of
+    // these two slots (planes i-NS-2 and i-NS-1 of its last pass)
+    issue(0, si);
+    issue(1, si + 1 == NSL ? 0 : si + 1);
+    for (int i = 0; i < P; i++) {
+      if (!FRESH) ok = mbar_wait(smem_addr(&bar[si]), phase) && ok;
+      float fw[KQ][2][CPT];  // the last stage's new values: the z+1 values of the next stage
 #pragma unroll
-        for (int k = 0; k < KQ; k++) {
-          const int r = rb + k * RK;
-          if (r >= s && r <= R - 1 - s) {
-            const int ro = k * RK * HH;
-            float s0[CPT], s1[CPT], xv[CPT];
+      for (int s = 1; s <= NS; s++) {
+        const int j = i - s;
+        if (j >= s && j <= P - 1 - s) {  // uniform over the CTA
+          const int c = (s - 1) & 1, o = 1 - c;
+          const int first = FRESH ? (s <= 2 ? s : 0) : 0;
+          // x = 2h + bb: the parity is the same for all of the thread's rows (RK is even)
+          const int bb = (c + y0 - NS + rb + z0 - NS + j + 1) & 1;
+          float* S = ssm + slot(s) * SL + (rb << LG);
+          const float* Sm = ssm + slot(s + 1) * SL + (rb << LG);
+          const float* Sp = ssm + slot(s - 1) * SL + (rb << LG);
 #pragma unroll
-            for (int q = 0; q < CPT; q++) s0[q] = s1[q] = xv[q] = 0.f;
-            if (first != 1) {
+          for (int k = 0; k < KQ; k++) {
+            const int r = rb + k * RK;
+            if (r >= s && r <= R - 1 - s) {
+              const int ro = k * RK * HH;
+              float s0[CPT], s1[CPT], xv[CPT];
 #pragma unroll
-              for (int var = 0; var < 2; var++) {
-                const int ao = (2 * var + o) * AR + ro;
-                float a[CPT], zp[CPT], zm[CPT], ym[CPT], yp[CPT];
-                // the other colour of this plane was the z+1 value of the
-                // pass over plane j-1, unchanged since
-                if (CARRY && j > s) {
+              for (int q = 0; q < CPT; q++) s0[q] = s1[q] = xv[q] = 0.f;
+              if (first != 1) {
 #pragma unroll
-                  for (int q = 0; q < CPT; q++) a[q] = cz[s - 1][CARRY ? k : 0][var][q];
-                } else {
-                  ldv<CPT>(S + ao + hc, a);
+                for (int var = 0; var < 2; var++) {
+                  const int ao = (2 * var + o) * AR + ro;
+                  float a[CPT], zp[CPT], zm[CPT], ym[CPT], yp[CPT];
+                  // the other colour of this plane was the z+1 value of the
+                  // pass over plane j-1, unchanged since
+                  if (CARRY && j > s) {
+#pragma unroll
+                    for (int q = 0; q < CPT; q++) a[q] = cz[s - 1][CARRY ? k : 0][var][q];
+                  } else {
+                    ldv<CPT>(S + ao + hc, a);
+                  }
+                  if (s == 1) {
+                    ldv<CPT>(Sp + ao + hc, zp);
+                  } else {
+#pragma unroll
+                    for (int q = 0; q < CPT; q++) zp[q] = fw[k][var][q];
+                  }
+                  if (CARRY) {
+#pragma unroll
+                    for (int q = 0; q < CPT; q++) cz[s - 1][CARRY ? k : 0][var][q] = zp[q];
+                  }
+                  ldv<CPT>(Sm + ao + hc, zm);
+                  ldv<CPT>(S + ao - HH + hc, ym);
+                  ldv<CPT>(S + ao + HH + hc, yp);
+                  // a[xm] + a[xp] with xm, xp = h, h+1 (bb = 1) or h-1, h (bb = 0)
+                  const float edge = S[ao + (bb ? hp : hm)];
+                  float* acc = var ? s1 : s0;
+#pragma unroll
+                  for (int q = 0; q < CPT; q++) {
+                    const float lft = bb ? a[q] : (q ? a[q - 1] : edge);
+                    const float rgt = bb ? (q + 1 < CPT ? a[q + 1] : edge) : a[q];
+                    float t = lft + rgt + ym[q] + yp[q];
+                    t += zm[q] + zp[q];
+                    acc[q] = t;
+                  }
                 }
-                if (s == 1) {
-                  ldv<CPT>(Sp + ao + hc, zp);
-                } else {
-#pragma unroll
-                  for (int q = 0; q < CPT; q++) zp[q] = fw[k][var][q];
-                }
-                if (CARRY) {
-#pragma unroll
-                  for (int q = 0; q < CPT; q++) cz[s - 1][CARRY ? k : 0][var][q] = zp[q];
-                }
-                ldv<CPT>(Sm + ao + hc, zm);
-                ldv<CPT>(S + ao - HH + hc, ym);
-                ldv<CPT>(S + ao + HH + hc, yp);
-                // a[xm] + a[xp] with xm, xp = h, h+1 (bb = 1) or h-1, h (bb = 0)
-                const float edge = S[ao + (bb ? hp : hm)];
-                float* acc = var ? s1 : s0;
-#pragma unroll
-                for (int q = 0; q < CPT; q++) {
-                  const float lft = bb ? a[q] : (q ? a[q - 1] : edge);
-                  const float rgt = bb ? (q + 1 < CPT ? a[q + 1] : edge) : a[q];
-                  float t = lft + rgt + ym[q] + yp[q];
-                  t += zm[q] + zp[q];
-                  acc[q] = t;
-                }
+                if (first == 0) ldv<CPT>(S + c * AR + ro + hc, xv);
               }
-              if (first == 0) ldv<CPT>(S + c * AR + ro + hc, xv);
-            }
-            float r0[CPT], r1[CPT];
+              float r0[CPT], r1[CPT];
 #pragma unroll
-            for (int q = 0; q < CPT; q++) {
-              newton_cell(L, v[s - 1][k][0][q], xv[q], s0[q], s1[q], v[s - 1][k][1][q], v[s - 1][k][2][q], r0[q],
-                          r1[q]);
-              if (!ok) r0[q] = r1[q] = nanf("");  // a copy that never landed: poison the pass
-              fw[k][0][q] = r0[q], fw[k][1][q] = r1[q];
+              for (int q = 0; q < CPT; q++) {
+                newton_cell(L, v[s - 1][k][0][q], xv[q], s0[q], s1[q], v[s - 1][k][1][q], v[s - 1][k][2][q], r0[q],
+                            r1[q]);
+                if (!ok) r0[q] = r1[q] = nanf("");  // a copy that never landed: poison the pass
+                fw[k][0][q] = r0[q], fw[k][1][q] = r1[q];
+              }
+              stv<CPT>(S + c * AR + ro + hc, r0);
+              stv<CPT>(S + (2 + c) * AR + ro + hc, r1);
             }
-            stv<CPT>(S + c * AR + ro + hc, r0);
-            stv<CPT>(S + (2 + c) * AR + ro + hc, r1);
           }
         }
+        load(s, i + 1 - s);  // the next pass's cells of this stage, in flight while the others compute
       }
-      load(s, i + 1 - s);  // the next pass's cells of this stage, in flight while the others compute
-    }
-    __syncthreads();  // rows y+-1 of this pass are read by the next; the slot below is free
-    issue(i + 2, slot(NSL - 2));  // plane i + 2 into the slot of plane i - NS - 1, which stage NS read last
-    const int j = i - NS;
-    if (j >= NS && j <= P - 1 - NS) {  // plane j is final: rows NS .. NS+TY-1 of the slot
-      const float* S = ssm + slot(NS) * SL + NS * HH;
-      float* D = EO + (unsigned)(((z0 - NS + j) * n1 + y0) * HH);
-      constexpr int n4 = (TY * HH) >> 2;
+      __syncthreads();  // rows y+-1 of this pass are read by the next; the slot below is free
+      issue(i + 2, slot(NSL - 2));  // plane i + 2 into the slot of plane i - NS - 1, which stage NS read last
+      const int j = i - NS;
+      if (j >= NS && j <= P - 1 - NS) {  // plane j is final: rows NS .. NS+TY-1 of the slot
+        const float* S = ssm + slot(NS) * SL + NS * HH;
+        float* D = EO + (unsigned)(((z0 - NS + j) * n1 + y0) * HH);
+        constexpr int n4 = (TY * HH) >> 2;
 #pragma unroll
-      for (int q = threadIdx.x; q < 4 * n4; q += NT) {
-        const int a = q / n4, t = q - a * n4;
-        reinterpret_cast<float4*>(D + (unsigned)a * half)[t] = reinterpret_cast<const float4*>(S + a * AR)[t];
+        for (int q = threadIdx.x; q < 4 * n4; q += NT) {
+          const int a = q / n4, t = q - a * n4;
+          reinterpret_cast<float4*>(D + (unsigned)a * half)[t] = reinterpret_cast<const float4*>(S + a * AR)[t];
+        }
       }
+      if (++si == NSL) si = 0, phase ^= 1u;
     }
-    if (++si == NSL) si = 0, phase ^= 1u;
   }
   if (!ok)  // a wait gave up: give the copies still in flight a bounded time to land before the block exits
     for (int b = 0; b < NSL; b++) mbar_wait(smem_addr(&bar[b]), 0u), mbar_wait(smem_addr(&bar[b]), 1u);
@@ -2078,11 +2092,46 @@ int e_tensor_map(Hier& H, const BoxLev& L, long long oe, CUtensorMap* m) {
   return BSAMG_OK;
 }
 
+// The split of a level of `tiles` y-tiles of n2 planes over at most `ctas`
+// CTAs: a CTA passes over its planes and 2 NS more for every tile it works
+// on, so the line is cut by passes, not by planes, into the smallest number
+// of passes a CTA that the CTAs suffice for.  Every SM has its share whatever
+// the extents (256^3: 150 CTAs of 64 passes, 166 us, instead of 128 CTAs, four
+// to a tile, of 72 passes, 182 us).
+// A CTA goes on to the next tile only for kSmTail planes or more.
+constexpr int kSmTail = 4;
+int smooth_split(int tiles, int n2, int ctas, SmoothSplit& S) {
+  const int total = tiles * n2;
+  auto cut = [&](int passes) {  // the CTAs it takes; more than `ctas` count as one more
+    int k = 0;
+    for (int p = 0; p < total && k <= ctas; k++) {
+      if (k < ctas) S.start[k] = p;
+      for (int left = passes; p < total;) {
+        const int room = left - 2 * kSmStages, rest = n2 - p % n2;
+        if (room < std::min(rest, left == passes ? 1 : kSmTail)) break;
+        const int take = std::min(room, rest);
+        p += take;
+        left -= take + 2 * kSmStages;
+      }
+    }
+    return k;
+  };
+  int lo = std::min(kSmMinPlanes, n2) + 2 * kSmStages, hi = total + tiles * 2 * kSmStages;
+  while (lo < hi) {
+    const int mid = (lo + hi) / 2;
+    if (cut(mid) <= ctas) hi = mid;
+    else lo = mid + 1;
+  }
+  const int k = cut(lo);
+  S.start[k] = total;
+  return k;
+}
+
 // out_oe = e after two red-black passes from e at in.oe (fresh: from zero)
 int bx_smooth(Hier& H, const BoxLev& in, long long out_oe, bool fresh) {
   const int ty = smooth_rows(in);
-  const int ytiles = in.n[1] / ty;
-  int nz = std::max(1, std::min(H.box_sms / ytiles, in.n[2] / kSmMinPlanes));
+  SmoothSplit split;
+  const int ctas = smooth_split(in.n[1] / ty, in.n[2], std::max(1, std::min(H.box_sms, kSmMaxCtas)), split);
   size_t smem = (size_t)smooth_slots(kSmStages) * smooth_slot_floats(ty, in.hh) * sizeof(float);
   static std::atomic<unsigned long long> attr;  // the kernels' shared-memory limit, per device
   if (needs_setup(attr, H.ctx->device)) {
@@ -2096,7 +2145,7 @@ int bx_smooth(Hier& H, const BoxLev& in, long long out_oe, bool fresh) {
   int r = e_tensor_map(H, in, in.oe, &emap);
   if (r) return r;
   auto ker = fresh ? k_bx_smooth<8, 128, true> : k_bx_smooth<8, 128, false>;
-  launch_after(ker, ytiles * nz, kSmThreads, smem, H.s, H.fpool, in, out_oe, nz, emap);
+  launch_after(ker, ctas, kSmThreads, smem, H.s, H.fpool, in, out_oe, split, emap);
   return after_launch(H, 1);
 }
 bool smooth_applies(const Hier& H, const BoxLev& L, int nsmooth) {
