@@ -103,13 +103,18 @@ __device__ __forceinline__ V2 var2(float* fp, long long off, long long half) {
   return {fp + off, fp + off + 2 * half};
 }
 
-// correction operator M(e) at a cell (see mixed.cu, mopn)
+// correction operator M(e) at a cell (see mixed.cu, mopn) whose variables'
+// neighbours sum to s0 and s1
+template <int DIM>
+__device__ __forceinline__ void mop_cell(const BoxLev& L, float x, float y, float pb, float s0, float s1, float& m0,
+                                         float& m1) {
+  const float k = DIM == 2 ? 4.0f : 6.0f;
+  m0 = x - L.c0 * (s1 - k * y);
+  m1 = y - x * (3.0f * pb * (pb + x) + x * x) + L.c1 * (s0 - k * x);
+}
 template <int DIM>
 __device__ __forceinline__ void mop(V2 E, const BoxLev& L, const Loc<DIM>& l, float pb, float& m0, float& m1) {
-  float x = E.v0[l.own], y = E.v1[l.own];
-  const float k = DIM == 2 ? 4.0f : 6.0f;
-  m0 = x - L.c0 * (nsum<DIM>(E.v1, l) - k * y);
-  m1 = y - x * (3.0f * pb * (pb + x) + x * x) + L.c1 * (nsum<DIM>(E.v0, l) - k * x);
+  mop_cell<DIM>(L, E.v0[l.own], E.v1[l.own], pb, nsum<DIM>(E.v0, l), nsum<DIM>(E.v1, l), m0, m1);
 }
 
 // the undivided Laplacian as a sum of neighbour differences: for a smooth
@@ -767,31 +772,28 @@ __global__ void __launch_bounds__(NT, 1) k_bx_smooth(float* __restrict__ fp, Box
 // RestrictSolution and the fine half of CoarseLoadingFunction in one pass
 // over the fine cells: coarse e = ec = R(e), coarse pb = R(pb) and coarse
 // g = R(g - M(e)); the coarse operator M_c(ec) needs the neighbours' ec, so
-// k_bx_coarse_op adds it in a second (coarse-sized) pass.  Every fine value
-// is loaded before the first store; six blocks per SM (40 registers, no
-// spills) against five uncapped: 30 vs 37 us averaged over the levels.
-template <int DIM>
-__device__ __forceinline__ void restrict_load_at(float* __restrict__ fp, const BoxLev& F, const BoxLev& C, int X,
-                                                 int Y, int Z) {
+// k_bx_coarse_op adds it in a second (coarse-sized) pass.  2D:
+__global__ void __launch_bounds__(256, 6) k_bx_restrict_load(float* __restrict__ fp, BoxLev F, BoxLev C) {
+  after_previous();
+  const int X = blockIdx.x * blockDim.x + threadIdx.x, Y = blockIdx.y * blockDim.y + threadIdx.y;
+  if (X >= C.n[0] || Y >= C.n[1]) return;
   V2 Ef = var2(fp, F.oe, F.half), Gf = var2(fp, F.og, F.half);
   const float* PBf = fp + F.opb;
   float s0 = 0.f, s1 = 0.f, s2 = 0.f, R0 = 0.f, R1 = 0.f;
-  const int nz = DIM == 3 ? 2 : 1;
-  for (int dz = 0; dz < nz; dz++)
-    for (int dy = 0; dy < 2; dy++)
-      for (int dx = 0; dx < 2; dx++) {
-        Loc<DIM> l(F, 2 * X + dx, 2 * Y + dy, DIM == 3 ? 2 * Z + dz : 0);
-        float pb = PBf[l.own];
-        s0 += Ef.v0[l.own];
-        s1 += Ef.v1[l.own];
-        s2 += pb;
-        float m0, m1;
-        mop<DIM>(Ef, F, l, pb, m0, m1);
-        R0 += Gf.v0[l.own] - m0;
-        R1 += Gf.v1[l.own] - m1;
-      }
-  const float w = DIM == 2 ? 0.25f : 0.125f;
-  Loc<DIM> lc(C, X, Y, Z);
+  for (int dy = 0; dy < 2; dy++)
+    for (int dx = 0; dx < 2; dx++) {
+      Loc<2> l(F, 2 * X + dx, 2 * Y + dy, 0);
+      float pb = PBf[l.own];
+      s0 += Ef.v0[l.own];
+      s1 += Ef.v1[l.own];
+      s2 += pb;
+      float m0, m1;
+      mop<2>(Ef, F, l, pb, m0, m1);
+      R0 += Gf.v0[l.own] - m0;
+      R1 += Gf.v1[l.own] - m1;
+    }
+  const float w = 0.25f;
+  Loc<2> lc(C, X, Y, 0);
   V2 Ec = var2(fp, C.oe, C.half), ECc = var2(fp, C.oec, C.half), Gc = var2(fp, C.og, C.half);
   Ec.v0[lc.own] = ECc.v0[lc.own] = s0 * w;
   Ec.v1[lc.own] = ECc.v1[lc.own] = s1 * w;
@@ -799,12 +801,103 @@ __device__ __forceinline__ void restrict_load_at(float* __restrict__ fp, const B
   Gc.v0[lc.own] = R0 * w;
   Gc.v1[lc.own] = R1 * w;
 }
-template <int DIM>
-__global__ void __launch_bounds__(256, 6) k_bx_restrict_load(float* __restrict__ fp, BoxLev F, BoxLev C) {
+
+// 3D: a thread owns two coarse cells of a row, whose fine cells are, in each
+// colour's array, two consecutive values of four rows: it loads every value
+// once, as a vector (72 vectors and 16 single ones for what cell by cell are
+// 272 loads).  The pass waits for memory (cell by cell at 40 registers it took
+// 135 us at 256^3 against 50 us for its bytes), so that fewer and wider loads,
+// more of them in flight, are what counts: 215 -> 234 steps/s of 256^3 with
+// five CTAs of 128 threads an SM at 96 registers; at 64 registers 225, with
+// four cells a thread at 128 registers 232.  The sums keep the order of the
+// cells, and the bits.
+constexpr int kRestrictThreads = 128;
+constexpr int kRestrictCells = 2;  // coarse cells a thread; a level's extents are even
+__global__ void __launch_bounds__(kRestrictThreads, 5) k_bx_restrict_rows(float* __restrict__ fp, BoxLev F, BoxLev C) {
   after_previous();
-  int X = blockIdx.x * blockDim.x + threadIdx.x;
-  int Y = blockIdx.y * blockDim.y + threadIdx.y;
-  if (X < C.n[0] && Y < C.n[1]) restrict_load_at<DIM>(fp, F, C, X, Y, blockIdx.z);
+  constexpr int CPT = kRestrictCells;
+  const int X = CPT * (int)(blockIdx.x * blockDim.x + threadIdx.x), Y = blockIdx.y * blockDim.y + threadIdx.y;
+  const int Z = blockIdx.z;
+  if (X >= C.n[0] || Y >= C.n[1]) return;
+  const unsigned hh = (unsigned)F.hh, n1 = (unsigned)F.n[1], n2 = (unsigned)F.n[2], half = (unsigned)F.half;
+  const unsigned h = (unsigned)X;  // fine x = 2 X + dx is position X of its colour's row
+  const unsigned hl = h ? h - 1 : hh - 1, hr = h + CPT < hh ? h + CPT : 0u;
+  const unsigned y0 = 2u * (unsigned)Y, z0 = 2u * (unsigned)Z;
+  // the rows below and above the cell's two in y and z
+  const unsigned yo[2] = {y0 ? y0 - 1 : n1 - 1, y0 + 2 < n1 ? y0 + 2 : 0u};
+  const unsigned zo[2] = {z0 ? z0 - 1 : n2 - 1, z0 + 2 < n2 ? z0 + 2 : 0u};
+  const float* const E = fp + F.oe;
+  const float* const G = fp + F.og;
+  const float* const PB = fp + F.opb;
+  float e[2][2][2][2][CPT];  // [variable][colour][dz][dy]
+#pragma unroll
+  for (int dz = 0; dz < 2; dz++)
+#pragma unroll
+    for (int dy = 0; dy < 2; dy++)
+#pragma unroll
+      for (int a = 0; a < 4; a++)
+        ldv<CPT>(E + (a * half + ((z0 + dz) * n1 + y0 + dy) * hh + h), e[a >> 1][a & 1][dz][dy]);
+  float t0[CPT], t1[CPT], t2[CPT], R0[CPT], R1[CPT];
+#pragma unroll
+  for (int q = 0; q < CPT; q++) t0[q] = t1[q] = t2[q] = R0[q] = R1[q] = 0.f;
+#pragma unroll
+  for (int dz = 0; dz < 2; dz++)
+#pragma unroll
+    for (int dy = 0; dy < 2; dy++) {
+      const unsigned r = ((z0 + dz) * n1 + y0 + dy) * hh;
+      const unsigned ry = ((z0 + dz) * n1 + yo[dy]) * hh + h, rz = (zo[dz] * n1 + y0 + dy) * hh + h;
+      const int c0 = (dy + dz + 1) & 1;  // the colour of the cells dx = 0 (2X, 2Y and 2Z are even)
+      float oy[2][2][CPT], oz[2][2][CPT], pb[2][CPT], g[2][2][CPT], edge[2][2];
+#pragma unroll
+      for (int a = 0; a < 4; a++) {
+        ldv<CPT>(E + (a * half + ry), oy[a >> 1][a & 1]);
+        ldv<CPT>(E + (a * half + rz), oz[a >> 1][a & 1]);
+        ldv<CPT>(G + (a * half + r + h), g[a >> 1][a & 1]);
+      }
+#pragma unroll
+      for (int v = 0; v < 2; v++) {
+        ldv<CPT>(PB + (v * half + r + h), pb[v]);
+        edge[v][0] = E[(2 * v + 1 - c0) * half + r + hl];
+        edge[v][1] = E[(2 * v + c0) * half + r + hr];
+      }
+#pragma unroll
+      for (int dx = 0; dx < 2; dx++) {
+        const int c = (c0 + dx) & 1, o = 1 - c;
+#pragma unroll
+        for (int q = 0; q < CPT; q++) {
+          float s[2];
+#pragma unroll
+          for (int v = 0; v < 2; v++) {
+            const float* w = e[v][o][dz][dy];
+            const float xm = dx ? w[q] : (q ? w[q ? q - 1 : 0] : edge[v][0]);
+            const float xp = dx ? (q + 1 < CPT ? w[q + 1 < CPT ? q + 1 : 0] : edge[v][1]) : w[q];
+            const float ym = dy ? e[v][o][dz][0][q] : oy[v][o][q], yp = dy ? oy[v][o][q] : e[v][o][dz][1][q];
+            const float zm = dz ? e[v][o][0][dy][q] : oz[v][o][q], zp = dz ? oz[v][o][q] : e[v][o][1][dy][q];
+            s[v] = xm + xp + ym + yp;
+            s[v] += zm + zp;
+          }
+          const float x = e[0][c][dz][dy][q], y = e[1][c][dz][dy][q];
+          float m0, m1;
+          mop_cell<3>(F, x, y, pb[c][q], s[0], s[1], m0, m1);
+          t0[q] += x;
+          t1[q] += y;
+          t2[q] += pb[c][q];
+          R0[q] += g[0][c][q] - m0;
+          R1[q] += g[1][c][q] - m1;
+        }
+      }
+    }
+  const float w = 0.125f;
+  const unsigned ch = (unsigned)C.half, cr = ((unsigned)Z * (unsigned)C.n[1] + (unsigned)Y) * (unsigned)C.hh;
+#pragma unroll
+  for (int q = 0; q < CPT; q++) {
+    const unsigned i = (colour<3>(X + q, Y, Z) ? ch : 0u) + cr + ((unsigned)(X + q) >> 1);
+    fp[C.oe + i] = fp[C.oec + i] = t0[q] * w;
+    fp[C.oe + 2 * ch + i] = fp[C.oec + 2 * ch + i] = t1[q] * w;
+    fp[C.opb + i] = t2[q] * w;
+    fp[C.og + i] = R0[q] * w;
+    fp[C.og + 2 * ch + i] = R1[q] * w;
+  }
 }
 // coarse g += M_c(ec), the coarse operator on the restricted correction
 template <int DIM>
@@ -2167,6 +2260,19 @@ int bx_relax(Hier& H, int level, int c, int first) {
   return BSAMG_OK;
 }
 
+int bx_restrict_load(Hier& H, const BoxLev& F, const BoxLev& C) {
+  if (H.ndims == 2) {
+    const Launch sh = shape(C.n[0], C.n[1], 1);
+    launch_after(k_bx_restrict_load, sh.g, sh.b, 0, H.s, H.fpool, F, C);
+    return after_launch(H, 1);
+  }
+  const int nx = C.n[0] / kRestrictCells, tx = std::min(nx, kRestrictThreads);
+  const int ty = std::max(1, std::min(kRestrictThreads / tx, C.n[1]));
+  launch_after(k_bx_restrict_rows, dim3((nx + tx - 1) / tx, (C.n[1] + ty - 1) / ty, C.n[2]), dim3(tx, ty), 0, H.s,
+               H.fpool, F, C);
+  return after_launch(H, 1);
+}
+
 // coarse: the V-cycle's coarsest level, smoothed in FP64 arithmetic
 int bx_level_relax(Hier& H, int level, int nsmooth, bool fresh, bool coarse = false) {
   for (int pass = 1; pass <= nsmooth; pass++)
@@ -2284,7 +2390,7 @@ bool cycle_layout(Hier& H, int top, int minlevel, int nsmooth, int share, int ba
     L.c0 = P.c0, L.c1 = P.c1, L.tmp3 = P.tmp3, L.a12 = P.a12;
     L.hx = dv(P.n[0] / 2), L.d1 = dv(P.n[1]), L.hc = dv(P.n[0] / 2), L.dc1 = dv(std::max(1, P.n[1] / 2));
     // the sums of the restriction keep the order of each size of level: small
-    // levels colour by colour, the others as k_bx_restrict_load
+    // levels colour by colour, the others as k_bx_restrict_load and _rows
     L.by_colour = 2 * P.half <= 8192;
     if (x + 1 < A.nl) scratch = std::max(scratch, 4 * pairs);
     if (o * 4 > kUniSmemMax || A.nl > 15) return false;  // (a named barrier a level)
@@ -2348,7 +2454,7 @@ int bx_vcycle_from(Hier& H, int level, int minlevel, int nsmooth, bool fresh, co
     Launch sc = shape(C.n[0], C.n[1], C.n[2]);
     int r = bx_smooth(H, F, F.oe2, fresh);
     if (r) return r;
-    BX_LAUNCH(H, sc, k_bx_restrict_load, H.fpool, Fb, C);
+    if ((r = bx_restrict_load(H, Fb, C))) return r;
     BX_LAUNCH(H, sc, k_bx_coarse_op, H.fpool, C);
     if ((r = bx_vcycle_from(H, level - 1, minlevel, nsmooth, false, cyc, cyc_smem, cyc_at))) return r;
     BX_LAUNCH(H, sc, k_bx_prolong, H.fpool, Fb, C);
@@ -2359,7 +2465,7 @@ int bx_vcycle_from(Hier& H, int level, int minlevel, int nsmooth, bool fresh, co
   if (level > minlevel) {
     BoxLev &F = B(H, level), &C = B(H, level - 1);
     Launch sc = shape(C.n[0], C.n[1], C.n[2]);
-    BX_LAUNCH(H, sc, k_bx_restrict_load, H.fpool, F, C);
+    if ((r = bx_restrict_load(H, F, C))) return r;
     BX_LAUNCH(H, sc, k_bx_coarse_op, H.fpool, C);
     if ((r = bx_vcycle_from(H, level - 1, minlevel, nsmooth, false, cyc, cyc_smem, cyc_at))) return r;
     BX_LAUNCH(H, sc, k_bx_prolong, H.fpool, F, C);
