@@ -14,7 +14,7 @@
 //
 // Measured (GB300), a 3D CH sweep of 256^3, a colour: 38 FP64 instructions a
 // cell, 612 us; 27 with the sums and about 500 integer ones, 440 us; 16 with
-// the two quotients, 321 us.  The residual norm: 16 instead of 32.
+// the two quotients, 312 us.  The residual norm: 16 instead of 32.
 #pragma once
 #ifndef FXP_CPU  // a test compiles this file for the host, with the intrinsics it spells out
 #include <cuda_runtime.h>
@@ -45,20 +45,22 @@ struct Acc {
 
 __device__ __forceinline__ int exponent(double a) { return (__double2hiint(a) >> 20) & 0x7ff; }
 
-// What decides whether the frame serves: the largest exponent, the smallest
-// one of a nonzero operand, and the significands of subnormal ones
+// What decides whether the frame serves: the largest high word without its
+// sign, and the smallest magnitude of a nonzero operand (its high word, the
+// low one as a last bit, less one so that zeros come out largest)
 struct Range {
-  int E, lo;
-  unsigned sub;
+  int top;
+  unsigned low;
 };
 __device__ __forceinline__ void widen(Range& R, double a) {
-  const int hi = __double2hiint(a), e = (hi >> 20) & 0x7ff;
-  R.E = max(R.E, e);
-  R.lo = min(R.lo, e ? e : 0x7ff);
-  R.sub |= e ? 0u : ((unsigned)hi << 1) | (unsigned)__double2loint(a);
+  const int hi = __double2hiint(a) & 0x7fffffff;
+  R.top = max(R.top, hi);
+  R.low = min(R.low, ((unsigned)hi | min((unsigned)__double2loint(a), 1u)) - 1u);
 }
+// (a subnormal operand lies 2^-32 below any E >= 130)
 __device__ __forceinline__ bool serves(const Range& R) {
-  return R.E - R.lo < 32 && (unsigned)(R.E - 130) < 1800u && R.sub == 0;
+  const int E = R.top >> 20;
+  return E - (int)(R.low >> 20) < 32 && (unsigned)(E - 130) < 1800u;
 }
 
 // add h:l:x, negated when sign is -1
@@ -77,18 +79,16 @@ __device__ __forceinline__ void add96(Acc& A, unsigned h, unsigned l, unsigned x
   A.x = (unsigned)s;
 #endif
 }
-// add the magnitude hi:lo (a significand shifted to the frame of exponent
-// E - d, F bits above its place) moved down by d
-__device__ __forceinline__ void add_shifted(Acc& A, unsigned hi, unsigned lo, int d, int sign) {
-  add96(A, hi >> d, __funnelshift_r(lo, hi, d), __funnelshift_r(0u, lo, d), sign);
-}
+// add a; top: the largest exponent E and ones below it, so that the
+// subtraction of a high word borrows nothing from its exponent's place
 template <int F>
-__device__ __forceinline__ void add_value(Acc& A, double a, int E) {
+__device__ __forceinline__ void add_value(Acc& A, double a, int top) {
   const int hi = __double2hiint(a);
   const unsigned lo = (unsigned)__double2loint(a);
-  const int e = (hi >> 20) & 0x7ff, d = (E - e) & 31;
-  const unsigned m = ((unsigned)hi & 0xfffffu) | (e ? 0x100000u : 0u);  // a zero adds nothing
-  add_shifted(A, __funnelshift_l(lo, m, F), lo << F, d, hi >> 31);
+  const unsigned d = (unsigned)(top - hi) >> 20;  // E - e in the low five bits, which are all a funnel shift takes
+  const unsigned m = ((unsigned)hi & 0xfffffu) | (unsigned)min(hi & 0x7fffffff, 0x100000);  // a zero adds nothing
+  const unsigned h = __funnelshift_l(lo, m, F), l = lo << F;
+  add96(A, __funnelshift_r(h, 0u, d), __funnelshift_r(l, h, d), __funnelshift_r(0u, l, d), hi >> 31);
 }
 // round the partial sum to 53 significant bits, ties to even
 __device__ __forceinline__ void round53(Acc& A) {
@@ -131,14 +131,14 @@ __device__ __forceinline__ double pack(const Acc& A, int E, bool& ok) {
 // (seven bits above a significand and the sign leave room for six of them)
 template <int N>
 __device__ __forceinline__ double sum(const double (&a)[N]) {
-  Range R{0, 0x7ff, 0u};
+  Range R{0, 0xffffffffu};
 #pragma unroll
   for (int i = 0; i < N; i++) widen(R, a[i]);
-  const int E = R.E;
+  const int E = R.top >> 20, top = R.top | 0xfffff;
   Acc A{0, 0u, 0u};
 #pragma unroll
   for (int i = 0; i < N; i++) {
-    add_value<7>(A, a[i], E);
+    add_value<7>(A, a[i], top);
     if (i) round53(A);
   }
   bool ok;
@@ -163,13 +163,6 @@ __device__ __forceinline__ double sum6(const double (&a)[6]) {
   return __dadd_rn(sum<5>({a[0], a[1], a[2], a[3], a[4]}), a[5]);
 }
 
-// RN(sum(a) - RN(6 c)): the undivided Laplacian of the six neighbours (the
-// norm of 160x96x128 with the centre in the frame too 88 us, so 82, with five
-// terms 85)
-__device__ __forceinline__ double lap6(const double (&a)[6], double c) {
-  return __dadd_rn(sum<6>(a), -__dmul_rn(6.0, c));
-}
-
 // RN(3 x): a significand times three has 54 or 55 bits
 __device__ __forceinline__ double triple(double x) {
   const int hi = __double2hiint(x), e = (hi >> 20) & 0x7ff;
@@ -190,6 +183,13 @@ __device__ __forceinline__ double scaled(double x) {
   double y = __hiloint2double(hi + K * (1 << 20), __double2loint(x));
   if ((unsigned)(e - 8) >= 2030u) y = plain_mul(x, K < 0 ? 1.0 / (1 << (K < 0 ? -K : 0)) : 1.0 * (1 << (K > 0 ? K : 0)));
   return y;
+}
+
+// RN(sum(a) - RN(6 c)): the undivided Laplacian of the six neighbours (the
+// norm of 160x96x128 with the centre in the frame too 88 us, so 80, with five
+// terms 83; 3 c on the integer pipe as well made the norm of 250^3 532 -> 568)
+__device__ __forceinline__ double lap6(const double (&a)[6], double c) {
+  return __dadd_rn(sum<6>(a), -__dmul_rn(6.0, c));
 }
 
 // ---- quotients ----
