@@ -377,18 +377,25 @@ __device__ __forceinline__ void correct_b(const View<typename TR::T>& V, const V
           }
         }
     }
+    // every fine value is loaded before the first store, which the next load
+    // would have to wait for (V.q is both)
+    int at[4 * NZ];
 #pragma unroll
     for (int m = 0; m < 4 * NZ; m++) {
       const int i = 2 * ci + (m & 1), j = 2 * cj + ((m >> 1) & 1), k = DIM == 3 ? 2 * ck + (m >> 2) : 1;
-      if (i < 1 || i > g.n0 || j < 1 || j > (DIM == 3 ? g.n1 : g.N) || (DIM == 3 && (k < 1 || k > g.N))) continue;
-      const int c = gcell<DIM>(g, i, j, k);
-      T w[TR::NV];
+      const bool in = i >= 1 && i <= g.n0 && j >= 1 && j <= (DIM == 3 ? g.n1 : g.N) && (DIM != 3 || (k >= 1 && k <= g.N));
+      at[m] = in ? gcell<DIM>(g, i, j, k) : -1;
 #pragma unroll
-      for (int v = 0; v < TR::NV; v++) {
-        w[v] = V.q[v * g.sq + c] + out[m][v];
-        V.q[v * g.sq + c] = w[v];
-      }
-      push<TR, DIM>(V.q, g, i, j, k, w, false, bc, par);
+      for (int v = 0; v < TR::NV; v++)
+        if (in) out[m][v] = V.q[v * g.sq + at[m]] + out[m][v];
+    }
+#pragma unroll
+    for (int m = 0; m < 4 * NZ; m++) {
+      if (at[m] < 0) continue;
+#pragma unroll
+      for (int v = 0; v < TR::NV; v++) V.q[v * g.sq + at[m]] = out[m][v];
+      push<TR, DIM>(V.q, g, 2 * ci + (m & 1), 2 * cj + ((m >> 1) & 1), DIM == 3 ? 2 * ck + (m >> 2) : 1, out[m], false, bc,
+                    par);
     }
   }
 }
