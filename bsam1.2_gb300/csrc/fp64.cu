@@ -266,7 +266,7 @@ int launch_update_source(const LaunchCtx& c, const Blk* blk, int nblk) {
 int launch_norm_partial(const LaunchCtx& c, const Blk* blk, int nblk, double* partial, int store_rf) {
   return ops_of(c).norm_partial(c, blk, nblk, partial, store_rf);
 }
-int launch_norm_finish(cudaStream_t s, const double* partial, int nblk, int nrvars, double count, int errortype,
+int launch_norm_finish(LaunchStream s, const double* partial, int nblk, int nrvars, double count, int errortype,
                        double* out, int* nonfinite, double* host, double* one) {
   int n = 1;
   if (nblk > 2048) {

@@ -728,6 +728,8 @@ int pinned_slot_take(Hier& H) {
   if (c->free_slots.empty()) return BSAMG_ERR_BUDGET;
   H.pinned_slot = c->free_slots.back();
   c->free_slots.pop_back();
+  H.crowded = kPinnedSlots - (int)c->free_slots.size() > kFewHiers;
+  H.launch_order();
   H.h_norm = c->pinned + (size_t)H.pinned_slot * kSlotDoubles;
   H.h_nonfinite = reinterpret_cast<int*>(H.h_norm + 8);
   return BSAMG_OK;
@@ -784,7 +786,7 @@ int commit(Hier& H) {
     H.reserved = need;
   }
   H.bytes += need;
-  CK(cudaStreamCreateWithFlags(&H.s, cudaStreamNonBlocking));
+  CK(cudaStreamCreateWithFlags(&H.s.s, cudaStreamNonBlocking));
   // stream-ordered allocations: creating or destroying a hierarchy never
   // synchronises the device, so other hierarchies' work keeps running
   CK(dev_alloc(H, (void**)&H.pool, H.pool_elems * sizeof(double)));

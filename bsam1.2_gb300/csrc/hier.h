@@ -80,6 +80,11 @@ struct TableUpload {
   }
 };
 
+// tail_cells up to which a hierarchy is set for a single run's latency (the default)
+constexpr long long kTailLatency = 2048;
+// hierarchies of a context that one run keeps (its states, a regrid's old and new one)
+constexpr int kFewHiers = 8;
+
 struct Hier {
   bsamg_ctx* ctx = nullptr;
   int ndims = 2, nrvars = 2, mbc = 1, problem = 1;
@@ -121,7 +126,11 @@ struct Hier {
   // coarse tail of the V-cycle (levels <= tail_level run in one CTA); the
   // recorded programs per (minlevel, nsmooth): device phases and their count
   int tail_level = -kMaxDepth - 2;
-  long long tail_cells = 2048;  // latency-friendly; a serving loop may raise it
+  long long tail_cells = kTailLatency;  // latency-friendly; a serving loop may raise it
+  // launches ahead of the previous kernel's end (launch_after) are for runs
+  // that have the GPU to themselves
+  bool crowded = false;  // committed beside more than kFewHiers hierarchies of the context
+  void launch_order() { s.early = !crowded && tail_cells <= kTailLatency; }
   // keys: (start level, minlevel, nsmooth) for V-cycles, (start level,
   // minlevel, -field) for FillDown
   using TailKey = std::tuple<int, int, int>;
@@ -202,7 +211,7 @@ struct Hier {
   size_t reserved = 0;  // bytes counted against the context budget
 
   LevelT lev[kNLev];
-  cudaStream_t s = nullptr;
+  LaunchStream s;
   double* d_partial = nullptr;
   int partial_cap = 0;
   double* d_norm = nullptr;      // [0] norm, [1] raw sum, plus scratch

@@ -12,11 +12,21 @@ namespace bsamg {
 
 constexpr int kNormOutLen = 8 + 3 * 128;
 
+// A stream and how launch_after uses it: as programmatic dependents, or in
+// the plain order.
+struct LaunchStream {
+  cudaStream_t s = nullptr;
+  bool early = true;
+  LaunchStream() = default;
+  LaunchStream(cudaStream_t st, bool e = true) : s(st), early(e) {}
+  operator cudaStream_t() const { return s; }
+};
+
 struct LaunchCtx {
   const PatchDev* P;  // device patch table
   double* pool;       // device FP64 pool
   float* fpool;       // device FP32 pool (mixed path), may be null
-  cudaStream_t s;
+  LaunchStream s;
   ProbParams pp;
   int ndims;
 };
@@ -251,7 +261,7 @@ int launch_norm_partial(const LaunchCtx& c, const Blk* blk, int nblk,
 // with `one` the norm also goes to *one.  out must hold
 // kNormOutLen doubles (out[8 ..] is scratch of the two-stage sum); the
 // partials hold nrvars values per block.
-int launch_norm_finish(cudaStream_t s, const double* partial, int nblk,
+int launch_norm_finish(LaunchStream s, const double* partial, int nblk,
                        int nrvars, double count, int errortype, double* out,
                        int* nonfinite, double* host = nullptr, double* one = nullptr);
 int launch_ghost_stage(const LaunchCtx& c, const GhostOp* ops, int n);
@@ -296,13 +306,17 @@ int tail_smem_attributes(int problem);
 // after_previous(): it lets the next kernel do the same and waits until the
 // one before has finished and its writes are visible.  Grids of many waves are
 // launched in the plain order: their early CTAs wait in the slots of the
-// running kernel's last wave (a step at 256^3 5.43 -> 5.56 ms).
+// running kernel's last wave (a step at 256^3 5.43 -> 5.56 ms).  Nor are those
+// of a hierarchy that shares the GPU with many (Hier::launch_order): CTAs that
+// wait hold the slots of the others' kernels (serving 200 requests a second,
+// early launches 1820 steps/s and a median of 310 ms, the plain order 2280 and
+// 40 ms).
 constexpr unsigned kEarlyCtas = 1024;
 __device__ __forceinline__ void after_previous() {
   asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory");
 }
 template <typename... P, typename... A>
-inline void launch_after(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... a) {
+inline void launch_after(void (*k)(P...), dim3 grid, dim3 block, size_t smem, LaunchStream s, A&&... a) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -312,7 +326,7 @@ inline void launch_after(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cu
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = (unsigned long long)grid.x * grid.y * grid.z <= kEarlyCtas ? 1 : 0;
+  cfg.numAttrs = s.early && (unsigned long long)grid.x * grid.y * grid.z <= kEarlyCtas ? 1 : 0;
   cudaLaunchKernelEx(&cfg, k, std::forward<A>(a)...);
 }
 #endif

@@ -1120,6 +1120,7 @@ void set_tail(Hier& H, long long cells) {
     progs->clear();
   }
   H.tail_cells = cells;
+  H.launch_order();
   H.tail_level = -kMaxDepth - 2;
   long long sum = 0;
   for (int l = H.minlevel; l <= H.maxlevel; l++) {
