@@ -53,6 +53,15 @@ struct Geo {
   int sy, sz, sq;
 };
 
+// How the rows of a level are dealt to the CTAs, as one of them sees it:
+// whether the level is shared out, whether it holds the domain's first and
+// last row, and the ranks below and above (around the domain) with the rows
+// of the one below.
+struct Part {
+  bool shared, first, last;
+  int lo, hi, lo_rows;
+};
+
 // One level as one CTA (or one launch) sees it: q, f, the coarse image c of
 // q, and x, the frozen data beside it (qold in q's layout, or base planes in
 // f's).  Pointers are to cell (0,0,0) of variable 1.
@@ -300,15 +309,18 @@ __device__ __forceinline__ typename TR::T ghosted_value(const typename TR::T* q,
 }
 
 template <class TR, int DIM>
-__device__ __forceinline__ typename TR::T slab_value(const typename TR::T* q, const Geo& g, int i, int j, int k, int v,
-                                                     const UniBC& bc, const typename TR::Par& par);
+__device__ __forceinline__ typename TR::T slab_value(const typename TR::T* q, const Geo& g, const Part& pt, int i,
+                                                     int j, int k, int v, const UniBC& bc,
+                                                     const typename TR::Par& par);
 
 // CorrectFine step 1 (afasroutines.f90:892-895, :934-938): the coarse image
 // becomes parent q - image, ghosts (and a slab's halo rows) included.  WHOLE:
-// a whole level, whose parent's edge and corner ghosts may be stale.
+// a whole level, whose parent's edge and corner ghosts may be stale; else pu
+// is the parent's part.
 template <class TR, int DIM, bool WHOLE>
-__device__ __forceinline__ void correct_a(const View<typename TR::T>& V, const View<typename TR::T>& U, int t0, int nt,
-                                          const UniBC& bc, const typename TR::Par& par) {
+__device__ __forceinline__ void correct_a(const View<typename TR::T>& V, const View<typename TR::T>& U,
+                                          const Part& pu, int t0, int nt, const UniBC& bc,
+                                          const typename TR::Par& par) {
   const Geo& gc = V.gc;
   const int units = (gc.n0 + 2) * (DIM == 3 ? gc.n1 + 2 : 1) * (gc.nr + 2);
   const int up = gc.r0 - U.g.r0;
@@ -322,7 +334,7 @@ __device__ __forceinline__ void correct_a(const View<typename TR::T>& V, const V
 #pragma unroll
     for (int v = 0; v < TR::NV; v++) {
       const typename TR::T u = WHOLE ? ghosted_value<TR, DIM>(U.q, U.g, i, pj, pk, v, bc, par)
-                                     : slab_value<TR, DIM>(U.q, U.g, i, pj, pk, v, bc, par);
+                                     : slab_value<TR, DIM>(U.q, U.g, pu, i, pj, pk, v, bc, par);
       V.c[v * gc.sq + c] = u - V.c[v * gc.sq + c];
     }
   }
@@ -522,7 +534,8 @@ __global__ void __launch_bounds__(kBlock) k_uni_correct_a(typename TR::Mem m, co
                                                           const __grid_constant__ UniPatch u, UniBC bc,
                                                           typename TR::Par par) {
   after_previous();
-  correct_a<TR, DIM, true>(global_view<TR, DIM>(p.p, p.d, m), global_view<TR, DIM>(u.p, u.d, m), UNI_T0, bc, par);
+  correct_a<TR, DIM, true>(global_view<TR, DIM>(p.p, p.d, m), global_view<TR, DIM>(u.p, u.d, m), Part{}, UNI_T0, bc,
+                           par);
 }
 template <class TR, int DIM>
 __global__ void __launch_bounds__(kBlock) k_uni_correct_b(typename TR::Mem m, const __grid_constant__ UniPatch p,
@@ -586,15 +599,6 @@ __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// How the rows of a level are dealt to the CTAs, as one of them sees it:
-// whether the level is shared out, whether it holds the domain's first and
-// last row, and the ranks below and above (around the domain) with the rows
-// of the one below.
-struct Part {
-  bool shared, first, last;
-  int lo, hi, lo_rows;
-};
-
 // Where the images of a slab's first and last row go: a halo row of the CTA
 // below (above), the slab's own ghost row beyond a wall (bc applied), or,
 // on a level one CTA holds, its own opposite ghost row.
@@ -650,12 +654,15 @@ __device__ __forceinline__ void push_slab(typename TR::T* q, const Geo& g, const
 }
 
 // The value at a cell of a slab's ghosted range whose edge and corner ghosts
-// may be stale: columns (and, in 3D, x rows) beyond a face from their
-// interior cell, the halo and ghost rows as they are
+// may be stale: columns and rows beyond a face from their interior cell, the
+// offset across x before the walls as SetGhost applies them (a wall's ghost
+// row, already through UserBC, would take the offset after it); the halo rows
+// as they are
 template <class TR, int DIM>
-__device__ __forceinline__ typename TR::T slab_value(const typename TR::T* q, const Geo& g, int i, int j, int k, int v,
-                                                     const UniBC& bc, const typename TR::Par& par) {
-  int nb = 0, sh = 0, si = i, sj = j;
+__device__ __forceinline__ typename TR::T slab_value(const typename TR::T* q, const Geo& g, const Part& pt, int i,
+                                                     int j, int k, int v, const UniBC& bc,
+                                                     const typename TR::Par& par) {
+  int nb = 0, sh = 0, si = i, sj = j, sk = k;
   if (i < 1 || i > g.n0) {
     if (bc.phys[0]) {
       si = i < 1 ? 1 : g.n0;
@@ -673,9 +680,15 @@ __device__ __forceinline__ typename TR::T slab_value(const typename TR::T* q, co
       sj = j < 1 ? g.n1 : 1;
     }
   }
-  typename TR::T u = TR::shift(q[v * g.sq + gcell<DIM>(g, si, sj, k)], sh, v, par);
-  if (nb > 0) u = TR::wall(u, bc.mask, v);
-  if (nb > 1) u = TR::wall(u, bc.mask, v);
+  int& row = DIM == 2 ? sj : sk;
+  if (bc.phys[DIM - 1] && ((row < 1 && pt.first) || (row > g.nr && pt.last))) {
+    row = row < 1 ? 1 : g.nr;
+    nb++;
+  }
+  typename TR::T u = TR::shift(q[v * g.sq + gcell<DIM>(g, si, sj, sk)], sh, v, par);
+#pragma unroll
+  for (int z = 0; z < DIM; z++)
+    if (z < nb) u = TR::wall(u, bc.mask, v);
   return u;
 }
 
@@ -914,7 +927,7 @@ __device__ __forceinline__ void load_cells(const View<typename TR::T>& V, const 
 // CorrectFine step 2 on a slab with the face images, one thread a fine cell
 template <class TR, int DIM, bool INLINE_A>
 __device__ __forceinline__ void correct_slab(const View<typename TR::T>& V, const View<typename TR::T>& U,
-                                             const Part& pt, int t, int nt, const UniBC& bc,
+                                             const Part& pt, const Part& pu, int t, int nt, const UniBC& bc,
                                              const typename TR::Par& par) {
   using T = typename TR::T;
   const Geo &g = V.g, &gc = V.gc;
@@ -932,8 +945,8 @@ __device__ __forceinline__ void correct_slab(const View<typename TR::T>& V, cons
     for (int v = 0; v < TR::NV; v++) {
       auto at = [&](int ii, int jj, int kk) -> T {
         if (!INLINE_A) return V.c[v * gc.sq + gcell<DIM>(gc, ii, jj, kk)];
-        return slab_value<TR, DIM>(U.q, U.g, ii, DIM == 2 ? jj + up : jj, kk + up, v, bc, par) -
-               slab_value<TR, DIM>(V.c, gc, ii, jj, kk, v, bc, par);
+        return slab_value<TR, DIM>(U.q, U.g, pu, ii, DIM == 2 ? jj + up : jj, kk + up, v, bc, par) -
+               slab_value<TR, DIM>(V.c, gc, pt, ii, jj, kk, v, bc, par);
       };
       auto row = [&](int jj, int kk) -> T {  // the x stage at coarse row (jj, kk)
         const T lo = at(ci, jj, kk), hi = at(ci + 1, jj, kk);
@@ -1039,10 +1052,10 @@ __global__ void __launch_bounds__(kUniThreads, 1) k_uni_cycle(const PatchDev* __
     if (A.L[x].mul && !A.L[x + 1].mul) all();  // CTA 0 has finished the levels it holds
     const View<T> V = slab_view<TR, DIM, false>(A, x, rank, pt), U = slab_view<TR, DIM, true>(A, x + 1, rank, pu);
     if (TR::kStoreRf) {
-      correct_a<TR, DIM, false>(V, U, t, nt, A.bc, par);
+      correct_a<TR, DIM, false>(V, U, pu, t, nt, A.bc, par);
       __syncthreads();
     }
-    correct_slab<TR, DIM, !TR::kStoreRf>(V, U, pt, t, nt, A.bc, par);
+    correct_slab<TR, DIM, !TR::kStoreRf>(V, U, pt, pu, t, nt, A.bc, par);
     sync(x);
     smooth(x);
   }
