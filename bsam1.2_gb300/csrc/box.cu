@@ -1827,7 +1827,9 @@ __global__ void __launch_bounds__(256) k_bx_merge(double* __restrict__ pool, lon
 // images.  e, g and pb stay in shared memory from cycle to cycle; qhi, qlo
 // and f stay where the other kernels keep them (a cluster barrier makes one
 // CTA's writes visible to the others).  Per cell it computes what the
-// separate kernels compute; the norms add the same squares in another order.
+// separate kernels compute; the norms add the same squares in another order,
+// in FP32 over a warp's cells (at most 128; there a CTA's 256 or 512) and in
+// FP64 from there.
 //
 // A step of such a box was some 14 launches and a graph with a conditional
 // loop of six launches a V-cycle; now it is this one, the fill of the coarse
@@ -1854,6 +1856,7 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_bx_solve(float* __restrict__
   after_previous();
   const int rank = A.ctas > 1 ? uni::my_rank() : 0;
   const int t = threadIdx.x, nt = blockDim.x;
+  static_assert(kCycThreads <= 16 * 32, "a half-warp adds the sums of the warps");
   __shared__ float wsum[2][kCycThreads / 32];
   __shared__ double part[2][32];  // two norms' worth: a CTA may start the next while another still adds up this one
   __shared__ double norm_now;
@@ -1911,17 +1914,17 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_bx_solve(float* __restrict__
     turn ^= 1;
     __syncthreads();
     if (t < 32) {
-      float a = t < nt / 32 ? wsum[0][t] : 0.f, b = t < nt / 32 ? wsum[1][t] : 0.f;
-      for (int o = 8; o > 0; o >>= 1) {
-        a += __shfl_down_sync(0xffffffffu, a, o);
-        b += __shfl_down_sync(0xffffffffu, b, o);
-      }
-      a = __shfl_sync(0xffffffffu, a, 0);
-      b = __shfl_sync(0xffffffffu, b, 0);
+      // in FP64 from a warp's cells on, half a warp a variable; the warps
+      // without a pair hold zeros, whose additions are left out
+      const int warps = (units + 31) >> 5;
+      double s = f2d((t & 15) < nt / 32 ? wsum[t >> 4][t & 15] : 0.f);
+      for (int o = 8; o > 0; o >>= 1)
+        if (o < warps) s += __shfl_down_sync(0xffffffffu, s, o, 16);
+      const double a = __shfl_sync(0xffffffffu, s, 0), b = __shfl_sync(0xffffffffu, s, 16);
       if (t < A.ctas) {  // to every CTA
         double* p = A.ctas > 1 ? uni::on_rank(sums, t) : sums;
-        p[rank] = f2d(a);
-        p[16 + rank] = f2d(b);
+        p[rank] = a;
+        p[16 + rank] = b;
       }
     }
     all();
