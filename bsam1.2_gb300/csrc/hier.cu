@@ -121,6 +121,13 @@ int enq_set_ghost(Hier& H, int level, int ipass) {
   return BSAMG_OK;
 }
 
+// before the first smoothing of a uniform level on which the caller may not
+// have set the ghosts (kern_uni.cuh k_uni_walls)
+int enq_entry_walls(Hier& H, int level, int nsmooth) {
+  if (nsmooth < 1 || !uni_level(H, level)) return BSAMG_OK;
+  return after_launch(H, uni64(H).walls(H.lc(), H.ubc, H.hP[uni_patch(H, level)]));
+}
+
 int enq_level_relax(Hier& H, int level, int nsmooth) {
   for (int pass = 1; pass <= nsmooth; pass++)
     for (int rb = 1; rb <= 2; rb++) {
@@ -519,8 +526,9 @@ namespace {
 
 int check_nonfinite(Hier& H) { return *H.h_nonfinite ? BSAMG_ERR_NONFINITE : BSAMG_OK; }
 
+// ghosts_set: SetGhost has just been done on the finest level
 int multigrid_iterations(Hier& H, int finest, int minlevel, int nsmooth, int maxvcycles, double tol,
-                         int errortype, int mode, int strict, int* ncycles, double* residuals) {
+                         int errortype, int mode, int strict, int* ncycles, double* residuals, bool ghosts_set) {
   if (finest > H.maxlevel || minlevel < H.minlevel || finest < 0 || minlevel > 0) return BSAMG_ERR_ARG;
   if (maxvcycles < 1 || nsmooth < 1 || (errortype != 1 && errortype != 2)) return BSAMG_ERR_ARG;
   if (mode != BSAMG_MODE_FP64 && mode != BSAMG_MODE_MIXED) return BSAMG_ERR_ARG;
@@ -541,6 +549,7 @@ int multigrid_iterations(Hier& H, int finest, int minlevel, int nsmooth, int max
   Hier::GraphRec* gr = nullptr;
   RET(capture_graph(H, std::make_tuple(mode, finest, minlevel, nsmooth, errortype),
                     [&] { return enq_iteration(H, finest, minlevel, nsmooth, errortype); }, &gr));
+  if (!ghosts_set) RET(enq_entry_walls(H, finest, nsmooth));
   int it;
   double r = 0.0;
   for (it = 1; it <= maxvcycles; it++) {
@@ -1183,6 +1192,7 @@ int bsamg_level_relax(bsamg_hier* h, int level, int nsmooth) {
   if (!h || !h->committed || !level_ok(*h, level) || nsmooth < 0) return BSAMG_ERR_ARG;
   RET(set_device(*h));
   h->box_g_valid = false;
+  RET(enq_entry_walls(*h, level, nsmooth));
   return enq_level_relax(*h, level, nsmooth);
 }
 
@@ -1205,6 +1215,7 @@ int bsamg_vcycle(bsamg_hier* h, int level, int minlevel, int nsmooth) {
     return BSAMG_ERR_ARG;
   RET(set_device(*h));
   h->box_g_valid = false;
+  RET(enq_entry_walls(*h, level, nsmooth));
   return enq_vcycle(*h, level, minlevel, nsmooth);
 }
 
@@ -1224,7 +1235,7 @@ int bsamg_multigrid_iterations(bsamg_hier* h, int finestlevel, int minlevel, int
   if (!h || !h->committed) return BSAMG_ERR_ARG;
   (void)updateauxfreq;  // both plugins have maux = 0: UpdateAuxInVcycle returns at :417
   return multigrid_iterations(*h, finestlevel, minlevel, nsmooth, maxvcycles, qerrortol, errortype, mode, strict,
-                              ncycles, residuals);
+                              ncycles, residuals, false);
 }
 
 int bsamg_time_step(bsamg_hier* h, int first, int finestlevel, int minlevel, int nsmooth, int maxvcycles,
@@ -1238,7 +1249,7 @@ int bsamg_time_step(bsamg_hier* h, int first, int finestlevel, int minlevel, int
   RET(enq_copy_q_to_qold(*h, minlevel, finestlevel));
   (void)updateauxfreq;
   return multigrid_iterations(*h, finestlevel, minlevel, nsmooth, maxvcycles, qerrortol, errortype, mode, strict,
-                              ncycles, residuals);
+                              ncycles, residuals, true);
 }
 
 int bsamg_sync(bsamg_hier* h) {

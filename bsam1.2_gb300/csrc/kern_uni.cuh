@@ -5,9 +5,10 @@
 // passed through the plugin's UserBC once per physical face it lies beyond.
 // The operations here push those images when they write the interior cell,
 // so a level needs no ghost pass of its own: a colour sweep reads the ghosts
-// the previous one left, and the images it writes are of its own colour,
-// which no cell of that colour reads (periodic extents are even; a physical
-// face's ghost is read only by the cell it images).  Every cell computes what
+// the previous one left (before the first: k_uni_walls), and the images it
+// writes are of its own colour, which no cell of that colour reads (periodic
+// extents are even; a physical face's ghost is read only by the cell it
+// images).  Every cell computes what
 // the stand-alone kernel of the operation computes, in the same order.
 //
 // The same operations run in two forms: as one launch per operation over a
@@ -449,7 +450,8 @@ __device__ __forceinline__ int shell_units(const Geo& g) {
   const int e0 = g.n0 + 2;
   return DIM == 3 ? 2 * e0 * (g.n1 + 2) + g.N * (2 * e0 + 2 * g.n1) : 2 * e0 + 2 * g.N;
 }
-template <class TR, int DIM>
+// WALLS: the ghosts beyond one wall of the cells of colour 2 only (k_uni_walls)
+template <class TR, int DIM, bool WALLS = false>
 __device__ __forceinline__ void set_ghost(typename TR::T* q, const Geo& g, const UniDim& d, int t0, int nt,
                                           const UniBC& bc, const typename TR::Par& par) {
   const int e0 = g.n0 + 2, cap = DIM == 3 ? e0 * (g.n1 + 2) : e0;
@@ -480,6 +482,18 @@ __device__ __forceinline__ void set_ghost(typename TR::T* q, const Geo& g, const
       }
     }
     const int jj = DIM == 2 ? row : j, kk = row;
+    if (WALLS) {
+      const int x[3] = {i, jj, kk}, n[3] = {g.n0, DIM == 3 ? g.n1 : g.N, g.N};
+      int beyond = 0, walls = 0, sum = 0;
+#pragma unroll
+      for (int b = 0; b < DIM; b++) {
+        const bool out = x[b] < 1 || x[b] > n[b];
+        beyond += out;
+        walls += out && bc.phys[b];
+        sum += x[b] < 1 ? 1 : (x[b] > n[b] ? n[b] : x[b]);
+      }
+      if (beyond != 1 || walls != 1 || !(sum & 1)) continue;
+    }
 #pragma unroll
     for (int v = 0; v < TR::NV; v++)
       q[v * g.sq + gcell<DIM>(g, i, jj, kk)] = ghosted_value<TR, DIM>(q, g, i, jj, kk, v, bc, par);
@@ -551,6 +565,18 @@ __global__ void __launch_bounds__(kBlock) k_uni_ghost(typename TR::Mem m, const 
   after_previous();
   const View<typename TR::T> V = global_view<TR, DIM>(p.p, p.d, m);
   set_ghost<TR, DIM>(V.q, V.g, p.d, UNI_T0, bc, par);
+}
+// The ghosts beyond the walls of a level whose ghosts the caller may not have
+// set, before its first smoothing.  SetGhost after the first colour's sweep
+// refreshes them for the second colour; the sweep here pushes its own
+// colour's only.  (The second colour's periodic images are read by the first
+// colour alone, which takes them as they are, here and there.)
+template <class TR, int DIM>
+__global__ void __launch_bounds__(kBlock) k_uni_walls(typename TR::Mem m, const __grid_constant__ UniPatch p, UniBC bc,
+                                                      typename TR::Par par) {
+  after_previous();
+  const View<typename TR::T> V = global_view<TR, DIM>(p.p, p.d, m);
+  set_ghost<TR, DIM, true>(V.q, V.g, p.d, UNI_T0, bc, par);
 }
 template <class TR, int DIM>
 __global__ void __launch_bounds__(kBlock) k_uni_fill(typename TR::Mem m, const __grid_constant__ UniPatch p,
@@ -1123,6 +1149,14 @@ struct UniLaunchers {
     else launch_after(k_uni_ghost<TR, 3>, nb, kBlock, 0, c.s, TR::mem(c), p, bc, TR::par(c));
     return 1;
   }
+  static int walls(const LaunchCtx& c, const UniBC& bc, const PatchDev& hp) {
+    if (!bc.phys[0] && !bc.phys[1] && !(c.ndims == 3 && bc.phys[2])) return 0;
+    const UniPatch p = uni_patch_of(hp);
+    const int nb = blocks(cells(hp.qn) - cells(hp.mx));
+    if (c.ndims == 2) launch_after(k_uni_walls<TR, 2>, nb, kBlock, 0, c.s, TR::mem(c), p, bc, TR::par(c));
+    else launch_after(k_uni_walls<TR, 3>, nb, kBlock, 0, c.s, TR::mem(c), p, bc, TR::par(c));
+    return 1;
+  }
   static int fill(const LaunchCtx& c, const UniBC& bc, const PatchDev& hp, const PatchDev& hu, int fields) {
     const UniPatch p = uni_patch_of(hp), u = uni_patch_of(hu);
     const int nb = blocks(cells(hp.cmx));
@@ -1183,7 +1217,7 @@ struct UniLaunchers {
   }
   static PluginUni table() {
     return PluginUni{TR::NV, TR::kXPlanes, TR::kXGhosted, (int)sizeof(typename TR::T), &relax, &restrict_load, &correct,
-                     &ghost, &fill, &fill_small, &cycle, &cycle_fit};
+                     &ghost, &walls, &fill, &fill_small, &cycle, &cycle_fit};
   }
 };
 

@@ -110,6 +110,7 @@ struct PluginUni {
   int (*restrict_load)(const LaunchCtx&, const UniBC&, int patch, const PatchDev& p, const PatchDev& u);
   int (*correct)(const LaunchCtx&, const UniBC&, const PatchDev& p, const PatchDev& u);
   int (*ghost)(const LaunchCtx&, const UniBC&, const PatchDev& p);
+  int (*walls)(const LaunchCtx&, const UniBC&, const PatchDev& p);
   int (*fill)(const LaunchCtx&, const UniBC&, const PatchDev& p, const PatchDev& u, int fields);
   int (*fill_small)(const LaunchCtx&, const UniCycle& A, int fields);
   int (*cycle)(const LaunchCtx&, const UniCycle& A, int smem);

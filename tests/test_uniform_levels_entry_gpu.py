@@ -1,9 +1,10 @@
 """Uniform levels (kern_uni.cuh) against the oracle: rows beyond a wall under a
-quasi-periodic offset."""
+quasi-periodic offset, and calls on a state whose ghosts the caller did not
+set."""
 import numpy as np
 import pytest
 
-from tests.test_uniform_levels_gpu import BIO, CH3, GROWTH, PX, W
+from tests.test_uniform_levels_gpu import BIO, CH2, CH3, GROWTH, PX, W
 
 pytestmark = pytest.mark.gpu
 
@@ -17,6 +18,16 @@ QPO = {
     "3d-wall-z": (CH3, (16, 24, 12), -1, (PX, PX, W), [0.25, -0.5]),
     "3d-above": (CH3, (32, 24, 20), -2, (PX, W, W), [0.25, -0.5]),
     "3d-growth": (GROWTH, (16, 16, 12), -2, (PX, W, W), [0.25, -0.5, 0.75]),
+}
+STALE = {
+    "2d-wall": (CH2, (40, 24), -3, (W, W), None),
+    "2d-above": (CH2, (96, 80), -3, (W, PX), None),
+    "2d-periodic": (CH2, (32, 48), -3, (PX, PX), None),
+    "2d-bio": (BIO, (72, 40), -3, (W, W), None),
+    "2d-bio-qpo": (BIO, (48, 32), -3, (PX, W), [0.25, -0.5]),
+    "3d-wall": (CH3, (20, 12, 28), -2, (W, W, W), None),
+    "3d-mixed": (CH3, (16, 12, 16), -2, (PX, W, PX), None),
+    "3d-growth": (GROWTH, (24, 16, 12), -2, (W, W, W), None),
 }
 
 
@@ -64,3 +75,20 @@ def test_offset_across_x_beside_a_wall(pkg, ctx, oracle_mod, case):
             h.vcycle(0, mn, 2)
     same_bits(g, o, QPO[case], ("q", "qc", "f", "rf"))
     g.close()
+
+
+@pytest.mark.parametrize("tail", [2048, 0])
+@pytest.mark.parametrize("case", list(STALE))
+def test_ghosts_the_caller_did_not_set(pkg, ctx, oracle_mod, case, tail):
+    """LevelRelax and the V-cycle read the ghosts they find in their first
+    colour sweep and SetGhost's from then on (afasroutines.f90:532-557)."""
+    spec = STALE[case]
+    mn = spec[2]
+    for call in (lambda h: h.level_relax(0, 1), lambda h: h.level_relax(mn, 2), lambda h: h.vcycle(0, mn, 2),
+                 lambda h: h.vcycle(-1, mn, 1),
+                 lambda h: h.multigrid_iterations(0, mn, nsmooth=2, maxvcycles=2, tol=1e-300)):
+        g, o = pair(pkg, ctx, oracle_mod, spec, 12)
+        g.set_tail_cells(tail)
+        call(g), call(o)
+        same_bits(g, o, spec, ("q", "f"))
+        g.close()
