@@ -155,8 +155,11 @@ int enq_vcycle(Hier& H, int level, int minlevel, int nsmooth) {
     if (level == minlevel) return BSAMG_OK;
     const int p = uni_patch(H, level), u = uni_patch(H, level - 1);
     RET(after_launch(H, U.restrict_load(H.lc(), H.ubc, p, H.hP[p], H.hP[u])));
+    // both write face ghosts; the last sweep of a smoothing writes the rest
+    if (nsmooth < 1) RET(enq_set_ghost(H, level - 1, 0));
     RET(enq_vcycle(H, level - 1, minlevel, nsmooth));
     RET(after_launch(H, U.correct(H.lc(), H.ubc, H.hP[p], H.hP[u])));
+    if (nsmooth < 1) RET(enq_set_ghost(H, level, 0));
     return enq_level_relax(H, level, nsmooth);
   }
   if (!H.rec && level <= H.tail_level && level >= minlevel) {

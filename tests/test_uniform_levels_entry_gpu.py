@@ -1,6 +1,6 @@
 """Uniform levels (kern_uni.cuh) against the oracle: rows beyond a wall under a
-quasi-periodic offset, and calls on a state whose ghosts the caller did not
-set."""
+quasi-periodic offset, calls on a state whose ghosts the caller did not set,
+and a V-cycle without smoothing."""
 import numpy as np
 import pytest
 
@@ -92,3 +92,16 @@ def test_ghosts_the_caller_did_not_set(pkg, ctx, oracle_mod, case, tail):
         call(g), call(o)
         same_bits(g, o, spec, ("q", "f"))
         g.close()
+
+
+@pytest.mark.parametrize("tail", [2048, 0])
+@pytest.mark.parametrize("case", list(STALE))
+def test_vcycle_without_smoothing(pkg, ctx, oracle_mod, case, tail):
+    spec = STALE[case]
+    g, o = pair(pkg, ctx, oracle_mod, spec, 13)
+    g.set_tail_cells(tail)
+    for h in (g, o):
+        h.set_ghost(0, 0)
+        h.vcycle(0, spec[2], 0)
+    same_bits(g, o, spec, ("q", "qc", "f", "rf"))
+    g.close()
