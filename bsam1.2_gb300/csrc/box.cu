@@ -2320,25 +2320,6 @@ int cycle_fit(int ndims, int ctas, int smem) {
   return n;
 }
 
-template <typename K, typename... Args>
-cudaError_t launch_cluster(K k, int ctas, int threads, int smem, cudaStream_t s, Args... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(ctas);
-  cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute at[2];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = ctas;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.numAttrs = 2;
-  return cudaLaunchKernelEx(&cfg, k, args...);
-}
-
 // The cluster's plan for the levels top .. minlevel with the first `share`
 // of them shared out; false when it does not fit (shared memory, pairs a
 // thread, the coarsest level's one pair a thread)

@@ -1172,22 +1172,8 @@ struct UniLaunchers {
     return 1;
   }
   static int cycle(const LaunchCtx& c, const UniCycle& A, int smem) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(A.ctas);
-    cfg.blockDim = dim3(A.threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = c.s;
-    cudaLaunchAttribute at[2];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = A.ctas;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 2;
-    cudaError_t e = c.ndims == 2 ? cudaLaunchKernelEx(&cfg, k_uni_cycle<TR, 2>, c.P, TR::mem(c), A, TR::par(c))
-                                 : cudaLaunchKernelEx(&cfg, k_uni_cycle<TR, 3>, c.P, TR::mem(c), A, TR::par(c));
+    auto k = c.ndims == 2 ? k_uni_cycle<TR, 2> : k_uni_cycle<TR, 3>;
+    cudaError_t e = launch_cluster(k, A.ctas, A.threads, smem, c.s, c.P, TR::mem(c), A, TR::par(c));
     return e == cudaSuccess ? 1 : -1;
   }
   // raise the kernel's limits (clusters above the portable 8 CTAs, dynamic

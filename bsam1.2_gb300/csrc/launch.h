@@ -329,6 +329,26 @@ inline void launch_after(void (*k)(P...), dim3 grid, dim3 block, size_t smem, La
   cfg.numAttrs = s.early && (unsigned long long)grid.x * grid.y * grid.z <= kEarlyCtas ? 1 : 0;
   cudaLaunchKernelEx(&cfg, k, std::forward<A>(a)...);
 }
+// the same for one cluster of `ctas` CTAs, the largest waiters there are: up to
+// 16 SMs' shared memory
+template <typename... P, typename... A>
+inline cudaError_t launch_cluster(void (*k)(P...), int ctas, int threads, int smem, LaunchStream s, A&&... a) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = ctas;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = s.early ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, k, std::forward<A>(a)...);
+}
 #endif
 
 }  // namespace bsamg
