@@ -314,7 +314,6 @@ int enq_copy_q_to_qold(Hier& H, int minlevel, int finest) {
 
 // the part of FillDown that enq_iteration leaves to the end of the loop
 int finish_fill_down(Hier& H, int finest, int minlevel) {
-  if (!H.uni) return BSAMG_OK;
   if (finest > 0) RET(enq_fill_down(H, 1, finest, 0));
   return uni_enq_fill(H, uni64(H), 3, 0, minlevel);
 }
@@ -561,7 +560,10 @@ int multigrid_iterations(Hier& H, int finest, int minlevel, int nsmooth, int max
     if (residuals) residuals[it - 1] = r;
     if (check_nonfinite(H) || r < tol) break;
   }
-  RET(finish_fill_down(H, finest, minlevel));
+  if (H.uni) {
+    RET(finish_fill_down(H, finest, minlevel));
+    RET(stream_wait(H));  // the step is finished when the call returns
+  }
   RET(check_nonfinite(H));
   bool conv = it <= maxvcycles;
   if (ncycles) *ncycles = conv ? it : maxvcycles;

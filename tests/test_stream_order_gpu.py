@@ -56,3 +56,12 @@ def test_raised_tail_cells_keep_the_plain_launch_order(pkg, ctx, cu):
     h.close()
     assert len(plain) == len(early) > 8
     assert 1 in early and set(plain) == {0}
+
+
+def test_a_step_is_finished_when_the_call_returns(pkg, ctx, cu):
+    """FillDown of q and f below level 0 included (some 100 us of kernels at 160^3)"""
+    h = box(pkg, ctx, (160, 160, 160), -4)
+    for s in range(3):
+        h.time_step(s == 0, 0, -4, tol=1e-30, maxvcycles=1, mode="fp64")
+        assert cu.cuStreamQuery(h.stream()) == 0
+    h.close()
