@@ -31,6 +31,12 @@
 //   static int stats(int ndims);       // bit 0: integral of phi, bit 1: CH energy
 //   // optional: false when relax and op read nothing of qold (default true)
 //   static constexpr bool kQold;
+//   // optional: true when the relaxations and operators read of a ghosted
+//   // array only the cell itself and its face neighbours (default false).
+//   // Levels of one patch then take the operations that write their own
+//   // ghosts (kern_uni.cuh), which set edge and corner ghosts only at the end
+//   // of a smoothing; a problem with wider stencils keeps SetGhost after each
+//   static constexpr bool kFaceStencils;
 //   // device, FP64, evaluated in the reference's order (the FP64 part of a
 //   // plugin file is compiled with --fmad=false):
 //   template <int DIM> __device__ static void relax(const Cell64&, const double* c, const ProbParams&);
@@ -172,12 +178,21 @@ template <class PL>
 struct UsesQold<PL, decltype((void)PL::kQold)> {
   static constexpr bool value = PL::kQold;
 };
+// PL::kFaceStencils where the plugin states it, else false
+template <class PL, class = void>
+struct FaceStencils {
+  static constexpr bool value = false;
+};
+template <class PL>
+struct FaceStencils<PL, decltype((void)PL::kFaceStencils)> {
+  static constexpr bool value = PL::kFaceStencils;
+};
 
 struct Plugin {
   int kind = 0;
   const char* name = nullptr;
   int nvars = 0, nparams = 0;
-  bool coeffs_only = false, box = false;
+  bool coeffs_only = false, box = false, face_stencils = false;
   void (*set_params)(ProbParams&, const double*, int) = nullptr;
   void (*coefficients)(const ProbParams&, int, double, double*) = nullptr;
   int (*bc_mask)(int) = nullptr;

@@ -31,6 +31,7 @@ int register_part() {
   p.nparams = PL::kNParams;
   p.coeffs_only = PL::kCoeffsOnly;
   p.box = PL::kBox;
+  p.face_stencils = FaceStencils<PL>::value;
   p.set_params = &PL::set_params;
   p.coefficients = &PL::coefficients;
   p.bc_mask = &PL::bc_mask;

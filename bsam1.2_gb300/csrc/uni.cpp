@@ -5,7 +5,7 @@
 namespace bsamg {
 
 bool uni_eligible(const Hier& H) {
-  if (H.mbc != 1) return false;
+  if (H.mbc != 1 || !find_plugin(H.problem)->face_stencils) return false;
   const HostPatch* root = nullptr;
   for (int l = 0; l >= H.minlevel; l--) {
     if (H.L(l).patches.size() != 1) return false;

@@ -7,7 +7,8 @@ namespace bsamg {
 
 // Levels minlevel .. 0 are each one patch covering its parent, one ghost
 // layer, every dimension periodic (even extents) or between physical faces;
-// then SetGhost on them is the image copy of kern_uni.cuh.
+// then SetGhost on them is the image copy of kern_uni.cuh.  The plugin's
+// stencils reach face neighbours only.
 bool uni_eligible(const Hier& H);
 // the boundary conditions of those levels
 UniBC uni_bc(const Hier& H);

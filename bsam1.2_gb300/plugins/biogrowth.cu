@@ -14,6 +14,7 @@ struct BioGrowth {
   static constexpr int kNParams = 5;  // dt, eps, gamma, lambda, c0
   static constexpr bool kCoeffsOnly = false;  // dt, gamma, lambda, c0 are kernel arguments
   static constexpr bool kBox = false;
+  static constexpr bool kFaceStencils = true;
   static constexpr bool kMixed = false;
   static constexpr int kMxBase = 0, kMxUpdate = 0;
 

@@ -16,6 +16,7 @@ struct CH {
   static constexpr bool kCoeffsOnly = true;
   static constexpr bool kBox = true;
   static constexpr bool kQold = false;  // relax and op read nothing of qold
+  static constexpr bool kFaceStencils = true;
   static constexpr bool kMixed = true;
   static constexpr int kMxBase = 1;    // phib
   static constexpr int kMxUpdate = 1;

@@ -17,6 +17,7 @@ struct Growth {
   static constexpr int kNParams = 6;  // dt, eps, gamma, lambda, c0, cpress
   static constexpr bool kCoeffsOnly = false;
   static constexpr bool kBox = false;
+  static constexpr bool kFaceStencils = true;
   static constexpr bool kMixed = true;
   static constexpr int kMxBase = 4;    // phib, nb, G, U
   static constexpr int kMxUpdate = 2;  // phib and nb follow qbar
