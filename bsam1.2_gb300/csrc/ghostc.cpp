@@ -663,8 +663,17 @@ struct PatchProg {
   std::vector<GhostOp> ops;
   std::vector<int> run;
 };
+// Work arrays that a thread keeps for the next patch, unless this one was large:
+// an adaptive level has many small patches, and a root of 256^3 cells would leave
+// 200 MB with every thread that ever compiled one.
+constexpr size_t kKeepBytes = 256 * 1024;
+template <typename T>
+void give_back_large(std::vector<T>& v) {
+  if (v.capacity() * sizeof(T) > kKeepBytes) std::vector<T>().swap(v);
+}
+
 // stage_ops of the operations that write one patch, which only conflict among
-// themselves (emit_patch); three arrays over its cells, kept between calls
+// themselves (emit_patch); three arrays over its cells
 void stage_patch(const HostPatch& P, int p, const std::vector<Em>& head, const std::vector<Em>& tail, PatchProg& out) {
   const int cells = P.qn[0] * P.qn[1] * P.qn[2], nh = (int)head.size(), m = nh + (int)tail.size();
   thread_local std::vector<int> last, wst, rst, stage;
@@ -715,6 +724,8 @@ void stage_patch(const HostPatch& P, int p, const std::vector<Em>& head, const s
   std::vector<int> fill(out.run.begin(), out.run.end() - 1);
   for (int x = 0; x < m; x++)
     if (!dead[x]) out.ops[fill[stage[x] * kTypes + op(x).op.type]++] = op(x).op;
+  for (std::vector<int>* v : {&last, &wst, &rst, &stage}) give_back_large(*v);
+  for (std::vector<char>* v : {&dead, &readf}) give_back_large(*v);
 }
 
 }  // namespace
@@ -757,12 +768,13 @@ void compile_set_ghost_all(const Hier& H, const std::vector<std::pair<int, int>>
     thread_local std::vector<Em> tail, heads[3];
     tail.clear();
     for (auto& h : heads) h.clear();
-    if (!emit_patch(*g.L, a, g.pass.data(), np, heads, tail)) {
+    if (emit_patch(*g.L, a, g.pass.data(), np, heads, tail))
+      for (int i = 0; i < np; i++)
+        stage_patch(H.patches[g.L->ps[a]], g.L->ps[a], heads[i], tail, g.prog[i * g.L->n + a]);
+    else
       g.alone = false;
-      return;
-    }
-    for (int i = 0; i < np; i++)
-      stage_patch(H.patches[g.L->ps[a]], g.L->ps[a], heads[i], tail, g.prog[i * g.L->n + a]);
+    give_back_large(tail);
+    for (auto& h : heads) give_back_large(h);
   });
   // a program: its patches' operations by (stage, type), then patch
   std::vector<std::pair<Level*, int>> progs;
