@@ -711,14 +711,14 @@ int upload_tables(Hier& H, const TableUpload& up) {
   if (!total) return BSAMG_OK;
   CK(dev_alloc(H, &H.tables, total));
   H.bytes += total;
-  std::vector<unsigned char> image(small);
+  std::vector<unsigned char>& image = H.table_image;
+  image.resize(small);
   unsigned char* const base = static_cast<unsigned char*>(H.tables);
   size_t at = 0, far = small;
   for (const auto& p : up.pieces) {
     const bool direct = p.bytes >= TableUpload::kDirect;
     size_t& o = direct ? far : at;
     *p.slot = base + o;
-    // a copy from pageable memory returns once the source has been staged
     if (direct) CK(cudaMemcpyAsync(base + o, p.data, p.bytes, cudaMemcpyHostToDevice, H.s));
     else std::memcpy(image.data() + o, p.data, p.bytes);
     o += al(p.bytes);
@@ -890,6 +890,7 @@ int commit(Hier& H) {
   CK(dev_alloc(H, (void**)&H.d_nonfinite, sizeof(int) * 4));
   RET(pinned_slot_take(H));
   CK(cudaStreamSynchronize(H.s));
+  std::vector<unsigned char>().swap(H.table_image);
   H.committed = true;
   H.regrid_ms[5] = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - tc0).count() -
                    H.regrid_ms[4];

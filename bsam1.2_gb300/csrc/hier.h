@@ -64,8 +64,8 @@ std::vector<std::vector<GhostOp>> set_ghost_sequences(const Hier& H, int level, 
 
 // The read-only tables of a commit (work lists, ghost programs) as one
 // allocation: an adaptive hierarchy has some eighty.  Small ones are gathered
-// and copied together, large ones copied from their vector, which stays in
-// place until upload_tables.
+// (Hier::table_image) and copied together, large ones copied from their
+// vector; both stay in place until the commit has waited for the stream.
 struct TableUpload {
   static constexpr size_t kDirect = 64 * 1024;
   struct Piece {
@@ -109,6 +109,7 @@ struct Hier {
   size_t e_len = 0;  // leading FP32 elements holding every patch's correction e
   size_t e_coarse_off = 0, e_coarse_len = 0;  // the part of it on levels < 0
   void* tables = nullptr;                     // every work list and ghost program of the commit
+  std::vector<unsigned char> table_image;     // its small tables while the commit's copy of them may run
   Blk* mx_norm_blk[kNLev] = {};               // padded interior lists (mixed norm)
   Blk* mx_prep_coarse = nullptr;              // interior lists of all levels < 0
   int mx_prep_coarse_n = 0;
