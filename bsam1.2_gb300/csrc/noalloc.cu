@@ -29,6 +29,7 @@
 // launch_norm_finish itself), so the two agree bit for bit.
 #include <cuda_runtime.h>
 
+#include <cstdint>
 #include <mutex>
 
 #include "../../include/bsamg.h"
@@ -143,8 +144,13 @@ extern "C" int bsamg_ch_residual_norm_noalloc(const double* q, const double* f, 
   // the hierarchy's own final reduction (two stages above 2048 blocks);
   // no non-finite flag: a NaN or Inf input shows as a NaN or Inf norm
   double* out = scratch + 2 * kMaxBlocks;
-  launch_norm_finish(s, scratch, nblk, 2, 2.0 * (double)cells, errortype, out, nullptr, nullptr, norm_out);
+  // an address that a kernel cannot store a double to is reached by a copy
+  const bool aligned = reinterpret_cast<uintptr_t>(norm_out) % alignof(double) == 0;
+  launch_norm_finish(s, scratch, nblk, 2, 2.0 * (double)cells, errortype, out, nullptr, nullptr,
+                     aligned ? norm_out : nullptr);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "bsamg_ch_residual_norm_noalloc launch");
-  return BSAMG_OK;
+  if (aligned) return BSAMG_OK;
+  e = cudaMemcpyAsync(norm_out, out, sizeof(double), cudaMemcpyDeviceToDevice, s);
+  return e == cudaSuccess ? BSAMG_OK : cuda_fail(e, "bsamg_ch_residual_norm_noalloc copy");
 }
