@@ -53,20 +53,31 @@ std::mutex g_mu;
 constexpr int kMaxDevices = 256;
 double* g_scratch_ptr[kMaxDevices] = {};
 
-int scratch_on_current_device(double** out) {
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return cuda_fail(e, "cudaGetDevice");
+int scratch_on_device(int dev, double** out) {
   if (dev < 0 || dev >= kMaxDevices) return BSAMG_ERR_UNSUPPORTED;
   std::lock_guard<std::mutex> lk(g_mu);
   if (!g_scratch_ptr[dev]) {
     void* p = nullptr;
-    e = cudaGetSymbolAddress(&p, g_norm_scratch);
+    cudaError_t e = cudaGetSymbolAddress(&p, g_norm_scratch);
     if (e != cudaSuccess) return cuda_fail(e, "cudaGetSymbolAddress(g_norm_scratch)");
     g_scratch_ptr[dev] = static_cast<double*>(p);
   }
   *out = g_scratch_ptr[dev];
   return BSAMG_OK;
+}
+
+// Whether the final kernel stores the norm itself: to a double's address in
+// memory of its own device.  Any other (unaligned, a peer's memory without
+// access enabled, the host's) would fault there or depend on the system, and
+// is left to a copy.
+bool kernel_can_store(const double* p, int dev) {
+  if (reinterpret_cast<uintptr_t>(p) % alignof(double)) return false;
+  cudaPointerAttributes at = {};
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();  // the copy reports it
+    return false;
+  }
+  return at.type == cudaMemoryTypeManaged || (at.type == cudaMemoryTypeDevice && at.device == dev);
 }
 
 template <int DIM>
@@ -126,9 +137,13 @@ extern "C" int bsamg_ch_residual_norm_noalloc(const double* q, const double* f, 
     cuda_fail(cudaSuccess, "bsamg_ch_residual_norm_noalloc: patch larger than BSAMG_NOALLOC_MAX_CELLS");
     return BSAMG_ERR_ARG;
   }
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return cuda_fail(e, "cudaGetDevice");
   double* scratch = nullptr;
-  int rc = scratch_on_current_device(&scratch);
+  int rc = scratch_on_device(dev, &scratch);
   if (rc != BSAMG_OK) return rc;
+  const bool store = kernel_can_store(norm_out, dev);
   // plugin coefficients exactly as the hierarchy computes them
   double h2 = h * h;
   double eps2 = eps * eps;
@@ -144,13 +159,11 @@ extern "C" int bsamg_ch_residual_norm_noalloc(const double* q, const double* f, 
   // the hierarchy's own final reduction (two stages above 2048 blocks);
   // no non-finite flag: a NaN or Inf input shows as a NaN or Inf norm
   double* out = scratch + 2 * kMaxBlocks;
-  // an address that a kernel cannot store a double to is reached by a copy
-  const bool aligned = reinterpret_cast<uintptr_t>(norm_out) % alignof(double) == 0;
   launch_norm_finish(s, scratch, nblk, 2, 2.0 * (double)cells, errortype, out, nullptr, nullptr,
-                     aligned ? norm_out : nullptr);
-  cudaError_t e = cudaGetLastError();
+                     store ? norm_out : nullptr);
+  e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "bsamg_ch_residual_norm_noalloc launch");
-  if (aligned) return BSAMG_OK;
+  if (store) return BSAMG_OK;
   e = cudaMemcpyAsync(norm_out, out, sizeof(double), cudaMemcpyDeviceToDevice, s);
   return e == cudaSuccess ? BSAMG_OK : cuda_fail(e, "bsamg_ch_residual_norm_noalloc copy");
 }
