@@ -82,8 +82,6 @@ struct TableUpload {
 
 // tail_cells up to which a hierarchy is set for a single run's latency (the default)
 constexpr long long kTailLatency = 2048;
-// hierarchies of a context that one run keeps (its states, a regrid's old and new one)
-constexpr int kFewHiers = 8;
 
 struct Hier {
   bsamg_ctx* ctx = nullptr;
@@ -130,8 +128,8 @@ struct Hier {
   long long tail_cells = kTailLatency;  // latency-friendly; a serving loop may raise it
   // launches ahead of the previous kernel's end (launch_after) are for runs
   // that have the GPU to themselves
-  bool crowded = false;  // committed beside more than kFewHiers hierarchies of the context
-  void launch_order() { s.early = !crowded && tail_cells <= kTailLatency; }
+  bool shared = false;  // a solve of it ran beside another one on the device (SolveRuns)
+  void launch_order() { s.early = !shared && tail_cells <= kTailLatency; }
   // keys: (start level, minlevel, nsmooth) for V-cycles, (start level,
   // minlevel, -field) for FillDown
   using TailKey = std::tuple<int, int, int>;

@@ -306,11 +306,11 @@ int tail_smem_attributes(int problem);
 // after_previous(): it lets the next kernel do the same and waits until the
 // one before has finished and its writes are visible.  Grids of many waves are
 // launched in the plain order: their early CTAs wait in the slots of the
-// running kernel's last wave (a step at 256^3 5.43 -> 5.56 ms).  Nor are those
-// of a hierarchy that shares the GPU with many (Hier::launch_order): CTAs that
+// running kernel's last wave (a step at 256^3 5.43 -> 5.56 ms).  So are those
+// of a hierarchy that shares the GPU with others (Hier::launch_order): CTAs that
 // wait hold the slots of the others' kernels (serving 200 requests a second,
 // early launches 1820 steps/s and a median of 310 ms, the plain order 2280 and
-// 40 ms).
+// 40 ms; see SolveRuns in hier.cu).
 constexpr unsigned kEarlyCtas = 1024;
 __device__ __forceinline__ void after_previous() {
   asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory");

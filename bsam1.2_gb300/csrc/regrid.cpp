@@ -678,6 +678,7 @@ int regrid(Hier& H, const bsamg_regrid_params& prm, bsamg_qinit_fn qinit, void* 
   nh->has_root_xupper = H.has_root_xupper;
   std::memcpy(nh->root_xupper, H.root_xupper, sizeof(H.root_xupper));
   nh->tail_cells = H.tail_cells;  // tuning carries over
+  nh->shared = H.shared;
   nh->box_sweep = H.box_sweep;
   nh->solve_mode = H.solve_mode;
   nh->solve_shape = H.solve_shape;
