@@ -473,8 +473,9 @@ class Hierarchy:
         _ck(lib().bsamg_set_box_sweep(self.h, int(kind)), "bsamg_set_box_sweep")
 
     def set_tail_cells(self, cells):
-        """Largest cumulative coarse-level size the mixed V-cycle runs inside
-        one thread block (bsamg_set_tail_cells; 0 disables)."""
+        """How the coarse end of a V-cycle runs: 0 an operation a launch, else
+        in one launch where the hierarchy allows; above the default 2048 set
+        for throughput (bsamg_set_tail_cells)."""
         _ck(lib().bsamg_set_tail_cells(self.h, cells), "bsamg_set_tail_cells")
 
     def set_solve(self, mode=1, ctas=16, threads=512, tile=64, solo_cells=8192):

@@ -2149,7 +2149,9 @@ int launch_staged(Hier& H, const BoxLev& L, int c, int first) {
 // cells (tiles of 8 rows; the ring fills 224 KB of shared memory), at least
 // one tile and its halo per plane.  Levels of 64-cell rows (tiles of 16 rows)
 // compile but measured slower than four sweeps on a GB300 (128^3: 62 against
-// 36 us: 64 CTAs), so they keep the sweeps.
+// 36 us, at a time when a level was cut into whole tiles by a quarter of the
+// planes, 64 CTAs there; not measured again with smooth_split), so they keep
+// the sweeps.
 int smooth_rows(const BoxLev& L) {
   const int ty = L.hh == 128 ? 8 : 0;
   return ty && L.n[1] % ty == 0 && L.n[1] >= ty + 2 * kSmStages ? ty : 0;

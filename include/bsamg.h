@@ -311,8 +311,10 @@ int bsamg_set_box_sweep(bsamg_hier* h, int kind);
  * instead of ~20 per level.  Results are bit-identical.  Default 2048; a
  * larger value trades a single run's latency for throughput when many
  * hierarchies share the GPU (kernels are then not launched ahead of the end of
- * the one before, either).  0: every operation its own launch.  Drops the
- * hierarchy's captured graphs. */
+ * the one before, either).  0: every operation its own launch.  The mixed path
+ * of a fully periodic box (bsamg_set_box_sweep) takes no notice of `cells`: the
+ * levels that fit one cluster launch run in one.  Drops the hierarchy's
+ * captured graphs. */
 int bsamg_set_tail_cells(bsamg_hier* h, long long cells);
 /* Tuning (no reference counterpart; replaces the loop of
  * MultigridIterations, afasroutines.f90:78-104, and the ApplyOnLevel loops
