@@ -764,8 +764,10 @@ def main():
         kdesc = "one-pass V(2,2) smoothing of the correction (four colour half-sweeps), finest level"
     # per colour half-sweep: e read (N*2*4) + g, phib and e write of that colour (N/2*(2*4+4+2*4)) = 18 N
     # (the per-sweep figure 4*N*V*s + N*s for the two colours); the one-pass smoothing performs four
-    # half-sweeps per launch (72 N) while moving 28 N (e, g, phib read once, e written once)
-    b_mixed = 18.0 * N * col_mixed
+    # half-sweeps per launch (72 N) while moving 28 N (e, g, phib read once, e written once), which the
+    # roofline counts; what the half-sweeps would have moved is given beside it
+    b_mixed = (28.0 if col_mixed == 4 else 18.0) * N
+    b_sweeps = 18.0 * N * col_mixed
     b_fp64 = 32.0 * N   # q read (N*2*8) + f read and q write of one colour (N/2*(2*8+2*8))
     ach = b_mixed / (ms_mixed * 1e-3) / 1e9
     ach64 = b_fp64 / (ms_fp64 * 1e-3) / 1e9
@@ -792,7 +794,8 @@ def main():
                      "achieved": ach, "peak": peak, "unit": "GB/s", "frac": ach / peak,
                      "peak_kind": peak_kind, "bytes_per_launch": b_mixed, "ms_per_launch": ms_mixed,
                      "half_sweeps_per_launch": col_mixed,
-                     "dram_bytes_needed": (28.0 if col_mixed == 4 else 18.0) * N,
+                     "in_half_sweep_bytes": {"bytes_per_launch": b_sweeps,
+                                             "of_peak": b_sweeps / (ms_mixed * 1e-3) / 1e9 / peak},
                      "traffic": ncu_traffic(args.workload, kmix)},
         "roofline_fp64": {"bound": "fp64 pipe", "kernel": "k_relax (FP64 colour sweep, finest level)",
                           "achieved_hbm": ach64, "peak_hbm": peak, "frac_hbm": ach64 / peak,
