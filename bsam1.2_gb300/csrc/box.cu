@@ -807,10 +807,11 @@ __global__ void __launch_bounds__(256, 6) k_bx_restrict_load(float* __restrict__
 // once, as a vector (72 vectors and 16 single ones for what cell by cell are
 // 272 loads).  The pass waits for memory (cell by cell at 40 registers it took
 // 135 us at 256^3 against 50 us for its bytes), so that fewer and wider loads,
-// more of them in flight, are what counts: 215 -> 234 steps/s of 256^3 with
-// five CTAs of 128 threads an SM at 96 registers; at 64 registers 225, with
-// four cells a thread at 128 registers 232.  The sums keep the order of the
-// cells, and the bits.
+// more of them in flight, are what counts: 200.6 -> 218.7 steps/s of 256^3
+// (bench.py --steps 20 --warmup 5) with five CTAs of 128 threads an SM at 96
+// registers; over a shorter run 234, at 64 registers 225, with four cells a
+// thread at 128 registers 232.  The sums keep the order of the cells, and the
+// bits.
 constexpr int kRestrictThreads = 128;
 constexpr int kRestrictCells = 2;  // coarse cells a thread; a level's extents are even
 __global__ void __launch_bounds__(kRestrictThreads, 5) k_bx_restrict_rows(float* __restrict__ fp, BoxLev F, BoxLev C) {
@@ -1010,6 +1011,10 @@ __global__ void __launch_bounds__(256) k_bx_prolong(float* __restrict__ fp, BoxL
 // 64^2 .. 2^2) with a launch per sweep above: ten steps at 128^2 7.8 -> 5.95
 // ms, five at 64^3 4.65 -> 4.15 ms, eight at 32^2 3.01 -> 2.68 ms, the same
 // bits.
+// 512 threads leave 128 registers, which do not hold two pairs' state in every
+// form: spill stores and loads of 68 and 140 bytes a thread in 2D, 284 and 504
+// in 3D (k_bx_solve, with its own state beside: 468 and 776, 900 and 1276),
+// one instruction in fifty of k_bx_cycle, one in twenty of k_bx_solve.
 struct CycLev {
   int n0, n1, N;       // extents (n1: 3D), rows
   int maxr;            // rows a CTA holds at most

@@ -14,7 +14,8 @@
 //
 // Measured (GB300), a 3D CH sweep of 256^3, a colour: 38 FP64 instructions a
 // cell, 612 us; 27 with the sums and about 500 integer ones, 440 us; 16 with
-// the two quotients, 312 us.  The residual norm: 16 instead of 32.
+// the two quotients, 312 us (each sum's last term is an FP64 addition again,
+// see sum6: 17).  The residual norm: 15 instead of 32.
 #pragma once
 #ifndef FXP_CPU  // a test compiles this file for the host, with the intrinsics it spells out
 #include <cuda_runtime.h>

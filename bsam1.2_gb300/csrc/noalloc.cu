@@ -89,9 +89,10 @@ __device__ __forceinline__ double lap(const double* a, int c, int sy, int sz) {
 // rf = f - Operator(q) (CH/problem.f90:393-422, :638-669) per interior cell,
 // sums of rf^2 over `group` consecutive runs of kBlock cells per CTA, in the
 // order of the hierarchy's norm on a one-patch level (whose blocks are the
-// same runs of cells).  Bound by the FP64 unit: about 12 of its instructions
-// a cell, the two Laplacians on the integer pipe beside them (31 with all of
-// them on it: 119 us for 160 x 96 x 128, now 82).
+// same runs of cells).  Bound by the FP64 unit and the integer ALU alike: 15
+// FP64 instructions a cell, the Laplacians' sums on the integer pipe beside
+// them (31 with all of them on the FP64 unit: 119 us for 160 x 96 x 128, now
+// 79 with the final sum).
 template <int DIM>
 __global__ void __launch_bounds__(kBlock, 4) k_norm_single(const double* __restrict__ q, const double* __restrict__ f,
                                                         int mx0, int mx1, int mx2, const __grid_constant__ UniDim d,
