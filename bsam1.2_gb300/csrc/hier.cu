@@ -145,6 +145,9 @@ int enq_level_relax(Hier& H, int level, int nsmooth) {
 // AFASVcycle, afasroutines.f90:495-529
 int enq_vcycle(Hier& H, int level, int minlevel, int nsmooth) {
   if (uni_level(H, level)) {
+    // no smoothing and no coarser level: the level stays as it is, edge and
+    // corner ghosts included, which the cluster's launch would set
+    if (level == minlevel && nsmooth < 1) return BSAMG_OK;
     const PluginUni& U = uni64(H);
     const Hier::UniPlan* pl = uni_plan(H, U, level, minlevel, nsmooth);
     if (pl && pl->top == level) {  // the rest of the V-cycle in one cluster launch
