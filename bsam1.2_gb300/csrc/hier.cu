@@ -552,9 +552,8 @@ std::atomic<int> SolveRuns::count_[64];
 
 int share_gpu(Hier& H) {
   H.shared = true;
-  if (!H.s.early) return BSAMG_OK;
+  if (H.tail_cells > kTailLatency) return BSAMG_OK;  // in the plain order already
   CK(cudaStreamSynchronize(H.s));
-  H.launch_order();
   drop_graphs(H);
   for (auto& kv : H.graph_donors)
     if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
@@ -571,6 +570,11 @@ int multigrid_iterations(Hier& H, int finest, int minlevel, int nsmooth, int max
   RET(set_device(H));
   const SolveRuns run(H.ctx->device);
   if (run.beside_others() && !H.shared) RET(share_gpu(H));
+  struct Order {  // of this solve's launches
+    Hier& H;
+    Order(Hier& h, bool mixed) : H(h) { H.launch_order(mixed); }
+    ~Order() { H.launch_order(); }
+  } order(H, mode == BSAMG_MODE_MIXED);
   if (!(mode == BSAMG_MODE_MIXED && H.box)) H.box_g_valid = false;  // the FP64 cycles change q
   // afasroutines.f90:57-76
   // the periodic-box mixed path forms f from qold itself

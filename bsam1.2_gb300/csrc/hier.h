@@ -129,7 +129,11 @@ struct Hier {
   // launches ahead of the previous kernel's end (launch_after) are for runs
   // that have the GPU to themselves
   bool shared = false;  // a solve of it ran beside another one on the device (SolveRuns)
-  void launch_order() { s.early = !shared && tail_cells <= kTailLatency; }
+  // the order of the launches that follow: a mixed solve's, or FP64 operations
+  void launch_order(bool mixed = false) {
+    const bool alone = !shared && tail_cells <= kTailLatency;
+    s.early = !alone ? 0 : (mixed ? kEarlyCtas : (ndims == 2 ? kEarlyCtas64 : 0));
+  }
   // keys: (start level, minlevel, nsmooth) for V-cycles, (start level,
   // minlevel, -field) for FillDown
   using TailKey = std::tuple<int, int, int>;

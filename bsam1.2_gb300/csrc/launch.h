@@ -12,13 +12,14 @@ namespace bsamg {
 
 constexpr int kNormOutLen = 8 + 3 * 128;
 
-// A stream and how launch_after uses it: as programmatic dependents, or in
-// the plain order.
+// A stream and how launch_after uses it: grids of up to `early` CTAs as
+// programmatic dependents, larger ones in the plain order.
+constexpr unsigned kEarlyCtas = 1024, kEarlyCtas64 = 152;
 struct LaunchStream {
   cudaStream_t s = nullptr;
-  bool early = true;
+  unsigned early = kEarlyCtas;
   LaunchStream() = default;
-  LaunchStream(cudaStream_t st, bool e = true) : s(st), early(e) {}
+  LaunchStream(cudaStream_t st) : s(st) {}
   operator cudaStream_t() const { return s; }
 };
 
@@ -304,14 +305,20 @@ int tail_smem_attributes(int problem);
 // which takes part of the launch latency off chains of small kernels (a V-cycle
 // of 30 to 110 launches: 2 to 5 % of it).  Its first statement is
 // after_previous(): it lets the next kernel do the same and waits until the
-// one before has finished and its writes are visible.  Grids of many waves are
-// launched in the plain order: their early CTAs wait in the slots of the
-// running kernel's last wave (a step at 256^3 5.43 -> 5.56 ms).  So are those
-// of a hierarchy that shares the GPU with others (Hier::launch_order): CTAs that
-// wait hold the slots of the others' kernels (serving 200 requests a second,
-// early launches 1820 steps/s and a median of 310 ms, the plain order 2280 and
-// 40 ms; see SolveRuns in hier.cu).
-constexpr unsigned kEarlyCtas = 1024;
+// one before has finished and its writes are visible.  CTAs that wait hold
+// slots, which is why not every launch is made so (Hier::launch_order):
+// - Grids of many waves: their early CTAs wait in the slots of the running
+//   kernel's last wave (a mixed step at 256^3 5.43 -> 5.56 ms).
+// - FP64 solves, whose kernels are bound by the FP64 unit and the integer
+//   pipe, want their CTAs spread evenly over the SMs, and early ones go where
+//   the running kernel left room.  In 2D, grids of up to a CTA an SM gain (a
+//   step of five V-cycles, early | plain: 128^2 0.882 | 0.909 ms, 256^2 1.146 |
+//   1.181; with grids of up to 1024 CTAs 512^2 lost, 1.964 | 1.763); in 3D all
+//   lost (64^3 1.976 | 1.770, 128^3 4.953 | 4.738; up to a CTA an SM still
+//   2 to 4 %; adaptive growth 33.6 | 31.4).
+// - Hierarchies that share the GPU with others: their CTAs hold the others'
+//   slots (serving 200 requests a second, early launches 1820 steps/s and a
+//   median of 310 ms, the plain order 2280 and 40 ms; see SolveRuns in hier.cu).
 __device__ __forceinline__ void after_previous() {
   asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory");
 }
@@ -326,7 +333,7 @@ inline void launch_after(void (*k)(P...), dim3 grid, dim3 block, size_t smem, La
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = s.early && (unsigned long long)grid.x * grid.y * grid.z <= kEarlyCtas ? 1 : 0;
+  cfg.numAttrs = (unsigned long long)grid.x * grid.y * grid.z <= s.early ? 1 : 0;
   cudaLaunchKernelEx(&cfg, k, std::forward<A>(a)...);
 }
 // the same for one cluster of `ctas` CTAs, the largest waiters there are: up to
