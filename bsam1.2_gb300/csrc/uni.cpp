@@ -150,12 +150,20 @@ const Hier::UniPlan* uni_plan(Hier& H, const PluginUni& U, int level, int minlev
   return it->second.A.nl ? &it->second : nullptr;
 }
 
+// Levels from which one CTA does the rest of FillDown: above, a launch a level
+// over the GPU is quicker.  The solves wait for it before they return (a step
+// of five V-cycles with the line at 16384 | 8192 | 4096 | 1024 cells: 128^2 FP64
+// 877 | 859 | 860 | 856 us, mixed 307 | 296 | 297 | 296, 128x64 FP64 784 | 784 |
+// 776 | 776, growth 24^3 mixed 937 | 839 | 839 | 844; a fill of q at 32^3 25.0 |
+// 25.0 | 25.1 | 24.0).
+constexpr long long kFillSmallCells = 4096;
+
 int uni_enq_fill(Hier& H, const PluginUni& U, int fields, int level, int minlevel) {
   const LaunchCtx c = H.lc();
   for (int l = level; l > minlevel; l--) {
     const int p = uni_patch(H, l);
     const HostPatch& P = H.patches[p];
-    if ((long long)P.mx[0] * P.mx[1] * P.mx[2] <= 16384 && l - minlevel < kNLev) {  // the rest in one CTA
+    if ((long long)P.mx[0] * P.mx[1] * P.mx[2] <= kFillSmallCells && l - minlevel < kNLev) {  // the rest in one CTA
       UniCycle A{};
       A.bc = H.ubc;
       for (int x = l; x >= minlevel; x--) {
